@@ -27,6 +27,7 @@
 #include <cstring>
 #include <string>
 
+#include "qk_attention_split.h"
 #include "qk_common.h"
 #include "qk_umma.cuh"
 
@@ -1906,6 +1907,7 @@ qk_status attention_sage_block_dev(qk_ctx *c, const float *dq, const float *dk, 
 // Device-buffer form of the exact face (also used by the decoder path).
 qk_status attention_exact_dev(qk_ctx *c, const float *q, const float *k, const float *v,
                               float *out, const qk_attention_shape *s, int causal) {
+    if (attention_split_takes(c, s, causal)) return attention_split_exact(c, q, k, v, out, s, causal);
     AttnDims dm = dims_of(s);
     size_t widest = s->head_dim > s->val_dim ? s->head_dim : s->val_dim;
     if (widest <= 16) return launch_exact<4>(c, q, k, v, out, dm, causal);

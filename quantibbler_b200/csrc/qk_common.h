@@ -62,6 +62,7 @@ struct qk_ctx {
     qk_scratch d_z, d_t, d_ptrs;
     // error word of the asynchronous tensor-core kernels, read back by qk_gpu_synchronize
     qk_scratch d_err;
+    qk_scratch d_terms; // 16-bit terms of k and v (exact attention)
     qk_scratch d_head;  // the LM head's bfloat16 split of the hidden state
     bool err_armed = false;  // sticky: set by the first launch that can raise the error word
     uint32_t wait_limit = 0;  // polls before a device-side wait gives up (0: the default)

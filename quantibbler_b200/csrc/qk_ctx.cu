@@ -168,6 +168,7 @@ void qk_gpu_free(qk_ctx *ctx) {
     ctx->d_t.release();
     ctx->d_ptrs.release();
     ctx->d_err.release();
+    ctx->d_terms.release();
     ctx->d_head.release();
     for (auto &ps : ctx->h_pinned) {
         if (ps.copied) cudaEventDestroy(ps.copied);

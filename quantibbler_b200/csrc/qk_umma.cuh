@@ -41,6 +41,15 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
                                           uint32_t limit) {
     return __all_sync(0xffffffffu, mbar_wait_lane(bar, parity, abort_flag, limit)) != 0;
 }
+// One lane of the converged warp, chosen by the hardware.  Issue tcgen05.mma and tcgen05.commit under this
+// and not under a comparison with the lane number: their operands live in uniform registers, and only
+// after elect does the compiler know that one lane is left (otherwise it loops over the lanes, and an MMA
+// costs its issuer over a hundred cycles).
+__device__ __forceinline__ bool elect_one() {
+    uint32_t is;
+    asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(is));
+    return is != 0;
+}
 __device__ __forceinline__ void umma_commit(uint64_t *bar) {
     asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(
                      smem_u32(bar))

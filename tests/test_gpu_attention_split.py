@@ -1,0 +1,101 @@
+"""Float32 attention as sums of 16-bit products (qk_attention_split.cu): the exact face from 192 keys on and the
+prefill attention of a bfloat16 cache, against 64-bit attention over the visible keys.
+
+Tolerance: float32 scores of magnitude s carry an error of about s 2^-23 into the weights, so 2e-6 of the
+largest output (scores here stay below 16); the plain float32 kernel is held to the reference's 1e-5."""
+
+import ctypes
+import math
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+from quantibbler_b200 import _lib  # noqa: E402
+from quantibbler_b200.gpu import AttentionShape, GpuContext  # noqa: E402
+
+
+@pytest.fixture(scope="module")
+def ctx():
+    return GpuContext.init()
+
+
+def visible_attention(q, k, v, causal, skew):
+    """q [H, Sq, d], k and v [KV, Sk, .]: 64 bits, every row over the keys it sees and no others."""
+    H, Sq, d = q.shape
+    out = np.zeros((H, Sq, v.shape[-1]))
+    with np.errstate(invalid="ignore", over="ignore"):
+        for h in range(H):
+            kk, vv = (t[h // (H // k.shape[0])].astype(np.float64) for t in (k, v))
+            for i in range(Sq):
+                n = i + skew + 1 if causal else kk.shape[0]
+                s = kk[:n] @ q[h, i].astype(np.float64) / math.sqrt(d)
+                p = np.exp(s - s.max())
+                out[h, i] = (p[:, None] * vv[:n]).sum(0) / p.sum()
+    return out
+
+
+def worst(got, want):
+    return np.abs(got - want).max() / np.abs(want).max()
+
+
+@pytest.mark.parametrize("H,KV,Sq,Sk,d,dv,causal", [
+    (2, 1, 192, 192, 128, 128, True),    # the shortest that takes this path
+    (1, 1, 257, 257, 64, 64, True),      # one key and one row past a tile
+    (4, 2, 129, 255, 80, 80, True),      # rows that see a third of a key block more than their tile's first
+    (2, 2, 1, 321, 40, 24, True),        # one row; head sizes off every multiple
+    (3, 1, 127, 320, 128, 64, False),
+    (2, 1, 200, 448, 65, 127, True),     # one channel past the first chunk; odd sizes
+    (1, 1, 130, 193, 1, 3, False),
+])
+def test_exact_face_at_the_edges_of_tiles(ctx, H, KV, Sq, Sk, d, dv, causal):
+    rng = np.random.default_rng(Sq * 1000 + Sk)
+    q, k, v = (rng.standard_normal(s).astype(np.float32) for s in ((H, Sq, d), (KV, Sk, d), (KV, Sk, dv)))
+    k += 2 * rng.standard_normal((KV, 1, d)).astype(np.float32)
+    got = ctx.attention(AttentionShape(1, H, KV, Sq, Sk, d, dv), q, k, v, causal).reshape(H, Sq, dv)
+    assert worst(got, visible_attention(q, k, v, causal, Sk - Sq)) < 2e-6
+
+
+@pytest.mark.parametrize("qs,ks,vs", [(1e-18, 1e18, 1e-30), (1e20, 1e-20, 1e30), (1.0, 0.0, 1.0), (1e-30, 1e-30, 3.0)])
+def test_exact_face_over_the_range_of_float32(ctx, qs, ks, vs):
+    rng = np.random.default_rng(5)
+    q, k, v = (rng.standard_normal((2, 200, 64)).astype(np.float32) * np.float32(x) for x in (qs, ks, vs))
+    v[0, :, 3] *= np.float32(1e-6)     # a channel far below the others keeps its own accuracy
+    got = ctx.attention(AttentionShape(1, 2, 2, 200, 200, 64, 64), q, k, v, True).reshape(2, 200, 64)
+    want = visible_attention(q, k, v, True, 0)
+    assert worst(got, want) < 2e-6
+    assert worst(got[0, :, 3], want[0, :, 3]) < 2e-6
+
+
+def test_exact_face_with_infinities_and_nan(ctx):
+    """Only the rows that see such a value are touched by it."""
+    rng = np.random.default_rng(6)
+    q, k, v = (rng.standard_normal((2, 260, 64)).astype(np.float32) for _ in range(3))
+    k[0, 150, 2], v[0, 200, 5], v[1, 130, 0], q[1, 40, 1] = np.inf, np.nan, -np.inf, np.nan
+    got = ctx.attention(AttentionShape(1, 2, 2, 260, 260, 64, 64), q, k, v, True).reshape(2, 260, 64)
+    want = visible_attention(q, k, v, True, 0)
+    fine = np.isfinite(want)
+    assert 0 < (~fine).sum() < want.size // 2
+    assert np.array_equal(np.isnan(got), np.isnan(want)) and np.array_equal(np.isposinf(got), np.isposinf(want))
+    assert np.abs(got[fine] - want[fine]).max() < 2e-6 * np.abs(want[fine]).max()
+
+
+@pytest.mark.parametrize("H,KV,T,p0", [(4, 1, 64, 0), (4, 2, 129, 0), (6, 2, 65, 63), (3, 3, 1, 70), (8, 1, 127, 130)])
+def test_prefill_attention_at_the_edges_of_tiles(ctx, H, KV, T, p0):
+    import torch
+    gen = torch.Generator("cuda").manual_seed(T + p0)
+    draw = lambda *s: torch.randn(s, device="cuda", generator=gen)  # noqa: E731
+    s_max = p0 + T + 5
+    q, ck, cv = draw(T, H * 128), draw(3, KV, s_max, 128).bfloat16(), draw(3, KV, s_max, 128).bfloat16()
+    ck[:, :, p0 + T:] = math.nan     # what no position has written yet is never read
+    cv[:, :, p0 + T:] = math.nan
+    ck[0], cv[2] = math.nan, math.nan
+    out = torch.zeros(T, H * 128, device="cuda")
+    torch.cuda.synchronize()
+    p = lambda t: ctypes.c_void_p(t.data_ptr())  # noqa: E731
+    _lib.check(_lib.lib().qk_prefill_attention(ctx.handle, p(q), p(ck), p(cv), _lib.QK_BF16, 1, p0, T, H, KV, 128, s_max, p(out)))
+    ctx.synchronize()
+    host = lambda t: t.float().cpu().numpy()  # noqa: E731
+    want = visible_attention(host(q.reshape(T, H, 128).transpose(0, 1)), host(ck[1, :, :p0 + T]), host(cv[1, :, :p0 + T]), True, p0)
+    assert worst(host(out.reshape(T, H, 128).transpose(0, 1)), want) < 2e-6
