@@ -433,7 +433,7 @@ split_attention_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
         }
         if (!ok) {
             *abort_flag = 1;
-            if (lane == 0) umma_commit(drain);  // the products still in flight
+            if (elect_one()) umma_commit(drain);  // the products still in flight
             __syncwarp();
             (void)mbar_wait(drain, 0, never, kWaitLimit);
         }

@@ -542,7 +542,7 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (lane == 0) {
+                if (elect_one()) {
                     const uint32_t a_addr = smem_u32(tiles + s * S::kStage), b_addr = a_addr + S::kABytes;
 #pragma unroll
                     for (int k = 0; k < kTcK / 16; ++k) {
@@ -558,12 +558,12 @@ dense_tc_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant
                 }
                 __syncwarp();
             }
-            if (!dead && lane == 0) umma_commit(&acc_full[acc]);
+            if (!dead && elect_one()) umma_commit(&acc_full[acc]);
             __syncwarp();
         }
         if (dead) {
             *abort_flag = 1;
-            if (lane == 0) umma_commit(drain);  // the products still in flight
+            if (elect_one()) umma_commit(drain);  // the products still in flight
             __syncwarp();
             (void)mbar_wait(drain, 0, never, g.wait_limit);
         }
@@ -841,7 +841,7 @@ dense_narrow_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
                 break;
             }
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (lane == 0) {
+            if (elect_one()) {
                 const uint32_t a_addr = smem_u32(tiles + s * S::kStage), b_addr = a_addr + S::kABytes;
 #pragma unroll
                 for (int k = 0; k < kTcK / 16; ++k) {
@@ -857,11 +857,11 @@ dense_narrow_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
             }
             __syncwarp();
         }
-        if (!dead && lane == 0) umma_commit(acc_full);
+        if (!dead && elect_one()) umma_commit(acc_full);
         __syncwarp();
         if (dead) {
             *abort_flag = 1;
-            if (lane == 0) umma_commit(drain);  // the products still in flight
+            if (elect_one()) umma_commit(drain);  // the products still in flight
             __syncwarp();
             (void)mbar_wait(drain, 0, never, g.wait_limit);
         }

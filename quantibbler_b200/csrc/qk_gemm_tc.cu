@@ -292,9 +292,7 @@ factorized_gemm_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid
         }
     } else if (warp == kMmaWarp) {
         // ------------------------------------------------------------ MMA issue
-        // The whole warp runs the loop and waits on the barriers; lane 0 alone issues.  (A
-        // lone diverged lane beside 31 lanes parked at the block barrier issues several
-        // times slower.)
+        // The whole warp runs the loop and waits on the barriers; one lane issues.
         const uint32_t idesc = umma_idesc(kBN);
         uint32_t gc = 0;
         bool dead = false;
@@ -316,7 +314,7 @@ factorized_gemm_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid
                     break;
                 }
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (lane == 0) {
+                if (elect_one()) {
                     const uint32_t a_addr = smem_u32(tiles + s * kStageBytes), b_addr = a_addr + kABytes;
 #pragma unroll
                     for (int k = 0; k < kBK / 16; ++k) {
@@ -332,7 +330,7 @@ factorized_gemm_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid
                 }
                 __syncwarp();
             }
-            if (!dead && lane == 0) umma_commit(&acc_full[acc]);
+            if (!dead && elect_one()) umma_commit(&acc_full[acc]);
             __syncwarp();
             u += kc1 - kc0;
         }

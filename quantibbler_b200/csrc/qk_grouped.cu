@@ -694,7 +694,7 @@ grouped_portion_umma_kernel(const __grid_constant__ CUtensorMap q_map, const __g
         }
     } else if (warp == 9) {
         const uint32_t idesc_s = portion_idesc(kUmKeys, 0), idesc_o = portion_idesc(a.vdim, 1);
-        auto scores = [&](uint32_t u, uint32_t j) {  // (lane 0)
+        auto scores = [&](uint32_t u, uint32_t j) {  // (one lane)
             const uint32_t q0 = smem_u32(qs + u * kUmTile), k0 = smem_u32(ks + (j % kUmStages) * kUmTile);
             for (uint32_t k = 0; k < a.dim / 16; ++k) {
                 const uint32_t at = k / 4 * kUmChunk + k % 4 * 32;
@@ -707,7 +707,7 @@ grouped_portion_umma_kernel(const __grid_constant__ CUtensorMap q_map, const __g
             }
             umma_commit(s_full + u);
         };
-        auto values = [&](uint32_t u, uint32_t j) {  // (lane 0)
+        auto values = [&](uint32_t u, uint32_t j) {  // (one lane)
             const uint32_t v0 = smem_u32(vs + (j % kUmStages) * kUmTile);
 #pragma unroll
             for (uint32_t k = 0; k < kUmKeys / 16; ++k) {
@@ -721,7 +721,7 @@ grouped_portion_umma_kernel(const __grid_constant__ CUtensorMap q_map, const __g
         };
         bool ok = mbar_wait(q_full, 0, abort_flag, wait_limit) && mbar_wait(k_full, 0, abort_flag, wait_limit);
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-        if (ok && lane == 0) {
+        if (ok && elect_one()) {
 #pragma unroll
             for (uint32_t u = 0; u < 2; ++u)
                 if (unit[u].n_blocks) scores(u, 0);
@@ -738,14 +738,14 @@ grouped_portion_umma_kernel(const __grid_constant__ CUtensorMap q_map, const __g
                 ok = mbar_wait(p_full + u, j & 1, abort_flag, wait_limit);
                 if (!ok) continue;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-                if (lane == 0) {
+                if (elect_one()) {
                     values(u, j);
                     if (j + 1 < unit[u].n_blocks) scores(u, j + 1);
                     else umma_commit(o_full + u);
                 }
                 __syncwarp();
             }
-            if (ok && lane == 0) {
+            if (ok && elect_one()) {
                 umma_commit(v_empty + s);
                 if (j + 1 < n_blocks) umma_commit(k_empty + s1);
             }
@@ -753,7 +753,7 @@ grouped_portion_umma_kernel(const __grid_constant__ CUtensorMap q_map, const __g
         }
         if (!ok) {
             *abort_flag = 1;
-            if (lane == 0) umma_commit(drain);  // the products still in flight
+            if (elect_one()) umma_commit(drain);  // the products still in flight
             __syncwarp();
             (void)mbar_wait(drain, 0, never, kUmWaitDefault);
         }
