@@ -280,6 +280,13 @@ qk_status qk_layers_apply_prefill(qk_ctx *ctx, const qk_layer *const *layers, si
 qk_status qk_layers_apply_prefill_gated(qk_ctx *ctx, const qk_layer *const *layers, size_t n_layers,
                                         const float *gate_dev, const float *up_dev, size_t n_tokens,
                                         float *const *y_devs);
+/* The same with the RMSNorm in front of the linears formed on the way: h = x (+ residual, may be null),
+ * x_out = h (may be null, may be x), and the linears read norm(h) * weight.  Same values as qk_rmsnorm
+ * under bfloat16 serving followed by qk_layers_apply_prefill, without the normed rows being written and
+ * read back.  Up to 8192 entries per row. */
+qk_status qk_layers_apply_prefill_normed(qk_ctx *ctx, const qk_layer *const *layers, size_t n_layers,
+                                         const float *x, const float *residual, const float *weight, float eps,
+                                         float *x_out, size_t n_tokens, float *const *y_devs);
 /* How the prefill calls above deal their work out (host arithmetic only; no device is touched):
  * problem p has tiles[p] output tiles of k_chunks[p] 64-wide k-chunks each, the units of
  * work are (tile, k-chunk) pairs in problem-major, tile-major order, and CTA i of *n_ctas

@@ -39,6 +39,7 @@
 #include <type_traits>
 
 #include "qk_common.h"
+#include "qk_decoder_dev.cuh"
 #include "qk_umma.cuh"
 
 namespace {
@@ -577,6 +578,69 @@ __global__ void scale_to_bf16_kernel(const float *__restrict__ x, const float *_
     *reinterpret_cast<uint4 *>(z + (size_t)t * pitch + k) = make_uint4(w[0], w[1], w[2], w[3]);
 }
 
+// The same with the RMSNorm in front of the linears formed on the way: h = x (+ residual), x_out = h,
+// z_p = bf16(s2_p * norm(h)), the norm with the thread count, element order, order of the sum and roundings
+// of the stand-alone norm kernel, hence the same bits.  One block per token, the row in registers.  What
+// it replaces at 2048 tokens of width 4096 is a norm kernel (61 us: every load of a row waited for the
+// store before it), its 34 MB output and the scaling kernel that read it back (27 to 39 us); here all loads
+// of a row go out before the first store.  x, residual: not restrict-qualified, x_out may be x, and a
+// read-only load might be moved above the dependency wait.
+constexpr int kNormThreads = 512, kNormPerThread = 16;
+struct NormArgs {
+    const float *x, *residual, *weight;
+    float *x_out;
+    float eps;
+};
+__global__ void __launch_bounds__(kNormThreads, 2)
+norm_scale_to_bf16_kernel(NormArgs n, ScaleArgs a, uint32_t n_problems, uint32_t d, uint32_t pitch) {
+    qk::pdl_launch();
+    __shared__ float red[kNormThreads / 32];
+    float w[kNormPerThread], keep[kNormPerThread];
+#pragma unroll
+    for (int r = 0; r < kNormPerThread; ++r) {  // (constants of the layer: before the dependency wait)
+        const uint32_t i = threadIdx.x + r * kNormThreads;
+        w[r] = i < d ? __ldg(n.weight + i) : 0.f;
+    }
+    qk::pdl_wait();
+    const size_t base = (size_t)blockIdx.x * d;
+#pragma unroll
+    for (int r = 0; r < kNormPerThread; ++r) {
+        const uint32_t i = threadIdx.x + r * kNormThreads;
+        keep[r] = i < d ? __ldcg(n.x + base + i) : 0.f;
+    }
+    if (n.residual) {
+        float more[kNormPerThread];
+#pragma unroll
+        for (int r = 0; r < kNormPerThread; ++r) {
+            const uint32_t i = threadIdx.x + r * kNormThreads;
+            more[r] = i < d ? __ldcg(n.residual + base + i) : 0.f;
+        }
+#pragma unroll
+        for (int r = 0; r < kNormPerThread; ++r) keep[r] += more[r];
+    }
+    float ss = 0.f;
+#pragma unroll
+    for (int r = 0; r < kNormPerThread; ++r) {
+        const uint32_t i = threadIdx.x + r * kNormThreads;
+        if (n.x_out && i < d) n.x_out[base + i] = keep[r];
+        keep[r] = round_bf16f(keep[r]);
+        ss += keep[r] * keep[r];
+    }
+    const float inv = 1.0f / sqrtf(block_sum(ss, red) / (float)d + n.eps);
+#pragma unroll
+    for (int r = 0; r < kNormPerThread; ++r) keep[r] = round_bf16f(keep[r] * inv * w[r]);
+    for (uint32_t p = 0; p < n_problems; ++p) {
+        const float *__restrict__ s2 = a.s2[p];
+        uint16_t *z = a.z[p] + (size_t)blockIdx.x * pitch;
+#pragma unroll
+        for (int r = 0; r < kNormPerThread; ++r) {
+            const uint32_t i = threadIdx.x + r * kNormThreads;
+            if (i < d) z[i] = (uint16_t)(round_bf16_hi(__float_as_uint(__ldg(s2 + i) * keep[r])) >> 16);
+        }
+        if (d + threadIdx.x < pitch) z[d + threadIdx.x] = 0;  // (the pitch exceeds d by less than 64)
+    }
+}
+
 constexpr size_t kSmemBytes = 1024 + kStages * kStageBytes + (2 * kStages + 5) * 8 + 16;
 static_assert(kSmemBytes <= 227 * 1024, "the stages must fit the 227 KB a CTA may have");
 
@@ -659,7 +723,8 @@ uint32_t pick_bn(size_t tokens) {
 }  // namespace
 
 static qk_status apply_prefill(qk_ctx *ctx, const qk_layer *const *layers, size_t n_layers, const float *x_dev,
-                               const float *up_dev, size_t n_tokens, float *const *y_devs) {
+                               const float *up_dev, size_t n_tokens, float *const *y_devs,
+                               const NormArgs *norm = nullptr) {
     if (n_layers == 0 || n_layers > (size_t)kMaxProblems)
         return qk::fail(QK_ERR_VALUE, "between 1 and %d layers per call, got %zu", kMaxProblems, n_layers);
     if (!layers || !y_devs) return qk::fail(QK_ERR_VALUE, "qk_layers_apply_prefill: null array");
@@ -673,6 +738,9 @@ static qk_status apply_prefill(qk_ctx *ctx, const qk_layer *const *layers, size_
             return qk::fail(QK_ERR_VALUE, "layers of one call share their input: layer %zu has din=%zu, "
                             "layer 0 has din=%zu", i, layers[i]->din, layers[0]->din);
     }
+    if (norm && layers[0]->din > (size_t)kNormThreads * kNormPerThread)
+        return qk::fail(QK_ERR_VALUE, "a normed input of the prefill may have %d entries, got %zu",
+                        kNormThreads * kNormPerThread, layers[0]->din);
     if (n_tokens == 0) return QK_OK;
     qk_ctx *c;
     qk_status st = qk::resolve_ctx(ctx, &c);
@@ -705,9 +773,13 @@ static qk_status apply_prefill(qk_ctx *ctx, const qk_layer *const *layers, size_
     }
     const int vec = ((uintptr_t)x_dev & 15) == 0 && ((uintptr_t)up_dev & 15) == 0 && (din & 3) == 0;
     const size_t total = n_tokens * (kp1 / 8);
-    (void)qk::launch_pdl(c->pdl, scale_to_bf16_kernel,
-                         dim3((unsigned)qk::ceil_div(total, 256), (unsigned)n_layers), dim3(256), 0, c->stream, x_dev,
-                         up_dev, sa, (uint32_t)n_tokens, (uint32_t)din, (uint32_t)kp1, vec);
+    if (norm)
+        (void)qk::launch_pdl(c->pdl, norm_scale_to_bf16_kernel, dim3((unsigned)n_tokens), dim3(kNormThreads), 0,
+                             c->stream, *norm, sa, (uint32_t)n_layers, (uint32_t)din, (uint32_t)kp1);
+    else
+        (void)qk::launch_pdl(c->pdl, scale_to_bf16_kernel,
+                             dim3((unsigned)qk::ceil_div(total, 256), (unsigned)n_layers), dim3(256), 0, c->stream,
+                             x_dev, up_dev, sa, (uint32_t)n_tokens, (uint32_t)din, (uint32_t)kp1, vec);
     QK_CUDA(cudaGetLastError());
     c->launches++;
     QK_CUDA(cudaFuncSetAttribute(factorized_gemm_tc_kernel<false>,
@@ -781,6 +853,14 @@ qk_status qk_layers_apply_prefill_gated(qk_ctx *ctx, const qk_layer *const *laye
     if (!gate_dev || !up_dev)
         return qk::fail(QK_ERR_VALUE, "qk_layers_apply_prefill_gated: gate and up must be given");
     return apply_prefill(ctx, layers, n_layers, gate_dev, up_dev, n_tokens, y_devs);
+}
+
+qk_status qk_layers_apply_prefill_normed(qk_ctx *ctx, const qk_layer *const *layers, size_t n_layers,
+                                         const float *x, const float *residual, const float *weight, float eps,
+                                         float *x_out, size_t n_tokens, float *const *y_devs) {
+    if (!x || !weight) return qk::fail(QK_ERR_VALUE, "qk_layers_apply_prefill_normed: x and weight must be given");
+    const NormArgs norm{x, residual, weight, x_out, eps};
+    return apply_prefill(ctx, layers, n_layers, x, nullptr, n_tokens, y_devs, &norm);
 }
 
 qk_status qk_prefill_work_split(size_t n_problems, const size_t *tiles, const size_t *k_chunks,

@@ -21,8 +21,8 @@ import numpy as np
 
 from . import _lib, tp
 from ._lib import QK_BF16, QK_F32, KernelError, check
-from .gpu import (DecodeStep, GpuContext, LayerPlan, PackedLayer, apply_prefill_many,
-                  apply_prefill_many_gated, make_feed)
+from .gpu import (PREFILL_NORM_MAX, DecodeStep, GpuContext, LayerPlan, PackedLayer, apply_prefill_many,
+                  apply_prefill_many_gated, apply_prefill_many_normed, make_feed)
 
 LINEARS = ("q", "k", "v", "o", "gate", "up", "down")
 
@@ -718,6 +718,18 @@ class Decoder(SlotDecoder):
             for name in names:
                 plan[name].apply()
 
+    def _normed_linears(self, li: int, names, pending, weight, feed, x_in, x_out, dsts) -> None:
+        """``_norm`` and the linears that read it; one call where the GEMM's scaling kernel can form the norm."""
+        cfg = self.cfg
+        if self.use_gemm and cfg.d_model <= PREFILL_NORM_MAX and not (pending is not None and self.fused_ar):
+            residual = None if pending is None else (self.delta_attn if pending == 0 else self.delta_mlp).data_ptr()
+            apply_prefill_many_normed([self.layers[li][n] for n in names], x_in.data_ptr(), residual,
+                                      weight.data_ptr(), cfg.rms_eps, x_out.data_ptr(), cfg.max_batch,
+                                      [dst.data_ptr() for dst in dsts])
+            return
+        self._norm(pending, weight, feed, x_in, x_out)
+        self._linears(li, names, self.h, dsts)
+
     def step(self) -> None:
         """One decode step for the whole batch: reads ``token_ids``/``positions``/``kv_len``,
         appends to the KV cache, leaves the greedy tokens in ``best_idx``."""
@@ -738,8 +750,8 @@ class Decoder(SlotDecoder):
             if normed:   # (norm and q,k,v in one pair of launches)
                 self.plans[li]["qkv_normed"].apply()
             else:
-                self._norm(pending, in_w, feeds["qkv"] if feeds else None, xa, xb)
-                self._linears(li, ["q", "k", "v"], self.h, [self.q, self.k, self.v])
+                self._normed_linears(li, ["q", "k", "v"], pending, in_w, feeds["qkv"] if feeds else None, xa, xb,
+                                     [self.q, self.k, self.v])
             xa, xb = xb, xa
             if self.qk_norms[li] is not None:
                 # every head is one row of head_dim values; x_out = x rewrites the projection
@@ -770,8 +782,8 @@ class Decoder(SlotDecoder):
             if normed:
                 self.plans[li]["gu_normed"].apply()
             else:
-                self._norm(0, post_w, feeds["gu"] if feeds else None, xa, xb)
-                self._linears(li, ["gate", "up"], self.h, [self.g, self.u])
+                self._normed_linears(li, ["gate", "up"], 0, post_w, feeds["gu"] if feeds else None, xa, xb,
+                                     [self.g, self.u])
             xa, xb = xb, xa
             if feeds:   # (the fed down plan needs no activation vector, only its digit table)
                 check(lib.qk_swiglu_feed(c, _p(self.g), _p(self.u), B, self.ff_loc, self.serving_tag,
@@ -826,6 +838,20 @@ class Decoder(SlotDecoder):
             for layer, dst in zip(layers, dsts):
                 layer.apply_device(src.data_ptr(), n_tokens, dst.data_ptr())
 
+    def _prefill_normed_linears(self, li: int, names, residual, weight, dsts, n_tokens: int) -> None:
+        """The stream takes up ``residual`` (if any) and the named linears read its norm; one call where the
+        GEMM's scaling kernel can form the norm."""
+        cfg, pf = self.cfg, self._pf
+        x, d = pf["x"], cfg.d_model
+        if cfg.serving == "bfloat16" and n_tokens >= cfg.gemm_min_batch and d <= PREFILL_NORM_MAX:
+            apply_prefill_many_normed([self.layers[li][n] for n in names], x.data_ptr(),
+                                      None if residual is None else residual.data_ptr(), weight.data_ptr(),
+                                      cfg.rms_eps, x.data_ptr(), n_tokens, [t.data_ptr() for t in dsts])
+            return
+        check(_lib.lib().qk_rmsnorm(self.ctx.handle, _p(x), None if residual is None else _p(residual), _p(weight),
+                                    n_tokens, d, cfg.rms_eps, self.serving_tag, _p(x), _p(pf["h"])))
+        self._prefill_linears(li, names, pf["h"], dsts, n_tokens)
+
     def _prefill_portion(self, part, seq: int, p0: int, reserve: int) -> None:
         torch, lib, c, cfg = self.torch, _lib.lib(), self.ctx.handle, self.cfg
         B, d, hd = cfg.max_batch, cfg.d_model, cfg.head_dim
@@ -839,9 +865,7 @@ class Decoder(SlotDecoder):
         pending = None
         for li in range(cfg.n_layers):
             in_w, post_w = self.norms[li]
-            check(lib.qk_rmsnorm(c, _p(pf["x"]), pending, _p(in_w), T, d, cfg.rms_eps,
-                                 self.serving_tag, _p(pf["x"]), _p(pf["h"])))
-            self._prefill_linears(li, ["q", "k", "v"], pf["h"], [pf["q"], pf["k"], pf["v"]], T)
+            self._prefill_normed_linears(li, ["q", "k", "v"], pending, in_w, [pf["q"], pf["k"], pf["v"]], T)
             if self.qk_norms[li] is not None:
                 for src, dst, wgt, heads in ((pf["q"], pf["qn"], self.qk_norms[li][0], self.h_loc),
                                              (pf["k"], pf["kn"], self.qk_norms[li][1], self.kv_loc)):
@@ -858,9 +882,7 @@ class Decoder(SlotDecoder):
             self._prefill_linears(li, ["o"], pf["attn"], [pf["delta"]], T)
             if self.tp_size > 1:
                 torch.distributed.all_reduce(pf["delta"][:T], group=self.group)
-            check(lib.qk_rmsnorm(c, _p(pf["x"]), _p(pf["delta"]), _p(post_w), T, d, cfg.rms_eps,
-                                 self.serving_tag, _p(pf["x"]), _p(pf["h"])))
-            self._prefill_linears(li, ["gate", "up"], pf["h"], [pf["g"], pf["u"]], T)
+            self._prefill_normed_linears(li, ["gate", "up"], pf["delta"], post_w, [pf["g"], pf["u"]], T)
             if cfg.serving == "bfloat16" and T >= cfg.gemm_min_batch:
                 apply_prefill_many_gated([self.layers[li]["down"]], pf["g"].data_ptr(), pf["u"].data_ptr(),
                                          T, [pf["delta"].data_ptr()])
@@ -869,7 +891,7 @@ class Decoder(SlotDecoder):
                 self._prefill_linears(li, ["down"], pf["a"], [pf["delta"]], T)
             if self.tp_size > 1:
                 torch.distributed.all_reduce(pf["delta"][:T], group=self.group)
-            pending = _p(pf["delta"])
+            pending = pf["delta"]
 
     def _portion_hidden(self, rows, out) -> None:
         cfg, pf = self.cfg, self._pf

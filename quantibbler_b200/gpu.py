@@ -399,6 +399,22 @@ def apply_prefill_many_gated(layers, gate_ptr: int, up_ptr: int, n_tokens: int, 
                                                    ctypes.c_void_p(up_ptr), int(n_tokens), outs))
 
 
+def apply_prefill_many_normed(layers, x_ptr: int, residual_ptr, weight_ptr: int, eps: float, x_out_ptr,
+                              n_tokens: int, y_ptrs) -> None:
+    """``apply_prefill_many`` on ``rmsnorm(x + residual) * weight`` (``residual_ptr`` may be None), the norm
+    formed inside the GEMM's scaling kernel, which also writes ``x + residual`` to ``x_out_ptr``.  Rows of
+    up to ``PREFILL_NORM_MAX`` entries.  Asynchronous."""
+    n = len(layers)
+    handles = (ctypes.c_void_p * n)(*[layer._h for layer in layers])
+    outs = (ctypes.c_void_p * n)(*[ctypes.c_void_p(p) for p in y_ptrs])
+    check(_lib.lib().qk_layers_apply_prefill_normed(
+        layers[0].ctx.handle, handles, n, ctypes.c_void_p(x_ptr), ctypes.c_void_p(residual_ptr),
+        ctypes.c_void_p(weight_ptr), float(eps), ctypes.c_void_p(x_out_ptr), int(n_tokens), outs))
+
+
+PREFILL_NORM_MAX = 8192
+
+
 def apply_noalloc(layer: PackedLayer, x_ptr: int, y_ptr: int) -> None:
     """One token through ``layer`` with the library allocating nothing: for hosts that own
     all device memory themselves (for example a server whose KV cache took what was left

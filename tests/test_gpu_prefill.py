@@ -146,3 +146,50 @@ def test_gated_prefill_equals_swiglu_then_prefill(gpu_ctx, shape):
     with pytest.raises(ValueError, match="gate and up"):
         apply_prefill_many_gated([layer], gate.data_ptr(), 0, n_tokens, [fused.data_ptr()])
     layer.close()
+
+
+@pytest.mark.parametrize("d,n_tokens,residual,in_place", [(64, 7, False, True), (520, 70, True, True),
+                                                          (4096, 33, True, False), (8192, 3, True, True)])
+def test_norm_inside_the_call(gpu_ctx, d, n_tokens, residual, in_place):
+    """The norm formed by the scaling kernel gives the bits of the norm kernel followed by the linears; the
+    row lengths are below one pass of a block, off its multiples, and the longest that is taken."""
+    import ctypes
+    import torch
+    from quantibbler_b200 import _lib
+    from quantibbler_b200.gpu import apply_prefill_many, apply_prefill_many_normed
+    layers = []
+    for i, (dout, r) in enumerate([(96, 40), (130, 33)]):
+        L = make_layer(dout, d, r, seed=d + i)
+        layers.append(PackedLayer(gpu_ctx, L["ub_rows"], L["vb_t_rows"], dout, d, r, L["s1"], L["s2"], None,
+                                  serving="bfloat16"))
+    gen = torch.Generator(device="cuda").manual_seed(d)
+    x = torch.randn(n_tokens, d, device="cuda", generator=gen)
+    more = torch.randn(n_tokens, d, device="cuda", generator=gen) if residual else None
+    weight = torch.randn(d, device="cuda", generator=gen)
+    out = lambda: [torch.full((n_tokens, n), float("nan"), device="cuda") for n in (96, 130)]  # noqa: E731
+    want, got = out(), out()
+    stream, h = torch.empty_like(x), torch.empty_like(x)
+    p = lambda t: ctypes.c_void_p(None if t is None else t.data_ptr())  # noqa: E731
+    torch.cuda.synchronize()
+    _lib.check(_lib.lib().qk_rmsnorm(gpu_ctx.handle, p(x), p(more), p(weight), n_tokens, d, 1e-5, _lib.QK_BF16,
+                                     p(stream), p(h)))
+    apply_prefill_many(layers, h.data_ptr(), n_tokens, [t.data_ptr() for t in want])
+    gpu_ctx.synchronize()
+    x_out = x if in_place else torch.empty_like(x)
+    torch.cuda.synchronize()
+    apply_prefill_many_normed(layers, x.data_ptr(), more.data_ptr() if residual else None, weight.data_ptr(), 1e-5,
+                              x_out.data_ptr(), n_tokens, [t.data_ptr() for t in got])
+    gpu_ctx.synchronize()
+    assert torch.equal(x_out, stream)
+    for a, b in zip(want, got):
+        assert torch.equal(a, b)
+
+
+def test_norm_inside_the_call_refuses_long_rows(gpu_ctx):
+    import torch
+    from quantibbler_b200.gpu import apply_prefill_many_normed
+    L = make_layer(16, 8200, 8, seed=1)
+    layer = PackedLayer(gpu_ctx, L["ub_rows"], L["vb_t_rows"], 16, 8200, 8, L["s1"], L["s2"], None, serving="bfloat16")
+    t = torch.zeros(8, 8200, device="cuda")
+    with pytest.raises(ValueError, match="8192 entries"):
+        apply_prefill_many_normed([layer], t.data_ptr(), None, t.data_ptr(), 1e-5, None, 8, [t.data_ptr()])
