@@ -372,17 +372,6 @@ __device__ __forceinline__ bool tc_epilogue_vote(bool ok) {
     return all != 0;
 }
 
-// 16 consecutive 32-bit columns of this thread's tensor-memory lane.
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&v)[16]) {
-    asm volatile(
-        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-          "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-        : "r"(taddr)
-        : "memory");
-}
-
 // A warp's 32 rows x 32 columns go through shared memory, so that eight lanes hold 32 consecutive
 // columns of a row, four each: whole lines for every load and store of the epilogue.
 constexpr int kEpiPitch = 36;  // floats per staged row

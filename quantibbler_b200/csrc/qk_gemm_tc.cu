@@ -11,25 +11,26 @@
 // The weights take the M side of the MMA (128 weight rows per tile) and the tokens the N
 // side (up to 256 tokens), so that the costly operand - the one that has to be expanded -
 // is the narrow one.  One persistent CTA per SM walks over its tiles with these roles:
-//   * warps 0..15, producers, in four groups of 128 threads; group g owns pipeline stage g
-//     and fills it for every fourth 64-wide k-chunk.  Thread i of a group owns weight row
-//     i of the tile: it reads the row's 64 bits of the chunk (two such loads ahead) and
-//     turns them into 64 bfloat16 +-1 values in registers (a multiply that spreads four
-//     bits to the tops of four bytes, one LOP3, two byte permutes per four weights: no
-//     table, because shared-memory bandwidth is what bounds this kernel), stored as eight
-//     16-byte pieces in the 128-byte-swizzled K-major layout
-//     the UMMA descriptors expect.  The group's first thread also starts the TMA copy
-//     (cp.async.bulk.tensor, one CTA per copy) of the chunk's activation tile, up to 256
-//     tokens x 64 k; rows beyond the token count are zero-filled by the copy;
+//   * warps 0..15, producers, in four groups of 128 threads; group g fills every fourth 64-wide
+//     k-chunk.  Thread i of a group owns weight row i of the tile: it reads the row's 64 bits of
+//     the chunk (two such loads ahead) and turns them into 64 bfloat16 +-1 values in registers (a
+//     multiply that spreads four bits to the tops of four bytes, one LOP3, two byte permutes per
+//     four weights: no table), stored as eight 16-byte pieces in the 128-byte-swizzled K-major
+//     layout the UMMA descriptors expect;
 //   * warp 16 issues tcgen05.mma (M = 128, N = tokens, K = 16 per instruction, four per
-//     stage) with the float32 accumulator in tensor memory; tcgen05.commit hands the stage
-//     back to its group.  The wait-issue-commit loop costs about 530 cycles per chunk
-//     whatever N is, which is why the token tile is as wide as it can be (N = 256 is 512
-//     cycles of tensor-core work per chunk);
+//     stage) with the float32 accumulator in tensor memory; tcgen05.commit hands the stage back;
 //   * warps 17..20, epilogue: tensor memory holds two accumulators, so the epilogue of one
 //     tile (tcgen05.ld, one weight row per thread so that a warp's stores to the
 //     token-major output are contiguous; rounding, scale, bias) overlaps the main loop of
-//     the next.
+//     the next.  The last tile of a CTA's run is finished by the producers as well;
+//   * warp 21 starts the TMA copies of the activation tile, up to 256 tokens x 64 k; rows
+//     beyond the token count are zero-filled by the copy.
+// What bounds it: with 256 tokens per tile a chunk takes 545 to 570 clocks where its products take 512,
+// at 1.45 GHz under the power cap, i.e. 1.6 PFLOP/s inside the loops, which is what cuBLAS reaches.  The
+// producers' positions used to cost three divisions per chunk and the copies waited behind the
+// expansion: 890 clocks.  Around the loops come 5 us of launch and first fetch per kernel and the last tile.
+// 14336 x 4096 of rank 2560 on 2048 tokens: 209 -> 162 us, 4096 x 4096 of rank 1102 on 64 tokens 29.7 -> 24.5 us.
+// Pairs of CTAs sharing the token tile (cta_group::2) came out no faster: 172 against 172 us.
 // All hand-offs go through mbarriers.  Every wait is bounded: on expiry the kernel records an
 // error code, frees its tensor memory and returns, and the host reports QK_ERR_TIMEOUT.
 #include <cuda.h>  // CUtensorMap types only; the encoder is fetched through the runtime
@@ -48,13 +49,15 @@ constexpr int kBM = 128;        // weight rows per tile (UMMA M)
 constexpr int kBNMax = 256;     // tokens per tile (UMMA N), a multiple of 16
 constexpr int kBK = 64;         // k per stage: one 128-byte swizzle row of bfloat16
 constexpr int kStages = 4;
-constexpr int kGroups = kStages;            // producer groups; group g fills stage g
+constexpr int kGroups = 4;                  // producer groups; group g fills every fourth chunk
 constexpr int kGroupThreads = 128;          // one thread per weight row of the tile
 constexpr int kProducerWarps = kGroups * kGroupThreads / 32;  // warps 0..15
 constexpr int kMmaWarp = kProducerWarps;                      // warp 16
 constexpr int kEpilogueWarp0 = kMmaWarp + 1;                  // warps 17..20
 constexpr int kEpilogueWarps = 4;
-constexpr int kThreads = (kEpilogueWarp0 + kEpilogueWarps) * 32;
+constexpr int kFinishWarps = kProducerWarps + kEpilogueWarps;  // what finishes a CTA's last tile
+constexpr int kCopyWarp = kEpilogueWarp0 + kEpilogueWarps;    // warp 21
+constexpr int kThreads = (kCopyWarp + 1) * 32;
 constexpr uint32_t kABytes = kBM * kBK * 2, kBBytes = kBNMax * kBK * 2;  // A: weights, B: tokens
 constexpr uint32_t kStageBytes = kABytes + kBBytes;
 constexpr uint32_t kTmemCols = 2 * kBNMax;    // two accumulators
@@ -108,6 +111,7 @@ struct GemmArgs {
     int *error;
     uint32_t tokens;
     uint32_t bn;           // tokens per tile
+    uint32_t tok_tiles;    // ... and how many such tiles there are
     uint32_t units;        // all tiles x their k_chunks: the work that is dealt out evenly to the CTAs
     float *partials;       // [CTAs][256][128] float32 accumulators of split tiles
     uint32_t *flags;       // [CTAs] flags[i] != 0: CTA i's partial is in place (its one reader clears it)
@@ -131,19 +135,71 @@ __device__ __forceinline__ UnitPos locate(const GemmArgs &g, uint32_t u) {
     return {pi, tile, local - tile * k, g.p[pi].unit_begin + tile * k};
 }
 
-// The epilogue of one output element: kFinal = false: out = bf16(acc) as the next stage's
-// activation (zero in the padding columns);  true: y = bf16(acc) * s1 + bias.
-template <bool kFinal>
-__device__ __forceinline__ void store_output(const Problem &g, uint32_t tok, uint32_t n, uint32_t acc_bits,
-                                             float scale, float bias) {
-    // one rounding to bfloat16, as packed_matmul's bf16 instantiation does
-    const uint32_t rb = round_bf16_hi(acc_bits);
-    if (kFinal) {
-        static_cast<float *>(g.out)[(size_t)tok * g.n_rows + n] = __uint_as_float(rb) * scale + bias;
-    } else {
-        static_cast<uint16_t *>(g.out)[(size_t)tok * g.out_pitch + n] =
-            n < g.n_rows ? (uint16_t)(rb >> 16) : (uint16_t)0;
+// The same position, moved on chunk by chunk without a division: what the roles that act on every chunk use
+// (the producers spent more instructions on three divisions per chunk than on expanding it).
+struct Walk {
+    uint32_t problem, kc, k, row_tile, row_tiles, tok_tile;
+    __device__ __forceinline__ Walk(const GemmArgs &g, uint32_t u) {
+        const UnitPos at = locate(g, u);
+        problem = at.problem;
+        kc = at.kc;
+        k = g.p[problem].k_chunks;
+        row_tiles = g.p[problem].row_tiles;
+        tok_tile = at.tile / row_tiles;
+        row_tile = at.tile - tok_tile * row_tiles;
     }
+    // true if the tile changed
+    __device__ __forceinline__ bool advance(const GemmArgs &g, uint32_t n) {
+        kc += n;
+        if (kc < k) return false;
+        do {
+            kc -= k;
+            if (++row_tile == row_tiles) {
+                row_tile = 0;
+                if (++tok_tile == g.tok_tiles && problem + 1 < g.n_problems) {
+                    tok_tile = 0;
+                    ++problem;
+                    k = g.p[problem].k_chunks;
+                    row_tiles = g.p[problem].row_tiles;
+                }
+            }
+        } while (kc >= k);
+        return true;
+    }
+};
+
+// The epilogue of kW accumulators of one weight row, tokens tok .. tok + kW: one rounding to bfloat16 (as
+// packed_matmul's bf16 instantiation does), then kFinal = false: the next stage's activation (zero in the padding
+// columns);  true: y = bf16(acc) * s1 + bias.
+template <bool kFinal, int kW>
+__device__ __forceinline__ void store_outputs(const Problem &g, uint32_t tok, uint32_t n_tokens, uint32_t n,
+                                              const uint32_t (&v)[kW], float scale, float bias) {
+    uint32_t two[kW / 2];
+#pragma unroll
+    for (int j = 0; j < kW; j += 2)
+        asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(two[j / 2]) : "f"(__uint_as_float(v[j + 1])), "f"(__uint_as_float(v[j])));
+    auto each = [&](auto limit) {
+        if constexpr (kFinal) {
+            float *dst = static_cast<float *>(g.out) + (size_t)tok * g.n_rows + n;
+#pragma unroll
+            for (int j = 0; j < kW; ++j) {
+                if (limit.value && tok + j >= n_tokens) break;
+                *dst = __uint_as_float((j & 1) ? two[j / 2] & 0xffff0000u : two[j / 2] << 16) * scale + bias;
+                dst += g.n_rows;
+            }
+        } else {
+            uint16_t *dst = static_cast<uint16_t *>(g.out) + (size_t)tok * g.out_pitch + n;
+            const uint32_t keep = n < g.n_rows ? 0xffffffffu : 0u;
+#pragma unroll
+            for (int j = 0; j < kW; ++j) {
+                if (limit.value && tok + j >= n_tokens) break;
+                *dst = (uint16_t)((two[j / 2] & keep) >> ((j & 1) * 16));
+                dst += g.out_pitch;
+            }
+        }
+    };
+    if (tok + kW <= n_tokens) each(std::false_type{});
+    else each(std::true_type{});
 }
 
 template <bool kFinal>
@@ -162,6 +218,7 @@ factorized_gemm_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid
     uint64_t *staged_bar = acc_empty + 2;   // a neighbour's partial accumulator has landed
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(staged_bar + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
+    volatile uint32_t *segments = tmem_slot + 2;  // of this CTA's run
 
     const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     const uint32_t kBN = g.bn;
@@ -190,13 +247,10 @@ factorized_gemm_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid
         const uint32_t n_src = min((at.tile % pr.row_tiles) * kBM + row, pr.n_rows - 1);
         return reinterpret_cast<const uint2 *>(pr.w_rows + (size_t)n_src * pr.w_stride) + at.kc;
     };
-    auto load_bits = [&](uint32_t gc) -> uint2 {
-        return gc < total_chunks ? *bits_at(gc) : make_uint2(0, 0);
-    };
     uint2 q0 = make_uint2(0, 0), q1 = q0;
     if (warp < kProducerWarps) {
-        q0 = load_bits(group);
-        q1 = load_bits(group + kGroups);
+        if (group < total_chunks) q0 = *bits_at(group);
+        if (group + kGroups < total_chunks) q1 = *bits_at(group + kGroups);
         // (a 128-byte line of a row holds sixteen chunks)
         for (uint32_t gc = group + 16; gc < total_chunks && gc < group + 16 * 8; gc += 16)
             asm volatile("prefetch.global.L2 [%0];" ::"l"(bits_at(gc)));
@@ -205,7 +259,7 @@ factorized_gemm_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid
             const CUtensorMap *m = lane == 0 ? &map0 : lane == 1 ? &map1 : lane == 2 ? &map2 : &map3;
             asm volatile("prefetch.tensormap [%0];" ::"l"(m) : "memory");
         }
-    } else if (kFinal && total_chunks) {
+    } else if (kFinal && total_chunks && warp < kCopyWarp) {
         const UnitPos at = locate(g, u_begin);
         const Problem &pr = g.p[at.problem];
         const uint32_t n = min((at.tile % pr.row_tiles) * kBM + (warp % 4) * 32 + lane, pr.n_rows - 1);
@@ -241,36 +295,83 @@ factorized_gemm_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid
     // waits, so that this kernel's completion implies the completion of everything before it.
     qk::pdl_wait();
     const uint32_t tmem_base = *tmem_slot;
+    bool ok = true;  // none of this warp's waits has run out
+
+    // ---- the epilogue's parts.  Thread = weight row n (tensor-memory lane; a warp reaches the 32 lanes of its
+    // number modulo 4), columns = tokens.
+    const size_t slot_elems = (size_t)kBNMax * kBM;
+    const uint32_t quarter = warp % 4, n_local = quarter * 32 + lane;
+    const uint32_t u_last = total_chunks ? max(u_begin, locate(g, u_end - 1).tile_begin) : u_begin;
+    struct Target {
+        const Problem *pr;
+        uint32_t n, t0;
+        float scale, bias;
+    };
+    auto target_of = [&](const UnitPos &at) -> Target {
+        const Problem &pr = g.p[at.problem];
+        const uint32_t token_tile = at.tile / pr.row_tiles, n = (at.tile - token_tile * pr.row_tiles) * kBM + n_local;
+        return {&pr, n, token_tile * kBN, (kFinal && pr.out_scale && n < pr.n_rows) ? pr.out_scale[n] : 1.f,
+                (kFinal && pr.out_bias && n < pr.n_rows) ? pr.out_bias[n] : 0.f};
+    };
+    // kW token columns: tensor memory -> registers, then the partial stored, or the other CTAs' shares added
+    // in CTA order and the finished outputs stored
+    auto columns = [&](const Target &to, uint32_t acc, uint32_t c0, bool partial, uint32_t n_staged, uint32_t last,
+                       auto width) {
+        constexpr int kW = decltype(width)::value;
+        uint32_t v[kW];
+        const uint32_t taddr = tmem_base + ((quarter * 32) << 16) + acc * kBNMax + c0;
+        if constexpr (kW == 32) tmem_ld32(taddr, v);
+        else tmem_ld16(taddr, v);
+        tmem_ld_wait();
+        if (partial) {
+            // the rest of a tile another CTA began: the raw accumulator, [token column][weight row]
+            float *part = g.partials + (size_t)blockIdx.x * slot_elems + (size_t)c0 * kBM + n_local;
+#pragma unroll
+            for (int j = 0; j < kW; ++j) part[j * kBM] = __uint_as_float(v[j]);
+            return;
+        }
+        for (uint32_t i = 0; i < n_staged; ++i) {  // in CTA order
+            const float *sp = reinterpret_cast<const float *>(tiles) + (size_t)i * (kBN * kBM) + c0 * kBM + n_local;
+#pragma unroll
+            for (int j = 0; j < kW; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + sp[j * kBM]);
+        }
+        for (uint32_t p = blockIdx.x + 1 + n_staged; p < last; ++p) {
+            const float *src = g.partials + (size_t)p * slot_elems + (size_t)c0 * kBM + n_local;
+            float got[kW];
+#pragma unroll
+            for (int j = 0; j < kW; ++j) got[j] = __ldcg(src + j * kBM);
+#pragma unroll
+            for (int j = 0; j < kW; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + got[j]);
+        }
+        if (kFinal ? to.n < to.pr->n_rows : to.n < to.pr->out_pitch)
+            store_outputs<kFinal, kW>(*to.pr, to.t0 + c0, g.tokens, to.n, v, to.scale, to.bias);
+    };
+    // publish the partial: the warps that stored it meet (which orders their stores before the one thread that
+    // goes on), and that thread raises the flag with a release at device scope, which is cumulative over what it
+    // has synchronised with
+    auto publish = [&](uint32_t n_threads) {
+        asm volatile("bar.sync 1, %0;" ::"r"(n_threads) : "memory");
+        if (warp == kEpilogueWarp0 && lane == 0)
+            asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(g.flags + blockIdx.x), "r"(1u) : "memory");
+    };
 
     if (warp < kProducerWarps) {
-        // ------------------------------------------------------------ producers
-        uint8_t *a_tile = tiles + group * kStageBytes, *b_tile = a_tile + kABytes;
-        uint64_t *my_full = &full[group], *my_empty = &empty[group];
-        const uint32_t dst_base = smem_u32(a_tile) + row * 128, swz = (row & 7) << 4;
-        uint32_t it = 0;
-        for (uint32_t gc = group; gc < total_chunks; gc += kGroups, ++it) {
+        // ------------------------------------------------------------ producers (group g: stage g)
+        const uint32_t swz = (row & 7) << 4, s = group;
+        const uint32_t dst_base = smem_u32(tiles + s * kStageBytes) + row * 128;
+        uint32_t phase = 1;
+        Walk ahead(g, min(u_begin + group + 2 * kGroups, g.units - 1));  // the chunk whose bits are asked for next
+        auto row_of = [&]() {
+            const Problem &pr = g.p[ahead.problem];
+            return pr.w_rows + (size_t)min(ahead.row_tile * kBM + row, pr.n_rows - 1) * pr.w_stride;
+        };
+        const uint8_t *bits = row_of();
+        for (uint32_t gc = group; gc < total_chunks; gc += kGroups) {
             const uint2 cur = q0;
-            q0 = q1;
-            q1 = load_bits(gc + 2 * kGroups);
-            if (!mbar_wait(my_empty, (it & 1) ^ 1, abort_flag, g.wait_limit)) {
+            if (!mbar_wait(&empty[s], phase, abort_flag, g.wait_limit)) {
+                ok = false;
                 *abort_flag = 1;
                 break;
-            }
-            if (row == 0) {
-                // tokens: one TMA box of 64 k x bn tokens, completing on the full barrier
-                const UnitPos at = locate(g, u_begin + gc);
-                const uint32_t kc = at.kc, t0 = (at.tile / g.p[at.problem].row_tiles) * kBN;
-                const CUtensorMap *b_map = at.problem == 0 ? &map0 : at.problem == 1 ? &map1
-                                         : at.problem == 2 ? &map2 : &map3;
-                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
-                                 smem_u32(my_full)),
-                             "r"(kBN * kBK * 2)
-                             : "memory");
-                asm volatile(
-                    "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes "
-                    "[%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(b_tile)),
-                    "l"(b_map), "r"(kc * kBK), "r"(t0), "r"(smem_u32(my_full))
-                    : "memory");
             }
 #pragma unroll
             for (int c = 0; c < 8; ++c) {
@@ -289,15 +390,21 @@ factorized_gemm_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid
             // generic-proxy writes must be visible to the tensor core's async proxy
             asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
             __syncwarp();
-            if (lane == 0) mbar_arrive(my_full);
+            if (lane == 0) mbar_arrive(&full[s]);
+            q0 = q1;
+            if (gc + 2 * kGroups < total_chunks) {
+                q1 = *reinterpret_cast<const uint2 *>(bits + ahead.kc * 8);
+                if (gc + 3 * kGroups < total_chunks && ahead.advance(g, kGroups)) bits = row_of();
+            }
+            phase ^= 1;
         }
     } else if (warp == kMmaWarp) {
         // ------------------------------------------------------------ MMA issue
         // The whole warp runs the loop and waits on the barriers; one lane issues.
         const uint32_t idesc = umma_idesc(kBN);
-        uint32_t gc = 0;
+        uint32_t gc = 0, seg = 0;
         bool dead = false;
-        for (uint32_t u = u_begin, seg = 0; u < u_end && !dead; ++seg) {
+        for (uint32_t u = u_begin; u < u_end && !dead; ++seg) {
             const UnitPos at = locate(g, u);
             const uint32_t kc0 = at.kc, kc1 = min(g.p[at.problem].k_chunks, kc0 + (u_end - u));
             const uint32_t acc = seg & 1;
@@ -335,43 +442,92 @@ factorized_gemm_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid
             __syncwarp();
             u += kc1 - kc0;
         }
+        ok = !dead;
         if (dead) *abort_flag = 1;
-    } else {
-        // ------------------------------------------------------------ epilogue
-        // thread = weight row n (tensor-memory lane; a warp reaches the 32 lanes of its number
-        // modulo 4), columns = tokens
-        const uint32_t quarter = warp % 4;
-        const size_t slot_elems = (size_t)kBNMax * kBM;
-        bool dead = false;
-        for (uint32_t u = u_begin, seg = 0; u < u_end && !dead; ++seg) {
-            const UnitPos at = locate(g, u);
-            const Problem &pr = g.p[at.problem];
-            const uint32_t tile = at.tile, kc0 = at.kc;
-            const uint32_t len = min(pr.k_chunks - kc0, u_end - u);
-            const uint32_t acc = seg & 1;
-            const uint32_t n_local = quarter * 32 + lane;
-            const uint32_t n = (tile % pr.row_tiles) * kBM + n_local;
-            const uint32_t t0 = (tile / pr.row_tiles) * kBN;
-            // CTAs [blockIdx.x + 1, last) hold the rest of this tile
-            uint32_t last = blockIdx.x + 1;
-            if (kc0 == 0 && len < pr.k_chunks) {
-                const uint32_t hi = at.tile_begin + pr.k_chunks;
-                while (last < gridDim.x && g.cta_begin[last] < hi) ++last;
+        if (lane == 0) *segments = seg;
+    } else if (warp == kCopyWarp) {
+        // ------------------------------------------------------------ token copies
+        // one TMA box of 64 k x bn tokens per chunk, completing on the full barrier
+        Walk at(g, min(u_begin, g.units - 1));
+        for (uint32_t gc = 0, s = 0, phase = 1; gc < total_chunks; ++gc) {
+            if (!mbar_wait(&empty[s], phase, abort_flag, g.wait_limit)) {
+                ok = false;
+                *abort_flag = 1;
+                break;
             }
-            // this CTA's own share of the tile first: once its accumulator is complete, every
-            // MMA of the CTA so far has read its operands
-            dead = !mbar_wait(&acc_full[acc], (seg >> 1) & 1, abort_flag, g.wait_limit);
-            // When this is the CTA's last segment the pipeline has drained and the stages are
-            // free: as many of the following CTAs' partials as fit there (each is contiguous,
-            // bn x 128 floats) come in by bulk copies instead of latency-bound loads, each one
-            // started the moment its flag is seen, so that the copies run while the later CTAs
-            // are still being waited for.  Any further partials are read directly.
-            const uint32_t part_bytes = kBN * kBM * 4;
-            uint32_t n_staged = 0;
-            if (last > blockIdx.x + 1 && u + len == u_end)
-                n_staged = min(last - blockIdx.x - 1, (uint32_t)(kStages * kStageBytes) / part_bytes);
-            const bool staged = n_staged > 0, issuer = warp == kEpilogueWarp0 && lane == 0;
-            for (uint32_t j = blockIdx.x + 1; j < last && !dead; ++j) {
+            if (lane == 0) {
+                const CUtensorMap *b_map = at.problem == 0 ? &map0 : at.problem == 1 ? &map1
+                                         : at.problem == 2 ? &map2 : &map3;
+                asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
+                                 smem_u32(&full[s])),
+                             "r"(kBN * kBK * 2)
+                             : "memory");
+                asm volatile(
+                    "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes "
+                    "[%0], [%1, {%2, %3}], [%4];" ::"r"(smem_u32(tiles + s * kStageBytes) + kABytes),
+                    "l"(b_map), "r"(at.kc * kBK), "r"(at.tok_tile * kBN), "r"(smem_u32(&full[s]))
+                    : "memory");
+            }
+            __syncwarp();
+            if (gc + 1 < total_chunks) at.advance(g, 1);
+            if (++s == kStages) {
+                s = 0;
+                phase ^= 1;
+            }
+        }
+    } else {
+        // ------------------------------------------------------------ epilogue of all segments but the last
+        uint32_t seg = 0;
+        for (uint32_t u = u_begin; u < u_last; ++seg) {
+            const UnitPos at = locate(g, u);
+            const uint32_t acc = seg & 1;
+            ok = mbar_wait(&acc_full[acc], (seg >> 1) & 1, abort_flag, g.wait_limit);
+            // one verdict for the four epilogue warps before any of them touches tensor memory
+            // or one of the epilogue's barriers
+            if (!epilogue_vote(ok, kEpilogueWarps * 32)) {
+                *abort_flag = 1;
+                ok = false;
+                break;
+            }
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const Target to = target_of(at);
+#pragma unroll 1
+            for (uint32_t c0 = 0; c0 < kBN && to.t0 + c0 < g.tokens; c0 += 32) {  // warp-uniform
+                if (kBN - c0 >= 32) columns(to, acc, c0, at.kc != 0, 0, 0, std::integral_constant<int, 32>{});
+                else columns(to, acc, c0, at.kc != 0, 0, 0, std::integral_constant<int, 16>{});
+            }
+            // the accumulator may be overwritten once every epilogue warp has read it
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            __syncwarp();
+            if (lane == 0) mbar_arrive(&acc_empty[acc]);
+            if (at.kc != 0) publish(kEpilogueWarps * 32);
+            u += g.p[at.problem].k_chunks - at.kc;
+        }
+    }
+    // ---------------------------------------------------------------- the last segment
+    // Nothing is left to overlap it with and the producers are idle, so twenty warps finish it, five to a
+    // quarter of the rows, 16 tokens each in turn.  With the four epilogue warps alone its columns took
+    // 4 us of a launch.
+    if (!__syncthreads_and(ok)) {
+        *abort_flag = 1;
+    } else if (total_chunks && warp != kMmaWarp && warp < kCopyWarp) {
+        const uint32_t seg = *segments - 1, acc = seg & 1, slot = warp < kMmaWarp ? warp / 4 : 4u;
+        const UnitPos at = locate(g, u_last);
+        // CTAs [blockIdx.x + 1, last) hold the rest of this tile
+        uint32_t last = blockIdx.x + 1;
+        if (at.kc == 0) {
+            const uint32_t hi = at.tile_begin + g.p[at.problem].k_chunks;
+            while (last < gridDim.x && g.cta_begin[last] < hi) ++last;
+        }
+        // once this CTA's own share is complete, every MMA of the CTA has read its operands
+        ok = mbar_wait(&acc_full[acc], (seg >> 1) & 1, abort_flag, g.wait_limit);
+        // The stages are free: as many of the following CTAs' partials as fit there (each is contiguous, bn x 128
+        // floats) come in by bulk copies, each one started the moment its flag is seen, so that the copies run
+        // while the later CTAs are still being waited for.  Any further partials are read directly.
+        const uint32_t part_bytes = kBN * kBM * 4;
+        const uint32_t n_staged = min(last - blockIdx.x - 1, (uint32_t)(kStages * kStageBytes) / part_bytes);
+        if (warp == kEpilogueWarp0) {
+            for (uint32_t j = blockIdx.x + 1; j < last && ok; ++j) {
                 uint32_t seen = 0;
                 for (uint32_t i = 0; i < g.wait_limit; ++i) {
                     asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(g.flags + j) : "memory");
@@ -380,9 +536,9 @@ factorized_gemm_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid
                     __nanosleep(64);
                 }
                 // every lane made its own acquire load; the warp goes on only if all saw it
-                dead = __all_sync(0xffffffffu, seen != 0) == 0;
-                const uint32_t slot = j - blockIdx.x - 1;
-                if (!dead && issuer && slot < n_staged) {
+                ok = __all_sync(0xffffffffu, seen != 0) != 0;
+                const uint32_t place = j - blockIdx.x - 1;
+                if (ok && lane == 0 && place < n_staged) {
                     // (the partial was written through the generic proxy and is read by the
                     // asynchronous one)
                     asm volatile("fence.proxy.async.global;" ::: "memory");
@@ -392,124 +548,43 @@ factorized_gemm_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid
                                  : "memory");
                     asm volatile(
                         "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::
-                            "r"(smem_u32(tiles) + slot * part_bytes),
+                            "r"(smem_u32(tiles) + place * part_bytes),
                         "l"(g.partials + (size_t)j * slot_elems), "r"(part_bytes), "r"(smem_u32(staged_bar))
                         : "memory");
                 }
             }
-            // (the barrier's one pending arrival keeps its phase open until every copy that was
-            // started has been accounted for; the issuer arrives whether or not its warp gave
-            // up, and every warp waits for the copies that are in flight before it votes)
-            if (issuer && staged) mbar_arrive(staged_bar);
-            if (staged && !mbar_wait(staged_bar, 0, abort_flag, g.wait_limit)) dead = true;
-            // one verdict for the four epilogue warps before any of them touches tensor memory
-            // or one of the epilogue's barriers
-            if (!epilogue_vote(!dead, kEpilogueWarps * 32)) {
-                *abort_flag = 1;
-                dead = true;
-                break;
-            }
+            // (the barrier's one pending arrival keeps its phase open until every copy that was started has
+            // been accounted for; it comes whether or not this warp gave up, and every warp waits for the
+            // copies in flight before it votes)
+            if (lane == 0) mbar_arrive(staged_bar);
+        }
+        if (!mbar_wait(staged_bar, 0, abort_flag, g.wait_limit)) ok = false;
+        // (one verdict before any of the warps touches tensor memory; with it the flags that one warp has
+        // seen are seen by all)
+        if (!epilogue_vote(ok, kFinishWarps * 32)) {
+            *abort_flag = 1;
+        } else {
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const bool n_live = kFinal ? n < pr.n_rows : n < pr.out_pitch;
-            const float scale = (kFinal && pr.out_scale && n < pr.n_rows) ? pr.out_scale[n] : 1.f;
-            const float bias = (kFinal && pr.out_bias && n < pr.n_rows) ? pr.out_bias[n] : 0.f;
-            float *part = g.partials + (size_t)blockIdx.x * slot_elems;
-            const float *staged_part = reinterpret_cast<const float *>(tiles);
-            // kW token columns at a time: tensor memory -> registers, the other CTAs' shares
-            // added in CTA order, then the partial or the finished outputs stored
-            auto columns = [&](uint32_t c0, auto width) {
-                constexpr int kW = decltype(width)::value;
-                uint32_t v[kW];
-                const uint32_t taddr = tmem_base + ((quarter * 32) << 16) + acc * kBNMax + c0;
-                if constexpr (kW == 32) {
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-                        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-                        "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]),
-                          "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]),
-                          "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]), "=r"(v[16]), "=r"(v[17]),
-                          "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-                          "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]),
-                          "=r"(v[30]), "=r"(v[31])
-                        : "r"(taddr)
-                        : "memory");
-                } else {
-                    asm volatile(
-                        "tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                        "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                        : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]),
-                          "=r"(v[6]), "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]),
-                          "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15])
-                        : "r"(taddr)
-                        : "memory");
-                }
-                asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-                if (kc0 != 0) {
-                    // the rest of a tile another CTA began: the raw accumulator,
-                    // [token column][weight row]
-#pragma unroll
-                    for (int j = 0; j < kW; ++j)
-                        part[(size_t)(c0 + j) * kBM + n_local] = __uint_as_float(v[j]);
-                    return;
-                }
-                for (uint32_t i = 0; i < n_staged; ++i) {  // in CTA order
-                    const float *sp = staged_part + (size_t)i * (kBN * kBM) + c0 * kBM + n_local;
-#pragma unroll
-                    for (int j = 0; j < kW; ++j)
-                        v[j] = __float_as_uint(__uint_as_float(v[j]) + sp[j * kBM]);
-                }
-                for (uint32_t p = blockIdx.x + 1 + n_staged; p < last; ++p) {
-                    const float *src = g.partials + (size_t)p * slot_elems + (size_t)c0 * kBM + n_local;
-                    float got[kW];
-#pragma unroll
-                    for (int j = 0; j < kW; ++j) got[j] = __ldcg(src + j * kBM);
-#pragma unroll
-                    for (int j = 0; j < kW; ++j) v[j] = __float_as_uint(__uint_as_float(v[j]) + got[j]);
-                }
-                if (n_live) {
-#pragma unroll
-                    for (int j = 0; j < kW; ++j) {
-                        const uint32_t tok = t0 + c0 + j;
-                        if (tok >= g.tokens) break;
-                        store_output<kFinal>(pr, tok, n, v[j], scale, bias);
-                    }
-                }
-            };
-            for (uint32_t c0 = 0; c0 < kBN;) {
-                if (t0 + c0 >= g.tokens) break;  // warp-uniform
-                if (kBN - c0 >= 32) {
-                    columns(c0, std::integral_constant<int, 32>{});
-                    c0 += 32;
-                } else {
-                    columns(c0, std::integral_constant<int, 16>{});
-                    c0 += 16;
-                }
-            }
-            // the accumulator may be overwritten once every epilogue warp has read it
-            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-            __syncwarp();
-            if (lane == 0) mbar_arrive(&acc_empty[acc]);
-            if (last > blockIdx.x + 1) {
+            const Target to = target_of(at);
+#pragma unroll 1
+            for (uint32_t c0 = slot * 16; c0 < kBN && to.t0 + c0 < g.tokens; c0 += 16 * (kFinishWarps / 4))
+                columns(to, acc, c0, at.kc != 0, n_staged, last, std::integral_constant<int, 16>{});
+            if (at.kc != 0) {
+                publish(kFinishWarps * 32);
+            } else if (last > blockIdx.x + 1) {
                 // every partial of this tile has been read: hand the flags back, cleared, for
                 // the next launch (this CTA is their only reader)
-                asm volatile("bar.sync 1, %0;" ::"r"(kEpilogueWarps * 32) : "memory");
+                asm volatile("bar.sync 1, %0;" ::"r"(kFinishWarps * 32) : "memory");
                 if (warp == kEpilogueWarp0 && lane == 0)
                     for (uint32_t j = blockIdx.x + 1; j < last; ++j) g.flags[j] = 0;
             }
-            if (kc0 != 0) {
-                // publish the partial: the four warps meet (which orders their stores before
-                // the one thread that goes on), and that thread raises the flag with a release
-                // at device scope, which is cumulative over what it has synchronised with
-                asm volatile("bar.sync 1, %0;" ::"r"(kEpilogueWarps * 32) : "memory");
-                if (warp == kEpilogueWarp0 && lane == 0)
-                    asm volatile("st.release.gpu.global.u32 [%0], %1;" ::"l"(g.flags + blockIdx.x), "r"(1u) : "memory");
-            }
-            u += len;
         }
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
+    // (given up: the copies and products still in flight end within microseconds, a millisecond is waited)
+    if (*abort_flag)
+        for (int i = 0; i < 1000; ++i) __nanosleep(1000);
     if (warp == kMmaWarp) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
                      "r"(kTmemCols)
@@ -676,9 +751,6 @@ qk_status encode_activation_map(const uint16_t *base, size_t rows, size_t pitch,
     return QK_OK;
 }
 
-// Tokens per tile.  The MMA warp's wait-issue-commit loop takes about 530 cycles per chunk
-// whatever N is, and N = 256 is 512 cycles of tensor-core work, so a narrower tile is never
-// faster per tile; it only helps when there are fewer tokens than that.
 // Which units each CTA takes.  Many tiles (a prompt): the units are dealt out evenly, a CTA's
 // run crossing tile borders wherever it falls.  Few tiles (a decode batch: at most half as
 // many tiles as CTAs): every tile goes to a whole number of CTAs in equal parts, so that no
@@ -716,8 +788,39 @@ unsigned plan_ctas(GemmArgs &g, size_t units, const size_t *tiles, size_t n_prob
     return (unsigned)n;
 }
 
-uint32_t pick_bn(size_t tokens) {
-    return tokens >= (size_t)kBNMax ? (uint32_t)kBNMax : (uint32_t)(qk::ceil_div(tokens, 16) * 16);
+// Tokens per tile of one stage: the width whose slowest CTA is done first.  A chunk costs what its products cost,
+// at least what the hand-offs cost (measured: 570 clocks at 256 tokens, 345 for narrow tiles), a run ends with
+// its last tile's epilogue, and a tile that CTAs share with the others' partials coming in one after the other.
+// A wide tile expands a weight bit for more tokens at once; a narrow one leaves fewer CTAs to a tile (4096 x 4096 of
+// rank 1102 on 256 tokens: 40 us with the widest tile, 29 with the one chosen here).
+uint32_t pick_bn(const GemmArgs &g, size_t n_problems, size_t tokens, unsigned sm_count) {
+    const uint32_t widest = (uint32_t)std::min<size_t>(kBNMax, qk::ceil_div(tokens, 16) * 16);
+    uint32_t best = widest;
+    uint64_t best_cost = ~0ull;
+    for (uint32_t bn : {widest, 128u, 64u, 32u}) {
+        if (bn > widest || (bn == widest && best_cost != ~0ull)) continue;
+        GemmArgs t = g;
+        size_t units = 0, tiles[kMaxProblems] = {};
+        for (size_t p = 0; p < n_problems; ++p) {
+            tiles[p] = g.p[p].row_tiles * qk::ceil_div(tokens, bn);
+            t.p[p].unit_begin = (uint32_t)units;
+            units += tiles[p] * g.p[p].k_chunks;
+        }
+        if (units >= (1ull << 32)) continue;
+        const unsigned n = plan_ctas(t, units, tiles, n_problems, sm_count);
+        uint32_t run = 0, sharers = 1;
+        for (unsigned i = 0, p = 0; i < n; ++i) {
+            run = std::max(run, t.cta_begin[i + 1] - t.cta_begin[i]);
+            while (p + 1 < n_problems && t.cta_begin[i] >= t.p[p + 1].unit_begin) ++p;
+            if ((t.cta_begin[i] - t.p[p].unit_begin) % t.p[p].k_chunks) sharers = 2;
+        }
+        for (size_t p = 0; p < n_problems; ++p)
+            sharers = std::max(sharers, (uint32_t)qk::ceil_div(t.p[p].k_chunks, run));
+        const uint64_t cost = (uint64_t)run * std::max(345u, 25 + bn * 17 / 8) + 1500 + 4 * bn +
+                              (sharers > 1 ? 2500 + (uint64_t)(sharers - 1) * bn * 13 : 0);
+        if (cost < best_cost) best = bn, best_cost = cost;
+    }
+    return best;
 }
 
 }  // namespace
@@ -786,26 +889,30 @@ static qk_status apply_prefill(qk_ctx *ctx, const qk_layer *const *layers, size_
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
     QK_CUDA(cudaFuncSetAttribute(factorized_gemm_tc_kernel<true>,
                                  cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
-    const uint32_t bn = pick_bn(n_tokens);
-    const size_t tok_tiles = qk::ceil_div(n_tokens, bn);
     uint32_t *flags = (uint32_t *)c->d_err.ptr + 64;  // after the error word's 256 bytes
     GemmArgs g1{}, g2{};
     CUtensorMap maps1[kMaxProblems], maps2[kMaxProblems];
-    size_t units1 = 0, units2 = 0, tiles1[kMaxProblems] = {}, tiles2[kMaxProblems] = {};
     for (size_t i = 0; i < n_layers; ++i) {
         const qk_layer *L = layers[i];
-        uint16_t *z = (uint16_t *)(base + i * z_bytes), *t = (uint16_t *)(base + t_off[i]);
-        if ((st = encode_activation_map(z, n_tokens, kp1, bn, &maps1[i])) != QK_OK) return st;
-        if ((st = encode_activation_map(t, n_tokens, kp2[i], bn, &maps2[i])) != QK_OK) return st;
-        const size_t rows1 = qk::ceil_div(kp2[i], kBM), rows2 = qk::ceil_div(L->dout, kBM);
-        g1.p[i] = Problem{L->vbt, t, nullptr, nullptr, (uint32_t)L->r, (uint32_t)(kp1 / kBK),
-                          (uint32_t)L->vbt_stride, (uint32_t)kp2[i], (uint32_t)rows1, (uint32_t)units1};
+        g1.p[i] = Problem{L->vbt, base + t_off[i], nullptr, nullptr, (uint32_t)L->r, (uint32_t)(kp1 / kBK),
+                          (uint32_t)L->vbt_stride, (uint32_t)kp2[i], (uint32_t)qk::ceil_div(kp2[i], kBM), 0};
         g2.p[i] = Problem{L->ub, y_devs[i], L->s1, L->bias, (uint32_t)L->dout, (uint32_t)(kp2[i] / kBK),
-                          (uint32_t)L->ub_stride, (uint32_t)L->dout, (uint32_t)rows2, (uint32_t)units2};
-        tiles1[i] = rows1 * tok_tiles;
-        tiles2[i] = rows2 * tok_tiles;
-        units1 += rows1 * tok_tiles * (kp1 / kBK);
-        units2 += rows2 * tok_tiles * (kp2[i] / kBK);
+                          (uint32_t)L->ub_stride, (uint32_t)L->dout, (uint32_t)qk::ceil_div(L->dout, kBM), 0};
+    }
+    const uint32_t bn1 = pick_bn(g1, n_layers, n_tokens, (unsigned)c->sm_count);
+    const uint32_t bn2 = pick_bn(g2, n_layers, n_tokens, (unsigned)c->sm_count);
+    const size_t tok_tiles1 = qk::ceil_div(n_tokens, bn1), tok_tiles2 = qk::ceil_div(n_tokens, bn2);
+    size_t units1 = 0, units2 = 0, tiles1[kMaxProblems] = {}, tiles2[kMaxProblems] = {};
+    for (size_t i = 0; i < n_layers; ++i) {
+        const uint16_t *z = (const uint16_t *)(base + i * z_bytes), *t = (const uint16_t *)(base + t_off[i]);
+        if ((st = encode_activation_map(z, n_tokens, kp1, bn1, &maps1[i])) != QK_OK) return st;
+        if ((st = encode_activation_map(t, n_tokens, kp2[i], bn2, &maps2[i])) != QK_OK) return st;
+        tiles1[i] = g1.p[i].row_tiles * tok_tiles1;
+        tiles2[i] = g2.p[i].row_tiles * tok_tiles2;
+        g1.p[i].unit_begin = (uint32_t)units1;
+        g2.p[i].unit_begin = (uint32_t)units2;
+        units1 += tiles1[i] * g1.p[i].k_chunks;
+        units2 += tiles2[i] * g2.p[i].k_chunks;
     }
     for (size_t i = n_layers; i < (size_t)kMaxProblems; ++i) {  // unused slots: valid descriptors
         maps1[i] = maps1[0];
@@ -822,7 +929,10 @@ static qk_status apply_prefill(qk_ctx *ctx, const qk_layer *const *layers, size_
     g1.n_problems = g2.n_problems = (uint32_t)n_layers;
     g1.error = g2.error = err;
     g1.tokens = g2.tokens = (uint32_t)n_tokens;
-    g1.bn = g2.bn = bn;
+    g1.bn = bn1;
+    g2.bn = bn2;
+    g1.tok_tiles = (uint32_t)tok_tiles1;
+    g2.tok_tiles = (uint32_t)tok_tiles2;
     g1.units = (uint32_t)units1;
     g2.units = (uint32_t)units2;
     g1.partials = g2.partials = partials;

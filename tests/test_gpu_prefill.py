@@ -148,6 +148,35 @@ def test_gated_prefill_equals_swiglu_then_prefill(gpu_ctx, shape):
     layer.close()
 
 
+@pytest.mark.parametrize("dout,din,r,n_tokens", [
+    (128, 64, 64, 1), (130, 4096, 1100, 16), (1000, 512, 65, 17), (260, 1024, 300, 33), (4096, 2048, 129, 65),
+    (256, 4096, 1024, 129), (4096, 4096, 1102, 256), (384, 14336, 200, 257), (1024, 1024, 300, 1000),
+    (4096, 64, 700, 2047)])
+def test_every_token_at_the_edges_of_the_tiles(gpu_ctx, dout, din, r, n_tokens):
+    """All outputs against plain float32 products with the same rounding points: token tiles of every width and
+    one token more, runs of one k-chunk, tiles shared by many CTAs.  Both sides round t and u to bfloat16; where
+    their float32 sums straddle a rounding border the results differ by one bfloat16 step, so the norm of the
+    difference stays below one step (2^-8) of the result."""
+    import torch
+    L = make_layer(dout, din, r, seed=dout + n_tokens, with_bias=True)
+    layer = PackedLayer(gpu_ctx, L["ub_rows"], L["vb_t_rows"], dout, din, r, L["s1"], L["s2"], L["bias"],
+                        serving="bfloat16")
+    gen = torch.Generator(device="cuda").manual_seed(n_tokens)
+    x = torch.randn(n_tokens, din, device="cuda", generator=gen)
+    y = torch.full((n_tokens, dout), float("nan"), device="cuda")
+    torch.cuda.synchronize()
+    for _ in range(2):      # (the second call finds the flags as the first left them)
+        layer.apply_prefill(x.data_ptr(), n_tokens, y.data_ptr())
+    gpu_ctx.synchronize()
+    dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).cuda()  # noqa: E731
+    signs = lambda rows, n: dev(oracle.unpack_signs(rows, n)).to(torch.float64)  # noqa: E731
+    z = (dev(L["s2"]) * x).to(torch.bfloat16).double()
+    t = (z @ signs(L["vb_t_rows"], din).T).float().to(torch.bfloat16).double()
+    u = (t @ signs(L["ub_rows"], r).T).float().to(torch.bfloat16).float()
+    want = u * dev(L["s1"]) + dev(L["bias"])
+    assert float((y - want).norm() / want.norm()) <= 2.0 ** -8
+
+
 @pytest.mark.parametrize("d,n_tokens,residual,in_place", [(64, 7, False, True), (520, 70, True, True),
                                                           (4096, 33, True, False), (8192, 3, True, True)])
 def test_norm_inside_the_call(gpu_ctx, d, n_tokens, residual, in_place):
