@@ -78,6 +78,8 @@ struct qk_ctx {
         bool in_flight = false;
     } h_pinned[kPinnedSlots];
     int h_pinned_next = 0;
+    // kernels whose dynamic shared memory limit this context has raised already, and to what (qk::allow_smem)
+    std::vector<std::pair<const void *, int>> smem_allowed;
     // the copy streams and events of the host-buffer pipeline (qk_groups_apply_host), made on first use
     cudaStream_t up_stream = nullptr, down_stream = nullptr;
     std::vector<cudaEvent_t> pipe_events;
@@ -152,6 +154,15 @@ cudaError_t launch_pdl(bool allow_overlap, void (*kernel)(KArgs...), dim3 grid, 
 // Returns the context to use for a call: `ctx` itself, or the process-wide default on
 // device 0 (created on first use) when `ctx` is null.
 qk_status resolve_ctx(qk_ctx *ctx, qk_ctx **out);
+// Raises a kernel's dynamic shared memory limit, once per context and size (the call costs the host a microsecond).
+template <typename Kernel>
+qk_status allow_smem(qk_ctx *c, Kernel *kernel, size_t bytes) {
+    for (const auto &seen : c->smem_allowed)
+        if (seen.first == (const void *)kernel && seen.second >= (int)bytes) return QK_OK;
+    QK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+    c->smem_allowed.emplace_back((const void *)kernel, (int)bytes);
+    return QK_OK;
+}
 // Makes sure the context's error word (an int, bits: 1 a prefill pipeline wait, 2 an all-reduce
 // inbox wait, 4 a token outside the KV cache, 8 a wait of the streaming GEMV, 16 a grid barrier of the
 // whole-step decode kernel) and the prefill's CTA flags after it exist.

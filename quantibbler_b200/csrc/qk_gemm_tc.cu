@@ -885,10 +885,8 @@ static qk_status apply_prefill(qk_ctx *ctx, const qk_layer *const *layers, size_
                              x_dev, up_dev, sa, (uint32_t)n_tokens, (uint32_t)din, (uint32_t)kp1, vec);
     QK_CUDA(cudaGetLastError());
     c->launches++;
-    QK_CUDA(cudaFuncSetAttribute(factorized_gemm_tc_kernel<false>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
-    QK_CUDA(cudaFuncSetAttribute(factorized_gemm_tc_kernel<true>,
-                                 cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBytes));
+    if ((st = qk::allow_smem(c, factorized_gemm_tc_kernel<false>, kSmemBytes)) != QK_OK) return st;
+    if ((st = qk::allow_smem(c, factorized_gemm_tc_kernel<true>, kSmemBytes)) != QK_OK) return st;
     uint32_t *flags = (uint32_t *)c->d_err.ptr + 64;  // after the error word's 256 bytes
     GemmArgs g1{}, g2{};
     CUtensorMap maps1[kMaxProblems], maps2[kMaxProblems];

@@ -92,6 +92,20 @@ struct StageParams {
     uint32_t ar_rank, ar_world, ar_total, ar_offset, ar_poll_limit;
 };
 
+// One layer for several tokens, its record handed over with the launch itself: token y's input, output and
+// intermediate lie y steps on.  (A record array on the device costs each call a copy that the first stage has to
+// wait for: 4096 x 4096 of rank 1024 on one token, 16.4 -> 13.1 us a call, 1024 x 1024 of rank 300 on 12 tokens 19.5 -> 11.4.)
+struct StageRun {
+    StageParams p;
+    size_t in_step, out_step;  // bytes
+};
+__device__ __forceinline__ StageParams run_params(const StageRun &run, uint32_t y) {
+    StageParams p = run.p;
+    p.in = static_cast<const uint8_t *>(p.in) + y * run.in_step;
+    p.out = static_cast<uint8_t *>(p.out) + y * run.out_step;
+    return p;
+}
+
 // ------------------------------------------------------------------ sign-select kernel
 constexpr int kWarpsPerBlock = 8;
 constexpr int kRowsPerWarp = 4;
@@ -1041,16 +1055,29 @@ bitslice_stage(const StageParams &p, uint8_t *table_smem, uint8_t *ring_smem,
 // One stage of the factorized linear.  grid.y is the instance, grid.x the blocks that
 // share its row groups.  smem: [digit table][ring].
 template <bool kRoundBf16, bool kFinal, bool kSmemDigits>
-__global__ void __launch_bounds__(512, 1)
-gemv_bitslice_kernel(const StageParams *__restrict__ many, uint32_t n_rows, uint32_t n_bits,
-                     uint32_t n_groups, uint32_t n_steps, uint32_t groups_per_warp) {
-    qk::pdl_launch();  // (bitslice_stage waits for the kernel before, after its weight prologue)
+__device__ __forceinline__ void streaming_form(const StageParams &p, uint32_t n_rows, uint32_t n_bits, uint32_t n_groups,
+                                               uint32_t n_steps, uint32_t groups_per_warp) {
     extern __shared__ __align__(128) uint8_t smem_dyn[];
-    const StageParams p = many[blockIdx.y];
     uint8_t *ring = smem_dyn + (kSmemDigits ? (size_t)n_steps * 4096 : 0);
     bitslice_stage<kRoundBf16, kFinal, kSmemDigits, false, false>(
         p, smem_dyn, ring, nullptr, nullptr, n_rows, n_bits, n_groups, n_steps, blockIdx.x,
         groups_per_warp, false);
+}
+template <bool kRoundBf16, bool kFinal, bool kSmemDigits>
+__global__ void __launch_bounds__(512, 1)
+gemv_bitslice_kernel(const StageParams *__restrict__ many, uint32_t n_rows, uint32_t n_bits,
+                     uint32_t n_groups, uint32_t n_steps, uint32_t groups_per_warp) {
+    qk::pdl_launch();  // (bitslice_stage waits for the kernel before, after its weight prologue)
+    const StageParams p = many[blockIdx.y];
+    streaming_form<kRoundBf16, kFinal, kSmemDigits>(p, n_rows, n_bits, n_groups, n_steps, groups_per_warp);
+}
+template <bool kRoundBf16, bool kFinal>
+__global__ void __launch_bounds__(512, 1)
+gemv_bitslice_run_kernel(const __grid_constant__ StageRun run, uint32_t n_rows, uint32_t n_bits, uint32_t n_groups,
+                         uint32_t n_steps, uint32_t groups_per_warp) {
+    qk::pdl_launch();
+    const StageParams p = run_params(run, blockIdx.y);
+    streaming_form<kRoundBf16, kFinal, true>(p, n_rows, n_bits, n_groups, n_steps, groups_per_warp);
 }
 
 // Low-latency form for few instances: one block per (row group, instance), the block's
@@ -1063,12 +1090,9 @@ gemv_bitslice_kernel(const StageParams *__restrict__ many, uint32_t n_rows, uint
 //   nothing, needs no shared memory for a table, and starts multiplying as soon as its first
 //   chunks have landed.  A stage-1 instance with a ticket then hands over to stage 2: the last
 //   of its blocks to finish builds the table of t.  smem: [ring][reduction buffer].
-template <bool kRoundBf16, bool kFinal, bool kFed = false>
-__global__ void __launch_bounds__(512)
-gemv_bitslice_splitk_kernel(const StageParams *__restrict__ many) {
-    qk::pdl_launch();  // (bitslice_stage waits for the kernel before, after its weight prologue)
+template <bool kRoundBf16, bool kFinal, bool kFed>
+__device__ __forceinline__ void splitk_form(const StageParams &p) {
     extern __shared__ __align__(128) uint8_t smem_dyn[];
-    const StageParams p = many[blockIdx.y];
     const uint32_t n_rows = p.n_rows, n_bits = p.n_bits;
     const uint32_t n_groups = (n_rows + kGroupRows - 1) / kGroupRows;
     const uint32_t n_steps = (n_bits + kStepBits - 1) / kStepBits;
@@ -1118,6 +1142,21 @@ gemv_bitslice_splitk_kernel(const StageParams *__restrict__ many) {
                               p.next_meta, tail_max, tail_sum, &tail_bad);
         }
     }
+}
+
+template <bool kRoundBf16, bool kFinal, bool kFed = false>
+__global__ void __launch_bounds__(512)
+gemv_bitslice_splitk_kernel(const StageParams *__restrict__ many) {
+    qk::pdl_launch();  // (bitslice_stage waits for the kernel before, after its weight prologue)
+    const StageParams p = many[blockIdx.y];
+    splitk_form<kRoundBf16, kFinal, kFed>(p);
+}
+template <bool kRoundBf16, bool kFinal>
+__global__ void __launch_bounds__(512)
+gemv_bitslice_splitk_run_kernel(const __grid_constant__ StageRun run) {
+    qk::pdl_launch();
+    const StageParams p = run_params(run, blockIdx.y);
+    splitk_form<kRoundBf16, kFinal, false>(p);
 }
 
 // Both stages of one layer instance in one block: t = Vb^T z stays in shared memory as
@@ -1750,9 +1789,16 @@ StagePlan plan_stage(const qk_ctx *c, const StageShape &s, size_t n_inst) {
 bool fed_plan_fits(const qk_ctx *c, const StageShape &s, size_t n_inst, size_t *warps, size_t *smem);
 constexpr size_t kSpreadTableSteps = 16;  // k-steps (of 512 inputs) from which the few-instance form gets its table made once
 
+// Whether a stage can take its records with the launch: every form but those whose table a kernel of its own makes.
+bool run_fits(const qk_ctx *c, const StageShape &s, size_t n_inst) {
+    return plan_stage(c, s, n_inst).smem_digits && s.n_steps < kSpreadTableSteps;
+}
+
+// many: the instances' records on the device; or null, and the instances are the tokens of `run` (run_fits).
 template <bool kFinal>
 qk_status launch_bitslice(qk_ctx *c, const StageParams *many, size_t n_inst, const StageShape &s,
-                          bool bf16, bool need_few = false) {
+                          bool bf16, bool need_few = false, const StageRun &run = StageRun{}) {
+    qk_status st;
     const StagePlan pl = plan_stage(c, s, n_inst);
     // Few instances: the streaming form would leave most SMs idle and make each warp walk
     // its chunks in sequence.  Give every row group a block whose warps split the k-steps.
@@ -1771,7 +1817,7 @@ qk_status launch_bitslice(qk_ctx *c, const StageParams *many, size_t n_inst, con
         if (ts != QK_OK) return ts;
         auto gemv = bf16 ? gemv_bitslice_splitk_kernel<true, kFinal, true>
                          : gemv_bitslice_splitk_kernel<false, kFinal, true>;
-        QK_CUDA(cudaFuncSetAttribute(gemv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
+        if ((st = qk::allow_smem(c, gemv, kSmemBudget)) != QK_OK) return st;
         dim3 grid((unsigned)s.n_groups, (unsigned)n_inst);
         (void)qk::launch_pdl(c->pdl, gemv, grid, dim3((unsigned)fed_warps * 32), fed_smem, c->stream, many);
         QK_CUDA(cudaGetLastError());
@@ -1782,10 +1828,17 @@ qk_status launch_bitslice(qk_ctx *c, const StageParams *many, size_t n_inst, con
         return qk::fail(QK_ERR_VALUE, "a plan that pushes its output into an all-reduce must fit the few-instance form");
     if (few && pl.smem_digits && sk_smem <= kSmemBudget) {
         dim3 grid((unsigned)s.n_groups, (unsigned)n_inst);
+        if (!many) {
+            auto one = bf16 ? gemv_bitslice_splitk_run_kernel<true, kFinal> : gemv_bitslice_splitk_run_kernel<false, kFinal>;
+            if ((st = qk::allow_smem(c, one, kSmemBudget)) != QK_OK) return st;
+            (void)qk::launch_pdl(c->pdl, one, grid, dim3((unsigned)sk_warps * 32), sk_smem, c->stream, run);
+            QK_CUDA(cudaGetLastError());
+            c->launches++;
+            return QK_OK;
+        }
         auto gemv = bf16 ? gemv_bitslice_splitk_kernel<true, kFinal>
                          : gemv_bitslice_splitk_kernel<false, kFinal>;
-        QK_CUDA(cudaFuncSetAttribute(gemv, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                     (int)kSmemBudget));
+        if ((st = qk::allow_smem(c, gemv, kSmemBudget)) != QK_OK) return st;
         (void)qk::launch_pdl(c->pdl, gemv, grid, dim3((unsigned)sk_warps * 32), sk_smem, c->stream, many);
         QK_CUDA(cudaGetLastError());
         c->launches++;
@@ -1797,12 +1850,21 @@ qk_status launch_bitslice(qk_ctx *c, const StageParams *many, size_t n_inst, con
         if (ts != QK_OK) return ts;
     }
     dim3 grid((unsigned)pl.blocks, (unsigned)n_inst);
+    if (!many) {
+        auto one = bf16 ? gemv_bitslice_run_kernel<true, kFinal> : gemv_bitslice_run_kernel<false, kFinal>;
+        if ((st = qk::allow_smem(c, one, kSmemBudget)) != QK_OK) return st;
+        (void)qk::launch_pdl(c->pdl, one, grid, dim3((unsigned)pl.warps_per_block * 32), pl.smem, c->stream, run,
+                             (uint32_t)s.n_rows, (uint32_t)s.n_bits, (uint32_t)s.n_groups, (uint32_t)s.n_steps,
+                             (uint32_t)pl.gpw);
+        QK_CUDA(cudaGetLastError());
+        c->launches++;
+        return QK_OK;
+    }
     auto gemv = pl.smem_digits ? (bf16 ? gemv_bitslice_kernel<true, kFinal, true>
                                        : gemv_bitslice_kernel<false, kFinal, true>)
                                : (bf16 ? gemv_bitslice_kernel<true, kFinal, false>
                                        : gemv_bitslice_kernel<false, kFinal, false>);
-    QK_CUDA(cudaFuncSetAttribute(gemv, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)kSmemBudget));
+    if ((st = qk::allow_smem(c, gemv, kSmemBudget)) != QK_OK) return st;
     (void)qk::launch_pdl(c->pdl, gemv, grid, dim3((unsigned)pl.warps_per_block * 32), pl.smem, c->stream,
                          many, (uint32_t)s.n_rows, (uint32_t)s.n_bits, (uint32_t)s.n_groups,
                          (uint32_t)s.n_steps, (uint32_t)pl.gpw);
@@ -1935,7 +1997,7 @@ qk_status launch_mixed_stage(qk_ctx *c, const StageParams *many, size_t n_inst, 
     if (!mixed_plan_fits(c, s, n_inst, &warps, &smem))
         return qk::fail(QK_ERR_VALUE, "a plan of mixed shapes must fit the few-instance form");
     auto gemv = bf16 ? gemv_bitslice_splitk_kernel<true, kFinal> : gemv_bitslice_splitk_kernel<false, kFinal>;
-    QK_CUDA(cudaFuncSetAttribute(gemv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
+    if (qk_status e = qk::allow_smem(c, gemv, kSmemBudget); e != QK_OK) return e;
     dim3 grid((unsigned)s.n_groups, (unsigned)n_inst);
     (void)qk::launch_pdl(c->pdl, gemv, grid, dim3((unsigned)warps * 32), smem, c->stream, many);
     QK_CUDA(cudaGetLastError());
@@ -1959,7 +2021,7 @@ qk_status launch_fed_stage(qk_ctx *c, const StageParams *many, size_t n_inst, co
         return qk::fail(QK_ERR_VALUE, "a fed plan must fit the few-instance form");
     auto gemv = bf16 ? gemv_bitslice_splitk_kernel<true, kFinal, true>
                      : gemv_bitslice_splitk_kernel<false, kFinal, true>;
-    QK_CUDA(cudaFuncSetAttribute(gemv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
+    if (qk_status e = qk::allow_smem(c, gemv, kSmemBudget); e != QK_OK) return e;
     dim3 grid((unsigned)s.n_groups, (unsigned)n_inst);
     (void)qk::launch_pdl(c->pdl, gemv, grid, dim3((unsigned)warps * 32), smem, c->stream, many);
     QK_CUDA(cudaGetLastError());
@@ -1979,7 +2041,7 @@ qk_status launch_normed_stage1(qk_ctx *c, const StageParams *many, size_t n_inst
     if (!normed_plan_fits(c, s, n_inst, &smem))
         return qk::fail(QK_ERR_VALUE, "a normed plan must fit the few-instance form");
     auto gemv = bf16 ? gemv_bitslice_splitk_kernel<true, false> : gemv_bitslice_splitk_kernel<false, false>;
-    QK_CUDA(cudaFuncSetAttribute(gemv, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmemBudget));
+    if (qk_status e = qk::allow_smem(c, gemv, kSmemBudget); e != QK_OK) return e;
     dim3 grid((unsigned)s.n_groups, (unsigned)n_inst);
     (void)qk::launch_pdl(c->pdl, gemv, grid, dim3(512), smem, c->stream, many);
     QK_CUDA(cudaGetLastError());
@@ -2080,6 +2142,16 @@ qk_status apply_group(qk_ctx *c, const qk_layer *const *layers, size_t n_layers,
         return qk::fail(QK_ERR_VALUE, "%zu layer-token instances exceed one launch (65535)", n_inst);
     const InstanceScratch sc = scratch_of(l0);
     if ((st = c->d_t.reserve(n_inst * sc.total)) != QK_OK) return st;
+    const StageShape s1 = stage1_shape(l0), s2 = stage2_shape(l0);
+    if (n_layers == 1 && c->gemv_kernel == 1 && n_tokens < (size_t)c->sm_count && run_fits(c, s1, n_tokens) &&
+        run_fits(c, s2, n_tokens)) {
+        StageParams h[2];
+        fill_params(h, layers, 1, 1, x_dev, y_dev, (uint8_t *)c->d_t.ptr, 0, 0);
+        const bool bf16 = l0->serving == QK_BF16;
+        const StageRun first{h[0], l0->din * sizeof(float), sc.total}, last{h[1], sc.total, l0->dout * sizeof(float)};
+        if ((st = launch_bitslice<false>(c, nullptr, n_tokens, s1, bf16, false, first)) != QK_OK) return st;
+        return launch_bitslice<true>(c, nullptr, n_tokens, s2, bf16, false, last);
+    }
     if ((st = c->d_ptrs.reserve(2 * n_inst * sizeof(StageParams))) != QK_OK) return st;
     void *hp;
     int slot;

@@ -525,3 +525,28 @@ def test_layer_from_container_streams_equals_layer_from_rows(gpu_ctx, shape, ser
                                    L["s2"], L["bias"], serving=serving)
     a.close()
     b.close()
+
+
+@pytest.mark.parametrize("serving", ["float32", "bfloat16"])
+@pytest.mark.parametrize("shape,n_tokens", [((96, 160, 72), 1), ((130, 1100, 515), 5), ((1024, 1024, 300), 32),
+                                            ((4096, 4096, 1024), 3), ((200, 7680, 65), 2), ((64, 8192, 64), 2)])
+def test_tokens_of_one_layer_match_single_tokens_and_a_group(gpu_ctx, shape, n_tokens, serving):
+    """One layer on several tokens takes its record with the launch (rows of up to 15 k-steps; beyond, and in a
+    group, from an array on the device): the same bits each way, from the few-instance form to the streaming one."""
+    import torch
+    from quantibbler_b200.gpu import LayerGroup
+    dout, din, r = shape
+    L = make_layer(dout, din, r, seed=dout + n_tokens, with_bias=True)
+    layer = PackedLayer(gpu_ctx, L["ub_rows"], L["vb_t_rows"], dout, din, r, L["s1"], L["s2"], L["bias"], serving=serving)
+    gen = torch.Generator(device="cuda").manual_seed(r)
+    x = torch.randn(n_tokens, din, device="cuda", generator=gen)
+    y, single, grouped = (torch.full((n_tokens, dout), float("nan"), device="cuda") for _ in range(3))
+    torch.cuda.synchronize()
+    layer.apply_device(x.data_ptr(), n_tokens, y.data_ptr())
+    for i in range(n_tokens):
+        layer.apply_device(x[i].data_ptr(), 1, single[i].data_ptr())
+    group = LayerGroup(gpu_ctx, [layer] * n_tokens, x.data_ptr(), grouped.data_ptr())
+    group.apply()
+    gpu_ctx.synchronize()
+    assert bool(torch.isfinite(y).all())
+    assert torch.equal(y, single) and torch.equal(y, grouped)
