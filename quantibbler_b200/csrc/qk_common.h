@@ -163,6 +163,11 @@ qk_status allow_smem(qk_ctx *c, Kernel *kernel, size_t bytes) {
     c->smem_allowed.emplace_back((const void *)kernel, (int)bytes);
     return QK_OK;
 }
+// Causal attention of `tokens` bfloat16 query rows at positions p0 .. against the rows 0 .. p0 + tokens - 1 of kv
+// ([key][heads x dim, then heads x vdim]) by the tcgen05 portion kernel of qk_grouped.cu.  dim and vdim: multiples of 16
+// from 64 to 128; all rows 16-byte aligned.
+qk_status causal_portion(qk_ctx *c, const void *q, size_t q_stride, const void *kv, size_t kv_row, size_t p0, size_t tokens,
+                         size_t heads, size_t dim, size_t vdim, float scale, void *out, size_t out_stride);
 // Makes sure the context's error word (an int, bits: 1 a prefill pipeline wait, 2 an all-reduce
 // inbox wait, 4 a token outside the KV cache, 8 a wait of the streaming GEMV, 16 a grid barrier of the
 // whole-step decode kernel) and the prefill's CTA flags after it exist.

@@ -1065,6 +1065,40 @@ qk_status launch_append(qk_ctx *c, const qk_grouped_call *d, const GroupedArgs &
 
 }  // namespace
 
+qk_status qk::causal_portion(qk_ctx *c, const void *q, size_t q_stride, const void *kv, size_t kv_row, size_t p0,
+                             size_t tokens, size_t heads, size_t dim, size_t vdim, float scale, void *out,
+                             size_t out_stride) {
+    qk_status st = qk::error_word(c);
+    if (st != QK_OK) return st;
+    c->err_armed = true;
+    GroupedArgs a{};
+    a.out = out;
+    a.error = (int *)c->d_err.ptr;
+    a.tokens = (uint32_t)tokens;
+    a.heads = a.kv_heads = (uint32_t)heads;
+    a.dim = (uint32_t)dim;
+    a.vdim = (uint32_t)vdim;
+    a.s_max = (uint32_t)(p0 + tokens);
+    a.n_slots = 1;
+    a.proj_stride = (uint32_t)q_stride;
+    a.out_stride = (uint32_t)out_stride;
+    a.bias_len = 1;
+    a.p0 = (uint32_t)p0;
+    a.scale = scale;
+    a.out_bf16 = 1;
+    CUtensorMap qm, km, vm;
+    const cuuint64_t q_dims[2] = {heads * dim, tokens}, q_strides[1] = {q_stride * 2};
+    const cuuint64_t k_dims[3] = {dim, p0 + tokens, heads}, k_strides[2] = {kv_row * 2, dim * 2};
+    const cuuint64_t v_dims[3] = {vdim, p0 + tokens, heads}, v_strides[2] = {kv_row * 2, vdim * 2};
+    const cuuint32_t box[3] = {64, 128, 1};
+    if ((st = encode_bf16_map(q, 2, q_dims, q_strides, box, &qm)) != QK_OK) return st;
+    if ((st = encode_bf16_map(kv, 3, k_dims, k_strides, box, &km)) != QK_OK) return st;
+    if ((st = encode_bf16_map((const uint16_t *)kv + heads * dim, 3, v_dims, v_strides, box, &vm)) != QK_OK) return st;
+    const dim3 grid(a.heads, (unsigned)qk::ceil_div(tokens, 2 * kUmRows)), block(kUmThreads);
+    QK_GROUPED(c, grouped_portion_umma_kernel, grid, block, kUmSmem, qm, km, vm, a, c->wait_limit ? c->wait_limit : kUmWaitDefault);
+    return QK_OK;
+}
+
 extern "C" {
 
 size_t qk_grouped_scratch(size_t tokens, size_t heads, size_t kv_heads, size_t vdim_stride, size_t n_splits) {

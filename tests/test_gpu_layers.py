@@ -255,6 +255,15 @@ def test_window_attention_expanded(dev, dim, vdim, window, p0, tokens):
     assert not out[:, heads * vdim:].any()
 
 
+@pytest.mark.parametrize("dim,vdim,window,p0,tokens", [
+    (64, 64, 1000, 0, 17), (128, 128, 300, 44, 256), (128, 128, 299, 44, 256), (80, 112, 2048, 0, 257),
+    (64, 128, 600, 300, 129), (128, 64, 385, 0, 385)])
+def test_window_that_hides_nothing(dev, dim, vdim, window, p0, tokens):
+    """A window as long as the sequence is causal attention and takes the tcgen05 kernel; one entry shorter it takes the
+    band.  Tiles of 128 rows and 128 keys and one more, head sizes off the 64-channel chunks, the same gate."""
+    test_window_attention_expanded(dev, dim, vdim, window, p0, tokens)
+
+
 def test_late_positions_keep_their_angles(dev):
     """Sinusoidal positions near 10^6: float32 angles would be wrong in the second digit."""
     ctx, torch, L = dev
