@@ -1,15 +1,11 @@
 // Float32 attention on tcgen05: both products on the 16-bit tensor cores, every float32 operand as a
 // sum of 16-bit terms, so that the result is as exact as float32 multiply-adds.
 //
-// Two uses of one kernel (layouts and masks as the kernels it stands beside):
-//   * Exact (the exact attention face, attention_exact_kernel's contract): q, k, v float32.  Each is
-//     two float16 terms, hi + lo, after scaling by a power of two (q per row, k per kv head, v per
-//     channel) that puts the largest magnitude at 2^14..2^15: what the two terms leave out is at most
-//     2^-24 of the value or 2^-40 of the largest one.  x y = lo hi' + hi lo' + hi hi' (lo lo' is below
-//     2^-24).  The terms of k and v are made once per call by two small kernels.
-//   * Cached (prefill attention against a bfloat16 cache, prefill_attention_mma_kernel's contract):
-//     k and v are bfloat16 as they lie in the cache, q and the weights three bfloat16 terms (exact to
-//     2^-25), three products each.
+// The exact attention face (attention_exact_kernel's contract, layouts and masks): q, k, v float32.  Each
+// is two float16 terms, hi + lo, after scaling by a power of two (q per row, k per kv head, v per
+// channel) that puts the largest magnitude at 2^14..2^15: what the two terms leave out is at most
+// 2^-24 of the value or 2^-40 of the largest one.  x y = lo hi' + hi lo' + hi hi' (lo lo' is below
+// 2^-24).  The terms of k and v are made once per call by two small kernels.
 //
 // What bounds it: shared memory (operand reads of the tensor core and the copies' writes, 128 bytes a
 // clock) and the instructions per score.  A CTA owns 128 query rows of one head; two units of four
@@ -23,9 +19,8 @@
 // A row whose result is not finite (infinities or NaN among its operands, an overflow) is computed
 // again by plain float32 arithmetic: the 16-bit terms of such values are not defined.
 //
-// Measured (32 / 8 heads of 128, causal, 2048 tokens): exact face 3014 us on float32 multiply-adds, 167 us here
-// (the six products alone take the tensor core about 46); against the cache 501 us on mma.sync,
-// 155 us here.
+// Measured (32 / 8 heads of 128, causal, 2048 tokens): 3014 us on float32 multiply-adds, 167 us here
+// (the six products alone take the tensor core about 46).
 #include <cuda_fp16.h>
 
 #include <algorithm>
@@ -42,35 +37,29 @@ constexpr uint32_t kChunkBytes = kKeys * 128;            // ... 64 channels of i
 constexpr uint32_t kQChunkBytes = kRows * 128, kQTermBytes = 2 * kQChunkBytes;
 constexpr uint32_t kThreads = 320, kLoadWarp = 8, kMmaWarp = 9;
 constexpr uint32_t kTmemCols = 512, kUnitCols = 256, kOutCol = 128;  // unit: scores and weights, outputs
-// Columns of term n of the weights (32 each).  The third goes over the scores: its columns 8 p .. 8 p + 7
-// are written when scores 0 .. 16 p + 15 have been read.
-__device__ __forceinline__ constexpr uint32_t weight_col(uint32_t n) { return n == 0 ? 64 : n == 1 ? 96 : 0; }
+__device__ __forceinline__ constexpr uint32_t weight_col(uint32_t n) { return 64 + 32 * n; }  // of the weights' term n
 constexpr float kLog2E = 1.4426950408889634f;
-constexpr float kWeightScale = 16384.f;                  // exact: weights are multiplied with v times this
+constexpr float kWeightScale = 16384.f;                  // weights are multiplied with v times this
 constexpr uint32_t kWaitLimit = 1u << 22;
 constexpr uint32_t kMaxPeakChunks = 64;
 
-template <bool kExact>
-struct Shape {
-    static constexpr uint32_t q_terms = kExact ? 2 : 3, kv_terms = kExact ? 2 : 1, p_terms = q_terms;
-    static constexpr uint32_t stages = kExact ? 2 : 4;
-    static constexpr uint32_t stage_bytes = 2 * kv_terms * kTermBytes;
-    static constexpr uint32_t smem = 1024 + q_terms * kQTermBytes + stages * stage_bytes + 1024 + 512;
-};
-static_assert(Shape<true>::smem <= 227 * 1024 && Shape<false>::smem <= 227 * 1024, "shared memory of a CTA");
-static_assert(Shape<true>::stages * Shape<true>::stage_bytes >= 65536 + 1024, "the units' exchange");
-static_assert(Shape<false>::stages * Shape<false>::stage_bytes >= 65536 + 1024, "the units' exchange");
+constexpr uint32_t kTerms = 2;                           // of every operand
+constexpr uint32_t kStages = 2, kStageBytes = 2 * kTerms * kTermBytes;
+constexpr uint32_t kSmem = 1024 + kTerms * kQTermBytes + kStages * kStageBytes + 1024 + 512;
+static_assert(kSmem <= 227 * 1024, "shared memory of a CTA");
+constexpr uint32_t kSwapFloats = 2 * 64 * kRows, kStatFloats = 2 * 2 * kRows;  // the units' exchange: outputs, then m and l
+static_assert(kStages * kStageBytes >= (kSwapFloats + kStatFloats) * 4, "the units' exchange lies in the ring");
 
 struct Args {
     const float *q;
     float *out;
-    const void *k, *v;           // the operands as the caller has them (rows that are computed again)
+    const float *k, *v;          // the operands as the caller has them (rows that are computed again)
     size_t kv_plane;             // values of one kv head's plane of k; rows of it are d long
     size_t v_plane;
-    const float *k_mul;          // exact: per plane, the power of two that k's terms were divided by
-    const float *v_mul;          // exact: per plane and channel, the same of v
+    const float *k_mul;          // per plane, the power of two that k's terms were divided by
+    const float *v_mul;          // per plane and channel, the same of v
     size_t q_batch, q_head, q_row, o_batch, o_head, o_row;  // strides in values
-    uint32_t heads, kv_heads, seq_q, seq_kv, d, dv, dpad, dvpad, first_plane;
+    uint32_t heads, kv_heads, seq_q, seq_kv, d, dv, dpad, dvpad;
     int skew;                    // row i sees keys 0 .. i + skew (causal)
     int causal;
     float scale;                 // 1 / sqrt(d)
@@ -88,11 +77,9 @@ __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t *v) {
                  "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
                  : "memory");
 }
-// M = 128, N = n; float16 or bfloat16 (both operands alike) -> float32; b_mn: B is MN-major
-template <bool kExact>
+// M = 128, N = n; float16 x float16 -> float32; b_mn: B is MN-major
 __device__ __forceinline__ uint32_t instruction(uint32_t n, uint32_t b_mn) {
-    const uint32_t type = kExact ? 0u : (1u << 7) | (1u << 10);
-    return (1u << 4) | type | (b_mn << 16) | ((n >> 3) << 17) | ((kRows >> 4) << 24);
+    return (1u << 4) | (b_mn << 16) | ((n >> 3) << 17) | ((kRows >> 4) << 24);
 }
 // MN-major tile in chunks of 64 channels (rows of 128 bytes, swizzled): chunks kChunkBytes apart
 __device__ __forceinline__ uint64_t desc_mn(uint32_t smem_addr) {
@@ -122,11 +109,6 @@ __device__ __forceinline__ bool vote(bool ok) {
         : "memory");
     return all != 0;
 }
-__device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
-    uint32_t r;
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
-    return r;
-}
 __device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) {
     uint32_t r;
     asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
@@ -134,21 +116,10 @@ __device__ __forceinline__ uint32_t pack_f16x2(float lo, float hi) {
 }
 __device__ __forceinline__ float2 unpack_f16x2(uint32_t u) { return __half22float2(*reinterpret_cast<__half2 *>(&u)); }
 // Two values as their terms: t[0] the leading one.
-template <bool kExact>
 __device__ __forceinline__ void split2(float a, float b, uint32_t *t) {
-    if (kExact) {
-        t[0] = pack_f16x2(a, b);
-        const float2 h = unpack_f16x2(t[0]);
-        t[1] = pack_f16x2(a - h.x, b - h.y);
-    } else {
-        t[0] = pack_bf16x2(a, b);
-        a -= __uint_as_float(t[0] << 16);
-        b -= __uint_as_float(t[0] & 0xffff0000u);
-        t[1] = pack_bf16x2(a, b);
-        a -= __uint_as_float(t[1] << 16);
-        b -= __uint_as_float(t[1] & 0xffff0000u);
-        t[2] = pack_bf16x2(a, b);
-    }
+    t[0] = pack_f16x2(a, b);
+    const float2 h = unpack_f16x2(t[0]);
+    t[1] = pack_f16x2(a - h.x, b - h.y);
 }
 // The power of two that brings a magnitude `peak` to [2^14, 2^15), and the one that undoes it.  Peaks
 // outside 2^-100 .. 2^126 (zero, infinity and NaN among them) take the nearest end of that range.
@@ -164,7 +135,7 @@ __device__ __forceinline__ float undo(uint32_t peak_bits, int e) {
     return peak_bits >= 0x7f800000u ? __int_as_float(0x7fffffff) : pow2(e - 14);
 }
 
-// ------------------------------------------------------------------ terms of k and v (exact)
+// ------------------------------------------------------------------ terms of k and v
 // Largest magnitude (as the bits of a float32) of a chunk of a plane's rows: of the whole chunk for k, per
 // channel for v.  Grid (chunks, planes, k or v); a thread owns a channel, so that rows are read whole.
 __global__ void __launch_bounds__(256)
@@ -230,21 +201,15 @@ kv_terms_kernel(const float *__restrict__ k, const float *__restrict__ v, const 
     for (uint32_t r = blockIdx.x * kKeys + threadIdx.x / pairs; r < row1; r += 256 / pairs) {
         const float a = c < n ? src[(size_t)r * n + c] * m0 : 0.f, b = c + 1 < n ? src[(size_t)r * n + c + 1] * m1 : 0.f;
         uint32_t t[2];
-        split2<true>(a, b, t);
+        split2(a, b, t);
         *reinterpret_cast<uint32_t *>(dst + (size_t)r * pad + c) = t[0];
         *reinterpret_cast<uint32_t *>(dst + ((size_t)seq + r) * pad + c) = t[1];
     }
 }
 
 // ------------------------------------------------------------------ a row by plain arithmetic
-template <bool kExact>
-__device__ __forceinline__ float plain_load(const void *p, size_t i) {
-    return kExact ? static_cast<const float *>(p)[i] : __uint_as_float((uint32_t)static_cast<const uint16_t *>(p)[i] << 16);
-}
 // One query row by one warp: lanes own keys for the scores, channels for the outputs.  32 keys at a time.
-template <bool kExact>
-__device__ __noinline__ void plain_row(const Args &a, const float *q, const void *k, size_t k0, const void *v, size_t v0,
-                                       float *out, int n_keys) {
+__device__ __noinline__ void plain_row(const Args &a, const float *q, const float *k, const float *v, float *out, int n_keys) {
     const uint32_t lane = threadIdx.x % 32;
     float o[4] = {}, m = -INFINITY, l = 0.f;
     for (int j0 = 0; j0 < n_keys; j0 += 32) {
@@ -252,7 +217,7 @@ __device__ __noinline__ void plain_row(const Args &a, const float *q, const void
         float s = -INFINITY;
         if (j < n_keys) {
             float dot = 0.f;
-            for (uint32_t c = 0; c < a.d; ++c) dot = fmaf(q[c], plain_load<kExact>(k, k0 + (size_t)j * a.d + c), dot);
+            for (uint32_t c = 0; c < a.d; ++c) dot = fmaf(q[c], k[(size_t)j * a.d + c], dot);
             s = dot * a.scale;
         }
         float top = s;
@@ -268,7 +233,7 @@ __device__ __noinline__ void plain_row(const Args &a, const float *q, const void
             l += w;
 #pragma unroll
             for (int e = 0; e < 4; ++e)
-                if (lane + 32 * e < a.dv) o[e] = fmaf(w, plain_load<kExact>(v, v0 + (size_t)(j0 + i) * a.dv + lane + 32 * e), o[e]);
+                if (lane + 32 * e < a.dv) o[e] = fmaf(w, v[(size_t)(j0 + i) * a.dv + lane + 32 * e], o[e]);
         }
     }
 #pragma unroll
@@ -277,25 +242,24 @@ __device__ __noinline__ void plain_row(const Args &a, const float *q, const void
 }
 
 // ------------------------------------------------------------------ the kernel
-template <bool kExact, uint32_t kChunks>  // kChunks: head size in chunks of 64 channels (padded)
+template <uint32_t kChunks>  // kChunks: head size in chunks of 64 channels (padded)
 __global__ void __launch_bounds__(kThreads, 1)
 split_attention_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_constant__ CUtensorMap v_map, Args a) {
-    using S = Shape<kExact>;
     qk::pdl_launch();
     extern __shared__ __align__(1024) uint8_t raw_smem[];
     uint8_t *qs = reinterpret_cast<uint8_t *>(((uintptr_t)raw_smem + 1023) & ~(uintptr_t)1023);
-    uint8_t *ring = qs + S::q_terms * kQTermBytes;
-    float *row_peak = reinterpret_cast<float *>(ring + S::stages * S::stage_bytes);  // [2][128]
+    uint8_t *ring = qs + kTerms * kQTermBytes;
+    float *row_peak = reinterpret_cast<float *>(ring + kStages * kStageBytes);  // [2][128]
     uint64_t *q_full = reinterpret_cast<uint64_t *>(row_peak + 256);
-    uint64_t *k_full = q_full + 1, *k_empty = k_full + S::stages, *v_full = k_empty + S::stages, *v_empty = v_full + S::stages;
-    uint64_t *s_full = v_empty + S::stages, *p_full = s_full + 2, *o_full = p_full + 2, *drain = o_full + 2;
+    uint64_t *k_full = q_full + 1, *k_empty = k_full + kStages, *v_full = k_empty + kStages, *v_empty = v_full + kStages;
+    uint64_t *s_full = v_empty + kStages, *p_full = s_full + 2, *o_full = p_full + 2, *drain = o_full + 2;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     volatile int *never = reinterpret_cast<volatile int *>(tmem_slot + 2);
     uint32_t *bad_rows = tmem_slot + 3;  // [4] rows whose result is not finite
     const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const uint32_t head = blockIdx.x % a.heads, batch = blockIdx.x / a.heads, kvh = head / (a.heads / a.kv_heads);
-    const uint32_t plane = a.first_plane + batch * a.kv_heads + kvh;
+    const uint32_t plane = batch * a.kv_heads + kvh;
     const uint32_t row0 = (gridDim.y - 1 - blockIdx.y) * kRows;   // (late rows see most keys: they go first)
     const uint32_t rows = min(kRows, a.seq_q - row0);
     const uint32_t n_keys = a.causal ? min(a.seq_kv, (uint32_t)((int)(row0 + rows) + a.skew)) : a.seq_kv;
@@ -303,7 +267,7 @@ split_attention_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
     const uint32_t d_chunks = kChunks, v_chunks = a.dvpad / 64;
     if (threadIdx.x == 0) {
         mbar_init(q_full, 8);
-        for (uint32_t s = 0; s < S::stages; ++s) {
+        for (uint32_t s = 0; s < kStages; ++s) {
             mbar_init(k_full + s, 1);
             mbar_init(k_empty + s, 1);
             mbar_init(v_full + s, 1);
@@ -337,18 +301,18 @@ split_attention_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
 
     if (warp == kLoadWarp) {
         for (uint32_t g = 0; g < n_blocks; ++g) {
-            const uint32_t s = g % S::stages, parity = ((g / S::stages) & 1) ^ 1;
-            uint8_t *stage = ring + s * S::stage_bytes;
+            const uint32_t s = g % kStages, parity = ((g / kStages) & 1) ^ 1;
+            uint8_t *stage = ring + s * kStageBytes;
             if (!mbar_wait(k_empty + s, parity, abort_flag, a.wait_limit)) {
                 *abort_flag = 1;
                 break;
             }
             if (lane == 0) {
-                mbar_expect(k_full + s, S::kv_terms * d_chunks * kChunkBytes);
-                for (uint32_t t = 0; t < S::kv_terms; ++t)
+                mbar_expect(k_full + s, kTerms * d_chunks * kChunkBytes);
+                for (uint32_t t = 0; t < kTerms; ++t)
                     for (uint32_t c = 0; c < d_chunks; ++c)
                         tma_load_3d(smem_u32(stage + t * kTermBytes + c * kChunkBytes), &k_map, c * 64, g * kKeys,
-                                    plane * S::kv_terms + t, k_full + s);
+                                    plane * kTerms + t, k_full + s);
             }
             fetched_k = g + 1;
             __syncwarp();
@@ -357,69 +321,69 @@ split_attention_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
                 break;
             }
             if (lane == 0) {
-                mbar_expect(v_full + s, S::kv_terms * v_chunks * kChunkBytes);
-                for (uint32_t t = 0; t < S::kv_terms; ++t)
+                mbar_expect(v_full + s, kTerms * v_chunks * kChunkBytes);
+                for (uint32_t t = 0; t < kTerms; ++t)
                     for (uint32_t c = 0; c < v_chunks; ++c)
-                        tma_load_3d(smem_u32(stage + (S::kv_terms + t) * kTermBytes + c * kChunkBytes), &v_map, c * 64,
-                                    g * kKeys, plane * S::kv_terms + t, v_full + s);
+                        tma_load_3d(smem_u32(stage + (kTerms + t) * kTermBytes + c * kChunkBytes), &v_map, c * 64,
+                                    g * kKeys, plane * kTerms + t, v_full + s);
             }
             fetched_v = g + 1;
             __syncwarp();
         }
     } else if (warp == kMmaWarp) {
-        const uint32_t idesc_s = instruction<kExact>(kKeys, 0), idesc_o = instruction<kExact>(a.dvpad, 1);
+        const uint32_t idesc_s = instruction(kKeys, 0), idesc_o = instruction(a.dvpad, 1);
         // (descriptors differ in their address field alone: sixteen bytes a unit)
         const uint64_t q_desc = umma_desc(smem_u32(qs)), k_desc = umma_desc(smem_u32(ring));
-        const uint64_t v_desc = desc_mn(smem_u32(ring) + S::kv_terms * kTermBytes);
+        const uint64_t v_desc = desc_mn(smem_u32(ring) + kTerms * kTermBytes);
         // scores of block g into its unit's columns: small terms first
         auto scores = [&](uint32_t g) {  // (one lane)
-            const uint64_t kd = k_desc + (uint64_t)((g % S::stages) * (S::stage_bytes >> 4));
+            const uint64_t kd = k_desc + (uint64_t)((g % kStages) * (kStageBytes >> 4));
             const uint32_t dst = tmem + kUnitCols * (g & 1);
 #pragma unroll
             for (uint32_t i = 0; i < 3; ++i) {
-                const uint32_t tq = kExact ? (i == 0 ? 1 : 0) : 2 - i, tk = kExact ? (i == 1 ? 1 : 0) : 0;
+                const uint32_t tq = i == 0 ? 1 : 0, tk = i == 1 ? 1 : 0;
 #pragma unroll
                 for (uint32_t k = 0; k < 4 * kChunks; ++k)
                     mma_ss(dst, q_desc + ((tq * kQTermBytes + k / 4 * kQChunkBytes + k % 4 * 32) >> 4),
                            kd + ((tk * kTermBytes + k / 4 * kChunkBytes + k % 4 * 32) >> 4), idesc_s, i + k != 0);
             }
-            umma_commit(k_empty + g % S::stages);
+            umma_commit(k_empty + g % kStages);
             umma_commit(s_full + (g & 1));
         };
         auto values = [&](uint32_t g) {  // (one lane)
-            const uint64_t vd = v_desc + (uint64_t)((g % S::stages) * (S::stage_bytes >> 4));
+            const uint64_t vd = v_desc + (uint64_t)((g % kStages) * (kStageBytes >> 4));
             const uint32_t unit = tmem + kUnitCols * (g & 1);
 #pragma unroll
             for (uint32_t i = 0; i < 3; ++i) {
-                const uint32_t tp = kExact ? (i == 0 ? 1 : 0) : 2 - i, tv = kExact ? (i == 1 ? 1 : 0) : 0;
+                const uint32_t tp = i == 0 ? 1 : 0, tv = i == 1 ? 1 : 0;
 #pragma unroll
                 for (uint32_t k = 0; k < kKeys / 16; ++k)
                     mma_ts(unit + kOutCol, unit + weight_col(tp) + k * 8, vd + ((tv * kTermBytes + k * 2048) >> 4), idesc_o,
                            i + k != 0);
             }
-            umma_commit(v_empty + g % S::stages);
+            umma_commit(v_empty + g % kStages);
             umma_commit(o_full + (g & 1));
         };
         bool ok = mbar_wait(q_full, 0, abort_flag, a.wait_limit);
         for (uint32_t g = 0; g < 2 && g < n_blocks && ok; ++g) {
-            ok = mbar_wait(k_full + g % S::stages, 0, abort_flag, a.wait_limit);
+            ok = mbar_wait(k_full + g % kStages, 0, abort_flag, a.wait_limit);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (elect_one()) scores(g);
             __syncwarp();
         }
         for (uint32_t g = 0; g < n_blocks && ok; ++g) {
-            ok = mbar_wait(v_full + g % S::stages, (g / S::stages) & 1, abort_flag, a.wait_limit);
+            ok = mbar_wait(v_full + g % kStages, (g / kStages) & 1, abort_flag, a.wait_limit);
             if (ok) ok = mbar_wait(p_full + (g & 1), (g >> 1) & 1, abort_flag, a.wait_limit);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
             if (elect_one()) values(g);
             __syncwarp();
             if (g + 2 >= n_blocks) continue;
-            ok = mbar_wait(k_full + (g + 2) % S::stages, ((g + 2) / S::stages) & 1, abort_flag, a.wait_limit);
+            ok = mbar_wait(k_full + (g + 2) % kStages, ((g + 2) / kStages) & 1, abort_flag, a.wait_limit);
             if (!ok) break;
             asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            if (elect_one()) scores(g + 2);   // (over the weights of block g: products run in the order of issue)
+            if (elect_one()) scores(g + 2);   // (over scores that the unit has read: it has handed in their weights)
             __syncwarp();
         }
         if (!ok) {
@@ -449,25 +413,22 @@ split_attention_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
                     for (int e = 0; e < 4; ++e) x[c + e] = live && ch + e < a.d ? q_row[ch + e] : 0.f;
                 }
             }
-            float mul = 1.f;
-            if (kExact) {
-                uint32_t top = 0;
+            uint32_t top = 0;
 #pragma unroll
-                for (int c = 0; c < 64; ++c) top = max(top, __float_as_uint(x[c]) & 0x7fffffffu);
-                row_peak[u * 128 + r] = __uint_as_float(top);
-                asm volatile("bar.sync 3, 256;" ::: "memory");
-                const int e = peak_exponent(max(top, __float_as_uint(row_peak[(u ^ 1) * 128 + r])));
-                mul = pow2(14 - e);
-                f = f * pow2(e - 14) * a.k_mul[plane];
-            }
+            for (int c = 0; c < 64; ++c) top = max(top, __float_as_uint(x[c]) & 0x7fffffffu);
+            row_peak[u * 128 + r] = __uint_as_float(top);
+            asm volatile("bar.sync 3, 256;" ::: "memory");
+            const int e = peak_exponent(max(top, __float_as_uint(row_peak[(u ^ 1) * 128 + r])));
+            const float mul = pow2(14 - e);
+            f = f * pow2(e - 14) * a.k_mul[plane];
             if (u < d_chunks) {
 #pragma unroll
                 for (int c = 0; c < 8; ++c) {
-                    uint32_t t[4][3];
+                    uint32_t t[4][kTerms];
 #pragma unroll
-                    for (int e = 0; e < 4; ++e) split2<kExact>(x[8 * c + 2 * e] * mul, x[8 * c + 2 * e + 1] * mul, t[e]);
+                    for (int e = 0; e < 4; ++e) split2(x[8 * c + 2 * e] * mul, x[8 * c + 2 * e + 1] * mul, t[e]);
 #pragma unroll
-                    for (int n = 0; n < (int)S::q_terms; ++n)
+                    for (int n = 0; n < (int)kTerms; ++n)
                         *reinterpret_cast<uint4 *>(qs + n * kQTermBytes + u * kQChunkBytes + r * 128 + ((c ^ (r & 7)) << 4)) =
                             make_uint4(t[0][n], t[1][n], t[2][n], t[3][n]);
                 }
@@ -518,7 +479,7 @@ split_attention_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
             float2 sum = make_float2(0.f, 0.f);
 #pragma unroll
             for (int part = 0; part < 4; ++part) {
-                uint32_t s[16], t[S::p_terms][8];
+                uint32_t s[16], t[kTerms][8];
                 tmem_ld16(unit + 16 * part, s);
                 tmem_ld_wait();
 #pragma unroll
@@ -531,14 +492,14 @@ split_attention_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
                     x = make_float2(ex2(x.x), ex2(x.y));
                     sum = __fadd2_rn(sum, x);
                     // (times 2^14 afterwards: added to the exponent's argument it would cost four bits of it)
-                    if (kExact) x = __fmul2_rn(x, make_float2(kWeightScale, kWeightScale));
-                    uint32_t w[3];
-                    split2<kExact>(x.x, x.y, w);
+                    x = __fmul2_rn(x, make_float2(kWeightScale, kWeightScale));
+                    uint32_t w[kTerms];
+                    split2(x.x, x.y, w);
 #pragma unroll
-                    for (int n = 0; n < (int)S::p_terms; ++n) t[n][e] = w[n];
+                    for (int n = 0; n < (int)kTerms; ++n) t[n][e] = w[n];
                 }
 #pragma unroll
-                for (int n = 0; n < (int)S::p_terms; ++n) tmem_st8(unit + weight_col(n) + 8 * part, t[n]);
+                for (int n = 0; n < (int)kTerms; ++n) tmem_st8(unit + weight_col(n) + 8 * part, t[n]);
             }
             l = fmaf(l, alpha, sum.x + sum.y);
             asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
@@ -570,7 +531,7 @@ split_attention_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
         // product has been read out, every copy consumed once both units are here).
         ok = vote<3, 256>(ok);
         if (ok) {
-            float *swap = reinterpret_cast<float *>(ring), *stat = swap + 2 * 64 * 128;  // [unit][64][128], [unit][m, l][128]
+            float *swap = reinterpret_cast<float *>(ring), *stat = swap + kSwapFloats;  // [unit][64][128], [unit][m, l][128]
             float *mine = swap + u * 64 * 128;
 #pragma unroll
             for (int c = 0; c < 64; ++c) mine[c * 128 + r] = u ? o[c] : o[64 + c];
@@ -582,7 +543,7 @@ split_attention_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
             const float w1 = ex2(m - base), w2 = ex2(m2 - base);
             const float inv = 1.0f / (l * w1 + l2 * w2), a1 = w1 * inv, a2 = w2 * inv;
             const float *other = swap + (u ^ 1) * 64 * 128;
-            const float *v_mul = kExact ? a.v_mul + (size_t)plane * a.dvpad : nullptr;
+            const float *v_mul = a.v_mul + (size_t)plane * a.dvpad;
             float *dst = a.out + batch * a.o_batch + head * a.o_head + (size_t)min(i, a.seq_q - 1) * a.o_row;
             const bool wide = (a.dv & 3) == 0 && (a.o_row & 3) == 0 && ((uintptr_t)dst & 15) == 0;
             float worst = 0.f;
@@ -595,7 +556,7 @@ split_attention_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
                 for (int e = 0; e < 4; ++e) {
                     const float own = u ? o[64 + c + e] : o[c + e];
                     x[e] = fmaf(own, a1, other[(c + e) * 128 + r] * a2);
-                    if (kExact) x[e] *= v_mul[ch + e] * (1.f / kWeightScale);
+                    x[e] *= v_mul[ch + e] * (1.f / kWeightScale);
                     worst = fmaxf(worst, fabsf(x[e] * 0.f) == 0.f ? 0.f : 1.f);
                 }
                 if (wide) {
@@ -612,9 +573,9 @@ split_attention_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
             for (uint32_t n = warp; n < kRows; n += 8) {
                 if (!(bad_rows[n / 32] >> (n % 32) & 1)) continue;
                 const uint32_t row = row0 + n;
-                plain_row<kExact>(a, a.q + batch * a.q_batch + head * a.q_head + (size_t)row * a.q_row, a.k, plane * a.kv_plane,
-                                  a.v, plane * a.v_plane, a.out + batch * a.o_batch + head * a.o_head + (size_t)row * a.o_row,
-                                  a.causal ? min((int)row + a.skew + 1, (int)a.seq_kv) : (int)a.seq_kv);
+                plain_row(a, a.q + batch * a.q_batch + head * a.q_head + (size_t)row * a.q_row, a.k + plane * a.kv_plane,
+                          a.v + plane * a.v_plane, a.out + batch * a.o_batch + head * a.o_head + (size_t)row * a.o_row,
+                          a.causal ? min((int)row + a.skew + 1, (int)a.seq_kv) : (int)a.seq_kv);
             }
         }
     }
@@ -622,10 +583,10 @@ split_attention_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     if (warp == kLoadWarp && *abort_flag) {  // the copies still in flight
-        for (uint32_t g = fetched_k > S::stages ? fetched_k - S::stages : 0; g < fetched_k; ++g)
-            (void)mbar_wait(k_full + g % S::stages, (g / S::stages) & 1, never, kWaitLimit);
-        for (uint32_t g = fetched_v > S::stages ? fetched_v - S::stages : 0; g < fetched_v; ++g)
-            (void)mbar_wait(v_full + g % S::stages, (g / S::stages) & 1, never, kWaitLimit);
+        for (uint32_t g = fetched_k > kStages ? fetched_k - kStages : 0; g < fetched_k; ++g)
+            (void)mbar_wait(k_full + g % kStages, (g / kStages) & 1, never, kWaitLimit);
+        for (uint32_t g = fetched_v > kStages ? fetched_v - kStages : 0; g < fetched_v; ++g)
+            (void)mbar_wait(v_full + g % kStages, (g / kStages) & 1, never, kWaitLimit);
     }
     if (warp == kMmaWarp)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");
@@ -640,16 +601,15 @@ qk_status plane_map(const void *base, size_t pad, size_t seq, size_t planes, siz
     return encode_bf16_map(base, 3, dims, strides, box, out);
 }
 
-template <bool kExact>
 qk_status launch_split(qk_ctx *c, const CUtensorMap &km, const CUtensorMap &vm, Args &a, size_t batch) {
     qk_status st = qk::error_word(c);
     if (st != QK_OK) return st;
     a.error = (int *)c->d_err.ptr;
     a.wait_limit = c->wait_limit ? c->wait_limit : kWaitLimit;
-    auto kernel = a.dpad == 64 ? split_attention_kernel<kExact, 1> : split_attention_kernel<kExact, 2>;
-    QK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Shape<kExact>::smem));
+    auto kernel = a.dpad == 64 ? split_attention_kernel<1> : split_attention_kernel<2>;
+    QK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kSmem));
     const dim3 grid((unsigned)(batch * a.heads), (unsigned)qk::ceil_div(a.seq_q, kRows));
-    (void)qk::launch_pdl(c->pdl, kernel, grid, dim3(kThreads), (size_t)Shape<kExact>::smem, c->stream, km, vm, a);
+    (void)qk::launch_pdl(c->pdl, kernel, grid, dim3(kThreads), (size_t)kSmem, c->stream, km, vm, a);
     QK_CUDA(cudaGetLastError());
     c->launches++;
     c->err_armed = true;
@@ -711,28 +671,7 @@ qk_status attention_split_exact(qk_ctx *c, const float *q, const float *k, const
     a.d = (uint32_t)s->head_dim, a.dv = (uint32_t)s->val_dim, a.dpad = (uint32_t)dpad, a.dvpad = (uint32_t)dvpad;
     a.skew = (int)seq - (int)s->seq_q, a.causal = causal != 0;
     a.scale = 1.0f / sqrtf((float)s->head_dim);
-    return launch_split<true>(c, km, vm, a, s->batch);
-}
-
-qk_status attention_split_cached(qk_ctx *c, const float *q, const void *cache_k, const void *cache_v, size_t seq,
-                                 size_t first_position, size_t n_tokens, size_t n_heads, size_t n_kv_heads, size_t s_max,
-                                 float *out) {
-    CUtensorMap km, vm;
-    qk_status st;
-    // (rows past the portion's last position read as zeros)
-    const size_t live = first_position + n_tokens, planes = (seq + 1) * n_kv_heads, d = 128;
-    if ((st = plane_map(cache_k, d, live, planes, s_max * d * 2, &km)) != QK_OK) return st;
-    if ((st = plane_map(cache_v, d, live, planes, s_max * d * 2, &vm)) != QK_OK) return st;
-    Args a{};
-    a.q = q, a.out = out, a.k = cache_k, a.v = cache_v;
-    a.kv_plane = a.v_plane = s_max * d;
-    a.q_row = a.o_row = n_heads * d, a.q_head = a.o_head = d;
-    a.heads = (uint32_t)n_heads, a.kv_heads = (uint32_t)n_kv_heads;
-    a.seq_q = (uint32_t)n_tokens, a.seq_kv = (uint32_t)live;
-    a.d = a.dv = a.dpad = a.dvpad = (uint32_t)d, a.first_plane = (uint32_t)(seq * n_kv_heads);
-    a.skew = (int)first_position, a.causal = 1;
-    a.scale = 1.0f / sqrtf((float)d);
-    return launch_split<false>(c, km, vm, a, 1);
+    return launch_split(c, km, vm, a, s->batch);
 }
 
 }  // namespace qk

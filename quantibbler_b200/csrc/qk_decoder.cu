@@ -18,7 +18,6 @@
 
 #include <cmath>
 
-#include "qk_attention_split.h"
 #include "qk_common.h"
 #include "qk_digits.cuh"
 #include "qk_decoder_dev.cuh"
@@ -1511,12 +1510,6 @@ qk_status qk_prefill_attention(qk_ctx *ctx, const float *q, const void *cache_k,
     if (first_position + n_tokens > s_max)
         return qk::fail(QK_ERR_VALUE, "positions %zu..%zu do not fit the KV cache of %zu positions",
                         first_position, first_position + n_tokens - 1, s_max);
-    // (64 positions are one key block; below that the mma.sync kernel's short tiles win: 16 tokens of 32
-    // heads at position 0 9.8 against 11.1 us, 64 tokens 12.9 against 11.9, 16 tokens at 2000 168 against 59)
-    const bool mma_sync = kv_dtype == QK_BF16 && head_dim == 128 && c->decode_attention_kernel != 0;
-    if (mma_sync && first_position + n_tokens >= 64)
-        return qk::attention_split_cached(c, q, cache_k, cache_v, seq, first_position, n_tokens, n_heads, n_kv_heads, s_max,
-                                          out);
     if (kv_dtype != QK_BF16 || head_dim != 128 || (group != 1 && group != 2 && group % 4 != 0) ||
         c->decode_attention_kernel == 0) {
         // any other shape: the plain kernel

@@ -1,8 +1,10 @@
-"""Float32 attention as sums of 16-bit products (qk_attention_split.cu): the exact face from 192 keys on and the
-prefill attention of a bfloat16 cache, against 64-bit attention over the visible keys.
+"""Float32 attention as sums of 16-bit products: the exact face from 192 keys on (qk_attention_split.cu) and the
+prefill attention of a bfloat16 cache (qk_decoder.cu), against 64-bit attention over the visible keys.
 
 Tolerance: float32 scores of magnitude s carry an error of about s 2^-23 into the weights, so 2e-6 of the
-largest output (scores here stay below 16); the plain float32 kernel is held to the reference's 1e-5."""
+largest output (scores here stay below 16); the plain float32 kernel is held to the reference's 1e-5.  The
+prefill kernel adds to a row's output on the tensor core, which truncates: six products per 32 keys, each off by up
+to 2^-23 of what is there."""
 
 import ctypes
 import math
@@ -98,4 +100,4 @@ def test_prefill_attention_at_the_edges_of_tiles(ctx, H, KV, T, p0):
     ctx.synchronize()
     host = lambda t: t.float().cpu().numpy()  # noqa: E731
     want = visible_attention(host(q.reshape(T, H, 128).transpose(0, 1)), host(ck[1, :, :p0 + T]), host(cv[1, :, :p0 + T]), True, p0)
-    assert worst(host(out.reshape(T, H, 128).transpose(0, 1)), want) < 2e-6
+    assert worst(host(out.reshape(T, H, 128).transpose(0, 1)), want) < 2e-6 + 6 * math.ceil((p0 + T) / 32) * 2.0 ** -23

@@ -296,6 +296,65 @@ def test_prefill_attention_against_exact_oracle(gpu_ctx, case):
     assert np.abs(got - want).max() <= 1e-5 * max(1.0, np.abs(want).max())
 
 
+def _prefill_attention(ctx, q, ck, cv, p0, s_max):
+    """q [T, heads, 128] at positions p0 .. of sequence 0 of a bfloat16 cache [1, kv heads, s_max, 128]."""
+    import ctypes
+    import torch
+    from quantibbler_b200 import _lib
+    out = torch.full_like(q, float("nan"))
+    torch.cuda.synchronize()
+    p = lambda t: ctypes.c_void_p(t.data_ptr())
+    _lib.check(_lib.lib().qk_prefill_attention(ctx.handle, p(q), p(ck), p(cv), _lib.QK_BF16, 0, p0, q.shape[0], q.shape[1],
+                                               ck.shape[1], 128, s_max, p(out)))
+    ctx.synchronize()
+    return out
+
+
+@pytest.mark.parametrize("heads,kv_heads", [(4, 1), (2, 2), (4, 2), (6, 2), (16, 2)])
+def test_prefill_attention_does_not_depend_on_the_portion(gpu_ctx, heads, kv_heads):
+    """A position's output has the same bits whether its prompt comes in one portion or in several, and
+    whatever follows it: every portion takes the same kernel."""
+    import torch
+    gen = torch.Generator("cuda").manual_seed(heads)
+    T = 333
+    q = torch.randn(T, heads, 128, device="cuda", generator=gen)
+    ck, cv = (torch.randn(1, kv_heads, T + 3, 128, device="cuda", generator=gen).bfloat16() for _ in range(2))
+    whole = _prefill_attention(gpu_ctx, q, ck, cv, 0, T + 3)
+    edges = [0, 1, 17, 63, 64, 129, 200, T]
+    parts = [_prefill_attention(gpu_ctx, q[a:b].contiguous(), ck, cv, a, T + 3) for a, b in zip(edges, edges[1:])]
+    assert torch.equal(whole, torch.cat(parts))
+
+
+def test_prefill_attention_of_a_cache_on_no_16_byte_boundary(gpu_ctx):
+    """A group of three query heads takes the plain kernel, which reads a bfloat16 cache from any address."""
+    import torch
+    gen = torch.Generator("cuda").manual_seed(3)
+    T, s_max = 70, 75
+    q = torch.randn(T, 6, 128, device="cuda", generator=gen)
+    store = torch.randn(2, 1 + 2 * s_max * 128, device="cuda", generator=gen).bfloat16()
+    ck, cv = (row[1:].view(1, 2, s_max, 128) for row in store)
+    assert ck.data_ptr() % 16
+    got = _prefill_attention(gpu_ctx, q, ck, cv, 0, s_max)
+    assert torch.equal(got, _prefill_attention(gpu_ctx, q, ck.clone(), cv.clone(), 0, s_max))
+
+
+def test_prefill_attention_of_a_long_prompt_against_64_bits(gpu_ctx):
+    """2048 positions, the last portion of them.  The tensor core truncates when it adds: a row's output takes up
+    six products per 32 keys, 384 in all, each off by up to 2^-23 of what is there, hence 384 x 2^-23 of the
+    largest output (the scores' own error, s 2^-23 with s below 16, is small beside it)."""
+    import torch
+    gen = torch.Generator("cuda").manual_seed(8)
+    heads, kv_heads, n, p0 = 8, 2, 2048, 1500
+    q = torch.randn(n - p0, heads, 128, device="cuda", generator=gen)
+    ck, cv = (torch.randn(1, kv_heads, n, 128, device="cuda", generator=gen).bfloat16() for _ in range(2))
+    got = _prefill_attention(gpu_ctx, q, ck, cv, p0, n).double()
+    seen = torch.arange(p0, n, device="cuda")[:, None] >= torch.arange(n, device="cuda")
+    for h in range(heads):
+        s = (q[:, h].double() @ ck[0, h // 4].double().T) * 128 ** -0.5
+        want = torch.softmax(s.masked_fill(~seen, -float("inf")), -1) @ cv[0, h // 4].double()
+        assert float((got[:, h] - want).abs().max()) < 384 * 2.0 ** -23 * float(want.abs().max())
+
+
 @pytest.mark.parametrize("cfg_kw,tol", [
     (dict(), 2e-4),                                                      # small heads, float32 everywhere
     (dict(n_heads=8, n_kv_heads=2, head_dim=128, d_model=256, kv_dtype="bfloat16"), 2e-4),
