@@ -41,17 +41,18 @@ constexpr int kQT = 64;  // queries per block (4 lanes each)
 constexpr int kTK = 32;  // keys per shared-memory tile
 
 // ------------------------------------------------------------------ exact attention
-template <int DPL>
-__global__ void __launch_bounds__(256)
-attention_exact_kernel(const float *__restrict__ q, const float *__restrict__ k,
-                       const float *__restrict__ v, float *__restrict__ out, AttnDims dm,
-                       int causal) {
+// The rows of one block; kMarked: only those whose bit of `rows` is set, and a value that a row does not see is not
+// multiplied with its weight of zero either (it may be an infinity or NaN).
+template <int DPL, bool kMarked>
+__device__ __forceinline__ void exact_rows(const float *__restrict__ q, const float *__restrict__ k,
+                                           const float *__restrict__ v, float *__restrict__ out, const AttnDims &dm,
+                                           int causal, uint64_t rows) {
     constexpr int PITCH = DPL + 4;  // +4 floats: the four parts of a key land in distinct banks
     extern __shared__ float sm[];
     float *Ks = sm, *Vs = sm + kTK * 4 * PITCH;
     const int qi = threadIdx.x >> 2, part = threadIdx.x & 3;
     const int i = blockIdx.x * kQT + qi;
-    const bool valid = i < (int)dm.Sq;
+    const bool valid = i < (int)dm.Sq && (!kMarked || (rows >> qi & 1));
     const int h = blockIdx.y, b = blockIdx.z, kvh = h / dm.group;
     const float scale = 1.0f / sqrtf((float)dm.d);
 
@@ -106,6 +107,7 @@ attention_exact_kernel(const float *__restrict__ q, const float *__restrict__ k,
         for (int e = 0; e < DPL; ++e) o[e] *= alpha;
 #pragma unroll
         for (int kk = 0; kk < kTK; ++kk) {
+            if (kMarked && j0 + kk > last_key) break;
             const float p = expf(s[kk] - m_new);
             l += p;
             const float *vr = Vs + (kk * 4 + part) * PITCH;
@@ -122,6 +124,28 @@ attention_exact_kernel(const float *__restrict__ q, const float *__restrict__ k,
             if (c < (int)dm.dv) orow[c] = o[e] / l;  // a row with no admissible key is 0/0 = NaN
         }
     }
+}
+
+template <int DPL>
+__global__ void __launch_bounds__(256)
+attention_exact_kernel(const float *__restrict__ q, const float *__restrict__ k,
+                       const float *__restrict__ v, float *__restrict__ out, AttnDims dm,
+                       int causal) {
+    exact_rows<DPL, false>(q, k, v, out, dm, causal, 0);
+}
+
+// The rows that attention_split_exact has marked, after it on the stream.  Nearly always there are none: a block
+// reads two words and leaves: 32 heads of 128 on 2048 tokens, causal, 166 us with this launch, 168 when the rows
+// were recomputed by the warps that found them.  With every row marked 3080 us, 2958 by attention_exact_kernel alone.
+template <int DPL>
+__global__ void __launch_bounds__(256)
+attention_marked_kernel(const float *__restrict__ q, const float *__restrict__ k, const float *__restrict__ v,
+                        float *__restrict__ out, AttnDims dm, int causal, const uint32_t *marked) {
+    qk::pdl_wait();
+    const uint32_t tiles = (dm.Sq + 127) / 128;
+    const uint2 bits = *reinterpret_cast<const uint2 *>(
+        marked + (((size_t)blockIdx.z * dm.H + blockIdx.y) * tiles + blockIdx.x / 2) * 4 + (blockIdx.x & 1) * 2);
+    if (bits.x | bits.y) exact_rows<DPL, true>(q, k, v, out, dm, causal, (uint64_t)bits.y << 32 | bits.x);
 }
 
 // ------------------------------------------------------------------ Sage quantisers
@@ -1678,14 +1702,24 @@ AttnDims dims_of(const qk_attention_shape *s) {
             (uint32_t)s->val_dim, (uint32_t)(s->n_heads / s->n_kv_heads)};
 }
 
+// marked: only these rows (attention_split_exact's marks); null: all.
 template <int DPL>
 qk_status launch_exact(qk_ctx *c, const float *q, const float *k, const float *v, float *out,
-                       const AttnDims &dm, int causal) {
+                       const AttnDims &dm, int causal, const uint32_t *marked) {
     size_t smem = 2 * kTK * 4 * (DPL + 4) * sizeof(float);
     if (smem > 48 * 1024)
         QK_CUDA(cudaFuncSetAttribute(attention_exact_kernel<DPL>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     dim3 grid((unsigned)qk::ceil_div(dm.Sq, kQT), dm.H, dm.B);
+    if constexpr (DPL <= 32) {  // (head sizes that attention_split_exact takes)
+        if (marked) {
+            (void)qk::launch_pdl(c->pdl, attention_marked_kernel<DPL>, grid, dim3(256), smem, c->stream, q, k, v, out, dm,
+                                 causal, marked);
+            QK_CUDA(cudaGetLastError());
+            c->launches++;
+            return QK_OK;
+        }
+    }
     attention_exact_kernel<DPL><<<grid, 256, smem, c->stream>>>(q, k, v, out, dm, causal);
     QK_CUDA(cudaGetLastError());
     c->launches++;
@@ -1907,13 +1941,15 @@ qk_status attention_sage_block_dev(qk_ctx *c, const float *dq, const float *dk, 
 // Device-buffer form of the exact face (also used by the decoder path).
 qk_status attention_exact_dev(qk_ctx *c, const float *q, const float *k, const float *v,
                               float *out, const qk_attention_shape *s, int causal) {
-    if (attention_split_takes(c, s, causal)) return attention_split_exact(c, q, k, v, out, s, causal);
+    const uint32_t *marked = nullptr;
+    if (attention_split_takes(c, s, causal))
+        if (qk_status st = attention_split_exact(c, q, k, v, out, s, causal, &marked); st != QK_OK) return st;
     AttnDims dm = dims_of(s);
     size_t widest = s->head_dim > s->val_dim ? s->head_dim : s->val_dim;
-    if (widest <= 16) return launch_exact<4>(c, q, k, v, out, dm, causal);
-    if (widest <= 64) return launch_exact<16>(c, q, k, v, out, dm, causal);
-    if (widest <= 128) return launch_exact<32>(c, q, k, v, out, dm, causal);
-    return launch_exact<64>(c, q, k, v, out, dm, causal);
+    if (widest <= 16) return launch_exact<4>(c, q, k, v, out, dm, causal, marked);
+    if (widest <= 64) return launch_exact<16>(c, q, k, v, out, dm, causal, marked);
+    if (widest <= 128) return launch_exact<32>(c, q, k, v, out, dm, causal, marked);
+    return launch_exact<64>(c, q, k, v, out, dm, causal, marked);
 }
 
 }  // namespace qk

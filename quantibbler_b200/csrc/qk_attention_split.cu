@@ -3,9 +3,22 @@
 //
 // The exact attention face (attention_exact_kernel's contract, layouts and masks): q, k, v float32.  Each
 // is two float16 terms, hi + lo, after scaling by a power of two (q per row, k per kv head, v per
-// channel) that puts the largest magnitude at 2^14..2^15: what the two terms leave out is at most
-// 2^-24 of the value or 2^-40 of the largest one.  x y = lo hi' + hi lo' + hi hi' (lo lo' is below
-// 2^-24).  The terms of k and v are made once per call by two small kernels.
+// channel) that puts the largest magnitude at 2^14..2^15.  What the two terms leave out is at most 2^-23
+// of the value, or 2^-39 of the largest one where that is more; of a product lo hi' + hi lo' + hi hi' are
+// formed, the missing lo lo' is at most 2^-22 of it.  (Measured over random operands the result is nearer
+// to 64 bits than float32 multiply-adds: 3.1e-7 against 4.8e-7 at 2048 keys.)  The terms of k and v are
+// made once per call by two small kernels.
+//
+// The 2^-39 of the largest value is the one error that float32 arithmetic does not have: a large key or
+// value somewhere in the sequence, seen by a row or not, costs the others bits.  So every row checks at its
+// end what that can have cost it: each score at most f d 2^-9 (f: the factor from scaled scores to log2
+// units; d channels of two operands of at most 2^15, off by 2^-25), each output channel at most
+// (1 + 2 n / l) 2^-25 of its multiplier (v off by 2^-25; n weights of at most 2^14, off by 2^-25, on values of
+// at most 2^15).  Where the first exceeds 2^-21 and 2^-21 of the row's largest score, or the second 2^-21 of the
+// row's largest output, the row is marked, and attention_marked_kernel (qk_attention.cu) computes it again
+// by float32 multiply-adds, as it does rows that are not finite (infinities or NaN among their operands, an
+// overflow).  For normal operands both stay below that by a factor of a hundred; one entry of 10^4 among
+// values of 1 is where marks begin.
 //
 // What bounds it: shared memory (operand reads of the tensor core and the copies' writes, 128 bytes a
 // clock) and the instructions per score.  A CTA owns 128 query rows of one head; two units of four
@@ -15,9 +28,6 @@
 // tensor memory as the A operand; v is read as it lies (MN-major B).
 // The tensor core truncates when it adds, so sums must stay short: a block's product with v starts
 // from zero, small terms first, and is added to the row's output in registers, in float32, rounded.
-//
-// A row whose result is not finite (infinities or NaN among its operands, an overflow) is computed
-// again by plain float32 arithmetic: the 16-bit terms of such values are not defined.
 //
 // Measured (32 / 8 heads of 128, causal, 2048 tokens): 3014 us on float32 multiply-adds, 167 us here
 // (the six products alone take the tensor core about 46).
@@ -40,6 +50,7 @@ constexpr uint32_t kTmemCols = 512, kUnitCols = 256, kOutCol = 128;  // unit: sc
 __device__ __forceinline__ constexpr uint32_t weight_col(uint32_t n) { return 64 + 32 * n; }  // of the weights' term n
 constexpr float kLog2E = 1.4426950408889634f;
 constexpr float kWeightScale = 16384.f;                  // weights are multiplied with v times this
+constexpr float kScoreRoom = 0x1p-12f, kValueRoom = 16.f;  // 2^-21 over the 2^-9 and the 2^-25 of the bounds above
 constexpr uint32_t kWaitLimit = 1u << 22;
 constexpr uint32_t kMaxPeakChunks = 64;
 
@@ -53,9 +64,7 @@ static_assert(kStages * kStageBytes >= (kSwapFloats + kStatFloats) * 4, "the uni
 struct Args {
     const float *q;
     float *out;
-    const float *k, *v;          // the operands as the caller has them (rows that are computed again)
-    size_t kv_plane;             // values of one kv head's plane of k; rows of it are d long
-    size_t v_plane;
+    uint32_t *marked;            // [batch x heads][tiles of 128 rows][4]: bits of the rows to be computed again
     const float *k_mul;          // per plane, the power of two that k's terms were divided by
     const float *v_mul;          // per plane and channel, the same of v
     size_t q_batch, q_head, q_row, o_batch, o_head, o_row;  // strides in values
@@ -130,9 +139,10 @@ __host__ __device__ __forceinline__ int peak_exponent(uint32_t peak_bits) {
 __device__ __forceinline__ float pow2(int e) { return __int_as_float((e + 127) << 23); }  // -126 <= e <= 127
 
 // The multiplier that undoes the scaling; NaN for a plane or channel that holds an infinity or NaN (its other
-// values have been scaled away), so that the rows that use it are computed by plain arithmetic.
+// values have been scaled away), so that the rows that use it are computed by plain arithmetic; zero for zeros,
+// which are exact.
 __device__ __forceinline__ float undo(uint32_t peak_bits, int e) {
-    return peak_bits >= 0x7f800000u ? __int_as_float(0x7fffffff) : pow2(e - 14);
+    return peak_bits >= 0x7f800000u ? __int_as_float(0x7fffffff) : peak_bits == 0 ? 0.f : pow2(e - 14);
 }
 
 // ------------------------------------------------------------------ terms of k and v
@@ -207,40 +217,6 @@ kv_terms_kernel(const float *__restrict__ k, const float *__restrict__ v, const 
     }
 }
 
-// ------------------------------------------------------------------ a row by plain arithmetic
-// One query row by one warp: lanes own keys for the scores, channels for the outputs.  32 keys at a time.
-__device__ __noinline__ void plain_row(const Args &a, const float *q, const float *k, const float *v, float *out, int n_keys) {
-    const uint32_t lane = threadIdx.x % 32;
-    float o[4] = {}, m = -INFINITY, l = 0.f;
-    for (int j0 = 0; j0 < n_keys; j0 += 32) {
-        const int j = j0 + (int)lane;
-        float s = -INFINITY;
-        if (j < n_keys) {
-            float dot = 0.f;
-            for (uint32_t c = 0; c < a.d; ++c) dot = fmaf(q[c], k[(size_t)j * a.d + c], dot);
-            s = dot * a.scale;
-        }
-        float top = s;
-        for (int off = 16; off > 0; off >>= 1) top = fmaxf(top, __shfl_xor_sync(0xffffffffu, top, off));
-        const float m_new = fmaxf(m, top);
-        if (m_new == -INFINITY) continue;   // (the same in every lane)
-        const float alpha = expf(m - m_new), p = expf(s - m_new);
-        m = m_new;
-        l *= alpha;
-        for (int e = 0; e < 4; ++e) o[e] *= alpha;
-        for (int i = 0; i < min(32, n_keys - j0); ++i) {
-            const float w = __shfl_sync(0xffffffffu, p, i);
-            l += w;
-#pragma unroll
-            for (int e = 0; e < 4; ++e)
-                if (lane + 32 * e < a.dv) o[e] = fmaf(w, v[(size_t)(j0 + i) * a.dv + lane + 32 * e], o[e]);
-        }
-    }
-#pragma unroll
-    for (int e = 0; e < 4; ++e)
-        if (lane + 32 * e < a.dv) out[lane + 32 * e] = o[e] / l;
-}
-
 // ------------------------------------------------------------------ the kernel
 template <uint32_t kChunks>  // kChunks: head size in chunks of 64 channels (padded)
 __global__ void __launch_bounds__(kThreads, 1)
@@ -256,7 +232,7 @@ split_attention_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
     volatile int *never = reinterpret_cast<volatile int *>(tmem_slot + 2);
-    uint32_t *bad_rows = tmem_slot + 3;  // [4] rows whose result is not finite
+    uint32_t *marks = tmem_slot + 3;  // [4] rows to be computed again
     const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const uint32_t head = blockIdx.x % a.heads, batch = blockIdx.x / a.heads, kvh = head / (a.heads / a.kv_heads);
     const uint32_t plane = batch * a.kv_heads + kvh;
@@ -281,7 +257,7 @@ split_attention_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
         mbar_init(drain, 1);
         *abort_flag = 0;
         *never = 0;
-        for (int i = 0; i < 4; ++i) bad_rows[i] = 0;
+        for (int i = 0; i < 4; ++i) marks[i] = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&k_map) : "memory");
         asm volatile("prefetch.tensormap [%0];" ::"l"(&v_map) : "memory");
@@ -541,12 +517,13 @@ split_attention_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
             const float m2 = stat[(u ^ 1) * 256 + r], l2 = stat[(u ^ 1) * 256 + 128 + r];
             const float top = fmaxf(m, m2), base = top == -INFINITY ? 0.f : top;
             const float w1 = ex2(m - base), w2 = ex2(m2 - base);
-            const float inv = 1.0f / (l * w1 + l2 * w2), a1 = w1 * inv, a2 = w2 * inv;
+            const float sum = l * w1 + l2 * w2, inv = 1.0f / sum, a1 = w1 * inv, a2 = w2 * inv;
             const float *other = swap + (u ^ 1) * 64 * 128;
             const float *v_mul = a.v_mul + (size_t)plane * a.dvpad;
             float *dst = a.out + batch * a.o_batch + head * a.o_head + (size_t)min(i, a.seq_q - 1) * a.o_row;
             const bool wide = (a.dv & 3) == 0 && (a.o_row & 3) == 0 && ((uintptr_t)dst & 15) == 0;
-            float worst = 0.f;
+            float largest = 0.f, v_unit = 0.f;   // this unit's largest output and multiplier
+            bool mark = !(f * (float)a.d <= kScoreRoom * fmaxf(1.f, fabsf(top)));
 #pragma unroll
             for (int c = 0; c < 64; c += 4) {
                 const uint32_t ch = u * 64 + c;
@@ -557,7 +534,9 @@ split_attention_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
                     const float own = u ? o[64 + c + e] : o[c + e];
                     x[e] = fmaf(own, a1, other[(c + e) * 128 + r] * a2);
                     x[e] *= v_mul[ch + e] * (1.f / kWeightScale);
-                    worst = fmaxf(worst, fabsf(x[e] * 0.f) == 0.f ? 0.f : 1.f);
+                    mark = mark || !(fabsf(x[e]) < INFINITY);
+                    largest = fmaxf(largest, fabsf(x[e]));
+                    v_unit = fmaxf(v_unit, v_mul[ch + e]);
                 }
                 if (wide) {
                     *reinterpret_cast<float4 *>(dst + ch) = make_float4(x[0], x[1], x[2], x[3]);
@@ -567,16 +546,14 @@ split_attention_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
                         if (ch + e < a.dv) dst[ch + e] = x[e];
                 }
             }
-            const uint32_t bad = __ballot_sync(0xffffffffu, worst != 0.f);
-            if (lane == 0 && bad) atomicOr(bad_rows + warp % 4, bad);
+            row_peak[u * 128 + r] = largest;
             asm volatile("bar.sync 3, 256;" ::: "memory");
-            for (uint32_t n = warp; n < kRows; n += 8) {
-                if (!(bad_rows[n / 32] >> (n % 32) & 1)) continue;
-                const uint32_t row = row0 + n;
-                plain_row(a, a.q + batch * a.q_batch + head * a.q_head + (size_t)row * a.q_row, a.k + plane * a.kv_plane,
-                          a.v + plane * a.v_plane, a.out + batch * a.o_batch + head * a.o_head + (size_t)row * a.o_row,
-                          a.causal ? min((int)row + a.skew + 1, (int)a.seq_kv) : (int)a.seq_kv);
-            }
+            largest = fmaxf(largest, row_peak[(u ^ 1) * 128 + r]);
+            mark = mark || !((1.f + 2.f * (float)seen / sum) * v_unit <= kValueRoom * largest);
+            const uint32_t bits = __ballot_sync(0xffffffffu, mark && r < rows);
+            if (lane == 0 && bits) atomicOr(marks + warp % 4, bits);
+            asm volatile("bar.sync 3, 256;" ::: "memory");
+            if (threadIdx.x < 4) a.marked[((size_t)blockIdx.x * gridDim.y + row0 / kRows) * 4 + threadIdx.x] = marks[threadIdx.x];
         }
     }
     __syncwarp();
@@ -636,14 +613,15 @@ bool attention_split_takes(qk_ctx *c, const qk_attention_shape *s, int causal) {
 }
 
 qk_status attention_split_exact(qk_ctx *c, const float *q, const float *k, const float *v, float *out,
-                                const qk_attention_shape *s, int causal) {
+                                const qk_attention_shape *s, int causal, const uint32_t **marked) {
     const size_t planes = s->batch * s->n_kv_heads, seq = s->seq_kv;
     const size_t dpad = s->head_dim <= 64 ? 64 : 128, dvpad = s->val_dim <= 64 ? 64 : 128;
     const size_t chunk_rows = std::max<size_t>(kKeys, ceil_div(seq, kMaxPeakChunks)), chunks = ceil_div(seq, chunk_rows);
     auto up = [](size_t n) { return (n + 255) / 256 * 256; };
     const size_t k_bytes = up(planes * 2 * seq * dpad * 2), v_bytes = up(planes * 2 * seq * dvpad * 2);
     const size_t peak_bytes = up(planes * chunks * 256 * 4), kmul_bytes = up(planes * 4);
-    qk_status st = c->d_terms.reserve(k_bytes + v_bytes + peak_bytes + kmul_bytes + up(planes * dvpad * 4));
+    const size_t vmul_bytes = up(planes * dvpad * 4), mark_bytes = s->batch * s->n_heads * ceil_div(s->seq_q, kRows) * 16;
+    qk_status st = c->d_terms.reserve(k_bytes + v_bytes + peak_bytes + kmul_bytes + vmul_bytes + mark_bytes);
     if (st != QK_OK) return st;
     uint8_t *base = (uint8_t *)c->d_terms.ptr;
     uint16_t *kt = (uint16_t *)base, *vt = (uint16_t *)(base + k_bytes);
@@ -661,8 +639,9 @@ qk_status attention_split_exact(qk_ctx *c, const float *q, const float *k, const
     if ((st = plane_map(kt, dpad, seq, planes * 2, seq * dpad * 2, &km)) != QK_OK) return st;
     if ((st = plane_map(vt, dvpad, seq, planes * 2, seq * dvpad * 2, &vm)) != QK_OK) return st;
     Args a{};
-    a.q = q, a.out = out, a.k = k, a.v = v;
-    a.kv_plane = seq * s->head_dim, a.v_plane = seq * s->val_dim;
+    a.q = q, a.out = out;
+    a.marked = (uint32_t *)((uint8_t *)v_mul + vmul_bytes);
+    *marked = a.marked;
     a.k_mul = k_mul, a.v_mul = v_mul;
     a.q_row = s->head_dim, a.q_head = s->seq_q * s->head_dim, a.q_batch = s->n_heads * a.q_head;
     a.o_row = s->val_dim, a.o_head = s->seq_q * s->val_dim, a.o_batch = s->n_heads * a.o_head;

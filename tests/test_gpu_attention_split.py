@@ -83,6 +83,76 @@ def test_exact_face_with_infinities_and_nan(ctx):
     assert np.abs(got[fine] - want[fine]).max() < 2e-6 * np.abs(want[fine]).max()
 
 
+@pytest.mark.parametrize("Sk", [191, 192, 260])
+@pytest.mark.parametrize("entry", [1e4, 1e6, 1e8, 1e12, 1e30])
+@pytest.mark.parametrize("place", ["last key", "a key's channel where q is zero", "seen key", "last value", "seen value",
+                                   "a value in every 64", "half of a query"])
+def test_exact_face_with_a_large_entry_among_small_ones(ctx, place, entry, Sk):
+    """A row is as exact as its own operands allow, whatever lies elsewhere in the sequence: every row is held to its
+    own largest output.  (A score s is off by about s 2^-23, which weighs fully where it decides over a large value.)"""
+    rng = np.random.default_rng(Sk)
+    q, k, v = (rng.standard_normal((2, Sk, 64)).astype(np.float32) for _ in range(3))
+    at_most = 8                  # of the scores that bear on an output
+    if place == "last key":
+        k[0, -1, 3] = entry
+    elif place == "a key's channel where q is zero":
+        q[:, :, 7], k[0, :, 7] = 0, entry
+    elif place == "seen key":
+        k[0, 10, 3], q[0, :, 3] = entry, -np.abs(q[0, :, 3])     # (its score is far below the others)
+    elif place == "last value":
+        v[0, -1, 3] = entry
+    elif place == "seen value":
+        v[0, 10, 3], k[0, 10], at_most = entry, -3 * q[0, 150], 30
+    elif place == "a value in every 64":
+        v[0, 63::64, 3] = -entry
+    else:
+        q[0, :, 32:] *= 1 / np.float32(entry)
+        k[0, :, 32:] *= np.float32(entry)
+        q[0, :, :32] *= 0.5
+    got = ctx.attention(AttentionShape(1, 2, 2, Sk, Sk, 64, 64), q, k, v, True).reshape(2, Sk, 64)
+    want = visible_attention(q, k, v, True, 0)
+    assert (np.abs(got - want).max(-1) <= 2 * at_most * 2.0 ** -23 * np.abs(want).max(-1)).all()
+
+
+def test_exact_face_of_zeros(ctx):
+    """Zeros are exact: a plane, a channel, the values that the first rows see."""
+    rng = np.random.default_rng(7)
+    q, k, v = (rng.standard_normal((3, 256, 128)).astype(np.float32) for _ in range(3))
+    v[0], k[1], v[2, :100], v[2, :, 70:] = 0, 0, 0, 0
+    got = ctx.attention(AttentionShape(1, 3, 3, 256, 256, 128, 128), q, k, v, True).reshape(3, 256, 128)
+    want = visible_attention(q, k, v, True, 0)
+    assert not got[0].any() and not got[2, :100].any() and not got[2, :, 70:].any()
+    assert np.abs(got - want).max() < 2e-6 * np.abs(want).max()
+
+
+def test_exact_face_where_every_product_loses_the_same(ctx):
+    """Mantissas of 1 + 2^-11 are a high term of 1 and a low one of 2^-11, whose product is not formed: 2^-22 of every
+    product, with one sign.  A score s is off by s 2^-22, an output by 2^-22 and by twice the largest score error."""
+    rng = np.random.default_rng(9)
+    q, k, v = (rng.choice([-1.0, 1.0], (1, 256, 64)).astype(np.float32) * np.float32(1 + 2.0 ** -11) for _ in range(3))
+    got = ctx.attention(AttentionShape(1, 1, 1, 256, 256, 64, 64), q, k, v, False).reshape(1, 256, 64)
+    scores = np.abs(q[0].astype(np.float64) @ k[0].T / 8).max()
+    assert np.abs(got - visible_attention(q, k, v, False, 0)).max() <= (1 + 2 * scores) * 2.0 ** -22 * np.abs(v).max()
+
+
+@pytest.mark.parametrize("causal", [True, False])
+def test_exact_face_of_2048_keys(ctx, causal):
+    import torch
+    gen = torch.Generator("cuda").manual_seed(11)
+    q, k, v = (torch.randn(1, h, 2048, 128, device="cuda", generator=gen) for h in (8, 2, 2))
+    k += 2 * torch.randn(1, 2, 1, 128, device="cuda", generator=gen)
+    y = torch.full_like(q, math.nan)
+    torch.cuda.synchronize()
+    ctx.attention_dev(AttentionShape(1, 8, 2, 2048, 2048, 128, 128), q.data_ptr(), k.data_ptr(), v.data_ptr(), causal, y.data_ptr())
+    ctx.synchronize()
+    kk, vv = (t.double().repeat_interleave(4, 1) for t in (k, v))
+    s = q.double() @ kk.transpose(2, 3) * 128 ** -0.5
+    if causal:
+        s = s.masked_fill(torch.ones(2048, 2048, dtype=torch.bool, device="cuda").triu(1), -math.inf)
+    want = torch.softmax(s, -1) @ vv
+    assert float((y - want).abs().max()) < 2e-6 * float(want.abs().max())
+
+
 @pytest.mark.parametrize("H,KV,T,p0", [(4, 1, 64, 0), (4, 2, 129, 0), (6, 2, 65, 63), (3, 3, 1, 70), (8, 1, 127, 130)])
 def test_prefill_attention_at_the_edges_of_tiles(ctx, H, KV, T, p0):
     import torch
