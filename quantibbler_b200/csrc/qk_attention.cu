@@ -1942,8 +1942,10 @@ qk_status attention_sage_block_dev(qk_ctx *c, const float *dq, const float *dk, 
 qk_status attention_exact_dev(qk_ctx *c, const float *q, const float *k, const float *v,
                               float *out, const qk_attention_shape *s, int causal) {
     const uint32_t *marked = nullptr;
-    if (attention_split_takes(c, s, causal))
-        if (qk_status st = attention_split_exact(c, q, k, v, out, s, causal, &marked); st != QK_OK) return st;
+    if (attention_split_takes(c, s, causal)) {
+        const qk_status st = attention_split_exact(c, q, k, v, out, s, causal, &marked);
+        if (st != QK_OK && st != QK_ERR_ALLOC) return st;  // (without memory for the terms: all rows below)
+    }
     AttnDims dm = dims_of(s);
     size_t widest = s->head_dim > s->val_dim ? s->head_dim : s->val_dim;
     if (widest <= 16) return launch_exact<4>(c, q, k, v, out, dm, causal, marked);

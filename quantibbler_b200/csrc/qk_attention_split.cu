@@ -579,8 +579,6 @@ qk_status plane_map(const void *base, size_t pad, size_t seq, size_t planes, siz
 }
 
 qk_status launch_split(qk_ctx *c, const CUtensorMap &km, const CUtensorMap &vm, Args &a, size_t batch) {
-    qk_status st = qk::error_word(c);
-    if (st != QK_OK) return st;
     a.error = (int *)c->d_err.ptr;
     a.wait_limit = c->wait_limit ? c->wait_limit : kWaitLimit;
     auto kernel = a.dpad == 64 ? split_attention_kernel<1> : split_attention_kernel<2>;
@@ -621,7 +619,9 @@ qk_status attention_split_exact(qk_ctx *c, const float *q, const float *k, const
     const size_t k_bytes = up(planes * 2 * seq * dpad * 2), v_bytes = up(planes * 2 * seq * dvpad * 2);
     const size_t peak_bytes = up(planes * chunks * 256 * 4), kmul_bytes = up(planes * 4);
     const size_t vmul_bytes = up(planes * dvpad * 4), mark_bytes = s->batch * s->n_heads * ceil_div(s->seq_q, kRows) * 16;
-    qk_status st = c->d_terms.reserve(k_bytes + v_bytes + peak_bytes + kmul_bytes + vmul_bytes + mark_bytes);
+    qk_status st = error_word(c);
+    if (st != QK_OK) return st;
+    st = c->d_terms.reserve(k_bytes + v_bytes + peak_bytes + kmul_bytes + vmul_bytes + mark_bytes);
     if (st != QK_OK) return st;
     uint8_t *base = (uint8_t *)c->d_terms.ptr;
     uint16_t *kt = (uint16_t *)base, *vt = (uint16_t *)(base + k_bytes);
@@ -641,7 +641,6 @@ qk_status attention_split_exact(qk_ctx *c, const float *q, const float *k, const
     Args a{};
     a.q = q, a.out = out;
     a.marked = (uint32_t *)((uint8_t *)v_mul + vmul_bytes);
-    *marked = a.marked;
     a.k_mul = k_mul, a.v_mul = v_mul;
     a.q_row = s->head_dim, a.q_head = s->seq_q * s->head_dim, a.q_batch = s->n_heads * a.q_head;
     a.o_row = s->val_dim, a.o_head = s->seq_q * s->val_dim, a.o_batch = s->n_heads * a.o_head;
@@ -650,7 +649,9 @@ qk_status attention_split_exact(qk_ctx *c, const float *q, const float *k, const
     a.d = (uint32_t)s->head_dim, a.dv = (uint32_t)s->val_dim, a.dpad = (uint32_t)dpad, a.dvpad = (uint32_t)dvpad;
     a.skew = (int)seq - (int)s->seq_q, a.causal = causal != 0;
     a.scale = 1.0f / sqrtf((float)s->head_dim);
-    return launch_split(c, km, vm, a, s->batch);
+    if ((st = launch_split(c, km, vm, a, s->batch)) != QK_OK) return st;
+    *marked = a.marked;
+    return QK_OK;
 }
 
 }  // namespace qk

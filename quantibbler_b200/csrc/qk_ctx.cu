@@ -13,6 +13,7 @@ qk_status qk_scratch::reserve(size_t bytes) {
     cudaError_t e = cudaMalloc(&ptr, want);
     if (e != cudaSuccess) {
         ptr = nullptr;
+        cudaGetLastError();  // (or the next launch would be taken for the one that failed)
         return qk::fail(QK_ERR_ALLOC, "device allocation of %zu bytes failed: %s", want,
                         cudaGetErrorString(e));
     }

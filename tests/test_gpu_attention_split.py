@@ -153,6 +153,26 @@ def test_exact_face_of_2048_keys(ctx, causal):
     assert float((y - want).abs().max()) < 2e-6 * float(want.abs().max())
 
 
+def test_exact_face_without_room_for_the_terms(ctx):
+    """Heads of one channel, padded to 64: the terms would take 251 GB where k and v take 4.  The call goes through all
+    the same, and so does the next."""
+    import torch
+    B, n = 60000, 8192
+    gen = torch.Generator("cuda").manual_seed(12)
+    k, v = (torch.randn(B, n, device="cuda", generator=gen) for _ in range(2))
+    q, y = torch.randn(B, device="cuda", generator=gen), torch.full((B,), math.nan, device="cuda")
+    torch.cuda.synchronize()
+    ctx.attention_dev(AttentionShape(B, 1, 1, 1, n, 1, 1), q.data_ptr(), k.data_ptr(), v.data_ptr(), False, y.data_ptr())
+    ctx.synchronize()
+    some = slice(None, None, 61)
+    weights = torch.softmax(q[some, None].double() * k[some].double(), -1)
+    want = (weights * v[some]).sum(-1)
+    # (8192 additions in turn, each off by half a unit of the running sum: of the weights, and of the products)
+    assert bool(torch.isfinite(y).all())
+    assert bool(((y[some] - want).abs() <= 2 * n * 2.0 ** -24 * (weights * v[some].abs()).sum(-1)).all())
+    test_exact_face_at_the_edges_of_tiles(ctx, 1, 1, 257, 257, 64, 64, True)
+
+
 @pytest.mark.parametrize("H,KV,T,p0", [(4, 1, 64, 0), (4, 2, 129, 0), (6, 2, 65, 63), (3, 3, 1, 70), (8, 1, 127, 130)])
 def test_prefill_attention_at_the_edges_of_tiles(ctx, H, KV, T, p0):
     import torch
