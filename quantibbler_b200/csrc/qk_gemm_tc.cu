@@ -31,8 +31,9 @@
 // expansion: 890 clocks.  Around the loops come 5 us of launch and first fetch per kernel and the last tile.
 // 14336 x 4096 of rank 2560 on 2048 tokens: 209 -> 162 us, 4096 x 4096 of rank 1102 on 64 tokens 29.7 -> 24.5 us.
 // Pairs of CTAs sharing the token tile (cta_group::2) came out no faster: 172 against 172 us.
-// All hand-offs go through mbarriers.  Every wait is bounded: on expiry the kernel records an
-// error code, frees its tensor memory and returns, and the host reports QK_ERR_TIMEOUT.
+// All hand-offs go through mbarriers.  Every wait is bounded: on expiry the kernel waits for its
+// own copies and products in flight, records an error code, frees its tensor memory and returns,
+// and the host reports QK_ERR_TIMEOUT.
 #include <cuda.h>  // CUtensorMap types only; the encoder is fetched through the runtime
 
 #include <algorithm>
@@ -216,9 +217,12 @@ factorized_gemm_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid
     uint64_t *acc_full = empty + kStages;   // [2]
     uint64_t *acc_empty = acc_full + 2;     // [2]
     uint64_t *staged_bar = acc_empty + 2;   // a neighbour's partial accumulator has landed
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(staged_bar + 1);
+    uint64_t *drain = staged_bar + 1;       // (given up) the products that were issued are done
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-    volatile uint32_t *segments = tmem_slot + 2;  // of this CTA's run
+    volatile int *never = reinterpret_cast<volatile int *>(tmem_slot + 2);  // the flag of waits that nothing cuts short
+    volatile uint32_t *segments = tmem_slot + 3;  // of this CTA's run
+    volatile uint32_t *copied = tmem_slot + 4;    // chunks whose token copies were started
 
     const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     const uint32_t kBN = g.bn;
@@ -277,7 +281,9 @@ factorized_gemm_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid
             mbar_init(&acc_empty[a], kEpilogueWarps);
         }
         mbar_init(staged_bar, 1);
+        mbar_init(drain, 1);
         *abort_flag = 0;
+        *never = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == kMmaWarp) {
@@ -296,6 +302,8 @@ factorized_gemm_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid
     qk::pdl_wait();
     const uint32_t tmem_base = *tmem_slot;
     bool ok = true;  // none of this warp's waits has run out
+    uint32_t chunk = 0;      // (producers, copy warp) the chunk this warp has come to
+    bool staging = false;    // (one epilogue warp) the others' partials are being fetched
 
     // ---- the epilogue's parts.  Thread = weight row n (tensor-memory lane; a warp reaches the 32 lanes of its
     // number modulo 4), columns = tokens.
@@ -366,7 +374,8 @@ factorized_gemm_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid
             return pr.w_rows + (size_t)min(ahead.row_tile * kBM + row, pr.n_rows - 1) * pr.w_stride;
         };
         const uint8_t *bits = row_of();
-        for (uint32_t gc = group; gc < total_chunks; gc += kGroups) {
+        uint32_t gc = group;
+        for (; gc < total_chunks; gc += kGroups) {
             const uint2 cur = q0;
             if (!mbar_wait(&empty[s], phase, abort_flag, g.wait_limit)) {
                 ok = false;
@@ -398,6 +407,7 @@ factorized_gemm_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid
             }
             phase ^= 1;
         }
+        chunk = gc;
     } else if (warp == kMmaWarp) {
         // ------------------------------------------------------------ MMA issue
         // The whole warp runs the loop and waits on the barriers; one lane issues.
@@ -449,7 +459,8 @@ factorized_gemm_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid
         // ------------------------------------------------------------ token copies
         // one TMA box of 64 k x bn tokens per chunk, completing on the full barrier
         Walk at(g, min(u_begin, g.units - 1));
-        for (uint32_t gc = 0, s = 0, phase = 1; gc < total_chunks; ++gc) {
+        uint32_t gc = 0;
+        for (uint32_t s = 0, phase = 1; gc < total_chunks; ++gc) {
             if (!mbar_wait(&empty[s], phase, abort_flag, g.wait_limit)) {
                 ok = false;
                 *abort_flag = 1;
@@ -475,6 +486,8 @@ factorized_gemm_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid
                 phase ^= 1;
             }
         }
+        chunk = gc;
+        if (lane == 0) *copied = gc;
     } else {
         // ------------------------------------------------------------ epilogue of all segments but the last
         uint32_t seg = 0;
@@ -527,6 +540,7 @@ factorized_gemm_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid
         const uint32_t part_bytes = kBN * kBM * 4;
         const uint32_t n_staged = min(last - blockIdx.x - 1, (uint32_t)(kStages * kStageBytes) / part_bytes);
         if (warp == kEpilogueWarp0) {
+            staging = true;
             for (uint32_t j = blockIdx.x + 1; j < last && ok; ++j) {
                 uint32_t seen = 0;
                 for (uint32_t i = 0; i < g.wait_limit; ++i) {
@@ -582,9 +596,23 @@ factorized_gemm_tc_kernel(const __grid_constant__ CUtensorMap map0, const __grid
     }
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
-    // (given up: the copies and products still in flight end within microseconds, a millisecond is waited)
-    if (*abort_flag)
-        for (int i = 0; i < 1000; ++i) __nanosleep(1000);
+    if (*abort_flag) {
+        // Given up: wait for the copies and products still in flight.  A stage's barrier counts its copy and its
+        // four producer warps; a producer that has not come to the last chunk copied into its stage (the copy
+        // runs one chunk ahead of it at most) arrives for that chunk all the same.
+        if (warp < kProducerWarps) {
+            if (lane == 0 && chunk < *copied) mbar_arrive(&full[group]);
+        } else if (warp == kCopyWarp) {
+            for (uint32_t gc = chunk > (uint32_t)kStages ? chunk - kStages : 0; gc < chunk; ++gc)
+                (void)mbar_wait(&full[gc % kStages], (gc / kStages) & 1, never, kWaitLimitDefault);
+        } else if (warp == kMmaWarp) {
+            if (elect_one()) umma_commit(drain);
+            __syncwarp();
+            (void)mbar_wait(drain, 0, never, kWaitLimitDefault);
+        } else if (staging) {
+            (void)mbar_wait(staged_bar, 0, never, kWaitLimitDefault);
+        }
+    }
     if (warp == kMmaWarp) {
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base),
                      "r"(kTmemCols)
@@ -716,7 +744,7 @@ norm_scale_to_bf16_kernel(NormArgs n, ScaleArgs a, uint32_t n_problems, uint32_t
     }
 }
 
-constexpr size_t kSmemBytes = 1024 + kStages * kStageBytes + (2 * kStages + 5) * 8 + 16;
+constexpr size_t kSmemBytes = 1024 + kStages * kStageBytes + (2 * kStages + 6) * 8 + 24;
 static_assert(kSmemBytes <= 227 * 1024, "the stages must fit the 227 KB a CTA may have");
 
 // cuTensorMapEncodeTiled, obtained through the runtime so that the library does not link

@@ -1,7 +1,7 @@
 """Failure paths that end in a status, not in a fault: a device-side wait that runs out,
-and a token that does not fit the KV cache.  Neither test makes the GPU fault, trap or hang:
-the wait is a bounded poll of ordinary memory that nothing writes, the out-of-range token is
-skipped by a bounds check."""
+and a token that does not fit the KV cache.  No test makes the GPU fault, trap or hang:
+the waits are bounded polls of ordinary memory or of a kernel's own barriers, the out-of-range
+token is skipped by a bounds check."""
 
 import ctypes
 
@@ -247,3 +247,42 @@ def test_allreduce_inside_plans_on_one_gpu_and_its_wait_running_out(gpu_ctx):
     LayerPlan(gpu_ctx, [(q, hn[b].data_ptr(), y2[b].data_ptr()) for b in range(n_tok)]).apply()
     gpu_ctx.synchronize()
     assert torch.equal(y2, y_ref)
+
+
+def _gives_up(ctx, call):
+    """Whether ``call`` reports a pipeline wait that ran out, in one of twenty tries with a single poll per wait."""
+    prev = ctx.set_wait_limit(1)
+    try:
+        for _ in range(20):
+            call()
+            try:
+                ctx.synchronize()
+            except DeviceError as e:
+                assert "pipeline barrier of a tcgen05 kernel" in str(e)
+                return True
+    finally:
+        ctx.set_wait_limit(prev)
+    return False
+
+
+def test_prefill_gemm_waits_run_out():
+    """One poll per wait: somewhere a CTA that finishes a tile finds another's share of it not there yet, or a
+    stage not filled.  The kernel waits for its own copies and products and ends, the call is reported, and
+    the context works on."""
+    import torch
+    from quantibbler_b200.gpu import GpuContext, PackedLayer
+    from tests.conftest import make_layer
+    ctx = GpuContext.init()
+    L = make_layer(1024, 2048, 300, seed=3)
+    layer = PackedLayer(ctx, L["ub_rows"], L["vb_t_rows"], 1024, 2048, 300, L["s1"], L["s2"], None, serving="bfloat16")
+    x = torch.randn(500, 2048, device="cuda")
+    y = torch.zeros(500, 1024, device="cuda")
+    torch.cuda.synchronize()
+    assert _gives_up(ctx, lambda: layer.apply_prefill(x.data_ptr(), 500, y.data_ptr()))
+    ctx.synchronize()            # reported once, then clear
+    z, w = torch.zeros_like(x), torch.ones(2048, device="cuda")
+    torch.cuda.synchronize()
+    _lib.check(_lib.lib().qk_rmsnorm(ctx.handle, _p(x), None, _p(w), 500, 2048, 0.0, _lib.QK_F32, None, _p(z)))
+    ctx.synchronize()
+    assert float((z - x / x.pow(2).mean(1, keepdim=True).sqrt()).abs().max()) < 1e-5
+    layer.close()
