@@ -362,12 +362,7 @@ split_attention_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
             if (elect_one()) scores(g + 2);   // (over scores that the unit has read: it has handed in their weights)
             __syncwarp();
         }
-        if (!ok) {
-            *abort_flag = 1;
-            if (elect_one()) umma_commit(drain);  // the products still in flight
-            __syncwarp();
-            (void)mbar_wait(drain, 0, never, kWaitLimit);
-        }
+        if (!ok) *abort_flag = 1;
     } else {
         const uint32_t u = warp / 4, r = threadIdx.x % 128;
         const uint32_t i = row0 + r;                      // query row
@@ -564,6 +559,11 @@ split_attention_kernel(const __grid_constant__ CUtensorMap k_map, const __grid_c
             (void)mbar_wait(k_full + g % kStages, (g / kStages) & 1, never, kWaitLimit);
         for (uint32_t g = fetched_v > kStages ? fetched_v - kStages : 0; g < fetched_v; ++g)
             (void)mbar_wait(v_full + g % kStages, (g / kStages) & 1, never, kWaitLimit);
+    }
+    if (warp == kMmaWarp && *abort_flag) {  // the products still in flight (whichever warp gave up)
+        if (elect_one()) umma_commit(drain);
+        __syncwarp();
+        (void)mbar_wait(drain, 0, never, kWaitLimit);
     }
     if (warp == kMmaWarp)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kTmemCols) : "memory");

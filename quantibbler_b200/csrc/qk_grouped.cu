@@ -751,12 +751,7 @@ grouped_portion_umma_kernel(const __grid_constant__ CUtensorMap q_map, const __g
             }
             __syncwarp();
         }
-        if (!ok) {
-            *abort_flag = 1;
-            if (elect_one()) umma_commit(drain);  // the products still in flight
-            __syncwarp();
-            (void)mbar_wait(drain, 0, never, kUmWaitDefault);
-        }
+        if (!ok) *abort_flag = 1;
     } else {
         const uint32_t u = warp / 4, r = threadIdx.x % 128;
         const PortionUnit me = u ? unit[1] : unit[0];
@@ -888,6 +883,11 @@ grouped_portion_umma_kernel(const __grid_constant__ CUtensorMap q_map, const __g
             (void)mbar_wait(k_full + j % kUmStages, (j / kUmStages) & 1, never, kUmWaitDefault);
             (void)mbar_wait(v_full + j % kUmStages, (j / kUmStages) & 1, never, kUmWaitDefault);
         }
+    }
+    if (warp == 9 && *abort_flag) {  // the products still in flight (whichever warp gave up)
+        if (elect_one()) umma_commit(drain);
+        __syncwarp();
+        (void)mbar_wait(drain, 0, never, kUmWaitDefault);
     }
     if (warp == 9)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(kUmTmemCols) : "memory");

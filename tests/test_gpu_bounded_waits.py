@@ -286,3 +286,34 @@ def test_prefill_gemm_waits_run_out():
     ctx.synchronize()
     assert float((z - x / x.pow(2).mean(1, keepdim=True).sqrt()).abs().max()) < 1e-5
     layer.close()
+
+
+def test_attention_waits_run_out():
+    """The exact face and the causal portion kernel: with one poll per wait a call may give up, in any of its roles; it
+    is reported if it does, and the next call is right."""
+    import torch
+    from quantibbler_b200.gpu import AttentionShape, GpuContext
+    ctx, lib = GpuContext.init(), _lib.lib()
+    H, S, d = 4, 700, 128
+    q, k, v = (torch.randn(1, H, S, d, device="cuda") for _ in range(3))
+    y = torch.zeros_like(q)
+    qb = q[0].transpose(0, 1).bfloat16().contiguous()                                     # [position][head][channel]
+    kv = torch.cat([t[0].transpose(0, 1).reshape(S, H * d) for t in (k, v)], 1).bfloat16().contiguous()
+    out = torch.zeros(S, H * d, device="cuda", dtype=torch.bfloat16)
+    torch.cuda.synchronize()
+
+    def exact():
+        ctx.attention_dev(AttentionShape(1, H, H, S, S, d, d), q.data_ptr(), k.data_ptr(), v.data_ptr(), True, y.data_ptr())
+
+    def portion():
+        _lib.check(lib.qk_window_attention(ctx.handle, _p(qb), H * d, _p(kv), 2 * H * d, 0, S, 0, S, H, d, d, d, S,
+                                           d ** -0.5, _p(out), H * d))
+
+    want = torch.nn.functional.scaled_dot_product_attention(q.double(), k.double(), v.double(), is_causal=True)[0]
+    for call in (exact, portion):
+        _gives_up(ctx, call)
+        call()
+        ctx.synchronize()
+    assert float((y[0] - want).abs().max()) < 2e-6 * float(want.abs().max())
+    got = out.reshape(S, H, d).transpose(0, 1)
+    assert float((got - want).abs().max()) < 1e-2 * float(want.abs().max())   # (operands rounded to bfloat16)
