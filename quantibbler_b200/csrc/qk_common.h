@@ -171,5 +171,6 @@ qk_status causal_portion(qk_ctx *c, const void *q, size_t q_stride, const void *
 // Makes sure the context's error word (an int, bits: 1 a prefill pipeline wait, 2 an all-reduce
 // inbox wait, 4 a token outside the KV cache, 8 a wait of the streaming GEMV, 16 a grid barrier of the
 // whole-step decode kernel) and the prefill's CTA flags after it exist.
+constexpr size_t kErrorBlockBytes = 256 + 4096;
 qk_status error_word(qk_ctx *c);
 }  // namespace qk

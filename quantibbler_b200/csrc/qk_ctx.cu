@@ -82,9 +82,9 @@ qk_status resolve_ctx(qk_ctx *ctx, qk_ctx **out) {
 
 qk_status error_word(qk_ctx *c) {
     if (c->d_err.ptr) return QK_OK;
-    qk_status st = c->d_err.reserve(256 + 4096);
+    qk_status st = c->d_err.reserve(kErrorBlockBytes);
     if (st != QK_OK) return st;
-    QK_CUDA(cudaMemsetAsync(c->d_err.ptr, 0, 256 + 4096, c->stream));
+    QK_CUDA(cudaMemsetAsync(c->d_err.ptr, 0, kErrorBlockBytes, c->stream));
     return QK_OK;
 }
 
@@ -192,7 +192,9 @@ qk_status qk_gpu_synchronize(qk_ctx *ctx) {
         QK_CUDA(cudaMemcpyAsync(&h_err, c->d_err.ptr, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
         QK_CUDA(cudaStreamSynchronize(c->stream));
         if (h_err) {
-            QK_CUDA(cudaMemsetAsync(c->d_err.ptr, 0, sizeof(int), c->stream));
+            // (with it the prefill GEMM's flags: a CTA that gave up has left flags of partial sums unread, and a
+            // later launch would take those sums for its own)
+            QK_CUDA(cudaMemsetAsync(c->d_err.ptr, 0, qk::kErrorBlockBytes, c->stream));
             if (h_err & 4)
                 return qk::fail(QK_ERR_VALUE,
                                 "a token's position or sequence index lies outside the KV cache; "

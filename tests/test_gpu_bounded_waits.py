@@ -268,7 +268,7 @@ def _gives_up(ctx, call):
 def test_prefill_gemm_waits_run_out():
     """One poll per wait: somewhere a CTA that finishes a tile finds another's share of it not there yet, or a
     stage not filled.  The kernel waits for its own copies and products and ends, the call is reported, and
-    the context works on."""
+    the context works on: partial sums that were left behind are not taken for a later call's."""
     import torch
     from quantibbler_b200.gpu import GpuContext, PackedLayer
     from tests.conftest import make_layer
@@ -276,10 +276,19 @@ def test_prefill_gemm_waits_run_out():
     L = make_layer(1024, 2048, 300, seed=3)
     layer = PackedLayer(ctx, L["ub_rows"], L["vb_t_rows"], 1024, 2048, 300, L["s1"], L["s2"], None, serving="bfloat16")
     x = torch.randn(500, 2048, device="cuda")
-    y = torch.zeros(500, 1024, device="cuda")
+    other = -2 * x
+    y, want = (torch.zeros(500, 1024, device="cuda") for _ in range(2))
     torch.cuda.synchronize()
-    assert _gives_up(ctx, lambda: layer.apply_prefill(x.data_ptr(), 500, y.data_ptr()))
-    ctx.synchronize()            # reported once, then clear
+    layer.apply_prefill(x.data_ptr(), 500, want.data_ptr())
+    for _ in range(3):
+        assert _gives_up(ctx, lambda: layer.apply_prefill(other.data_ptr(), 500, y.data_ptr()))
+        ctx.synchronize()        # reported once, then clear
+        for _ in range(2):
+            y.zero_()
+            torch.cuda.synchronize()
+            layer.apply_prefill(x.data_ptr(), 500, y.data_ptr())
+            ctx.synchronize()
+            assert torch.equal(y, want)
     z, w = torch.zeros_like(x), torch.ones(2048, device="cuda")
     torch.cuda.synchronize()
     _lib.check(_lib.lib().qk_rmsnorm(ctx.handle, _p(x), None, _p(w), 500, 2048, 0.0, _lib.QK_F32, None, _p(z)))
