@@ -1981,7 +1981,7 @@ qk_status qk_gpu_attention(qk_ctx *ctx, const qk_attention_shape *shape, const f
         return st;
     QK_CUDA(cudaMemcpyAsync(out, c->d_out.ptr, ob, cudaMemcpyDeviceToHost, c->stream));
     QK_CUDA(cudaStreamSynchronize(c->stream));
-    return QK_OK;
+    return qk::report_errors(c, 1);  // (a wait that ran out: the result is unfinished)
 }
 
 qk_status qk_gpu_attention_sage(qk_ctx *ctx, const qk_attention_shape *shape, const float *query,
@@ -2009,7 +2009,7 @@ qk_status qk_gpu_attention_sage(qk_ctx *ctx, const qk_attention_shape *shape, co
         return st;
     QK_CUDA(cudaMemcpyAsync(out, c->d_out.ptr, ob, cudaMemcpyDeviceToHost, c->stream));
     QK_CUDA(cudaStreamSynchronize(c->stream));
-    return QK_OK;
+    return qk::report_errors(c, 1);  // (a wait that ran out: the result is unfinished)
 }
 
 qk_status qk_gpu_attention_dev(qk_ctx *ctx, const qk_attention_shape *shape, const float *q_dev,

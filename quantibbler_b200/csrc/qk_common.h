@@ -173,4 +173,5 @@ qk_status causal_portion(qk_ctx *c, const void *q, size_t q_stride, const void *
 // whole-step decode kernel) and the prefill's CTA flags after it exist.
 constexpr size_t kErrorBlockBytes = 256 + 4096;
 qk_status error_word(qk_ctx *c);
+qk_status report_errors(qk_ctx *c, int which);
 }  // namespace qk

@@ -88,6 +88,29 @@ qk_status error_word(qk_ctx *c) {
     return QK_OK;
 }
 
+// Reads the error word once the stream is idle.  If it holds one of the bits `which`, it is cleared and reported.
+qk_status report_errors(qk_ctx *c, int which) {
+    // (armed: kernels that can raise the error word have been launched on this context, or captured
+    // into a graph that may be replayed at any time, which is why the check stays armed)
+    if (!c->err_armed) return QK_OK;
+    int h_err = 0;
+    QK_CUDA(cudaMemcpyAsync(&h_err, c->d_err.ptr, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+    QK_CUDA(cudaStreamSynchronize(c->stream));
+    if (!(h_err & which)) return QK_OK;
+    // (with it the prefill GEMM's flags: a CTA that gave up has left flags of partial sums unread, and a
+    // later launch would take those sums for its own)
+    QK_CUDA(cudaMemsetAsync(c->d_err.ptr, 0, kErrorBlockBytes, c->stream));
+    if (h_err & 4)
+        return fail(QK_ERR_VALUE,
+                    "a token's position or sequence index lies outside the KV cache; "
+                    "the token was skipped");
+    return fail(QK_ERR_TIMEOUT, "a bounded device-side wait gave up:%s%s%s%s",
+                (h_err & 1) ? " a pipeline barrier of a tcgen05 kernel (prefill GEMM, dense linear, attention);" : "",
+                (h_err & 2) ? " the inbox of a fused all-reduce (a peer did not send);" : "",
+                (h_err & 8) ? " a ring or table barrier of the streaming GEMV;" : "",
+                (h_err & 16) ? " a grid barrier of the whole-step decode kernel;" : "");
+}
+
 }  // namespace qk
 
 extern "C" {
@@ -185,29 +208,7 @@ qk_status qk_gpu_synchronize(qk_ctx *ctx) {
     QK_CUDA(cudaSetDevice(c->device));
     QK_CUDA(cudaStreamSynchronize(c->stream));
     std::lock_guard<std::mutex> lock(c->mu);
-    if (c->err_armed) {
-        // Kernels that can raise the error word have been launched on this context (or captured
-        // into a graph that may be replayed at any time, which is why the check stays armed).
-        int h_err = 0;
-        QK_CUDA(cudaMemcpyAsync(&h_err, c->d_err.ptr, sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-        QK_CUDA(cudaStreamSynchronize(c->stream));
-        if (h_err) {
-            // (with it the prefill GEMM's flags: a CTA that gave up has left flags of partial sums unread, and a
-            // later launch would take those sums for its own)
-            QK_CUDA(cudaMemsetAsync(c->d_err.ptr, 0, qk::kErrorBlockBytes, c->stream));
-            if (h_err & 4)
-                return qk::fail(QK_ERR_VALUE,
-                                "a token's position or sequence index lies outside the KV cache; "
-                                "the token was skipped");
-            return qk::fail(QK_ERR_TIMEOUT, "a bounded device-side wait gave up:%s%s%s%s",
-                            (h_err & 1) ? " a pipeline barrier of a tcgen05 kernel (prefill GEMM, dense linear, Sage attention);" : "",
-                            (h_err & 2) ? " the inbox of a fused all-reduce (a peer did not send);"
-                                        : "",
-                            (h_err & 8) ? " a ring or table barrier of the streaming GEMV;" : "",
-                            (h_err & 16) ? " a grid barrier of the whole-step decode kernel;" : "");
-        }
-    }
-    return QK_OK;
+    return qk::report_errors(c, ~0);
 }
 
 void *qk_gpu_stream(qk_ctx *ctx) {

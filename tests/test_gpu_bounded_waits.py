@@ -326,3 +326,36 @@ def test_attention_waits_run_out():
     assert float((y[0] - want).abs().max()) < 2e-6 * float(want.abs().max())
     got = out.reshape(S, H, d).transpose(0, 1)
     assert float((got - want).abs().max()) < 1e-2 * float(want.abs().max())   # (operands rounded to bfloat16)
+
+
+def test_host_attention_reports_a_wait_that_ran_out():
+    """The host-buffer face says so when a pipeline wait has run out before its result is there, its own or one of a call
+    in front of it on the stream (here the prefill GEMM's, whose waits can be made to run out)."""
+    import torch
+    from quantibbler_b200.gpu import AttentionShape, GpuContext, PackedLayer
+    from tests.conftest import make_layer
+    ctx = GpuContext.init()
+    L = make_layer(1024, 2048, 300, seed=3)
+    layer = PackedLayer(ctx, L["ub_rows"], L["vb_t_rows"], 1024, 2048, 300, L["s1"], L["s2"], None, serving="bfloat16")
+    x, y = torch.randn(500, 2048, device="cuda"), torch.zeros(500, 1024, device="cuda")
+    rng = np.random.default_rng(4)
+    shape = AttentionShape(1, 2, 2, 300, 300, 128, 128)
+    q, k, v = (rng.standard_normal((2, 300, 128)).astype(np.float32) for _ in range(3))
+    torch.cuda.synchronize()
+    faces = (lambda: ctx.attention(shape, q, k, v, True), lambda: ctx.attention_sage(shape, q, k, v, True, 64))
+    for face in faces:
+        want = face()
+        reported = False
+        for _ in range(20):
+            prev = ctx.set_wait_limit(1)
+            layer.apply_prefill(x.data_ptr(), 500, y.data_ptr())
+            ctx.set_wait_limit(prev)
+            try:
+                face()
+            except DeviceError as e:
+                assert "pipeline barrier of a tcgen05 kernel" in str(e)
+                reported = True
+                break
+        assert reported
+        assert np.array_equal(face(), want)      # reported once, then clear
+    layer.close()
