@@ -809,6 +809,14 @@ grouped_portion_umma_kernel(const __grid_constant__ CUtensorMap q_map, const __g
                     s[e] = __ffma2_rn(make_float2(__uint_as_float(raw[e / 16][e % 16 * 2]), __uint_as_float(raw[e / 16][e % 16 * 2 + 1])),
                                       f2, b2);
             }
+            if (nearest < 0) {  // (the band's -inf does not hide an infinity or NaN)
+                const int seen = pos - (int)(j * kUmKeys);
+#pragma unroll
+                for (int e = 0; e < kUmKeys / 2; ++e) {
+                    s[e].x = 2 * e <= seen ? s[e].x : -INFINITY;
+                    s[e].y = 2 * e + 1 <= seen ? s[e].y : -INFINITY;
+                }
+            }
 #pragma unroll
             for (int e = 0; e < kUmKeys / 2; ++e) mx[e % 4] = fmaxf(mx[e % 4], fmaxf(s[e].x, s[e].y));
             const float top = fmaxf(fmaxf(mx[0], mx[1]), fmaxf(mx[2], mx[3]));

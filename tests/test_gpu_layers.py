@@ -264,6 +264,28 @@ def test_window_that_hides_nothing(dev, dim, vdim, window, p0, tokens):
     test_window_attention_expanded(dev, dim, vdim, window, p0, tokens)
 
 
+def test_a_key_that_is_not_finite_reaches_only_the_rows_that_see_it(dev):
+    """Scores of unseen keys are left out, not added to -inf: an infinite or NaN key changes no earlier row."""
+    ctx, torch, L = dev
+    heads, d, n, P = 2, 128, 300, ctypes.c_void_p
+    g = torch.Generator(device="cuda").manual_seed(1)
+    q = torch.randn(n, heads * d, device="cuda", generator=g).bfloat16()
+    kv = torch.randn(n, 2 * heads * d, device="cuda", generator=g).bfloat16()
+
+    def run():
+        out = torch.zeros(n, heads * d, device="cuda", dtype=torch.bfloat16)
+        check(_lib.lib().qk_window_attention(ctx.handle, P(q.data_ptr()), heads * d, P(kv.data_ptr()), 2 * heads * d, 0, n,
+                                             0, n, heads, d, d, d, n, d ** -0.5, P(out.data_ptr()), heads * d))
+        ctx.synchronize()
+        return out.reshape(n, heads, d)
+
+    want = run()
+    kv[90, 5], kv[200, 5], kv[250, d + 5] = float("inf"), float("nan"), float("-inf")
+    got = run()
+    assert torch.equal(got[:90, 0], want[:90, 0]) and torch.equal(got[:250, 1], want[:250, 1])
+    assert bool(got[200:, 0].isnan().all())
+
+
 def test_late_positions_keep_their_angles(dev):
     """Sinusoidal positions near 10^6: float32 angles would be wrong in the second digit."""
     ctx, torch, L = dev
