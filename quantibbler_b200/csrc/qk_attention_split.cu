@@ -602,12 +602,7 @@ bool attention_split_takes(qk_ctx *c, const qk_attention_shape *s, int causal) {
     if (s->seq_kv < 192) return false;
     if (ceil_div(s->seq_q, kRows) > 65535 || s->batch * s->n_kv_heads > 65535 || s->seq_kv > (1u << 30)) return false;
     // (a captured graph may be replayed after the scratch has moved: a recording keeps the plain kernel)
-    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
-    if (cudaStreamIsCapturing(c->stream, &capture) != cudaSuccess) {
-        (void)cudaGetLastError();
-        return false;
-    }
-    return capture == cudaStreamCaptureStatusNone;
+    return !capturing(c);
 }
 
 qk_status attention_split_exact(qk_ctx *c, const float *q, const float *k, const float *v, float *out,

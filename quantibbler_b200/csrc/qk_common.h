@@ -154,6 +154,8 @@ cudaError_t launch_pdl(bool allow_overlap, void (*kernel)(KArgs...), dim3 grid, 
 // Returns the context to use for a call: `ctx` itself, or the process-wide default on
 // device 0 (created on first use) when `ctx` is null.
 qk_status resolve_ctx(qk_ctx *ctx, qk_ctx **out);
+// Whether calls on the context's stream are being recorded (or would disturb a recording): nothing may be allocated.
+bool capturing(qk_ctx *c);
 // Raises a kernel's dynamic shared memory limit, once per context and size (the call costs the host a microsecond).
 template <typename Kernel>
 qk_status allow_smem(qk_ctx *c, Kernel *kernel, size_t bytes) {

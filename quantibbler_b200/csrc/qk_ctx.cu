@@ -80,6 +80,15 @@ qk_status resolve_ctx(qk_ctx *ctx, qk_ctx **out) {
     return QK_OK;
 }
 
+bool capturing(qk_ctx *c) {
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    if (cudaStreamIsCapturing(c->stream, &capture) != cudaSuccess) {
+        (void)cudaGetLastError();
+        return true;
+    }
+    return capture != cudaStreamCaptureStatusNone;
+}
+
 qk_status error_word(qk_ctx *c) {
     if (c->d_err.ptr) return QK_OK;
     qk_status st = c->d_err.reserve(kErrorBlockBytes);

@@ -958,11 +958,13 @@ qk_status qk_window_attention(qk_ctx *ctx, const void *q, size_t q_stride, const
                         key0, key0 + n_keys - 1, first_position, first_position + tokens - 1);
     // A window that hides nothing leaves causal attention, which the tcgen05 portion kernel does; the band below is
     // bound by mma.sync and its fragments' loads (2048-token prompt through four such layers, 32 heads of 128:
-    // 8315 -> 7685 us, 240 -> 80 us a call; 20 tokens 1030 -> 928 us: it pays from the shortest portions on).
+    // 8315 -> 7685 us, 240 -> 80 us a call; 20 tokens 1030 -> 928 us: it pays from the shortest portions on).  It needs
+    // the context's error word, which a call that is being recorded cannot allocate.
     auto aligned = [](const void *p) { return ((uintptr_t)p & 15) == 0; };
     if (key0 == 0 && window >= first_position + tokens && vdim == vdim_stride && dim_stride % 16 == 0 &&
         vdim_stride % 16 == 0 && std::min(dim_stride, vdim_stride) >= 64 && std::max(dim_stride, vdim_stride) <= 128 &&
-        out_stride % 8 == 0 && aligned(q) && aligned(kv) && aligned(out) && c->decode_attention_kernel != 0)
+        out_stride % 8 == 0 && aligned(q) && aligned(kv) && aligned(out) && c->decode_attention_kernel != 0 &&
+        (c->d_err.ptr || !qk::capturing(c)))
         return qk::causal_portion(c, q, q_stride, kv, kv_row, first_position, tokens, heads, dim_stride, vdim, scale, out,
                                   out_stride);
     BandArgs a{};

@@ -286,6 +286,35 @@ def test_a_key_that_is_not_finite_reaches_only_the_rows_that_see_it(dev):
     assert bool(got[200:, 0].isnan().all())
 
 
+def test_window_attention_as_a_context_s_first_call_under_capture(dev):
+    """A recording allocates nothing: the call takes the kernel that needs no error word."""
+    _, torch, L = dev
+    from quantibbler_b200.gpu import GpuContext
+    ctx, P = GpuContext.init(), ctypes.c_void_p
+    heads, d, n = 2, 64, 100
+    q, kv = (torch.randn(n, m * heads * d, device="cuda").bfloat16() for m in (1, 2))
+    out = torch.zeros(n, heads * d, device="cuda", dtype=torch.bfloat16)
+    side, graph = torch.cuda.Stream(), torch.cuda.CUDAGraph()
+
+    def call():
+        check(_lib.lib().qk_window_attention(ctx.handle, P(q.data_ptr()), heads * d, P(kv.data_ptr()), 2 * heads * d, 0, n,
+                                             0, n, heads, d, d, d, n, d ** -0.5, P(out.data_ptr()), heads * d))
+
+    torch.cuda.synchronize()
+    ctx.set_stream(side.cuda_stream)
+    with torch.cuda.graph(graph, stream=side):
+        call()
+    graph.replay()
+    torch.cuda.synchronize()
+    recorded = out.clone()
+    out.zero_()
+    torch.cuda.synchronize()
+    call()
+    ctx.synchronize()
+    assert float((recorded.float() - out.float()).abs().max()) < 1e-2 * float(out.float().abs().max())
+    del graph
+
+
 def test_late_positions_keep_their_angles(dev):
     """Sinusoidal positions near 10^6: float32 angles would be wrong in the second digit."""
     ctx, torch, L = dev
