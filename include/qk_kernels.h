@@ -290,7 +290,8 @@ qk_status qk_layers_apply_prefill_gated(qk_ctx *ctx, const qk_layer *const *laye
 /* The same with the RMSNorm in front of the linears formed on the way: h = x (+ residual, may be null),
  * x_out = h (may be null, may be x), and the linears read norm(h) * weight.  Same values as qk_rmsnorm
  * under bfloat16 serving followed by qk_layers_apply_prefill, without the normed rows being written and
- * read back.  Up to 8192 entries per row. */
+ * read back.  Up to 8192 entries per row.  weight is a constant of the model like the layers' scales: it may be read
+ * while the work in front of the call is still running, so that work must not write it. */
 qk_status qk_layers_apply_prefill_normed(qk_ctx *ctx, const qk_layer *const *layers, size_t n_layers,
                                          const float *x, const float *residual, const float *weight, float eps,
                                          float *x_out, size_t n_tokens, float *const *y_devs);

@@ -739,6 +739,10 @@ grouped_portion_umma_kernel(const __grid_constant__ CUtensorMap q_map, const __g
                 if (!ok) continue;
                 asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
                 if (elect_one()) {
+                    // The next scores go over the weights that this product reads.  Nothing waits in between: the
+                    // products of one thread are carried out in the order of issue (the ISA says so for one
+                    // accumulator and shape; that it holds from one accumulator to the next is observed: the
+                    // outputs repeat bit for bit and agree with the row kernels).
                     values(u, j);
                     if (j + 1 < unit[u].n_blocks) scores(u, j + 1);
                     else umma_commit(o_full + u);
