@@ -41,12 +41,22 @@ constexpr int kQT = 64;  // queries per block (4 lanes each)
 constexpr int kTK = 32;  // keys per shared-memory tile
 
 // ------------------------------------------------------------------ exact attention
-// The rows of one block; kMarked: only those whose bit of `rows` is set, and a value that a row does not see is not
-// multiplied with its weight of zero either (it may be an infinity or NaN).
+// kMarked: only the rows that attention_split_exact has marked, after it on the stream.  Nearly always there are
+// none: a block reads two words and leaves: 32 heads of 128 on 2048 tokens, causal, 166 us with this launch, 168 when
+// the rows were recomputed by the warps that found them; with every row marked 3080 us, 2958 by this kernel alone.
 template <int DPL, bool kMarked>
-__device__ __forceinline__ void exact_rows(const float *__restrict__ q, const float *__restrict__ k,
-                                           const float *__restrict__ v, float *__restrict__ out, const AttnDims &dm,
-                                           int causal, uint64_t rows) {
+__global__ void __launch_bounds__(256)
+attention_exact_kernel(const float *__restrict__ q, const float *__restrict__ k,
+                       const float *__restrict__ v, float *__restrict__ out, AttnDims dm,
+                       int causal, const uint32_t *marked) {
+    [[maybe_unused]] uint64_t rows = 0;
+    if constexpr (kMarked) {
+        qk::pdl_wait();
+        const uint2 bits = *reinterpret_cast<const uint2 *>(
+            marked + (((size_t)blockIdx.z * dm.H + blockIdx.y) * ((dm.Sq + 127) / 128) + blockIdx.x / 2) * 4 + (blockIdx.x & 1) * 2);
+        rows = (uint64_t)bits.y << 32 | bits.x;
+        if (!rows) return;
+    }
     constexpr int PITCH = DPL + 4;  // +4 floats: the four parts of a key land in distinct banks
     extern __shared__ float sm[];
     float *Ks = sm, *Vs = sm + kTK * 4 * PITCH;
@@ -107,6 +117,7 @@ __device__ __forceinline__ void exact_rows(const float *__restrict__ q, const fl
         for (int e = 0; e < DPL; ++e) o[e] *= alpha;
 #pragma unroll
         for (int kk = 0; kk < kTK; ++kk) {
+            // (a value that a row does not see is not multiplied with its weight of zero: it may be an infinity or NaN)
             if (kMarked && j0 + kk > last_key) break;
             const float p = expf(s[kk] - m_new);
             l += p;
@@ -124,28 +135,6 @@ __device__ __forceinline__ void exact_rows(const float *__restrict__ q, const fl
             if (c < (int)dm.dv) orow[c] = o[e] / l;  // a row with no admissible key is 0/0 = NaN
         }
     }
-}
-
-template <int DPL>
-__global__ void __launch_bounds__(256)
-attention_exact_kernel(const float *__restrict__ q, const float *__restrict__ k,
-                       const float *__restrict__ v, float *__restrict__ out, AttnDims dm,
-                       int causal) {
-    exact_rows<DPL, false>(q, k, v, out, dm, causal, 0);
-}
-
-// The rows that attention_split_exact has marked, after it on the stream.  Nearly always there are none: a block
-// reads two words and leaves: 32 heads of 128 on 2048 tokens, causal, 166 us with this launch, 168 when the rows
-// were recomputed by the warps that found them.  With every row marked 3080 us, 2958 by attention_exact_kernel alone.
-template <int DPL>
-__global__ void __launch_bounds__(256)
-attention_marked_kernel(const float *__restrict__ q, const float *__restrict__ k, const float *__restrict__ v,
-                        float *__restrict__ out, AttnDims dm, int causal, const uint32_t *marked) {
-    qk::pdl_wait();
-    const uint32_t tiles = (dm.Sq + 127) / 128;
-    const uint2 bits = *reinterpret_cast<const uint2 *>(
-        marked + (((size_t)blockIdx.z * dm.H + blockIdx.y) * tiles + blockIdx.x / 2) * 4 + (blockIdx.x & 1) * 2);
-    if (bits.x | bits.y) exact_rows<DPL, true>(q, k, v, out, dm, causal, (uint64_t)bits.y << 32 | bits.x);
 }
 
 // ------------------------------------------------------------------ Sage quantisers
@@ -1708,19 +1697,19 @@ qk_status launch_exact(qk_ctx *c, const float *q, const float *k, const float *v
                        const AttnDims &dm, int causal, const uint32_t *marked) {
     size_t smem = 2 * kTK * 4 * (DPL + 4) * sizeof(float);
     if (smem > 48 * 1024)
-        QK_CUDA(cudaFuncSetAttribute(attention_exact_kernel<DPL>,
+        QK_CUDA(cudaFuncSetAttribute(attention_exact_kernel<DPL, false>,
                                      cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     dim3 grid((unsigned)qk::ceil_div(dm.Sq, kQT), dm.H, dm.B);
     if constexpr (DPL <= 32) {  // (head sizes that attention_split_exact takes)
         if (marked) {
-            (void)qk::launch_pdl(c->pdl, attention_marked_kernel<DPL>, grid, dim3(256), smem, c->stream, q, k, v, out, dm,
+            (void)qk::launch_pdl(c->pdl, attention_exact_kernel<DPL, true>, grid, dim3(256), smem, c->stream, q, k, v, out, dm,
                                  causal, marked);
             QK_CUDA(cudaGetLastError());
             c->launches++;
             return QK_OK;
         }
     }
-    attention_exact_kernel<DPL><<<grid, 256, smem, c->stream>>>(q, k, v, out, dm, causal);
+    attention_exact_kernel<DPL, false><<<grid, 256, smem, c->stream>>>(q, k, v, out, dm, causal, nullptr);
     QK_CUDA(cudaGetLastError());
     c->launches++;
     return QK_OK;

@@ -15,7 +15,7 @@
 // units; d channels of two operands of at most 2^15, off by 2^-25), each output channel at most
 // (1 + 2 n / l) 2^-25 of its multiplier (v off by 2^-25; n weights of at most 2^14, off by 2^-25, on values of
 // at most 2^15).  Where the first exceeds 2^-21 and 2^-21 of the row's largest score, or the second 2^-21 of the
-// row's largest output, the row is marked, and attention_marked_kernel (qk_attention.cu) computes it again
+// row's largest output, the row is marked, and attention_exact_kernel (qk_attention.cu) computes it again
 // by float32 multiply-adds, as it does rows that are not finite (infinities or NaN among their operands, an
 // overflow).  For normal operands both stay below that by a factor of a hundred; one entry of 10^4 among
 // values of 1 is where marks begin.
@@ -600,6 +600,11 @@ bool attention_split_takes(qk_ctx *c, const qk_attention_shape *s, int causal) {
     // Below 192 keys the float32 kernel is the more exact one (error against 64 bits at 128 keys 1.7e-7 to
     // 2.5e-7 there, 1.8e-7 to 2.6e-7 here; from 192 on equal, at 2048 4.8e-7 and 3.1e-7).
     if (s->seq_kv < 192) return false;
+    // Heads of up to 16 channels are padded to 64 here and cost the float32 kernel a quarter of what 64 do: up to 255
+    // keys they stay there (16 channels, 32 heads: 192 tokens 16.5 against 17.9 us, one query row on 192 keys in a batch
+    // of four 14.4 against 21.7; 256 tokens 22.6 against 18.1).  So do one to three value channels, where an output
+    // near zero marks its row (one channel, 32 heads, 384 tokens: 43 against 48 us).
+    if ((std::max(s->head_dim, s->val_dim) <= 16 && s->seq_kv < 256) || s->val_dim < 4) return false;
     if (ceil_div(s->seq_q, kRows) > 65535 || s->batch * s->n_kv_heads > 65535 || s->seq_kv > (1u << 30)) return false;
     // (a captured graph may be replayed after the scratch has moved: a recording keeps the plain kernel)
     return !capturing(c);

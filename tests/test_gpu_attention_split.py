@@ -153,23 +153,30 @@ def test_exact_face_of_2048_keys(ctx, causal):
     assert float((y - want).abs().max()) < 2e-6 * float(want.abs().max())
 
 
+@pytest.mark.parametrize("d,dv,Sk", [(16, 16, 255), (16, 16, 256), (17, 16, 192), (8, 3, 600), (8, 4, 600), (2, 1, 600)])
+def test_exact_face_where_its_kernels_meet(ctx, d, dv, Sk):
+    """Small heads, around the sizes from which the tensor-core form takes them.  (Outputs of few channels lie near zero at
+    times: the error is held against the head's largest.)"""
+    test_exact_face_at_the_edges_of_tiles(ctx, 4, 2, Sk - 65, Sk, d, dv, True)
+
+
 def test_exact_face_without_room_for_the_terms(ctx):
-    """Heads of one channel, padded to 64: the terms would take 251 GB where k and v take 4.  The call goes through all
+    """Heads of four channels, padded to 64: the terms would take 210 GB where k and v take 13.  The call goes through all
     the same, and so does the next."""
     import torch
-    B, n = 60000, 8192
+    B, n, d = 50000, 8192, 4
     gen = torch.Generator("cuda").manual_seed(12)
-    k, v = (torch.randn(B, n, device="cuda", generator=gen) for _ in range(2))
-    q, y = torch.randn(B, device="cuda", generator=gen), torch.full((B,), math.nan, device="cuda")
+    k, v = (torch.randn(B, n, d, device="cuda", generator=gen) for _ in range(2))
+    q, y = torch.randn(B, d, device="cuda", generator=gen), torch.full((B, d), math.nan, device="cuda")
     torch.cuda.synchronize()
-    ctx.attention_dev(AttentionShape(B, 1, 1, 1, n, 1, 1), q.data_ptr(), k.data_ptr(), v.data_ptr(), False, y.data_ptr())
+    ctx.attention_dev(AttentionShape(B, 1, 1, 1, n, d, d), q.data_ptr(), k.data_ptr(), v.data_ptr(), False, y.data_ptr())
     ctx.synchronize()
     some = slice(None, None, 61)
-    weights = torch.softmax(q[some, None].double() * k[some].double(), -1)
-    want = (weights * v[some]).sum(-1)
+    weights = torch.softmax(torch.einsum("bd,bnd->bn", q[some].double(), k[some].double()) / 2, -1)[..., None]
+    want = (weights * v[some]).sum(1)
     # (8192 additions in turn, each off by half a unit of the running sum: of the weights, and of the products)
     assert bool(torch.isfinite(y).all())
-    assert bool(((y[some] - want).abs() <= 2 * n * 2.0 ** -24 * (weights * v[some].abs()).sum(-1)).all())
+    assert bool(((y[some] - want).abs() <= 2 * n * 2.0 ** -24 * (weights * v[some].abs()).sum(1)).all())
     test_exact_face_at_the_edges_of_tiles(ctx, 1, 1, 257, 257, 64, 64, True)
 
 
