@@ -792,6 +792,16 @@ grouped_portion_umma_kernel(const __grid_constant__ CUtensorMap q_map, const __g
 #pragma unroll
             for (int c = 0; c < 4; ++c) tmem_ld32(s_tmem + 32 * c, raw[c]);
             tmem_ld_wait();
+            // whether a block that holds unseen keys has a score that is not finite (its product with zero is not zero)
+            bool strange = false;
+            if (nearest < 0) {
+                float2 odd[2] = {make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+#pragma unroll
+                for (int e = 0; e < kUmKeys / 2; ++e)
+                    odd[e % 2] = __ffma2_rn(make_float2(__uint_as_float(raw[e / 16][e % 16 * 2]), __uint_as_float(raw[e / 16][e % 16 * 2 + 1])),
+                                            make_float2(0.f, 0.f), odd[e % 2]);
+                strange = __any_sync(0xffffffffu, !(odd[0].x + odd[0].y + odd[1].x + odd[1].y == 0.f));
+            }
             const float2 f2 = make_float2(factor, factor);
             float mx[4] = {-INFINITY, -INFINITY, -INFINITY, -INFINITY};
             if (near) {
@@ -813,7 +823,7 @@ grouped_portion_umma_kernel(const __grid_constant__ CUtensorMap q_map, const __g
                     s[e] = __ffma2_rn(make_float2(__uint_as_float(raw[e / 16][e % 16 * 2]), __uint_as_float(raw[e / 16][e % 16 * 2 + 1])),
                                       f2, b2);
             }
-            if (nearest < 0) {  // (the band's -inf does not hide an infinity or NaN)
+            if (__builtin_expect(strange, 0)) {  // (the band's -inf does not hide an infinity or NaN)
                 const int seen = pos - (int)(j * kUmKeys);
 #pragma unroll
                 for (int e = 0; e < kUmKeys / 2; ++e) {

@@ -958,10 +958,13 @@ qk_status qk_window_attention(qk_ctx *ctx, const void *q, size_t q_stride, const
                         key0, key0 + n_keys - 1, first_position, first_position + tokens - 1);
     // A window that hides nothing leaves causal attention, which the tcgen05 portion kernel does; the band below is
     // bound by mma.sync and its fragments' loads (2048-token prompt through four such layers, 32 heads of 128:
-    // 8315 -> 7685 us, 240 -> 80 us a call; 20 tokens 1030 -> 928 us: it pays from the shortest portions on).  It needs
-    // the context's error word, which a call that is being recorded cannot allocate.
+    // 8315 -> 7685 us, 240 -> 80 us a call; 20 tokens 1030 -> 928 us).  Up to eight rows against few keys stay with the band,
+    // whose tiles are half as large: 32 heads, one row: 61 keys of 128 channels 5.7 against 7.3 us, 126 keys 8.0 against
+    // 7.3; eight rows: 133 keys of 64 channels 7.6 against 8.2, which adds 1.8 us per 64 keys there and 2.1 per 128 here.
+    // It needs the context's error word, which a call that is being recorded cannot allocate.
+    const bool short_call = tokens <= 8 && first_position + tokens <= (std::max(dim_stride, vdim_stride) <= 64 ? 192u : 64u);
     auto aligned = [](const void *p) { return ((uintptr_t)p & 15) == 0; };
-    if (key0 == 0 && window >= first_position + tokens && vdim == vdim_stride && dim_stride % 16 == 0 &&
+    if (key0 == 0 && window >= first_position + tokens && !short_call && vdim == vdim_stride && dim_stride % 16 == 0 &&
         vdim_stride % 16 == 0 && std::min(dim_stride, vdim_stride) >= 64 && std::max(dim_stride, vdim_stride) <= 128 &&
         out_stride % 8 == 0 && aligned(q) && aligned(kv) && aligned(out) && c->decode_attention_kernel != 0 &&
         (c->d_err.ptr || !qk::capturing(c)))

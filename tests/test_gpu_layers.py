@@ -257,7 +257,8 @@ def test_window_attention_expanded(dev, dim, vdim, window, p0, tokens):
 
 @pytest.mark.parametrize("dim,vdim,window,p0,tokens", [
     (64, 64, 1000, 0, 17), (128, 128, 300, 44, 256), (128, 128, 299, 44, 256), (80, 112, 2048, 0, 257),
-    (64, 128, 600, 300, 129), (128, 64, 385, 0, 385)])
+    (64, 128, 600, 300, 129), (128, 64, 385, 0, 385), (64, 64, 500, 184, 8), (64, 64, 500, 185, 8), (128, 128, 99, 56, 8),
+    (128, 128, 99, 57, 8), (128, 128, 99, 55, 9), (128, 128, 99, 0, 1)])
 def test_window_that_hides_nothing(dev, dim, vdim, window, p0, tokens):
     """A window as long as the sequence is causal attention and takes the tcgen05 kernel; one entry shorter it takes the
     band.  Tiles of 128 rows and 128 keys and one more, head sizes off the 64-channel chunks, the same gate."""
