@@ -29,7 +29,8 @@
 // at 1.45 GHz under the power cap, i.e. 1.6 PFLOP/s inside the loops, which is what cuBLAS reaches.  The
 // producers' positions used to cost three divisions per chunk and the copies waited behind the
 // expansion: 890 clocks.  Around the loops come 5 us of launch and first fetch per kernel and the last tile.
-// 14336 x 4096 of rank 2560 on 2048 tokens: 209 -> 162 us, 4096 x 4096 of rank 1102 on 64 tokens 29.7 -> 24.5 us.
+// 14336 x 4096 of rank 2560 on 2048 tokens: 213 -> 171 us a call in a burst of 20, 234 -> 192 back to back for a second,
+// under the power cap; 4096 x 4096 of rank 1102 on 64 tokens 29.7 -> 24.5 us.
 // Pairs of CTAs sharing the token tile (cta_group::2) came out no faster: 172 against 172 us.
 // All hand-offs go through mbarriers.  Every wait is bounded: on expiry the kernel waits for its
 // own copies and products in flight, records an error code, frees its tensor memory and returns,
@@ -823,6 +824,7 @@ unsigned plan_ctas(GemmArgs &g, size_t units, const size_t *tiles, size_t n_prob
 // rank 1102 on 256 tokens: 40 us with the widest tile, 29 with the one chosen here).
 uint32_t pick_bn(const GemmArgs &g, size_t n_problems, size_t tokens, unsigned sm_count) {
     const uint32_t widest = (uint32_t)std::min<size_t>(kBNMax, qk::ceil_div(tokens, 16) * 16);
+    if (widest <= 32) return widest;
     uint32_t best = widest;
     uint64_t best_cost = ~0ull;
     for (uint32_t bn : {widest, 128u, 64u, 32u}) {
