@@ -179,7 +179,7 @@ qk_status qk_gpu_sage_quantize(qk_ctx *ctx, const qk_attention_shape *shape, con
  * context's stream: for callers whose q, k, v already live on the GPU (a resident prefill).
  * Additive; the reference's API has only the host-slice forms above.
  *
- * The exact face has two kernels.  From 192 keys on, heads of up to 128 channels run on the tensor cores with q, k, v
+ * The exact face has two kernels.  From 192 keys on (256 for heads of up to 16 channels), heads of up to 128 channels run on the tensor cores with q, k, v
  * as sums of 16-bit terms (as exact as float32 arithmetic, other last bits); the terms of k and v live in the
  * context, in a buffer as large as the largest k and v so far (heads padded to 64 or 128 channels), until
  * qk_gpu_free.  Where that buffer cannot be had, and while a stream capture records the call (a graph may
