@@ -793,7 +793,8 @@ size_t qk_grouped_scratch(size_t tokens, size_t heads, size_t kv_heads, size_t v
 qk_status qk_grouped_portion(qk_ctx *ctx, const qk_grouped_call *call);
 
 /* Which GEMV kernel qk_layer_apply and the group calls use: 0 = sign-select SIMT, 1 = bit-sliced
- * INT8 tensor-core (default; many instances per launch run in the persistent streaming form),
+ * INT8 tensor-core (default; many instances per launch run in the persistent streaming form, few and
+ * small ones as integer sums with the same bits),
  * 3 = the same without the split-k form, 5 = the same with one block per instance instead of
  * the streaming form, 2 and 4 = as 5 with 16-warp resp. 4-warp blocks (measurement variants).
  * Returns the previous value; values out of range leave it unchanged. */

@@ -109,6 +109,7 @@ struct qk_group {
     size_t n_inst = 0;
     qk_layer shape;          // dimensions/strides of the member layers (the largest, if they differ)
     bool mixed = false;      // the members differ in shape: few-instance form only
+    size_t rows1 = 0, rows2 = 0;  // rows of the two stages over all members (plans)
     bool fed = false;        // the stage-1 tables are written by the kernels that produce the inputs
     bool normed = false;     // stage 1 applies an RMSNorm to its input itself (qk_plan_set_norm)
     bool pushed = false;     // the last stage pushes its outputs into all-reduce inboxes (qk_plan_set_allreduce)

@@ -23,6 +23,9 @@
 // conversion (relative 2^-47 of max|v|) and one rounding of the final sum: closer to
 // the exact sum than the reference's own float64 left-to-right loop.
 //
+// A launch of few and small instances is a chain of latencies, not a stream: it adds up the same whole numbers without
+// digits (qk_gemv_sum.cuh).
+//
 // Data layout in HBM (built once by qk_layer_create):
 //   * tiles: the factor's rows are cut into groups of 64 rows and k-steps of 512 bits.
 //     One (group, k-step) pair is a 4 KB chunk holding four 16-row x 512-bit tiles;
@@ -32,12 +35,13 @@
 //     index h*32 + 4*g + t, so lane (g,t) of a warp moves its own eight pieces of a
 //     chunk with eight fully coalesced 512-byte warp transfers.  Rows are padded to a
 //     multiple of 64 and bits to a multiple of 512 with zeros.
-//   * rows: the reference's per-row bitplanes padded to 16-byte rows; only the
-//     sign-select kernel reads it.
+//   * rows: the reference's per-row bitplanes padded to 16-byte rows; the sums and the
+//     sign-select kernel read it.
 //
 // Rounding points follow the reference: fp32 serving forms z = s2*x in float32 and
 // keeps t and u in float64 between the stages; bf16 serving rounds z, t and u to
 // bfloat16 exactly where apply_bf16 does.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <type_traits>
@@ -307,6 +311,12 @@ __device__ __forceinline__ void load_record(const StageParams &p, uint32_t r, ui
     else
         load_inputs<kInDouble, kRoundBf16, 8, Out>(p, index_of, n_bits, r < n_records, out);
 }
+
+}  // namespace
+
+#include "qk_gemv_sum.cuh"
+
+namespace {
 
 // Converts one instance's input vector to its digit table.
 //   kInDouble: the input is the float64 intermediate of the previous stage.
@@ -1786,12 +1796,85 @@ StagePlan plan_stage(const qk_ctx *c, const StageShape &s, size_t n_inst) {
     return pl;
 }
 
+// How a stage is cut for the few-instance form by sums.  total_rows: over all instances.
+struct SumPlan {
+    bool fits;
+    uint32_t rows, slice, ranks;
+    size_t blocks, smem;
+};
+constexpr size_t kSumSmem = 116 * 1024;  // at least: more than half of an SM's, so that it holds one block
+// Most weights of a launch (rows x entries over its instances).  The sums' time grows with them, by 0.24 us a million
+// (bfloat16 serving 0.2), from 2.6 us on; the digit form takes 5 to 10 us for its tables and 0.07 to 0.16 us a million after
+// that.  Measured, us a call, digits -> sums, float32 serving: 4096 x 4096 of rank 1024 on 1, 2, 3, 5 tokens 13.4 -> 8.3,
+// 14.1 -> 9.5, 14.3 -> 11.0, 17.0 -> 13.7 (21e6 weights a stage), on 8 tokens (34e6) 17.6 -> 27; 8192 x 3000 of rank 2560 on one token
+// (21e6) 16.0 -> 12.6; 14336 x 14336 of rank 2560 (37e6) 22.5 -> 22.9, bfloat16 serving 23.5 -> 20.7.  Where many
+// instances share the machine, the second stage's short tables cost little: 2048 outputs of rank 800 on 12 tokens (20e6)
+// take 6 us longer by sums, 1024 of rank 300 on 32 (10e6) 3 us less.
+double sum_most_weights(size_t n_inst, bool final, bool bf16) {
+    if (final && n_inst > 8) return 14e6;
+    return bf16 && n_inst <= 2 ? 50e6 : 30e6;
+}
+SumPlan sum_plan(const qk_ctx *c, const StageShape &s, size_t n_inst, size_t total_rows, bool final, bool bf16,
+                 bool normed = false) {
+    SumPlan pl{};
+    pl.ranks = (uint32_t)qk::ceil_div(s.n_bits, (size_t)kSumSlice);
+    if (c->gemv_kernel != 1 || pl.ranks > 8u || (normed && s.n_bits > 8 * kSumThreads) || s.n_groups > 65535 ||
+        (double)total_rows * (double)s.n_bits > sum_most_weights(n_inst, final, bf16))
+        return pl;
+    pl.slice = pl.ranks == 1 ? (uint32_t)s.n_bits
+                             : (uint32_t)(qk::ceil_div(qk::ceil_div(s.n_bits, (size_t)pl.ranks), (size_t)128) * 128);
+    // one wave of blocks, one per SM: rows enough that the instances' blocks together are no more
+    const size_t room = (size_t)c->sm_count / pl.ranks;
+    if (n_inst * 2 > room) return pl;
+    pl.rows = (uint32_t)std::max<size_t>(1, total_rows == n_inst * s.n_rows ? qk::ceil_div(s.n_rows, room / n_inst)
+                                                                           : qk::ceil_div(total_rows, room - n_inst));
+    // (an entry is float64 where it is the second stage's intermediate and not rounded to bfloat16)
+    pl.smem = std::max((size_t)sum_layout(pl.slice, pl.rows, final && !bf16 ? 8 : 4).bytes, kSumSmem);
+    pl.blocks = qk::ceil_div(s.n_rows, (size_t)pl.rows) * pl.ranks;
+    pl.fits = pl.smem <= kSmemBudget;
+    return pl;
+}
+
+// many: the instances' records on the device; or null, and the instances are the tokens of `run`.
+template <bool kFinal>
+qk_status launch_sums(qk_ctx *c, const StageParams *many, size_t n_inst, const SumPlan &pl, bool bf16,
+                      const StageRun &run = StageRun{}) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3((unsigned)pl.blocks, (unsigned)n_inst);
+    cfg.blockDim = dim3(kSumThreads);
+    cfg.dynamicSmemBytes = pl.smem;
+    cfg.stream = c->stream;
+    cudaLaunchAttribute attr[2];
+    attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[0].val.programmaticStreamSerializationAllowed = c->pdl ? 1 : 0;
+    attr[1].id = cudaLaunchAttributeClusterDimension;
+    attr[1].val.clusterDim.x = pl.ranks;
+    attr[1].val.clusterDim.y = 1;
+    attr[1].val.clusterDim.z = 1;
+    cfg.attrs = attr;
+    cfg.numAttrs = pl.ranks > 1 ? 2 : 1;
+    qk_status st;
+    if (many) {
+        auto kern = bf16 ? gemv_sum_kernel<true, kFinal> : gemv_sum_kernel<false, kFinal>;
+        if ((st = qk::allow_smem(c, kern, kSmemBudget)) != QK_OK) return st;
+        QK_CUDA(cudaLaunchKernelEx(&cfg, kern, many, pl.rows, pl.slice));
+    } else {
+        auto kern = bf16 ? gemv_sum_run_kernel<true, kFinal> : gemv_sum_run_kernel<false, kFinal>;
+        if ((st = qk::allow_smem(c, kern, kSmemBudget)) != QK_OK) return st;
+        QK_CUDA(cudaLaunchKernelEx(&cfg, kern, run, pl.rows, pl.slice));
+    }
+    c->launches++;
+    return QK_OK;
+}
+
 bool fed_plan_fits(const qk_ctx *c, const StageShape &s, size_t n_inst, size_t *warps, size_t *smem);
 constexpr size_t kSpreadTableSteps = 16;  // k-steps (of 512 inputs) from which the few-instance form gets its table made once
 
 // Whether a stage can take its records with the launch: every form but those whose table a kernel of its own makes.
-bool run_fits(const qk_ctx *c, const StageShape &s, size_t n_inst) {
-    return plan_stage(c, s, n_inst).smem_digits && s.n_steps < kSpreadTableSteps;
+bool run_fits(const qk_ctx *c, const StageShape &s, size_t n_inst, bool final, bool bf16) {
+    const StagePlan pl = plan_stage(c, s, n_inst);
+    return (pl.smem_digits && s.n_steps < kSpreadTableSteps) ||
+           (n_inst * pl.blocks < (size_t)c->sm_count && sum_plan(c, s, n_inst, n_inst * s.n_rows, final, bf16).fits);
 }
 
 // many: the instances' records on the device; or null, and the instances are the tokens of `run` (run_fits).
@@ -1807,6 +1890,10 @@ qk_status launch_bitslice(qk_ctx *c, const StageParams *many, size_t n_inst, con
     while (sk_warps > 4 && sk_bytes(sk_warps) > kSmemBudget) --sk_warps;
     const size_t sk_smem = sk_bytes(sk_warps);
     const bool few = c->gemv_kernel != 3 && n_inst * pl.blocks < (size_t)c->sm_count && s.n_groups <= 65535;
+    if (few && !need_few) {
+        const SumPlan sums = sum_plan(c, s, n_inst, n_inst * s.n_rows, kFinal, bf16);
+        if (sums.fits) return launch_sums<kFinal>(c, many, n_inst, sums, bf16, run);
+    }
     // A long input vector (the down projection's 14336 entries): every block of the few-instance
     // form would build the whole digit table for itself, about 10 us of the kernel's 16.  The
     // table is built once instead, by a small grid of its own that shares out the records, and
@@ -1992,7 +2079,11 @@ bool mixed_plan_fits(const qk_ctx *c, const StageShape &s, size_t n_inst, size_t
 
 template <bool kFinal>
 qk_status launch_mixed_stage(qk_ctx *c, const StageParams *many, size_t n_inst, const StageShape &s,
-                             bool bf16) {
+                             bool bf16, size_t total_rows, bool pushed = false) {
+    if (!pushed) {
+        const SumPlan sums = sum_plan(c, s, n_inst, total_rows, kFinal, bf16);
+        if (sums.fits) return launch_sums<kFinal>(c, many, n_inst, sums, bf16);
+    }
     size_t warps, smem;
     if (!mixed_plan_fits(c, s, n_inst, &warps, &smem))
         return qk::fail(QK_ERR_VALUE, "a plan of mixed shapes must fit the few-instance form");
@@ -2036,7 +2127,12 @@ bool normed_plan_fits(const qk_ctx *c, const StageShape &s, size_t n_inst, size_
     return *smem <= kSmemBudget && s.n_bits <= 16 * 512 && s.n_groups <= 65535 && n_inst <= 65535 &&
            n_inst * s.n_groups <= 8 * (size_t)c->sm_count;
 }
-qk_status launch_normed_stage1(qk_ctx *c, const StageParams *many, size_t n_inst, const StageShape &s, bool bf16) {
+qk_status launch_normed_stage1(qk_ctx *c, const StageParams *many, size_t n_inst, const StageShape &s, bool bf16,
+                               size_t total_rows, bool gathered) {
+    if (!gathered) {
+        const SumPlan sums = sum_plan(c, s, n_inst, total_rows, false, bf16, true);
+        if (sums.fits) return launch_sums<false>(c, many, n_inst, sums, bf16);
+    }
     size_t smem;
     if (!normed_plan_fits(c, s, n_inst, &smem))
         return qk::fail(QK_ERR_VALUE, "a normed plan must fit the few-instance form");
@@ -2050,22 +2146,25 @@ qk_status launch_normed_stage1(qk_ctx *c, const StageParams *many, size_t n_inst
 }
 
 qk_status launch_both(qk_ctx *c, const qk_layer *l0, const StageParams *d, size_t n_inst,
-                      int kernel, bool mixed = false, bool fed = false, bool normed = false, bool pushed = false) {
+                      int kernel, const qk_group *plan = nullptr) {
+    const bool mixed = plan && plan->mixed, fed = plan && plan->fed, normed = plan && plan->normed,
+               pushed = plan && plan->pushed;
+    const size_t rows1 = plan ? plan->rows1 : 0, rows2 = plan ? plan->rows2 : 0;  // (read for plans only)
     if (pushed && !normed && !fed) {
         // (the last stage pushes into the all-reduce inboxes: only the few-instance kernel does)
         const bool bf16 = l0->serving == QK_BF16;
-        qk_status e = mixed ? launch_mixed_stage<false>(c, d, n_inst, stage1_shape(l0), bf16)
+        qk_status e = mixed ? launch_mixed_stage<false>(c, d, n_inst, stage1_shape(l0), bf16, rows1)
                             : launch_bitslice<false>(c, d, n_inst, stage1_shape(l0), bf16);
         if (e != QK_OK) return e;
-        if (mixed) return launch_mixed_stage<true>(c, d + n_inst, n_inst, stage2_shape(l0), bf16);
+        if (mixed) return launch_mixed_stage<true>(c, d + n_inst, n_inst, stage2_shape(l0), bf16, rows2, true);
         return launch_bitslice<true>(c, d + n_inst, n_inst, stage2_shape(l0), bf16, true);
     }
     if (pushed) return qk::fail(QK_ERR_VALUE, "a normed or fed plan cannot push into an all-reduce");
     if (normed) {
         const bool bf16 = l0->serving == QK_BF16;
-        qk_status e = launch_normed_stage1(c, d, n_inst, stage1_shape(l0), bf16);
+        qk_status e = launch_normed_stage1(c, d, n_inst, stage1_shape(l0), bf16, rows1, plan->gathered);
         if (e != QK_OK) return e;
-        if (mixed) return launch_mixed_stage<true>(c, d + n_inst, n_inst, stage2_shape(l0), bf16);
+        if (mixed) return launch_mixed_stage<true>(c, d + n_inst, n_inst, stage2_shape(l0), bf16, rows2);
         return launch_bitslice<true>(c, d + n_inst, n_inst, stage2_shape(l0), bf16);
     }
     if (fed) {
@@ -2075,9 +2174,9 @@ qk_status launch_both(qk_ctx *c, const qk_layer *l0, const StageParams *d, size_
     }
     if (mixed) {
         // l0 holds the largest din, r and dout over the instances
-        qk_status e = launch_mixed_stage<false>(c, d, n_inst, stage1_shape(l0), l0->serving == QK_BF16);
+        qk_status e = launch_mixed_stage<false>(c, d, n_inst, stage1_shape(l0), l0->serving == QK_BF16, rows1);
         if (e != QK_OK) return e;
-        return launch_mixed_stage<true>(c, d + n_inst, n_inst, stage2_shape(l0), l0->serving == QK_BF16);
+        return launch_mixed_stage<true>(c, d + n_inst, n_inst, stage2_shape(l0), l0->serving == QK_BF16, rows2);
     }
     const bool bf16 = l0->serving == QK_BF16;
     const StageShape s1 = stage1_shape(l0), s2 = stage2_shape(l0);
@@ -2143,11 +2242,11 @@ qk_status apply_group(qk_ctx *c, const qk_layer *const *layers, size_t n_layers,
     const InstanceScratch sc = scratch_of(l0);
     if ((st = c->d_t.reserve(n_inst * sc.total)) != QK_OK) return st;
     const StageShape s1 = stage1_shape(l0), s2 = stage2_shape(l0);
-    if (n_layers == 1 && c->gemv_kernel == 1 && n_tokens < (size_t)c->sm_count && run_fits(c, s1, n_tokens) &&
-        run_fits(c, s2, n_tokens)) {
+    const bool bf16 = l0->serving == QK_BF16;
+    if (n_layers == 1 && c->gemv_kernel == 1 && n_tokens < (size_t)c->sm_count && run_fits(c, s1, n_tokens, false, bf16) &&
+        run_fits(c, s2, n_tokens, true, bf16)) {
         StageParams h[2];
         fill_params(h, layers, 1, 1, x_dev, y_dev, (uint8_t *)c->d_t.ptr, 0, 0);
-        const bool bf16 = l0->serving == QK_BF16;
         const StageRun first{h[0], l0->din * sizeof(float), sc.total}, last{h[1], sc.total, l0->dout * sizeof(float)};
         if ((st = launch_bitslice<false>(c, nullptr, n_tokens, s1, bf16, false, first)) != QK_OK) return st;
         return launch_bitslice<true>(c, nullptr, n_tokens, s2, bf16, false, last);
@@ -2426,6 +2525,7 @@ qk_status qk_group_create(qk_ctx *ctx, const qk_layer *const *layers, size_t n_l
     g->device = c->device;
     g->n_inst = n_layers;
     g->shape = *l0;  // dimensions and strides only; the pointers are not used
+    g->rows1 = n_layers * l0->r, g->rows2 = n_layers * l0->dout;
     const InstanceScratch sc = scratch_of(l0);
     cudaError_t e = cudaMalloc(&g->scratch, n_layers * sc.total);
     if (e == cudaSuccess) e = cudaMalloc(&g->params, 2 * n_layers * sizeof(StageParams));
@@ -2494,6 +2594,7 @@ static qk_status plan_create(qk_ctx *ctx, const qk_layer *const *layers, const f
     g->n_inst = n_inst;
     g->shape = widest;  // dimensions only (the largest over the instances); the pointers are not used
     g->mixed = mixed;
+    for (size_t i = 0; i < n_inst; ++i) g->rows1 += layers[i]->r, g->rows2 += layers[i]->dout;
     cudaError_t e = cudaMalloc(&g->scratch, n_inst * slice);
     if (e == cudaSuccess) e = cudaMalloc(&g->params, 2 * n_inst * sizeof(StageParams));
     if (e != cudaSuccess) {
@@ -2687,7 +2788,7 @@ qk_status qk_group_apply(qk_ctx *ctx, const qk_group *group) {
         }
     }
     return launch_both(c, &group->shape, (const StageParams *)group->params, group->n_inst,
-                       c->gemv_kernel, group->mixed, group->fed, group->normed, group->pushed);
+                       c->gemv_kernel, group);
 }
 
 qk_status qk_groups_apply_host(qk_ctx *ctx, const qk_group *const *groups, const size_t *first_row,
@@ -2730,7 +2831,7 @@ qk_status qk_groups_apply_host(qk_ctx *ctx, const qk_group *const *groups, const
         QK_CUDA(cudaEventRecord(uploaded, c->up_stream));
         QK_CUDA(cudaStreamWaitEvent(c->stream, uploaded, 0));
         st = launch_both(c, &groups[p]->shape, (const StageParams *)groups[p]->params, groups[p]->n_inst,
-                         c->gemv_kernel, groups[p]->mixed, groups[p]->fed);
+                         c->gemv_kernel, groups[p]);
         if (st != QK_OK) return st;
         QK_CUDA(cudaEventRecord(computed, c->stream));
         QK_CUDA(cudaStreamWaitEvent(c->down_stream, computed, 0));

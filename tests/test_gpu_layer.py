@@ -550,3 +550,47 @@ def test_tokens_of_one_layer_match_single_tokens_and_a_group(gpu_ctx, shape, n_t
     gpu_ctx.synchronize()
     assert bool(torch.isfinite(y).all())
     assert torch.equal(y, single) and torch.equal(y, grouped)
+
+
+@pytest.mark.parametrize("serving", ["float32", "bfloat16"])
+@pytest.mark.parametrize("shape", [(1, 1, 1), (33, 511, 129), (150, 512, 16), (77, 4097, 513), (40, 8192, 300), (300, 8193, 90),
+                                   (37, 20000, 33), (4100, 300, 1030)])
+def test_sums_give_the_bits_of_the_digit_forms(gpu_ctx, shape, serving):
+    """Few instances by sums (the default) against the digit tables (selector 3): entries of ordinary range, over sixty
+    powers of two, subnormal, near the end of float32, all equal, zero.  One whole number either way, hence the
+    same bits; vectors of more than 8192 entries are cut into slices with a grid each, where a float32 result may
+    round the other way."""
+    import torch
+    dout, din, r = shape
+    L = make_layer(dout, din, r, seed=dout + din + r + 1, with_bias=(dout % 2 == 1))
+    layer = PackedLayer(gpu_ctx, L["ub_rows"], L["vb_t_rows"], dout, din, r, L["s1"], L["s2"], L["bias"], serving=serving)
+    rng = np.random.default_rng(sum(shape))
+    x = rng.standard_normal((6, din))
+    x[1] *= 2.0 ** rng.integers(-60, 1, din)
+    x[2] *= 1e-39
+    x[3] *= 1e35
+    x[4] = 0.37
+    x[5] = 0.0
+    xs = torch.from_numpy(x.astype(np.float32)).cuda()
+    out = {}
+    for which in (1, 3):
+        prev = gpu_ctx.set_gemv_kernel(which)
+        try:
+            for n in (1, 6):
+                y = torch.full((6, dout), float("nan"), device="cuda")
+                torch.cuda.synchronize()
+                for first in range(0, 6, n):
+                    layer.apply_device(xs[first].data_ptr(), n, y[first].data_ptr())
+                gpu_ctx.synchronize()
+                out[which, n] = y.cpu().numpy()
+        finally:
+            gpu_ctx.set_gemv_kernel(prev)
+    layer.close()
+    assert np.array_equal(out[1, 1], out[1, 6], equal_nan=True)
+    if din <= 8192:
+        assert np.array_equal(out[1, 1], out[3, 1], equal_nan=True)
+    else:
+        # (the slices' grids are finer than the whole vector's by up to 2^-47 of its largest entry: a rounding to float32
+        # or bfloat16 of t, u or y may turn, by a unit in its last place of the terms' scale)
+        scale = np.abs(out[3, 1]).max(axis=1, keepdims=True)
+        assert (np.abs(out[1, 1] - out[3, 1]) <= (2 ** -8 if serving == "bfloat16" else 2 ** -22) * scale).all()
