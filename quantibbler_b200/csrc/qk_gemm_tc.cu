@@ -689,42 +689,46 @@ __global__ void scale_to_bf16_kernel(const float *__restrict__ x, const float *_
 // store before it), its 34 MB output and the scaling kernel that read it back (27 to 39 us); here all loads
 // of a row go out before the first store.  x, residual: not restrict-qualified, x_out may be x, and a
 // read-only load might be moved above the dependency wait.
-constexpr int kNormThreads = 512, kNormPerThread = 16;
+constexpr int kNormThreads = 512, kNormMost = 16;  // entries a thread at most
 struct NormArgs {
     const float *x, *residual, *weight;
     float *x_out;
     float eps;
 };
-__global__ void __launch_bounds__(kNormThreads, 2)
+// kPer: entries a thread, 8 for rows of up to 4096 and 16 for up to 8192.  With 8, three blocks fit an SM: a block is a
+// chain of latencies (the row, the sum, the stores), and rows in flight are what hides them.
+// An eight-layer prompt of 2048 tokens at width 4096 takes 9690 us with sixteen entries and two blocks, 9381 with these.
+template <int kPer>
+__global__ void __launch_bounds__(kNormThreads, kPer == 8 ? 3 : 2)
 norm_scale_to_bf16_kernel(NormArgs n, ScaleArgs a, uint32_t n_problems, uint32_t d, uint32_t pitch) {
     qk::pdl_launch();
     __shared__ float red[kNormThreads / 32];
-    float w[kNormPerThread], keep[kNormPerThread];
+    float w[kPer], keep[kPer];
 #pragma unroll
-    for (int r = 0; r < kNormPerThread; ++r) {  // (constants of the layer: before the dependency wait)
+    for (int r = 0; r < kPer; ++r) {  // (constants of the layer: before the dependency wait)
         const uint32_t i = threadIdx.x + r * kNormThreads;
         w[r] = i < d ? __ldg(n.weight + i) : 0.f;
     }
     qk::pdl_wait();
     const size_t base = (size_t)blockIdx.x * d;
 #pragma unroll
-    for (int r = 0; r < kNormPerThread; ++r) {
+    for (int r = 0; r < kPer; ++r) {
         const uint32_t i = threadIdx.x + r * kNormThreads;
         keep[r] = i < d ? __ldcg(n.x + base + i) : 0.f;
     }
     if (n.residual) {
-        float more[kNormPerThread];
+        float more[kPer];
 #pragma unroll
-        for (int r = 0; r < kNormPerThread; ++r) {
+        for (int r = 0; r < kPer; ++r) {
             const uint32_t i = threadIdx.x + r * kNormThreads;
             more[r] = i < d ? __ldcg(n.residual + base + i) : 0.f;
         }
 #pragma unroll
-        for (int r = 0; r < kNormPerThread; ++r) keep[r] += more[r];
+        for (int r = 0; r < kPer; ++r) keep[r] += more[r];
     }
     float ss = 0.f;
 #pragma unroll
-    for (int r = 0; r < kNormPerThread; ++r) {
+    for (int r = 0; r < kPer; ++r) {
         const uint32_t i = threadIdx.x + r * kNormThreads;
         if (n.x_out && i < d) n.x_out[base + i] = keep[r];
         keep[r] = round_bf16f(keep[r]);
@@ -732,12 +736,12 @@ norm_scale_to_bf16_kernel(NormArgs n, ScaleArgs a, uint32_t n_problems, uint32_t
     }
     const float inv = 1.0f / sqrtf(block_sum(ss, red) / (float)d + n.eps);
 #pragma unroll
-    for (int r = 0; r < kNormPerThread; ++r) keep[r] = round_bf16f(keep[r] * inv * w[r]);
+    for (int r = 0; r < kPer; ++r) keep[r] = round_bf16f(keep[r] * inv * w[r]);
     for (uint32_t p = 0; p < n_problems; ++p) {
         const float *__restrict__ s2 = a.s2[p];
         uint16_t *z = a.z[p] + (size_t)blockIdx.x * pitch;
 #pragma unroll
-        for (int r = 0; r < kNormPerThread; ++r) {
+        for (int r = 0; r < kPer; ++r) {
             const uint32_t i = threadIdx.x + r * kNormThreads;
             if (i < d) z[i] = (uint16_t)(round_bf16_hi(__float_as_uint(__ldg(s2 + i) * keep[r])) >> 16);
         }
@@ -871,9 +875,9 @@ static qk_status apply_prefill(qk_ctx *ctx, const qk_layer *const *layers, size_
             return qk::fail(QK_ERR_VALUE, "layers of one call share their input: layer %zu has din=%zu, "
                             "layer 0 has din=%zu", i, layers[i]->din, layers[0]->din);
     }
-    if (norm && layers[0]->din > (size_t)kNormThreads * kNormPerThread)
+    if (norm && layers[0]->din > (size_t)kNormThreads * kNormMost)
         return qk::fail(QK_ERR_VALUE, "a normed input of the prefill may have %d entries, got %zu",
-                        kNormThreads * kNormPerThread, layers[0]->din);
+                        kNormThreads * kNormMost, layers[0]->din);
     if (n_tokens == 0) return QK_OK;
     qk_ctx *c;
     qk_status st = qk::resolve_ctx(ctx, &c);
@@ -907,8 +911,9 @@ static qk_status apply_prefill(qk_ctx *ctx, const qk_layer *const *layers, size_
     const int vec = ((uintptr_t)x_dev & 15) == 0 && ((uintptr_t)up_dev & 15) == 0 && (din & 3) == 0;
     const size_t total = n_tokens * (kp1 / 8);
     if (norm)
-        (void)qk::launch_pdl(c->pdl, norm_scale_to_bf16_kernel, dim3((unsigned)n_tokens), dim3(kNormThreads), 0,
-                             c->stream, *norm, sa, (uint32_t)n_layers, (uint32_t)din, (uint32_t)kp1);
+        (void)qk::launch_pdl(c->pdl, din <= 8 * kNormThreads ? norm_scale_to_bf16_kernel<8> : norm_scale_to_bf16_kernel<16>,
+                             dim3((unsigned)n_tokens), dim3(kNormThreads), 0, c->stream, *norm, sa, (uint32_t)n_layers,
+                             (uint32_t)din, (uint32_t)kp1);
     else
         (void)qk::launch_pdl(c->pdl, scale_to_bf16_kernel,
                              dim3((unsigned)qk::ceil_div(total, 256), (unsigned)n_layers), dim3(256), 0, c->stream,
