@@ -23,6 +23,8 @@
 //   * attention_sage_kernel: integer dots with dp4a, any shape.  A key block's P codes all
 //     depend on the block's row maximum, so each block is swept twice there: once for the
 //     maximum, once for P and the PV product.
+#include <cuda_fp16.h>
+
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -142,15 +144,18 @@ attention_exact_kernel(const float *__restrict__ q, const float *__restrict__ k,
 // per (plane, pair of key blocks), laid out in global memory byte for byte as the kernel wants
 // them in shared memory, so that an iteration's operands arrive by one bulk copy:
 //   [K tile: 144 rows of 128 bytes: the 128 keys' codes, then 2 x 8 mean-digit rows]
-//   [V tile: 128 channel rows of 128 bytes: the codes of block a's 64 keys, then block b's]
-//   [scales: 128 key scales, 2 x 128 channel scales of V, 2 mean units (16 floats reserved)]
+//   [128 key scales, 2 mean units (16 floats reserved)]
+//   [V tiles of block a, of block b: 128 channel rows of 128 bytes: the codes of the block's 64 keys in float16]
+//   [2 x 128 channel scales of V]
+// (K's half and V's, from kURecVOff, are copied and used up apart.)
 // Tile rows are 128-byte-swizzled: the 16-byte piece p of row r sits at piece p ^ (r & 7).
-// What a ragged sequence leaves unwritten (keys past the end, a missing second block) is never
-// used: those scores are masked before the softmax and the second product is not folded in.
-constexpr uint32_t kURecKBytes = 144 * 128, kURecVBytes = 128 * 128;
-constexpr uint32_t kURecScaleOff = kURecKBytes + kURecVBytes, kURecScaleFloats = 128 + 2 * 128 + 16;
-constexpr uint32_t kURecBytes = kURecScaleOff + kURecScaleFloats * 4;  // what one bulk copy moves
-constexpr uint32_t kURecStride = (kURecBytes + 1023) / 1024 * 1024;
+// What a ragged sequence leaves unwritten (codes of keys past the end, of a missing second block) is never
+// used: those scores are masked before the softmax.  V's rows past the end are zeros, a missing second block's
+// tile and scales too: its product adds nothing.
+constexpr uint32_t kURecTileBytes = 144 * 128, kURecKBytes = kURecTileBytes + (128 + 16) * 4;
+constexpr uint32_t kURecVOff = (kURecKBytes + 1023) / 1024 * 1024, kURecVTileBytes = 128 * 128;
+constexpr uint32_t kURecVBytes = 2 * kURecVTileBytes + 2 * 128 * 4;
+constexpr uint32_t kURecStride = (kURecVOff + kURecVBytes + 1023) / 1024 * 1024;
 // Records of the block-scale variant (attention_sage_block_kernel): the same K tile, a
 // bfloat16 V tile per key block ([128 channels][64 keys], 16 KB each, block a then block b),
 // 128 key scales (one value per 64-key block, repeated) and the two mean units.
@@ -221,9 +226,7 @@ __global__ void sage_quant_k_kernel(const float *__restrict__ k, int8_t *__restr
                                     float *__restrict__ scale, float *__restrict__ mean,
                                     uint32_t S, uint32_t d, uint32_t dpad, uint32_t block,
                                     uint32_t n_blocks, int8_t *__restrict__ mean_digits,
-                                    float *__restrict__ mean_scale, uint8_t *__restrict__ rec,
-                                    uint32_t rec_stride = kURecStride, uint32_t rec_scale_off = kURecScaleOff,
-                                    uint32_t rec_mscale_at = 128 + 2 * 128, int block_scale = 0) {
+                                    float *__restrict__ mean_scale, uint8_t *__restrict__ rec) {
     extern __shared__ float mu[];  // d floats
     const uint32_t plane = blockIdx.y, jb = blockIdx.x;
     const uint32_t j0 = jb * block, j1 = min(S, j0 + block), kj = j1 - j0;
@@ -237,10 +240,10 @@ __global__ void sage_quant_k_kernel(const float *__restrict__ k, int8_t *__restr
     }
     __syncthreads();
     if (rec) {
-        // record form (d = dpad = 128, block = 64, 128 threads): thread c owns channel c of the
+        // record form of the block-scale variant (d = dpad = 128, block = 64, 128 threads): thread c owns channel c of the
         // digit rows, lane l of a warp owns channels 4 l .. 4 l + 3 of a key
         __shared__ float peak_rec[4];
-        uint8_t *rc = rec + ((size_t)plane * ((n_blocks + 1) / 2) + jb / 2) * rec_stride;
+        uint8_t *rc = rec + ((size_t)plane * ((n_blocks + 1) / 2) + jb / 2) * kBRecStride;
         const uint32_t half = jb % 2, c = threadIdx.x;
         float peak = fabsf(mu[c]);
         for (int off = 16; off > 0; off >>= 1) peak = fmaxf(peak, __shfl_xor_sync(0xffffffffu, peak, off));
@@ -259,32 +262,26 @@ __global__ void sage_quant_k_kernel(const float *__restrict__ k, int8_t *__restr
         rc[rec_tile_offset(row0 + 2, c)] = (uint8_t)(int8_t)d2;
 #pragma unroll
         for (uint32_t dr = 3; dr < 8; ++dr) rc[rec_tile_offset(row0 + dr, c)] = 0;
-        float *scales = reinterpret_cast<float *>(rc + rec_scale_off);
-        if (threadIdx.x == 0) scales[rec_mscale_at + half] = unit;
+        float *scales = reinterpret_cast<float *>(rc + kBRecScaleOff);
+        if (threadIdx.x == 0) scales[128 + half] = unit;
         const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-        float block_delta = 0.f;
-        if (block_scale) {
-            // one scale for the whole 64-key block (the benchmark specification's granularity)
-            __shared__ float block_peak[4];
-            float pk = 0.f;
-            for (uint32_t j = j0 + warp; j < j1; j += 4) {
-                const float4 x = *reinterpret_cast<const float4 *>(kp + (size_t)j * d + 4 * lane);
-                const float4 mm = *reinterpret_cast<const float4 *>(mu + 4 * lane);
-                pk = fmaxf(pk, fmaxf(fmaxf(fabsf(x.x - mm.x), fabsf(x.y - mm.y)), fmaxf(fabsf(x.z - mm.z), fabsf(x.w - mm.w))));
-            }
-            for (int off = 16; off > 0; off >>= 1) pk = fmaxf(pk, __shfl_xor_sync(0xffffffffu, pk, off));
-            if (lane == 0) block_peak[warp] = pk;
-            __syncthreads();
-            pk = fmaxf(fmaxf(block_peak[0], block_peak[1]), fmaxf(block_peak[2], block_peak[3]));
-            block_delta = pk > 0.f ? pk / 127.f : 1.f;
+        // one scale for the whole 64-key block (the benchmark specification's granularity)
+        __shared__ float block_peak[4];
+        float pk = 0.f;
+        for (uint32_t j = j0 + warp; j < j1; j += 4) {
+            const float4 x = *reinterpret_cast<const float4 *>(kp + (size_t)j * d + 4 * lane);
+            const float4 mm = *reinterpret_cast<const float4 *>(mu + 4 * lane);
+            pk = fmaxf(pk, fmaxf(fmaxf(fabsf(x.x - mm.x), fabsf(x.y - mm.y)), fmaxf(fabsf(x.z - mm.z), fabsf(x.w - mm.w))));
         }
+        for (int off = 16; off > 0; off >>= 1) pk = fmaxf(pk, __shfl_xor_sync(0xffffffffu, pk, off));
+        if (lane == 0) block_peak[warp] = pk;
+        __syncthreads();
+        pk = fmaxf(fmaxf(block_peak[0], block_peak[1]), fmaxf(block_peak[2], block_peak[3]));
+        const float delta = pk > 0.f ? pk / 127.f : 1.f;
         for (uint32_t j = j0 + warp; j < j1; j += 4) {
             const float4 x = *reinterpret_cast<const float4 *>(kp + (size_t)j * d + 4 * lane);
             const float4 mm = *reinterpret_cast<const float4 *>(mu + 4 * lane);
             const float e0 = x.x - mm.x, e1 = x.y - mm.y, e2 = x.z - mm.z, e3 = x.w - mm.w;
-            float pk = fmaxf(fmaxf(fabsf(e0), fabsf(e1)), fmaxf(fabsf(e2), fabsf(e3)));
-            for (int off = 16; off > 0; off >>= 1) pk = fmaxf(pk, __shfl_xor_sync(0xffffffffu, pk, off));
-            const float delta = block_scale ? block_delta : pk > 0.f ? pk / 127.f : 1.f;
             const uint32_t w = (uint32_t)(quant_code(e0, delta) & 0xff) | ((uint32_t)(quant_code(e1, delta) & 0xff) << 8) |
                                ((uint32_t)(quant_code(e2, delta) & 0xff) << 16) |
                                ((uint32_t)(quant_code(e3, delta) & 0xff) << 24);
@@ -408,7 +405,7 @@ __host__ __device__ inline uint32_t sage_tc_key_slot(uint32_t kk) {
 __global__ void sage_quant_v_kernel(const float *__restrict__ v, int8_t *__restrict__ codes,
                                     float *__restrict__ scale, uint32_t S, uint32_t dv,
                                     uint32_t block, uint32_t bpad, uint32_t n_blocks,
-                                    int permute, uint8_t *__restrict__ rec) {
+                                    int permute) {
     const uint32_t plane = blockIdx.y, jb = blockIdx.x;
     const uint32_t j0 = jb * block, j1 = min(S, j0 + block);
     const float *vp = v + (size_t)plane * S * dv;
@@ -438,20 +435,9 @@ __global__ void sage_quant_v_kernel(const float *__restrict__ v, int8_t *__restr
                         w[q] |= (uint32_t)(code & 0xff) << (8 * e);
                     }
                 }
-                if (rec) {  // record form (dv = 128): row c of the pair's V tile, the block's half of it
-                    uint8_t *rc = rec + ((size_t)plane * ((n_blocks + 1) / 2) + jb / 2) * kURecStride + kURecKBytes;
-                    *reinterpret_cast<uint4 *>(rc + rec_tile_offset(c, 64 * (jb % 2) + 16 * piece)) =
-                        make_uint4(w[0], w[1], w[2], w[3]);
-                } else {
-                    *reinterpret_cast<uint4 *>(cr + 16 * piece) = make_uint4(w[0], w[1], w[2], w[3]);
-                }
+                *reinterpret_cast<uint4 *>(cr + 16 * piece) = make_uint4(w[0], w[1], w[2], w[3]);
             }
-            if (rec) {
-                uint8_t *rc = rec + ((size_t)plane * ((n_blocks + 1) / 2) + jb / 2) * kURecStride;
-                reinterpret_cast<float *>(rc + kURecScaleOff)[128 + 128 * (jb % 2) + c] = delta;
-            } else {
-                scale[((size_t)plane * n_blocks + jb) * dv + c] = delta;
-            }
+            scale[((size_t)plane * n_blocks + jb) * dv + c] = delta;
             continue;
         }
         float peak = 0.f;
@@ -461,6 +447,139 @@ __global__ void sage_quant_v_kernel(const float *__restrict__ v, int8_t *__restr
             cr[permute ? sage_tc_key_slot(j - j0) : j - j0] =
                 j < j1 ? (int8_t)quant_code(vp[(size_t)j * dv + c], delta) : 0;
         scale[((size_t)plane * n_blocks + jb) * dv + c] = delta;
+    }
+}
+
+// ------------------------------------------------------------------ the records' preparation
+// psi_Q, gamma + psi_K and psi_V of the tcgen05 kernel in one launch (head_dim = val_dim = 128, key block 64), the arithmetic
+// of the quantisers above.  Blocks 0 .. 2 planes n_blocks - 1: a key block of K, then of V: the tile comes to shared memory
+// by coalesced loads that are all in flight together (a thread that sums or scans a channel in global memory waits for 64
+// loads, a few at a time).  The rest: kPrepRows query rows each, a warp four of them at a time.
+// 8192 tokens of 32 heads over 8: the whole call 978 -> 944 us against three launches; 64 tokens of 2 heads 34 -> 14.
+constexpr int kPrepThreads = 256, kPrepWarps = kPrepThreads / 32, kPrepRows = 4 * kPrepWarps;
+__global__ void __launch_bounds__(kPrepThreads)
+sage_prepare_kernel(const float *__restrict__ q, const float *__restrict__ k, const float *__restrict__ v,
+                    int8_t *__restrict__ q_codes, float *__restrict__ q_scale, float *__restrict__ k_mean,
+                    uint8_t *__restrict__ rec, uint32_t q_rows, uint32_t S, uint32_t n_blocks, uint32_t planes,
+                    float inv_sqrt_d) {
+    qk::pdl_launch();
+    qk::pdl_wait();
+    const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32, kv_blocks = 2 * planes * n_blocks;
+    auto peak4 = [](float4 x) { return fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))); };
+    auto warp_max = [](float m) {
+        for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+        return m;
+    };
+    auto codes4 = [](float4 x, float delta) {
+        return (uint32_t)(quant_code(x.x, delta) & 0xff) | ((uint32_t)(quant_code(x.y, delta) & 0xff) << 8) |
+               ((uint32_t)(quant_code(x.z, delta) & 0xff) << 16) | ((uint32_t)(quant_code(x.w, delta) & 0xff) << 24);
+    };
+    if (blockIdx.x >= kv_blocks) {
+        const uint32_t row0 = (blockIdx.x - kv_blocks) * kPrepRows + warp;
+        float4 x[4];
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            x[e] = *reinterpret_cast<const float4 *>(q + (size_t)min(row0 + kPrepWarps * e, q_rows - 1) * 128 + 4 * lane);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+            const uint32_t row = row0 + kPrepWarps * e;
+            if (row >= q_rows) break;
+            x[e].x *= inv_sqrt_d, x[e].y *= inv_sqrt_d, x[e].z *= inv_sqrt_d, x[e].w *= inv_sqrt_d;
+            const float peak = warp_max(peak4(x[e])), delta = peak > 0.f ? peak / 127.f : 1.f;
+            *reinterpret_cast<uint32_t *>(q_codes + (size_t)row * 128 + 4 * lane) = codes4(x[e], delta);
+            if (lane == 0) q_scale[row] = delta;
+        }
+        return;
+    }
+    __shared__ __align__(16) float tile[64][128];
+    __shared__ __align__(16) float mu[128];
+    __shared__ float peaks[kPrepThreads];
+    const bool is_v = blockIdx.x >= planes * n_blocks;
+    const uint32_t at = blockIdx.x - (is_v ? planes * n_blocks : 0), plane = at / n_blocks, jb = at % n_blocks;
+    const uint32_t j0 = jb * 64, kj = min(S - j0, 64u), half = jb % 2;
+    const float *src = (is_v ? v : k) + ((size_t)plane * S + j0) * 128;
+    uint8_t *rc = rec + ((size_t)plane * ((n_blocks + 1) / 2) + jb / 2) * kURecStride;
+    {
+        float4 x[8];
+#pragma unroll
+        for (int e = 0; e < 8; ++e) {
+            const uint32_t j = warp + kPrepWarps * e;
+            x[e] = *reinterpret_cast<const float4 *>(src + (size_t)min(j, kj - 1) * 128 + 4 * lane);
+            if (j >= kj) x[e] = make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+#pragma unroll
+        for (int e = 0; e < 8; ++e) *reinterpret_cast<float4 *>(&tile[warp + kPrepWarps * e][4 * lane]) = x[e];
+    }
+    __syncthreads();
+    const uint32_t c = tid % 128;
+    if (is_v) {
+        // a channel's scale over the block's keys, two threads a channel; codes as float16, those past the end are 0
+        const uint32_t first = 32 * (tid / 128);
+        float peak = 0.f;
+#pragma unroll 8
+        for (uint32_t j = first; j < first + 32; ++j) peak = fmaxf(peak, fabsf(tile[j][c]));
+        peaks[tid] = peak;
+        __syncthreads();
+        peak = fmaxf(peak, peaks[tid ^ 128]);
+        const float delta = peak > 0.f ? peak / 127.f : 1.f;
+        uint8_t *dst = rc + kURecVOff + half * kURecVTileBytes;
+        float *scales = reinterpret_cast<float *>(rc + kURecVOff + 2 * kURecVTileBytes);
+#pragma unroll
+        for (uint32_t piece = first / 8; piece < first / 8 + 4; ++piece) {
+            uint32_t w[4];
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+                const uint32_t j = 8 * piece + 2 * e;
+                const float lo = (float)quant_code(tile[j][c], delta), hi = (float)quant_code(tile[j + 1][c], delta);
+                asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(w[e]) : "f"(hi), "f"(lo));
+            }
+            *reinterpret_cast<uint4 *>(dst + rec_tile_offset(c, 16 * piece)) = make_uint4(w[0], w[1], w[2], w[3]);
+            if (half == 0 && jb + 1 == n_blocks)  // (no second block)
+                *reinterpret_cast<uint4 *>(dst + kURecVTileBytes + 128 * c + 16 * piece) = make_uint4(0, 0, 0, 0);
+        }
+        if (tid < 128) {
+            scales[128 * half + c] = delta;
+            if (half == 0 && jb + 1 == n_blocks) scales[128 + c] = 0.f;
+        }
+        return;
+    }
+    // the channels' means: sequential float32 sums over the keys, as the reference forms them
+    if (tid < 128) {
+        float sum = 0.f;
+#pragma unroll 16
+        for (uint32_t j = 0; j < kj; ++j) sum += tile[j][c];
+        const float mean = sum / (float)kj;
+        mu[c] = mean;
+        k_mean[((size_t)plane * n_blocks + jb) * 128 + c] = mean;
+        const float peak = warp_max(fabsf(mean));
+        if (lane == 0) peaks[warp] = peak;
+    }
+    __syncthreads();
+    const float peak = fmaxf(fmaxf(peaks[0], peaks[1]), fmaxf(peaks[2], peaks[3]));
+    const float unit = peak > 0.f ? peak / 8000000.f : 1.f;  // |fixed| <= 8e6 < 127 * 65536
+    float *scales = reinterpret_cast<float *>(rc + kURecTileBytes);
+    const uint32_t row0 = 128 + 8 * half;
+    if (tid < 128) {  // the mean's three digit rows
+        int d = (int)rintf(mu[c] / unit);
+        const int d2 = ((d + 128) & 255) - 128;
+        d = (d - d2) >> 8;
+        const int d1 = ((d + 128) & 255) - 128;
+        d = (d - d1) >> 8;
+        rc[rec_tile_offset(row0, c)] = (uint8_t)(int8_t)d;
+        rc[rec_tile_offset(row0 + 1, c)] = (uint8_t)(int8_t)d1;
+        rc[rec_tile_offset(row0 + 2, c)] = (uint8_t)(int8_t)d2;
+        if (c == 0) scales[128 + half] = unit;
+    } else {          // ... and the five rows of zeros: 160 words
+        for (uint32_t i = c; i < 160; i += 128) *reinterpret_cast<uint32_t *>(rc + (row0 + 3) * 128 + 4 * i) = 0;
+    }
+    const float4 mm = *reinterpret_cast<const float4 *>(mu + 4 * lane);
+#pragma unroll 4
+    for (uint32_t j = warp; j < kj; j += kPrepWarps) {
+        const float4 x = *reinterpret_cast<const float4 *>(&tile[j][4 * lane]);
+        const float4 e = make_float4(x.x - mm.x, x.y - mm.y, x.z - mm.z, x.w - mm.w);
+        const float pk = warp_max(peak4(e)), delta = pk > 0.f ? pk / 127.f : 1.f;
+        *reinterpret_cast<uint32_t *>(rc + rec_tile_offset(64 * half + j, 4 * lane)) = codes4(e, delta);
+        if (lane == 0) scales[64 * half + j] = delta;
     }
 }
 
@@ -938,45 +1057,59 @@ attention_sage_tc_kernel(SageArgs a, AttnDims dm, int causal) {
     }
 }
 
-// ------------------------------------------------------------------ Sage on tcgen05 (kind::i8)
-// The same arithmetic once more, with both integer products on the 5th-generation tensor
-// cores: tcgen05.mma kind::i8 (s8 x s8 -> s32) with the accumulators in tensor memory.  Built
-// for head_dim = val_dim = 128 and the Sage key block of 64 (benchmark configuration 2).
-//   * A CTA owns 128 queries; query row r is tensor-memory lane r.  Its 512 threads are four
-//     groups of 128: thread (g, r) works on row r's score columns 32 g .. 32 g + 31 of the
-//     iteration (groups 0, 1: the first Sage block; 2, 3: the second) and on output channels
-//     32 g .. 32 g + 31.  What a row's four threads have to agree on (the blocks' maxima and
-//     sums of P) goes through shared memory; every thread then derives the same running
-//     maximum, alphas and l.
-//   * One iteration covers TWO Sage blocks (128 keys): S = Qhat [Khat_a; Khat_b; mean digits]^T
-//     is one 128 x 144 x 128 product (the sixteen extra B rows are the digit rows of the two
-//     blocks' channel means, which give the per-row shift), then the online softmax runs block
-//     by block exactly as in the other kernels - block b's codes use the maximum after block a -
-//     and the two PV products (128 x 128 x 64 each, because V has one scale set per block) go
-//     to two accumulators that alias S, which has been read out by then.
-//   * Operands are staged by cp.async into 128-byte-swizzled K-major tiles (rows of 128 bytes:
-//     Q and K rows are 128 channels, P and V rows are the iteration's 128 keys, V_a and V_b
-//     side by side), two iterations ahead.  The P codes go from registers to shared memory and
-//     are the A operand of PV.
-//   * The products run beside the arithmetic: tensor memory holds two accumulator regions, S of
-//     iteration it + 1 is issued as soon as S of iteration it has been read out and runs while
-//     the threads exponentiate; PV of iteration it is issued at the end of the iteration and is
-//     folded into the output in the middle of the next one, after that one's scores.
-// All waits on the MMA barriers are bounded (bit 1 of the context's error word on expiry).
+// ------------------------------------------------------------------ Sage on tcgen05
+// The same arithmetic once more, with both products on the 5th-generation tensor cores.  Built for
+// head_dim = val_dim = 128 and the Sage key block of 64 (benchmark configuration 2).
+//   * A CTA owns 128 queries; query row r is tensor-memory lane r.  Four kinds of warps: two groups of eight for
+//     the SCORES, which take the iterations in turn, a row's 64 keys of one Sage block a thread; two groups of four for
+//     the OUTPUT, a row's 64 channels a thread; one that issues the products; one that copies.  While one score group
+//     waits for its products the other computes, and the output warps work beside both.  From one iteration to the next
+//     only the running maximum is handed over, as soon as it is known.
+//   * One iteration covers TWO Sage blocks (128 keys): S = Qhat [Khat_a; Khat_b]^T (kind::i8), the online
+//     softmax block by block exactly as in the other kernels - block b's codes use the maximum after block
+//     a -, then one PV product per block, because V has one scale set per block.
+//   * PV is kind::f16: P and V codes are whole numbers of at most 127, which float16 holds exactly, and a
+//     block's sums stay below 2^21, which the float32 accumulators hold exactly.  So the sums arrive as
+//     floats, and the output warps convert nothing (per score two conversions fewer on a pipe that takes two cycles
+//     for each).  S stays kind::i8: half the operand bytes, one conversion per score.
+//   * The Q . mean shift of a row comes from the blocks' mean digit rows, a product with N = 16 whose result
+//     lies in S's columns before S does (64 ..: free once the scores are P codes).
+//   * Tensor memory (512 columns): S of the two score groups at 0 and 128, the PV sums of the two blocks at 256 and
+//     384.  The scores, scaled, go back to S's columns between the two passes over them (maximum, exponentials); a block's P
+//     codes (float16, PV's A operand) take the first half of its scores' columns.
+// All waits are bounded (bit 1 of the context's error word on expiry).
+//
+// What bounds it: the chain of an iteration - scores to maximum, maximum to P codes, the products' issue - which two
+// groups in turn hide in part: issue slots 52 % busy, the special-function unit 27 % (4096 tokens).  8192 tokens of 32
+// heads over 8, causal, whole call: 1296 us by sixteen warps in step with both products in kind::i8, 1035 with groups of four
+// warps and one PV region, 978 as it is (944 with the preparation in one launch).  Taking the two tiles of a CTA in turn instead
+// of two iterations: 1146.
 constexpr int kUQ = 128, kUBlk = 64, kUKeys = 2 * kUBlk, kUD = 128;
 constexpr int kUThreads = 512, kUGroups = kUThreads / kUQ;
-// The warps whose lane 0 issues the S products, the record copies and the PV products.  Each of
+// The block-scale kernel's issuing warps (their lane 0): S products, record copies, PV products.  Each of
 // these instructions (tcgen05.mma, tcgen05.commit, the mbarrier operations, the bulk copy) takes
 // its thread a hundred cycles and more to issue, one after the other: spread over three warps
 // on three schedulers they overlap, and no warp falls far behind the others at the CTA barriers.
 constexpr uint32_t kUWarpS = 0, kUWarpRec = 5, kUWarpPV = 10;
-constexpr int kUSRows = kUKeys + 16;  // keys + 2 x 8 mean-digit rows: N of the S product
-constexpr uint32_t kUQBytes = kUQ * 128, kUPBytes = kUQ * 128;
+constexpr int kUSRows = kUKeys + 16;  // the block-scale kernel's N of the S product: keys + 2 x 8 mean-digit rows
+constexpr uint32_t kUQBytes = kUQ * 128;
 constexpr int kUBufs = 3;  // record buffers: an iteration's record is fetched two iterations ahead
-static_assert(kURecKBytes == kUSRows * 128 && kURecVBytes == kUD * 128, "the record holds the kernel's tiles");
-constexpr uint32_t kUSmemBytes = kUQBytes + kUBufs * kURecStride + kUPBytes + 2 * kUGroups * kUQ * 4 + 64;
-constexpr uint32_t kUTmemCols = 512, kUPVCol = 256;  // S (144 columns) at column 0, the two PV accumulators from column 256
+static_assert(kURecTileBytes == kUSRows * 128 && kURecVTileBytes == kUD * 128, "the record holds the kernel's tiles");
+constexpr int kUAllThreads = 896;  // scores, output, the issuing warp, the copying warp, two that leave at once
+constexpr uint32_t kUOutWarp = 16, kUIssueWarp = 24, kUCopyWarp = 25;
+constexpr int kUKBufs = 4, kUVBufs = 3, kUStats = 4;
+// Q tile, buffers of K and of V, [iteration % kUStats][alpha a, alpha b, sum a, sum b][row], maxima [group][row],
+// maxima of the blocks [group][block][row], barriers
+constexpr uint32_t kUSmemBytes = kUQBytes + kUKBufs * kURecVOff + kUVBufs * (kURecStride - kURecVOff) +
+                                 kUStats * 4 * kUQ * 4 + 6 * kUQ * 4 + 384;
+static_assert(kUSmemBytes + 1024 <= 227 * 1024, "the Sage kernel's shared memory");
+constexpr uint32_t kUTmemCols = 512, kUPVCol = 256;
+constexpr uint32_t kUDigitCol = 32;   // of S's columns: the digit sums of the group's next iteration, block b's 8 further
 constexpr uint32_t kUWaitLimitDefault = 1u << 22;
+// Registers a thread: the warps share what the block is launched with.
+constexpr uint32_t kURegsScores = 64, kURegsOutput = 112, kURegsIssue = 24, kURegsLaunch = 72;
+static_assert(512 * kURegsScores + 256 * kURegsOutput + 128 * kURegsIssue <= kUAllThreads * kURegsLaunch,
+              "setmaxnreg draws on the launch's registers");
 
 // s8 x s8 -> s32, both operands K-major, M = 128, N = n
 __device__ __forceinline__ uint32_t umma_idesc_i8(uint32_t n) {
@@ -990,334 +1123,460 @@ __device__ __forceinline__ void umma_i8(uint32_t d_tmem, uint64_t a_desc, uint64
         "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
+// f16 x f16 -> f32, A in tensor memory, B K-major, M = 128, N = n
+__device__ __forceinline__ uint32_t umma_idesc_f16(uint32_t n) {
+    return (1u << 4) | ((n >> 3) << 17) | ((uint32_t)(kUQ >> 4) << 24);
+}
+__device__ __forceinline__ void umma_f16_ts(uint32_t d_tmem, uint32_t a_tmem, uint64_t b_desc, uint32_t idesc,
+                                            uint32_t accumulate) {
+    asm volatile(
+        "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
+        " tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n}" ::"r"(d_tmem),
+        "r"(a_tmem), "l"(b_desc), "r"(idesc), "r"(accumulate)
+        : "memory");
+}
+__device__ __forceinline__ void tmem_ld4(uint32_t taddr, uint32_t (&v)[4]) {
+    asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
+                 : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3])
+                 : "r"(taddr)
+                 : "memory");
+}
+__device__ __forceinline__ void tmem_st16(uint32_t taddr, const uint32_t (&v)[16]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16};" ::"r"(taddr),
+        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+        "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
+    asm volatile(
+        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
+        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, "
+        "%23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
+        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
+        "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]),
+        "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]),
+        "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
+        : "memory");
+}
+__device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t (&v)[8]) {
+    asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(v[0]),
+                 "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7])
+                 : "memory");
+}
+// The wait for all loads so far, as the point from which `v`, the last one's registers, may be used.
+__device__ __forceinline__ void tmem_ld_wait16(uint32_t (&v)[16]) {
+    asm volatile("tcgen05.wait::ld.sync.aligned;"
+                 : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+                   "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])::"memory");
+}
+__device__ __forceinline__ void tmem_st_wait() { asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
+__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
 __device__ __forceinline__ float ex2_approx(float x) {
     float y;
     asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
     return y;
 }
 
-__global__ void __launch_bounds__(kUThreads, 1)
+struct SageBars {
+    uint64_t k[kUKBufs], k_free[kUKBufs], v[kUVBufs], v_free[kUVBufs];  // copies: landed; used up
+    // per score group
+    uint64_t digits[2], digits_read[2];  // the digit sums of the group's next iteration: there; read
+    uint64_t s[2], p[2];                 // S is there; P codes, alphas and sums are there
+    uint64_t max[2][4];                  // [group][warp]: the rows' maximum after the group's iteration
+    uint64_t pv[2], pv_read[2];          // the PV sums of an iteration's block a, b are there; read
+    uint64_t drain;
+    uint32_t tmem_slot;
+    int abort_flag, never;
+};
+static_assert(sizeof(SageBars) <= 384, "reserved for the barriers");
+
+__global__ void __launch_bounds__(kUAllThreads, 1)
 attention_sage_umma_kernel(SageArgs a, AttnDims dm, int causal, uint32_t wait_limit, int *error) {
     extern __shared__ __align__(1024) uint8_t sm_u_raw[];
     // (the swizzled tiles want 1024-byte alignment; the launch asks for 1 KB more than kUSmemBytes)
-    uint8_t *sm_u = sm_u_raw + ((1024 - (smem_u32(sm_u_raw) & 1023)) & 1023);
-    uint8_t *Qs = sm_u, *Rb = Qs + kUQBytes, *Ps = Rb + kUBufs * kURecStride;  // Q tile, record buffers, P tile
-    float *xm = reinterpret_cast<float *>(Ps + kUPBytes), *xe = xm + kUGroups * kUQ;  // [group][row]: block maxima, sums of P
-    uint64_t *bar_s = reinterpret_cast<uint64_t *>(xe + kUGroups * kUQ), *bar_pv = bar_s + 1, *bar_drain = bar_s + 2;
-    uint64_t *bar_rec = bar_s + 3;  // [kUBufs]: a record has landed in its buffer
-    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bar_rec + kUBufs);
-    volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
-    const uint32_t tid = threadIdx.x, warp = tid / 32;
-    const uint32_t g = tid / kUQ, r = tid % kUQ;  // column group, query row
-    const int my_blk = g / 2;
-    const int h = blockIdx.y, b = blockIdx.z, kvh = h / dm.group;
+    uint8_t *Qs = sm_u_raw + ((1024 - (smem_u32(sm_u_raw) & 1023)) & 1023), *Kb = Qs + kUQBytes;
+    constexpr uint32_t kKStride = kURecVOff, kVStride = kURecStride - kURecVOff;
+    uint8_t *Vb = Kb + kUKBufs * kKStride;
+    float *stats = reinterpret_cast<float *>(Vb + kUVBufs * kVStride), *maxima = stats + kUStats * 4 * kUQ;
+    float *block_max = maxima + 2 * kUQ;
+    SageBars *bars = reinterpret_cast<SageBars *>(block_max + 4 * kUQ);
+    volatile int *abort_flag = &bars->abort_flag;
+    const uint32_t tid = threadIdx.x, warp = tid / 32, r = tid % kUQ;
+    const int h = blockIdx.x, b = blockIdx.z, kvh = h / dm.group;
     const size_t plane = (size_t)b * dm.KV + kvh;
     // under causal masking the last query tiles have the most key blocks: start them first
-    const int q_tile = causal ? (int)gridDim.x - 1 - (int)blockIdx.x : (int)blockIdx.x;
-    const int q0 = q_tile * kUQ, i = q0 + (int)r;
-    const bool valid = i < (int)dm.Sq;
+    const int q0 = (causal ? (int)gridDim.y - 1 - (int)blockIdx.y : (int)blockIdx.y) * kUQ, i = q0 + (int)r;
     const size_t row_base = ((size_t)b * dm.H + h) * dm.Sq;
-    const int S = (int)dm.Skv, n_blocks = (int)a.n_blocks;
+    const int S = (int)dm.Skv, n_blocks = (int)a.n_blocks, Sq = (int)dm.Sq;
+    const bool valid = i < Sq;
+    const int n_it = ((causal ? min(Sq - 1, q0 + kUQ - 1) / kUBlk + 1 : n_blocks) + 1) / 2;
 
     if (tid == 0) {
-        mbar_init(bar_s, 1);
-        mbar_init(bar_pv, 1);
-        mbar_init(bar_drain, 2);
-        for (int bi = 0; bi < kUBufs; ++bi) mbar_init(bar_rec + bi, 1);
-        *abort_flag = 0;
+        for (int k = 0; k < kUKBufs; ++k) {
+            mbar_init(bars->k + k, 1);
+            mbar_init(bars->k_free + k, 8);
+        }
+        for (int k = 0; k < kUVBufs; ++k) {
+            mbar_init(bars->v + k, 1);
+            mbar_init(bars->v_free + k, 8);
+        }
+        for (int k = 0; k < 2; ++k) {
+            mbar_init(bars->digits + k, 1);
+            mbar_init(bars->digits_read + k, 8);
+            mbar_init(bars->s + k, 1);
+            mbar_init(bars->p + k, 8);
+            for (int w = 0; w < 4; ++w) mbar_init(&bars->max[k][w], 2);  // (a row's two warps)
+            mbar_init(bars->pv + k, k == 0 ? 2 : 1);  // (block a's counts the issuing thread too)
+            mbar_init(bars->pv_read + k, 8);
+        }
+        mbar_init(&bars->drain, 1);
+        bars->abort_flag = 0;
+        bars->never = 0;
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     if (warp == 0) {
-        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&bars->tmem_slot)),
                      "r"(kUTmemCols)
                      : "memory");
         asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
     }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    // a warp reaches the 32 lanes (rows) 32 (warp % 4) ..; the groups differ in their columns
-    const uint32_t tmem_base = *tmem_slot, my_tmem = tmem_base + (((warp % 4) * 32) << 16);
-
-    // 16-byte piece `piece` of row `row` of a swizzled tile
-    auto swz = [](uint8_t *tile, int row, int piece) { return tile + row * 128 + ((piece ^ (row & 7)) << 4); };
-    // The record of iteration `it` (keys 128 it .., the key blocks 2 it and 2 it + 1) into its
-    // buffer: one bulk copy, started by one thread, which completes on the buffer's barrier.
-    const uint8_t *rec_src = a.rec + plane * (size_t)((n_blocks + 1) / 2) * kURecStride;
-    auto stage = [&](int it) {
-        const uint32_t bar = smem_u32(bar_rec + it % kUBufs);
-        asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(bar), "r"(kURecBytes) : "memory");
-        asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
-                         smem_u32(Rb + (it % kUBufs) * kURecStride)),
-                     "l"(rec_src + (size_t)it * kURecStride), "r"(kURecBytes), "r"(bar)
-                     : "memory");
-    };
-
-    const int i_blk_max = min((int)dm.Sq - 1, q0 + kUQ - 1);
-    const int jb_hi = causal ? i_blk_max / kUBlk + 1 : n_blocks;
-    const int n_it = (jb_hi + 1) / 2;
-    for (int idx = tid; idx < kUQ * 8; idx += kUThreads) {
+    qk::pdl_launch();
+    qk::pdl_wait();
+    // the Q tile: 16-byte piece `piece` of row `row` at piece ^ (row & 7) (rows past the end repeat the last one)
+    for (int idx = tid; idx < kUQ * 8; idx += kUAllThreads) {
         const int row = idx / 8, piece = idx % 8;
-        cp_async16(swz(Qs, row, piece), a.qc + (row_base + min(q0 + row, (int)dm.Sq - 1)) * a.dpad + piece * 16);
+        cp_async16(Qs + row * 128 + ((piece ^ (row & 7)) << 4),
+                   a.qc + (row_base + min(q0 + row, Sq - 1)) * a.dpad + piece * 16);
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
-    const float dq = valid ? a.qs[row_base + i] : 1.f;
-
-    // channels 32 g .. 32 g + 31 of row r, in pairs: the per-element arithmetic of this kernel
-    // runs on the packed float32 instructions (two IEEE operations per issue slot: the same
-    // results, half the instructions)
-    float2 o[16];
-#pragma unroll
-    for (int c = 0; c < 16; ++c) o[c] = make_float2(0.f, 0.f);
-    float m = -INFINITY, l = 0.f;
-    float prev_alpha_a = 0.f, prev_alpha_b = 0.f;  // of the iteration whose PV is still to be folded in
-    const uint32_t idesc_s = umma_idesc_i8(kUSRows), idesc_pv = umma_idesc_i8(kUD);
-    const uint32_t limit = wait_limit ? wait_limit : kUWaitLimitDefault;
-    bool dead = false;
-    int dead_it = n_it;  // the iteration that gave up
-    uint32_t v[32];
-    auto issue_s = [&](int it) {  // S of iteration `it` (one thread)
-        const uint32_t kt = smem_u32(Rb + (it % kUBufs) * kURecStride);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-        for (int k = 0; k < kUD / 32; ++k)
-            umma_i8(tmem_base, umma_desc(smem_u32(Qs) + k * 32), umma_desc(kt + k * 32), idesc_s, k != 0);
-        umma_commit(bar_s);
-    };
-    // o = alpha * o + PV * dV for one key block: `v` holds the block's 32 integer sums of this
-    // thread's channels, `vd` points at their scales
-    auto fold_block = [&](float al, const float *vd) {
-        const float2 al2 = make_float2(al, al);
-        const float4 *vd4 = reinterpret_cast<const float4 *>(vd);
-#pragma unroll
-        for (int e = 0; e < 8; ++e) {
-            const float4 d = vd4[e];
-            o[2 * e] = __ffma2_rn(al2, o[2 * e],
-                                  __fmul2_rn(make_float2((float)(int)v[4 * e], (float)(int)v[4 * e + 1]), make_float2(d.x, d.y)));
-            o[2 * e + 1] = __ffma2_rn(al2, o[2 * e + 1],
-                                      __fmul2_rn(make_float2((float)(int)v[4 * e + 2], (float)(int)v[4 * e + 3]),
-                                                 make_float2(d.z, d.w)));
-        }
-    };
-    // the channel scales of V of iteration `it`, this thread's 32 channels of block a (block b: + kUD)
-    auto vscale_of = [&](int it) {
-        return reinterpret_cast<const float *>(Rb + (it % kUBufs) * kURecStride + kURecScaleOff) + kUKeys + 32 * g;
-    };
-    const bool lane0 = tid % 32 == 0;
-    if (warp == kUWarpRec && lane0) {
-        stage(0);
-        if (n_it > 1) stage(1);
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");  // (the Q tile)
+    asm volatile("cp.async.wait_group 0;" ::: "memory");
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-    // (if this wait gives up, no product is issued and every wait below gives up in turn)
-    const bool first_landed = warp != kUWarpRec || mbar_wait(bar_rec, 0, abort_flag, limit);
-    if (__syncthreads_and(first_landed) && warp == kUWarpS && lane0) issue_s(0);
-    __syncwarp();
-    for (int it = 0; it < n_it; ++it) {
-        const int buf = it % kUBufs;
-        const float *kscale = reinterpret_cast<const float *>(Rb + buf * kURecStride + kURecScaleOff);
-        const float *mscale = kscale + kUKeys + 2 * kUD;
-        // A warp whose wait gives up skips what needs the products and votes at the next CTA
-        // barrier: the verdict is taken by the whole CTA, nobody goes on to a barrier the others
-        // have left.
-        // (one warp saw this iteration's record land before a CTA barrier that lies behind us,
-        // which makes the record's scales visible to this thread)
-        bool ok = mbar_wait(bar_s, it & 1, abort_flag, limit);
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    tc_fence_before();
+    __syncthreads();
+    tc_fence_after();
+    // a warp reaches the 32 lanes (rows) 32 (warp % 4) ..
+    const uint32_t tmem_base = bars->tmem_slot, lanes = ((warp % 4) * 32) << 16;
+    const uint32_t limit = wait_limit ? wait_limit : kUWaitLimitDefault;
+    const bool lane0 = tid % 32 == 0;
+    int got_k = 0, got_v = 0;  // (the copying warp) copies asked for
+    bool ok = true;
 
-        // ---- this thread's 32 scores of its Sage block
-        const int jb = 2 * it + my_blk, j0 = jb * kUBlk, kj = min(kUBlk, S - j0);
-        const bool live = jb < jb_hi;
-        float shift = 0.f;
-        if (ok) {
-            uint32_t c0, c1, c2, c3;
-            asm volatile("tcgen05.ld.sync.aligned.32x32b.x4.b32 {%0, %1, %2, %3}, [%4];"
-                         : "=r"(c0), "=r"(c1), "=r"(c2), "=r"(c3)
-                         : "r"(my_tmem + kUKeys + 8 * my_blk)
-                         : "memory");
-            tmem_ld32(my_tmem + 32 * g, v);
-            tmem_ld_wait();
-            (void)c3;
-            shift = (((float)(int)c0 * 65536.f + (float)(int)c1 * 256.f) + (float)(int)c2) * mscale[my_blk] * dq;
-        }
-        // only the iteration on the diagonal, the last one of a ragged sequence, a tile with rows
-        // past the end and a missing second block need the per-element mask
-        const int it_j0 = it * kUKeys;
-        const bool masked = it_j0 + kUKeys > S || q0 + kUQ > (int)dm.Sq || !live || 2 * it + 1 >= jb_hi ||
-                            (causal && it_j0 + kUKeys - 1 > q0);
-        float s[32];
-        float bm = -INFINITY;
-        const float *ksc = kscale + 32 * g;
-        if (masked) {
-#pragma unroll
-            for (int e = 0; e < 32; ++e) {
-                const int kk = 32 * (int)(g % 2) + e, j = j0 + kk;
-                float sc = fmaf((float)(int)v[e] * dq, ksc[e], shift);
-                if (!live || kk >= kj || !valid || (causal && j > i)) sc = -INFINITY;
-                s[e] = sc;
-                bm = fmaxf(bm, sc);
-            }
-        } else {
-            const float2 dq2 = make_float2(dq, dq), shift2 = make_float2(shift, shift);
-            const float4 *ksc4 = reinterpret_cast<const float4 *>(ksc);
-#pragma unroll
-            for (int e = 0; e < 8; ++e) {
-                const float4 d = ksc4[e];
-                const float2 sa = __ffma2_rn(__fmul2_rn(make_float2((float)(int)v[4 * e], (float)(int)v[4 * e + 1]), dq2),
-                                             make_float2(d.x, d.y), shift2);
-                const float2 sb = __ffma2_rn(__fmul2_rn(make_float2((float)(int)v[4 * e + 2], (float)(int)v[4 * e + 3]), dq2),
-                                             make_float2(d.z, d.w), shift2);
-                s[4 * e] = sa.x, s[4 * e + 1] = sa.y, s[4 * e + 2] = sb.x, s[4 * e + 3] = sb.y;
-                bm = fmaxf(fmaxf(bm, fmaxf(sa.x, sa.y)), fmaxf(sb.x, sb.y));
-            }
-        }
-        xm[g * kUQ + r] = bm;
-        // the record of the next iteration was asked for an iteration ago
-        if (warp == kUWarpRec && it + 1 < n_it && ok)
-            ok = mbar_wait(bar_rec + (it + 1) % kUBufs, ((it + 1) / kUBufs) & 1, abort_flag, limit);
-        // after the barrier every thread has read S of this iteration out of tensor memory
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        if (!__syncthreads_and(ok)) {
-            dead = true;
-            dead_it = it;
-            break;
-        }
-        if (warp == kUWarpS && lane0 && it + 1 < n_it) issue_s(it + 1);  // runs while the threads exponentiate
-        __syncwarp();
-        // ---- the row's maxima after block a and after block b (the same in its four threads)
-        const float bm_a = fmaxf(xm[r], xm[kUQ + r]), bm_b = fmaxf(xm[2 * kUQ + r], xm[3 * kUQ + r]);
-        const float mn_a = fmaxf(m, bm_a);
-        const float alpha_a = (mn_a == -INFINITY) ? 0.f : expf(m - mn_a);
-        const float m_a = (mn_a == -INFINITY) ? m : mn_a;
-        const float mn_b = fmaxf(m_a, bm_b);
-        const float alpha_b = (mn_b == -INFINITY) ? 0.f : expf(m_a - mn_b);
-        const float m_b = (mn_b == -INFINITY) ? m_a : mn_b;
-        const float mn = my_blk ? mn_b : mn_a;
-        // P scaled by 127 (the static P scale): 127 exp(s - m) = exp2(s log2e - m log2e + log2 127).
-        // A masked score is -inf and so is `off` of a row without any key so far: their sum is
-        // -inf (never NaN), of which ex2 gives 0.
+    if (warp < kUOutWarp) {
+        // ---------------------------------------------------------------- scores: iterations g, g + 2, ..., block blk
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kURegsScores));
+        const uint32_t g = warp / 8, blk = warp / 4 % 2, my_s = tmem_base + lanes + 128 * g + 64 * blk;
+        const uint32_t my_digits = tmem_base + lanes + 128 * g + kUDigitCol + 8 * blk;
+        const float dq = valid ? a.qs[row_base + i] : 1.f;
+        const float2 dq2 = make_float2(dq, dq);
+        const int seen = !valid ? 0 : causal ? min(S, i + 1) : S;  // keys of the sequence that the row sees
         constexpr float kLog2e = 1.4426950408889634f, kLog2_127 = 6.988684686772166f;
-        const float off = (mn == -INFINITY) ? -INFINITY : kLog2_127 - mn * kLog2e;
-        const float2 log2e2 = make_float2(kLog2e, kLog2e), off2 = make_float2(off, off);
-        float2 es2 = make_float2(0.f, 0.f);  // the sums over the even and the odd columns
-        auto exp_piece = [&](int piece) {  // 16 of the thread's 32 columns: exponentiate, round, store the codes
-            uint32_t w[4];
+        const float2 log2e2 = make_float2(kLog2e, kLog2e);
+        // x + kRound - kRound rounds 0 <= x <= 2^22 to the nearest whole number, ties to even, like rint
+        constexpr float kRound = 12582912.f;
+        const float2 round2 = make_float2(kRound, kRound), unround2 = make_float2(-kRound, -kRound);
+        // A row's two warps meet: what they wrote is there for both; true when neither has given up (they leave together).
+        auto meet = [&](bool good) {
+            if (!good) *abort_flag = 1;
+            uint32_t all;
+            asm volatile(
+                "{\n .reg .pred p, q;\n setp.ne.b32 p, %1, 0;\n barrier.cta.red.and.pred q, %2, 64, p;\n"
+                " selp.u32 %0, 1, 0, q;\n}"
+                : "=r"(all)
+                : "r"((uint32_t)good), "r"(1 + 4 * g + warp % 4)
+                : "memory");
+            return all != 0;
+        };
+        float raw = 0.f;  // the row's digit sums of the block, put together
+        auto read_digits = [&](int it) {
+            ok = ok && mbar_wait(bars->digits + g, (it >> 1) & 1, abort_flag, limit);
+            tc_fence_after();
+            uint32_t d[4];
+            tmem_ld4(my_digits, d);
+            tmem_ld_wait();
+            raw = ((float)(int)d[0] * 65536.f + (float)(int)d[1] * 256.f) + (float)(int)d[2];
+            tc_fence_before();
+            __syncwarp();
+            if (lane0) mbar_arrive(bars->digits_read + g);
+        };
+        if ((int)g < n_it) read_digits((int)g);
+        for (int it = (int)g; it < n_it; it += 2) {
+            const int kbuf = it % kUKBufs;
+            const float *kscale = reinterpret_cast<const float *>(Kb + kbuf * kKStride + kURecTileBytes);
+            const float4 *ks4 = reinterpret_cast<const float4 *>(kscale + 64 * blk);
+            ok = ok && mbar_wait(bars->k + kbuf, (it / kUKBufs) & 1, abort_flag, limit);
+            const float shift = raw * kscale[kUKeys + blk] * dq;
+            const float2 shift2 = make_float2(shift, shift);
+            ok = ok && mbar_wait(bars->s + g, (it >> 1) & 1, abort_flag, limit);
+            tc_fence_after();
+            // ---- the scores, back into S's columns, and the block's maximum.  Only the iteration on the
+            // diagonal, the last one of a ragged sequence and a tile with rows past the end need the mask.
+            const int end = seen - it * kUKeys - 64 * (int)blk;  // keys of this block that the row sees
+            const bool masked = (it + 1) * kUKeys > S || q0 + kUQ > Sq || (causal && (it + 1) * kUKeys - 1 > q0);
+            uint32_t v[2][16];
+            tmem_ld16(my_s, v[0]);
+            float mx0 = -INFINITY, mx1 = -INFINITY;
 #pragma unroll
-            for (int q = 0; q < 4; ++q) {
-                int c[4];
+            for (int c = 0; c < 4; ++c) {
+                uint32_t(&w)[16] = v[c & 1];
+                tmem_ld_wait16(w);
+                if (c < 3) tmem_ld16(my_s + 16 * (c + 1), v[(c + 1) & 1]);
 #pragma unroll
-                for (int e = 0; e < 4; e += 2) {
-                    const int at = 16 * piece + 4 * q + e;
-                    const float2 arg = __ffma2_rn(make_float2(s[at], s[at + 1]), log2e2, off2);
+                for (int e = 0; e < 4; ++e) {
+                    const float4 d = ks4[4 * c + e];
+                    const float2 x = __ffma2_rn(__fmul2_rn(make_float2((float)(int)w[4 * e], (float)(int)w[4 * e + 1]), dq2),
+                                                make_float2(d.x, d.y), shift2);
+                    const float2 y = __ffma2_rn(__fmul2_rn(make_float2((float)(int)w[4 * e + 2], (float)(int)w[4 * e + 3]), dq2),
+                                                make_float2(d.z, d.w), shift2);
+                    w[4 * e] = __float_as_uint(x.x), w[4 * e + 1] = __float_as_uint(x.y);
+                    w[4 * e + 2] = __float_as_uint(y.x), w[4 * e + 3] = __float_as_uint(y.y);
+                }
+                if (masked) {
+#pragma unroll
+                    for (int e = 0; e < 16; ++e) w[e] = 16 * c + e < end ? w[e] : 0xff800000u;
+                }
+#pragma unroll
+                for (int e = 0; e < 16; e += 4) {
+                    mx0 = fmaxf(fmaxf(mx0, __uint_as_float(w[e])), __uint_as_float(w[e + 1]));
+                    mx1 = fmaxf(fmaxf(mx1, __uint_as_float(w[e + 2])), __uint_as_float(w[e + 3]));
+                }
+                tmem_st16(my_s + 16 * c, w);
+            }
+            block_max[(2 * g + blk) * kUQ + r] = fmaxf(mx0, mx1);
+            // (S and the digits of this iteration are done, the scales read)
+            __syncwarp();
+            if (lane0) mbar_arrive(bars->k_free + kbuf);
+            ok = meet(ok);
+            if (!ok) break;
+            // ---- the row's maxima after block a and after block b; the second is the other group's to go on from
+            float m = -INFINITY;
+            if (it > 0) {
+                ok = mbar_wait(&bars->max[1 - g][warp % 4], ((it - 1) >> 1) & 1, abort_flag, limit);
+                m = maxima[(1 - g) * kUQ + r];
+            }
+            const float mn_a = fmaxf(m, block_max[2 * g * kUQ + r]), mn_b = fmaxf(mn_a, block_max[(2 * g + 1) * kUQ + r]);
+            if (blk == 0) maxima[g * kUQ + r] = mn_b;
+            __syncwarp();
+            if (lane0) mbar_arrive(&bars->max[g][warp % 4]);
+            const float before = blk ? mn_a : m, mn = blk ? mn_b : mn_a;
+            // ---- P scaled by 127 (the static P scale): 127 exp(s - m) = exp2(s log2e - m log2e + log2 127).
+            // A masked score is -inf and so is `off` of a row without any key so far: their sum is
+            // -inf (never NaN), of which ex2 gives 0.
+            const float off = (mn == -INFINITY) ? -INFINITY : kLog2_127 - mn * kLog2e;
+            const float2 off2 = make_float2(off, off);
+            float *st = stats + ((it % kUStats) * 4 + blk) * kUQ + r;
+            st[0] = (mn == -INFINITY) ? 0.f : expf(before - mn);  // alpha
+            float sum = 0.f;
+            float2 es2 = make_float2(0.f, 0.f);  // the sums over the even and the odd ones of 32 columns
+            tmem_st_wait();
+            tmem_ld16(my_s, v[0]);
+#pragma unroll
+            for (int c = 0; c < 4; ++c) {
+                uint32_t(&w)[16] = v[c & 1];
+                tmem_ld_wait16(w);
+                if (c < 3) tmem_ld16(my_s + 16 * (c + 1), v[(c + 1) & 1]);
+                uint32_t codes[8];
+#pragma unroll
+                for (int e = 0; e < 8; ++e) {
+                    const float2 arg = __ffma2_rn(make_float2(__uint_as_float(w[2 * e]), __uint_as_float(w[2 * e + 1])), log2e2, off2);
                     const float2 pe = make_float2(ex2_approx(arg.x), ex2_approx(arg.y));
                     es2 = __fadd2_rn(es2, pe);
-                    c[e] = __float2int_rn(pe.x);  // in [0, 127]: rounds to nearest even like rint
-                    c[e + 1] = __float2int_rn(pe.y);
+                    const float2 code = __fadd2_rn(__fadd2_rn(pe, round2), unround2);
+                    asm("cvt.rn.f16x2.f32 %0, %1, %2;" : "=r"(codes[e]) : "f"(code.y), "f"(code.x));
                 }
-                w[q] = pack_codes(c);
+                tmem_st8(my_s + 8 * c, codes);  // (columns that have been read)
+                if (c == 1) {
+                    sum = es2.x + es2.y;
+                    es2 = make_float2(0.f, 0.f);
+                }
             }
-            *reinterpret_cast<uint4 *>(swz(Ps, (int)r, 2 * g + piece)) = make_uint4(w[0], w[1], w[2], w[3]);
-        };
-        // ---- the exponentials of this iteration (bound by the special-function unit) and, between
-        // them, the products of the iteration before folded into the output (bound by issue slots):
-        // with the warps of a scheduler at different places of this stretch the two overlap.  The
-        // PV accumulators have a tensor-memory region of their own, so they may stay there until
-        // the next PV product is issued after the second barrier.  (Both blocks of the iteration
-        // before exist: only the last iteration can lack its second block.)
-        bool pv_ok = true;
-        if (it > 0) {
-            pv_ok = mbar_wait(bar_pv, (it - 1) & 1, abort_flag, limit);
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            st[2 * kUQ] = sum + (es2.x + es2.y);
+            tmem_st_wait();
+            tc_fence_before();
+            __syncwarp();
+            if (lane0) mbar_arrive(bars->p + g);
+            if (it + 2 < n_it) read_digits(it + 2);
         }
-        const bool fold = it > 0 && pv_ok;
-        const float *vd_prev = vscale_of(it + kUBufs - 1);
-        if (fold) tmem_ld32(my_tmem + kUPVCol + 32 * g, v);
-        exp_piece(0);
-        if (fold) {
-            tmem_ld_wait();
-            fold_block(prev_alpha_a, vd_prev);
-            tmem_ld32(my_tmem + kUPVCol + kUD + 32 * g, v);
-        }
-        exp_piece(1);
-        if (fold) {
-            tmem_ld_wait();
-            fold_block(prev_alpha_b, vd_prev + kUD);
-        }
-        xe[g * kUQ + r] = es2.x + es2.y;
-        // ---- PV of this iteration: the P codes are in shared memory, the accumulators of the
-        // iteration before have been read out, and nobody reads that iteration's record any more
-        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-        if (!__syncthreads_and(pv_ok)) {
-            dead = true;
-            dead_it = it;
-            break;
-        }
-        if (lane0) {
-            if (warp == kUWarpPV) {
-                const uint32_t vt = smem_u32(Rb + buf * kURecStride + kURecKBytes);
-                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    } else if (warp < kUIssueWarp) {
+        // ---------------------------------------------------------------- output: 64 channels of a row a thread
+        asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kURegsOutput));
+        const uint32_t half = warp / 4 - kUOutWarp / 4, my_pv = tmem_base + lanes + kUPVCol + 64 * half;
+        float2 o[32];  // the channels in pairs
 #pragma unroll
-                for (int blk = 0; blk < 2; ++blk)
+        for (int c = 0; c < 32; ++c) o[c] = make_float2(0.f, 0.f);
+        float l = 0.f;
+        for (int it = 0; it < n_it && ok; ++it) {
+            const int vbuf = it % kUVBufs;
+            const float *st = stats + (it % kUStats) * 4 * kUQ + r;
+            const float4 *vs4 = reinterpret_cast<const float4 *>(Vb + vbuf * kVStride + 2 * kURecVTileBytes) + 16 * half;
 #pragma unroll
-                    for (int k = 0; k < 2; ++k)
-                        umma_i8(tmem_base + kUPVCol + kUD * blk, umma_desc(smem_u32(Ps) + (2 * blk + k) * 32),
-                                umma_desc(vt + (2 * blk + k) * 32), idesc_pv, k != 0);
-                umma_commit(bar_pv);
+            for (int blk = 0; blk < 2; ++blk) {
+                // (with block a's barrier come the alphas, the sums and the scales that the issuing thread has seen)
+                ok = ok && mbar_wait(bars->pv + blk, it & 1, abort_flag, limit);  // (given up: the loop ends below)
+                tc_fence_after();
+                const float alpha = st[blk * kUQ];
+                const float2 al2 = make_float2(alpha, alpha);
+                l = alpha * l + st[(2 + blk) * kUQ];
+                uint32_t v[2][16];
+                tmem_ld16(my_pv + kUD * blk, v[0]);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    uint32_t(&w)[16] = v[c & 1];
+                    tmem_ld_wait16(w);
+                    if (c < 3) {
+                        tmem_ld16(my_pv + kUD * blk + 16 * (c + 1), v[(c + 1) & 1]);
+                    } else {
+                        tc_fence_before();
+                        __syncwarp();
+                        if (lane0) mbar_arrive(bars->pv_read + blk);
+                    }
+                    // o = alpha * o + PV * dV, two channels an instruction
+#pragma unroll
+                    for (int e = 0; e < 4; ++e) {
+                        const float4 d = vs4[(kUD * blk + 16 * c) / 4 + e];
+                        float2 &x = o[8 * c + 2 * e], &y = o[8 * c + 2 * e + 1];
+                        x = __ffma2_rn(al2, x, __fmul2_rn(make_float2(__uint_as_float(w[4 * e]), __uint_as_float(w[4 * e + 1])),
+                                                          make_float2(d.x, d.y)));
+                        y = __ffma2_rn(al2, y, __fmul2_rn(make_float2(__uint_as_float(w[4 * e + 2]), __uint_as_float(w[4 * e + 3])),
+                                                          make_float2(d.z, d.w)));
+                    }
+                }
             }
-            if (warp == kUWarpRec && it + 2 < n_it) stage(it + 2);  // into the buffer of the iteration before
+            __syncwarp();
+            if (lane0) mbar_arrive(bars->v_free + vbuf);
         }
-        __syncwarp();
-        l = alpha_a * l + (xe[r] + xe[kUQ + r]);
-        l = alpha_b * l + (xe[2 * kUQ + r] + xe[3 * kUQ + r]);
-        m = m_b;
-        prev_alpha_a = alpha_a;
-        prev_alpha_b = alpha_b;
-    }
-    if (!dead) {
-        if (!__syncthreads_and(mbar_wait(bar_pv, (n_it - 1) & 1, abort_flag, limit))) {
-            dead = true;
-        } else {
-            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-            const float *vd_last = vscale_of(n_it - 1);
-            tmem_ld32(my_tmem + kUPVCol + 32 * g, v);
-            tmem_ld_wait();
-            fold_block(prev_alpha_a, vd_last);
-            if (2 * (n_it - 1) + 1 < jb_hi) {  // (the same for the whole CTA)
-                tmem_ld32(my_tmem + kUPVCol + kUD + 32 * g, v);
-                tmem_ld_wait();
-                fold_block(prev_alpha_b, vd_last + kUD);
+        if (ok && valid) {
+            float *dst = a.out + (row_base + i) * kUD + 64 * half;
+#pragma unroll
+            for (int c = 0; c < 32; c += 2)
+                *reinterpret_cast<float4 *>(dst + 2 * c) =
+                    make_float4(o[c].x / l, o[c].y / l, o[c + 1].x / l, o[c + 1].y / l);
+        }
+    } else {
+        asm volatile("setmaxnreg.dec.sync.aligned.u32 %0;" ::"n"(kURegsIssue));
+        if (warp == kUIssueWarp) {
+            // ------------------------------------------------------------ the products
+            const uint32_t idesc_s = umma_idesc_i8(kUKeys), idesc_d = umma_idesc_i8(16), idesc_pv = umma_idesc_f16(kUD);
+            const uint64_t q_desc = umma_desc(smem_u32(Qs)), k_desc0 = umma_desc(smem_u32(Kb)), v_desc0 = umma_desc(smem_u32(Vb));
+            // (one thread each; descriptors count in sixteen bytes)
+            auto issue_digits = [&](int it) {
+                const uint64_t d = k_desc0 + (((it % kUKBufs) * kKStride + kUKeys * 128) >> 4);
+#pragma unroll
+                for (int k = 0; k < kUD / 32; ++k)
+                    umma_i8(tmem_base + 128 * (it & 1) + kUDigitCol, q_desc + 2 * k, d + 2 * k, idesc_d, k != 0);
+                umma_commit(bars->digits + (it & 1));
+            };
+            auto issue_s = [&](int it) {
+                const uint64_t d = k_desc0 + (((it % kUKBufs) * kKStride) >> 4);
+#pragma unroll
+                for (int k = 0; k < kUD / 32; ++k)
+                    umma_i8(tmem_base + 128 * (it & 1), q_desc + 2 * k, d + 2 * k, idesc_s, k != 0);
+                umma_commit(bars->s + (it & 1));
+            };
+            auto issue_pv = [&](int it, int blk) {
+                const uint64_t d = v_desc0 + (((it % kUVBufs) * kVStride + blk * kURecVTileBytes) >> 4);
+#pragma unroll
+                for (int k = 0; k < kUBlk / 16; ++k)
+                    umma_f16_ts(tmem_base + kUPVCol + kUD * blk, tmem_base + 128 * (it & 1) + 64 * blk + 8 * k, d + 2 * k,
+                                idesc_pv, k != 0);
+                umma_commit(bars->pv + blk);
+                if (blk == 0) mbar_arrive(bars->pv);
+            };
+            for (int it = 0; it < 2 && it < n_it && ok; ++it) {
+                ok = mbar_wait(bars->k + it, 0, abort_flag, limit);
+                if (ok && elect_one()) issue_digits(it);
+                __syncwarp();
+            }
+            for (int it = 0; it < 2 && it < n_it && ok; ++it) {
+                ok = mbar_wait(bars->digits_read + it, 0, abort_flag, limit);
+                tc_fence_after();
+                if (ok && elect_one()) issue_s(it);
+                __syncwarp();
+            }
+            for (int it = 0; it < n_it && ok; ++it) {
+                const int g = it & 1;
+                const bool more = it + 2 < n_it;
+                ok = mbar_wait(bars->v + it % kUVBufs, (it / kUVBufs) & 1, abort_flag, limit);
+                if (more) ok = ok && mbar_wait(bars->k + (it + 2) % kUKBufs, ((it + 2) / kUKBufs) & 1, abort_flag, limit);
+                if (it > 0) ok = ok && mbar_wait(bars->pv_read, (it - 1) & 1, abort_flag, limit) &&
+                                 mbar_wait(bars->pv_read + 1, (it - 1) & 1, abort_flag, limit);
+                ok = ok && mbar_wait(bars->p + g, (it >> 1) & 1, abort_flag, limit);
+                if (!ok) break;
+                tc_fence_after();
+                if (elect_one()) {
+                    if (more) issue_digits(it + 2);  // (over scores that have become P codes)
+                    issue_pv(it, 0);
+                    issue_pv(it, 1);
+                }
+                __syncwarp();
+                if (!more) continue;
+                ok = mbar_wait(bars->digits_read + g, ((it + 2) >> 1) & 1, abort_flag, limit);
+                if (!ok) break;
+                tc_fence_after();
+                if (elect_one()) issue_s(it + 2);  // (over the P codes, behind the products that read them)
+                __syncwarp();
+            }
+        } else if (warp == kUCopyWarp) {
+            // ------------------------------------------------------------ the records' halves
+            const uint8_t *rec = a.rec + plane * (size_t)((n_blocks + 1) / 2) * kURecStride;
+            auto copy = [&](uint8_t *dst, const uint8_t *src, uint32_t bytes, uint64_t *bar) {
+                if (lane0) {
+                    asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(bar)), "r"(bytes)
+                                 : "memory");
+                    asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                                     smem_u32(dst)),
+                                 "l"(src), "r"(bytes), "r"(smem_u32(bar))
+                                 : "memory");
+                }
+                __syncwarp();
+            };
+            auto copy_k = [&](int it) {
+                copy(Kb + (it % kUKBufs) * kKStride, rec + (size_t)it * kURecStride, kURecKBytes, bars->k + it % kUKBufs);
+                got_k = it + 1;
+            };
+            auto copy_v = [&](int it) {
+                copy(Vb + (it % kUVBufs) * kVStride, rec + (size_t)it * kURecStride + kURecVOff, kURecVBytes,
+                     bars->v + it % kUVBufs);
+                got_v = it + 1;
+            };
+            for (int it = 0; it < kUKBufs && it < n_it; ++it) {
+                copy_k(it);
+                if (it < kUVBufs) copy_v(it);
+            }
+            for (int it = kUVBufs; it < n_it && ok; ++it) {
+                if (it + 1 >= kUKBufs && it + 1 < n_it) {
+                    ok = mbar_wait(bars->k_free + (it + 1) % kUKBufs, ((it + 1 - kUKBufs) / kUKBufs) & 1, abort_flag, limit);
+                    if (!ok) break;
+                    copy_k(it + 1);
+                }
+                ok = mbar_wait(bars->v_free + it % kUVBufs, ((it - kUVBufs) / kUVBufs) & 1, abort_flag, limit);
+                if (ok) copy_v(it);
             }
         }
     }
-    if (dead) {
+    if (!ok) *abort_flag = 1;
+    tc_fence_before();
+    __syncthreads();
+    if (*abort_flag) {
         // Given up: before tensor memory is handed back, the products that were issued must have
         // finished.  A commit on a barrier of its own arrives when everything issued so far is
         // done; it is waited for with the default (long) limit, not the one that just expired.
-        // The same for the records still on their way into shared memory: the one of the
-        // iteration that gave up and the one after it (later ones have not been asked for).
-        __syncthreads();
-        // (a commit covers the products its own thread has issued: both issuing threads commit)
-        if ((warp == kUWarpS || warp == kUWarpPV) && lane0) umma_commit(bar_drain);
-        __syncwarp();
-        if (warp == 0) {
-            volatile int never = 0;
-            (void)mbar_wait(bar_drain, 0, &never, kUWaitLimitDefault);
-            for (int k = dead_it; k < min(n_it, dead_it + 2); ++k)
-                (void)mbar_wait(bar_rec + k % kUBufs, (k / kUBufs) & 1, &never, kUWaitLimitDefault);
+        // The same for the copies still on their way into shared memory.
+        tc_fence_after();
+        if (warp == kUIssueWarp) {
+            if (elect_one()) umma_commit(&bars->drain);
+            __syncwarp();
+            (void)mbar_wait(&bars->drain, 0, &bars->never, kUWaitLimitDefault);
         }
+        for (int k = max(0, got_k - kUKBufs); k < got_k; ++k)
+            (void)mbar_wait(bars->k + k % kUKBufs, (k / kUKBufs) & 1, &bars->never, kUWaitLimitDefault);
+        for (int k = max(0, got_v - kUVBufs); k < got_v; ++k)
+            (void)mbar_wait(bars->v + k % kUVBufs, (k / kUVBufs) & 1, &bars->never, kUWaitLimitDefault);
+        tc_fence_before();
+        __syncthreads();
     }
-    if (dead) *abort_flag = 1;
-    if (valid && !dead) {
-        float *dst = a.out + (row_base + i) * kUD + 32 * g;
-#pragma unroll
-        for (int c = 0; c < 16; c += 2)
-            *reinterpret_cast<float4 *>(dst + 2 * c) =
-                make_float4(o[c].x / l, o[c].y / l, o[c + 1].x / l, o[c + 1].y / l);
-    }
-    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
-    __syncthreads();
     if (warp == 0)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(kUTmemCols)
                      : "memory");
@@ -1355,18 +1614,6 @@ __device__ __forceinline__ void umma_bf16(uint32_t d_tmem, uint64_t a_desc, uint
         "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
         : "memory");
 }
-__device__ __forceinline__ void tmem_st32(uint32_t taddr, const uint32_t (&v)[32]) {
-    asm volatile(
-        "tcgen05.st.sync.aligned.32x32b.x32.b32 [%0], "
-        "{%1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, %16, %17, %18, %19, %20, %21, %22, "
-        "%23, %24, %25, %26, %27, %28, %29, %30, %31, %32};" ::"r"(taddr),
-        "r"(v[0]), "r"(v[1]), "r"(v[2]), "r"(v[3]), "r"(v[4]), "r"(v[5]), "r"(v[6]), "r"(v[7]), "r"(v[8]), "r"(v[9]),
-        "r"(v[10]), "r"(v[11]), "r"(v[12]), "r"(v[13]), "r"(v[14]), "r"(v[15]), "r"(v[16]), "r"(v[17]), "r"(v[18]),
-        "r"(v[19]), "r"(v[20]), "r"(v[21]), "r"(v[22]), "r"(v[23]), "r"(v[24]), "r"(v[25]), "r"(v[26]), "r"(v[27]),
-        "r"(v[28]), "r"(v[29]), "r"(v[30]), "r"(v[31])
-        : "memory");
-}
-
 __global__ void __launch_bounds__(kUThreads, 1)
 attention_sage_block_kernel(SageArgs a, AttnDims dm, int causal, uint32_t wait_limit, int *error) {
     extern __shared__ __align__(1024) uint8_t sm_b_raw[];
@@ -1820,8 +2067,17 @@ uint8_t *sage_records(uint8_t *base, const SageLayout &L) {
 qk_status sage_quantize_dev(qk_ctx *c, const float *dq, const float *dk, const float *dv,
                             uint8_t *base, const AttnDims &dm, const SageLayout &L) {
     const size_t S = dm.Skv;
-    uint8_t *rec = L.umma ? sage_records(base, L) : nullptr;
     const float inv_sqrt_d = 1.0f / sqrtf((float)dm.d);  // gpu_attention.rs:720
+    if (L.umma) {
+        const size_t kv_blocks = 2 * L.planes * L.n_blocks, q_blocks = qk::ceil_div(L.qrows, (size_t)kPrepRows);
+        (void)qk::launch_pdl(c->pdl, sage_prepare_kernel, dim3((unsigned)(kv_blocks + q_blocks)), dim3(kPrepThreads), 0,
+                             c->stream, dq, dk, dv, (int8_t *)(base + L.o_qc), (float *)(base + L.o_qs),
+                             (float *)(base + L.o_km), sage_records(base, L), (uint32_t)L.qrows, (uint32_t)S,
+                             (uint32_t)L.n_blocks, (uint32_t)L.planes, inv_sqrt_d);
+        QK_CUDA(cudaGetLastError());
+        c->launches++;
+        return QK_OK;
+    }
     sage_quant_q_kernel<<<(unsigned)qk::ceil_div(L.qrows, 8), 256, 0, c->stream>>>(
         dq, (int8_t *)(base + L.o_qc), (float *)(base + L.o_qs), (uint32_t)L.qrows, dm.d,
         (uint32_t)L.dpad, inv_sqrt_d);
@@ -1830,11 +2086,11 @@ qk_status sage_quantize_dev(qk_ctx *c, const float *dq, const float *dk, const f
     sage_quant_k_kernel<<<kgrid, 128, dm.d * sizeof(float), c->stream>>>(
         dk, (int8_t *)(base + L.o_kc), (float *)(base + L.o_ks), (float *)(base + L.o_km), (uint32_t)S,
         dm.d, (uint32_t)L.dpad, (uint32_t)L.block, (uint32_t)L.n_blocks,
-        L.tc ? (int8_t *)(base + L.o_md) : nullptr, (float *)(base + L.o_ms), rec);
+        L.tc ? (int8_t *)(base + L.o_md) : nullptr, (float *)(base + L.o_ms), nullptr);
     QK_CUDA(cudaGetLastError());
     sage_quant_v_kernel<<<kgrid, 128, 0, c->stream>>>(
         dv, (int8_t *)(base + L.o_vc), (float *)(base + L.o_vs), (uint32_t)S, dm.dv,
-        (uint32_t)L.block, (uint32_t)L.bpad, (uint32_t)L.n_blocks, L.tc && !L.umma ? 1 : 0, rec);
+        (uint32_t)L.block, (uint32_t)L.bpad, (uint32_t)L.n_blocks, L.tc ? 1 : 0);
     QK_CUDA(cudaGetLastError());
     c->launches += 3;
     return QK_OK;
@@ -1860,9 +2116,9 @@ qk_status attention_sage_dev(qk_ctx *c, const float *dq, const float *dk, const 
         c->err_armed = true;
         QK_CUDA(cudaFuncSetAttribute(attention_sage_umma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                      (int)(kUSmemBytes + 1024)));
-        dim3 grid((unsigned)qk::ceil_div(dm.Sq, kUQ), dm.H, dm.B);
-        attention_sage_umma_kernel<<<grid, kUThreads, kUSmemBytes + 1024, c->stream>>>(a, dm, causal, c->wait_limit,
-                                                                                 (int *)c->d_err.ptr);
+        const dim3 grid(dm.H, (unsigned)qk::ceil_div((size_t)dm.Sq, (size_t)kUQ), dm.B);
+        (void)qk::launch_pdl(c->pdl, attention_sage_umma_kernel, grid, dim3(kUAllThreads), kUSmemBytes + 1024, c->stream, a,
+                             dm, causal, c->wait_limit, (int *)c->d_err.ptr);
         QK_CUDA(cudaGetLastError());
         c->launches++;
         return QK_OK;
@@ -1906,7 +2162,7 @@ qk_status attention_sage_block_dev(qk_ctx *c, const float *dq, const float *dk, 
     dim3 kgrid((unsigned)n_blocks, (unsigned)planes);
     sage_quant_k_kernel<<<kgrid, 128, dm.d * sizeof(float), c->stream>>>(
         dk, nullptr, nullptr, (float *)km, (uint32_t)S, dm.d, 128u, (uint32_t)kUBlk, (uint32_t)n_blocks, nullptr, nullptr,
-        rec, kBRecStride, kBRecScaleOff, (uint32_t)kUKeys, 1);
+        rec);
     QK_CUDA(cudaGetLastError());
     sage_v_bf16_record_kernel<<<kgrid, 128, 0, c->stream>>>(dv, rec, (uint32_t)S, (uint32_t)n_blocks);
     QK_CUDA(cudaGetLastError());
@@ -2098,21 +2354,26 @@ qk_status qk_gpu_sage_quantize(qk_ctx *ctx, const qk_attention_shape *shape, con
         // the tcgen05 kernel's records: undo the row swizzle
         const uint8_t *rec = host.data() + (qk::sage_records(base + o_scratch, L) - (base + o_scratch));
         const size_t n_rec = (L.n_blocks + 1) / 2;
+        auto float16_code = [](const uint8_t *p) {
+            __half v;
+            std::memcpy(&v, p, 2);
+            return (int8_t)__half2float(v);
+        };
         for (size_t p = 0; p < L.planes; ++p) {
             for (size_t j = 0; j < S; ++j) {
                 const uint8_t *rc = rec + (p * n_rec + j / 128) * kURecStride;
                 for (size_t ch = 0; ch < d; ++ch)
                     k_codes[(p * S + j) * d + ch] = (int8_t)rc[rec_tile_offset((uint32_t)(j % 128), (uint32_t)ch)];
-                std::memcpy(k_scale + p * S + j, rc + kURecScaleOff + 4 * (j % 128), 4);
+                std::memcpy(k_scale + p * S + j, rc + kURecTileBytes + 4 * (j % 128), 4);
             }
             for (size_t jb = 0; jb < L.n_blocks; ++jb) {
                 const uint8_t *rc = rec + (p * n_rec + jb / 2) * kURecStride;
-                std::memcpy(v_scale + (p * L.n_blocks + jb) * dv_, rc + kURecScaleOff + 4 * (128 + 128 * (jb % 2)),
+                std::memcpy(v_scale + (p * L.n_blocks + jb) * dv_, rc + kURecVOff + 2 * kURecVTileBytes + 4 * 128 * (jb % 2),
                             dv_ * 4);
                 for (size_t ch = 0; ch < dv_; ++ch)
                     for (size_t kk = 0; kk < L.block && jb * L.block + kk < S; ++kk)
                         v_codes[(p * S + jb * L.block + kk) * dv_ + ch] =
-                            (int8_t)rc[kURecKBytes + rec_tile_offset((uint32_t)ch, (uint32_t)(64 * (jb % 2) + kk))];
+                            float16_code(rc + kURecVOff + (jb % 2) * kURecVTileBytes + rec_tile_offset((uint32_t)ch, (uint32_t)(2 * kk)));
             }
         }
         return QK_OK;

@@ -323,6 +323,38 @@ def test_sage_tcgen05_kernel_matches_the_other_kernels(gpu_ctx, case):
         gpu_ctx.set_sage_kernel(default)
 
 
+@pytest.mark.parametrize("causal", [True, False])
+@pytest.mark.parametrize("seq", [64, 65, 127, 128, 129, 191, 192, 193, 320, 385, 513, 1100])
+def test_sage_tcgen05_kernel_at_the_edges_of_its_tiles(gpu_ctx, seq, causal):
+    """Ends of query tiles, key blocks, pairs of blocks and buffer rings against the mma.sync kernel, whose integer sums
+    it must reproduce (1e-5 as above: the order in which l is summed); the quantisers' codes as well.  An infinite
+    value and a query row of NaN stay where they belong."""
+    b, h, kvh, d, block = 2, 3, 1, 128, 64
+    rng = np.random.default_rng(seq + causal)
+    q = rng.standard_normal((b, h, seq, d), dtype=np.float32)
+    k = rng.standard_normal((b, kvh, seq, d), dtype=np.float32) \
+        + (2.0 * rng.standard_normal((1, kvh, 1, d))).astype(np.float32)
+    v = rng.standard_normal((b, kvh, seq, d), dtype=np.float32)
+    q[1, 2, seq // 2] = np.nan
+    v[0, 0, 0, 5] = np.inf      # (a key that every row sees: a block's infinite scale reaches all rows that pass over the block)
+    default = gpu_ctx.set_sage_kernel(1)
+    try:
+        with np.errstate(invalid="ignore"):
+            tc = run_sage(gpu_ctx, q, k, v, causal, block)
+            codes = gpu_ctx.sage_quantize(shape_of(q, k, v), q, k, v, block)
+            gpu_ctx.set_sage_kernel(2)
+            um = run_sage(gpu_ctx, q, k, v, causal, block)
+            same = gpu_ctx.sage_quantize(shape_of(q, k, v), q, k, v, block)
+    finally:
+        gpu_ctx.set_sage_kernel(default)
+    assert np.array_equal(np.isnan(um), np.isnan(tc))
+    fine = np.isfinite(tc)
+    assert np.array_equal(um[~fine], tc[~fine], equal_nan=True)
+    assert np.abs(um[fine] - tc[fine]).max() <= 1e-5 * np.abs(tc[fine]).max()
+    for name in codes:
+        assert np.array_equal(codes[name], same[name], equal_nan=True), name
+
+
 def test_attention_on_device_buffers(gpu_ctx):
     import torch
     rng = np.random.default_rng(11)
