@@ -551,7 +551,7 @@ __device__ __noinline__ void attention_groups(const StepArgs &a, const StepSmem 
             const uint32_t rows = min(a.gq, group - hsub * a.gq);
             for (uint32_t r = sb.tid / 32; r < rows; r += 4) {  // a warp per head
                 const size_t head = (size_t)b * a.n_heads + h0 + r;
-                decode_combine_warp<4, 32>(sb.tid % 32, a.partial + head * a.n_splits * 130, a.attn + head * 128,
+                decode_combine_warp<4, 8>(sb.tid % 32, a.partial + head * a.n_splits * 130, a.attn + head * 128,
                                           128, a.n_splits, 0, 32);
             }
         }

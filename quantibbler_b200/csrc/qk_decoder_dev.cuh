@@ -86,12 +86,19 @@ __device__ __forceinline__ void mma_bf16_full(float (&c)[4], uint32_t a0, uint32
         : "r"(a0), "r"(a1), "r"(a2), "r"(a3), "r"(b0), "r"(b1));
 }
 
-// x = hi + mid + lo with each term a bfloat16 (to 2^-25 of x)
-__device__ __forceinline__ void split3(float x, uint32_t &hi, uint32_t &mid, uint32_t &lo) {
-    hi = float_to_bf16_bits(x);
-    const float r1 = x - bf16_bits_to_float((uint16_t)hi);
-    mid = float_to_bf16_bits(r1);
-    lo = float_to_bf16_bits(r1 - bf16_bits_to_float((uint16_t)mid));
+// x = t[0] + t[1] + t[2] with each term a bfloat16 (to 2^-25 of x), for two values side by side: a in the low halves
+__device__ __forceinline__ uint32_t bf16_pair(float a, float b) {
+    uint32_t w;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(w) : "f"(b), "f"(a));
+    return w;
+}
+__device__ __forceinline__ void split3(float a, float b, uint32_t (&t)[3]) {
+#pragma unroll
+    for (int i = 0; i < 3; ++i) {
+        t[i] = bf16_pair(a, b);
+        a -= __uint_as_float(t[i] << 16);
+        b -= __uint_as_float(t[i] & 0xffff0000u);
+    }
 }
 
 constexpr int kMmaDecWarps = 4;
@@ -162,6 +169,43 @@ __device__ __forceinline__ void decode_attention_mma_body(
     const uint32_t warp = sb.tid / 32, lane = sb.tid % 32, g = lane >> 2, t = lane & 3;
     const float scale = 1.0f / sqrtf((float)d);
 
+    const uint16_t *kb = cache_k + ((size_t)b * n_kv + kvh) * s_max * d;
+    const uint16_t *vb = cache_v + ((size_t)b * n_kv + kvh) * s_max * d;
+    // Each warp streams its 16-key steps through a private ring of kBufs shared-memory buffers
+    // with cp.async, so the next kBufs - 1 steps' 8 KB of K and V each are in flight while this
+    // one is multiplied.  Row pitches 320 B (K) and 272 B (V) keep the 16-byte fragment reads
+    // conflict-free.
+    uint8_t *my_smem = sm.stage + warp * sm.warp_bytes;
+    auto fetch = [&](int j, int buf) {
+        uint8_t *kt = my_smem + buf * kMmaDecBufBytes, *vt = kt + 16 * kMmaDecKPitch;
+#pragma unroll
+        for (int q = 0; q < 8; ++q) {
+            const int idx = (int)lane + 32 * q, key = idx / 16, piece = idx % 16;
+            const int src_key = min(j + key, j_end - 1);      // a valid address even when unused
+            const uint32_t bytes = j + key < j_end ? 16u : 0u;  // 0: the 16 bytes are zero-filled
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                             (uint32_t)__cvta_generic_to_shared(kt + key * kMmaDecKPitch + piece * 16)),
+                         "l"(kb + (size_t)src_key * d + piece * 8), "r"(bytes)
+                         : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                             (uint32_t)__cvta_generic_to_shared(vt + key * kMmaDecVPitch + piece * 16)),
+                         "l"(vb + (size_t)src_key * d + piece * 8), "r"(bytes)
+                         : "memory");
+        }
+        asm volatile("cp.async.commit_group;" ::: "memory");
+    };
+    constexpr int kStride = 16 * kMmaDecWarps;  // keys between a warp's steps
+    const int j_first = j_begin + 16 * (int)warp;
+    auto fetch_first = [&] {
+#pragma unroll
+        for (int ahead = 0; ahead < kBufs - 1; ++ahead)
+            if (j_first + ahead * kStride < j_end) fetch(j_first + ahead * kStride, ahead);
+    };
+    // The first keys are on their way while q is brought into shape (1.8 us, and the keys' 1.0 us used to follow); not where
+    // the key being appended is among this block's: it is written first.
+    const bool appends = kRope && fresh.pos >= j_begin && fresh.pos < (int)((split + 1) * chunk);
+    if (!appends) fetch_first();
+
     // A fragments of q: MMA m (0..7) contracts channels 32 (m/2) + 8 t + 4 (m%2) + {0,1 | 2,3}
     constexpr int kTerms = kPacked ? 2 : 3;
     uint32_t qa[kTerms][8][2];
@@ -199,18 +243,16 @@ __device__ __forceinline__ void decode_attention_mma_body(
             for (int half = 0; half < 2; ++half)
 #pragma unroll
                 for (int pr = 0; pr < 2; ++pr) {
-                    uint32_t e0[3], e1[3];
+                    uint32_t e[3];
                     const float x0 = qrow < rows ? v[4 * half + 2 * pr] * scale : 0.f;
                     const float x1 = qrow < rows ? v[4 * half + 2 * pr + 1] * scale : 0.f;
-                    split3(x0, e0[0], e0[1], e0[2]);
-                    split3(x1, e1[0], e1[1], e1[2]);
+                    split3(x0, x1, e);
                     if (kPacked) {
-                        qa[0][2 * i + half][pr] = upper ? (e0[1] | (e1[1] << 16)) : (e0[0] | (e1[0] << 16));
-                        qa[1][2 * i + half][pr] = upper ? 0u : (e0[2] | (e1[2] << 16));
+                        qa[0][2 * i + half][pr] = upper ? e[1] : e[0];
+                        qa[1][2 * i + half][pr] = upper ? 0u : e[2];
                     } else {
 #pragma unroll
-                        for (int term = 0; term < kTerms; ++term)
-                            qa[term][2 * i + half][pr] = e0[term] | (e1[term] << 16);
+                        for (int term = 0; term < kTerms; ++term) qa[term][2 * i + half][pr] = e[term];
                     }
                 }
         }
@@ -220,32 +262,7 @@ __device__ __forceinline__ void decode_attention_mma_body(
     for (int nt = 0; nt < 16; ++nt) o[nt][0] = o[nt][1] = 0.f;
     float m = -INFINITY, l = 0.f;  // row g; l is this lane's share (its own key columns)
 
-    const uint16_t *kb = cache_k + ((size_t)b * n_kv + kvh) * s_max * d;
-    const uint16_t *vb = cache_v + ((size_t)b * n_kv + kvh) * s_max * d;
-    // Each warp streams its 16-key steps through a private ring of kBufs shared-memory buffers
-    // with cp.async, so the next kBufs - 1 steps' 8 KB of K and V each are in flight while this
-    // one is multiplied.  Row pitches 320 B (K) and 272 B (V) keep the 16-byte fragment reads
-    // conflict-free.
-    uint8_t *my_smem = sm.stage + warp * sm.warp_bytes;
-    auto fetch = [&](int j, int buf) {
-        uint8_t *kt = my_smem + buf * kMmaDecBufBytes, *vt = kt + 16 * kMmaDecKPitch;
-#pragma unroll
-        for (int q = 0; q < 8; ++q) {
-            const int idx = (int)lane + 32 * q, key = idx / 16, piece = idx % 16;
-            const int src_key = min(j + key, j_end - 1);      // a valid address even when unused
-            const uint32_t bytes = j + key < j_end ? 16u : 0u;  // 0: the 16 bytes are zero-filled
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
-                             (uint32_t)__cvta_generic_to_shared(kt + key * kMmaDecKPitch + piece * 16)),
-                         "l"(kb + (size_t)src_key * d + piece * 8), "r"(bytes)
-                         : "memory");
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
-                             (uint32_t)__cvta_generic_to_shared(vt + key * kMmaDecVPitch + piece * 16)),
-                         "l"(vb + (size_t)src_key * d + piece * 8), "r"(bytes)
-                         : "memory");
-        }
-        asm volatile("cp.async.commit_group;" ::: "memory");
-    };
-    if (kRope && fresh.pos >= j_begin && fresh.pos < (int)((split + 1) * chunk)) {
+    if (appends) {
         // this block's keys include the position being appended: rotate k, write k and v into
         // the cache (every block of the kv head that covers the position writes the same bits)
         if (fresh.valid) {
@@ -266,12 +283,8 @@ __device__ __forceinline__ void decode_attention_mma_body(
         }
         sb.sync();
     }
+    if (appends) fetch_first();
     int buf = 0;
-    constexpr int kStride = 16 * kMmaDecWarps;  // keys between a warp's steps
-    const int j_first = j_begin + 16 * (int)warp;
-#pragma unroll
-    for (int ahead = 0; ahead < kBufs - 1; ++ahead)
-        if (j_first + ahead * kStride < j_end) fetch(j_first + ahead * kStride, ahead);
     for (int j = j_first; j < j_end; j += kStride, buf = buf + 1 == kBufs ? 0 : buf + 1) {
         // (groups still allowed in flight = the steps after this one that have been started)
         if (j + (kBufs - 1) * kStride < j_end) {
@@ -341,15 +354,14 @@ __device__ __forceinline__ void decode_attention_mma_body(
         uint32_t pa[kTerms][2];
 #pragma unroll
         for (int nt = 0; nt < 2; ++nt) {
-            uint32_t e0[3], e1[3];
-            split3(p[nt][0], e0[0], e0[1], e0[2]);
-            split3(p[nt][1], e1[0], e1[1], e1[2]);
+            uint32_t e[3];
+            split3(p[nt][0], p[nt][1], e);
             if (kPacked) {
-                pa[0][nt] = upper ? (e0[1] | (e1[1] << 16)) : (e0[0] | (e1[0] << 16));
-                pa[1][nt] = upper ? 0u : (e0[2] | (e1[2] << 16));
+                pa[0][nt] = upper ? e[1] : e[0];
+                pa[1][nt] = upper ? 0u : e[2];
             } else {
 #pragma unroll
-                for (int term = 0; term < kTerms; ++term) pa[term][nt] = e0[term] | (e1[term] << 16);
+                for (int term = 0; term < kTerms; ++term) pa[term][nt] = e[term];
             }
         }
 #pragma unroll
@@ -406,13 +418,19 @@ __device__ __forceinline__ void decode_attention_mma_body(
             for (int e = 0; e < 2; ++e) mine[64 * (nt / 8) + 8 * (2 * t + e) + nt % 8] = o[nt][e];
     }
     sb.sync();
-    for (uint32_t idx = sb.tid; idx < rows * d; idx += 128) {
-        const uint32_t r = idx / d, c = idx % d;
-        float mm = -INFINITY;
-        for (int w = 0; w < kMmaDecWarps; ++w) mm = fmaxf(mm, sm.m(w)[r]);
-        float ll = 0.f, oo = 0.f;
+    // (a thread has one channel of every row: the weights of a row's warps are the same for all of them)
+    for (uint32_t r = 0; r < rows; ++r) {
+        float ms[kMmaDecWarps], mm = -INFINITY;
+#pragma unroll
         for (int w = 0; w < kMmaDecWarps; ++w) {
-            const float wt = sm.m(w)[r] == -INFINITY ? 0.f : expf(sm.m(w)[r] - mm);
+            ms[w] = sm.m(w)[r];
+            mm = fmaxf(mm, ms[w]);
+        }
+        const uint32_t c = sb.tid;
+        float ll = 0.f, oo = 0.f;
+#pragma unroll
+        for (int w = 0; w < kMmaDecWarps; ++w) {
+            const float wt = ms[w] == -INFINITY ? 0.f : expf(ms[w] - mm);
             ll += sm.l(w)[r] * wt;
             oo += sm.o(w)[r * d + c] * wt;
         }
@@ -429,11 +447,13 @@ __device__ __forceinline__ void decode_attention_mma_body(
 // ONE warp: p = that head's n_splits <= 128 partials {m, l, o[d]}; the warp produces the
 // channels c0 + lane + i * c_stride, i < kCh (those below d).  The loads of kBatch splits are
 // issued together, the products are added in split order, so the result does not depend on
-// kCh or kBatch.  No shared memory, no block barrier.
+// kCh or kBatch.  No shared memory, no block barrier.  (Sixteen splits of four heads by the last block of a step at batch 1:
+// 4 to 8 us with the loads of 32 splits unrolled and four rounds of weights, whatever the number of splits.)
 template <int kCh, int kBatch>
 __device__ __forceinline__ void decode_combine_warp(uint32_t lane, const float *__restrict__ p,
                                                     float *__restrict__ out, uint32_t d, uint32_t n_splits,
                                                     uint32_t c0, uint32_t c_stride) {
+    const uint32_t rounds = (n_splits + 31) / 32;  // (at most four)
     float ms[4], ls[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -443,9 +463,10 @@ __device__ __forceinline__ void decode_combine_warp(uint32_t lane, const float *
     }
     float mm = fmaxf(fmaxf(ms[0], ms[1]), fmaxf(ms[2], ms[3]));
     for (int off = 16; off > 0; off >>= 1) mm = fmaxf(mm, __shfl_xor_sync(0xffffffffu, mm, off));
-    float wv[4], ll = 0.f;
+    float wv[4] = {}, ll = 0.f;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
+        if (i >= (int)rounds) break;
         wv[i] = ms[i] == -INFINITY ? 0.f : expf(ms[i] - mm);
         float part = ls[i] * wv[i];
         for (int off = 16; off > 0; off >>= 1) part += __shfl_xor_sync(0xffffffffu, part, off);
