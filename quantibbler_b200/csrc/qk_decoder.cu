@@ -619,13 +619,17 @@ decode_attention_rope_kernel(const float *__restrict__ q, const float *__restric
 // A CTA of four warps owns 64 query rows that share one kv head: `hw` = min(group, 4) query
 // heads times 4/hw blocks of 16 positions, one (head, position block) per warp, so that a K/V
 // tile staged in shared memory serves the whole GQA group.  Q is split once into its three
-// terms in shared memory; K/V tiles of 32 keys are double-buffered with cp.async; all
-// fragments come from ldmatrix (row pitch 272 bytes: conflict-free), a step ahead of their products; a channel tile's
-// three terms are added with other tiles' between them (2048 tokens of 32 heads: 531 -> 463 us, the terms' split by
-// hardware conversions included).
+// terms in shared memory; K and V of a tile of 32 keys have one buffer each and come in by cp.async
+// during the other's product, so that three CTAs fit an SM; all fragments come from ldmatrix (row pitch
+// 272 bytes: conflict-free), a step ahead of their products; a channel tile's three terms are added with
+// other tiles' between them.
+// What bounds it: the legacy tensor pipe, 54 % busy with two CTAs to an SM, and the chains around it.  2048 tokens of 32
+// heads, us: two CTAs with double buffers 531, the order of the products and the terms' split by hardware
+// conversions 463, three CTAs and the longest blocks first 341.
 constexpr int kPfKeys = 32, kPfPitch = 136;  // keys per tile; bf16 elements per staged row
 constexpr int kPfQBytes = 3 * 64 * kPfPitch * 2, kPfTileBytes = kPfKeys * kPfPitch * 2;
-constexpr int kPfSmem = kPfQBytes + 4 * kPfTileBytes;
+constexpr int kPfSmem = kPfQBytes + 2 * kPfTileBytes;
+static_assert(3 * (kPfSmem + 1024) <= 227 * 1024, "three CTAs fit an SM");
 
 __device__ __forceinline__ void ldsm_x4(uint32_t (&r)[4], uint32_t addr) {
     asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];"
@@ -645,7 +649,7 @@ __device__ __forceinline__ void mma_bf16_full(float (&c)[4], const uint32_t (&a)
         : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, 3)
 prefill_attention_mma_kernel(const float *__restrict__ q, const uint16_t *__restrict__ cache_k,
                              const uint16_t *__restrict__ cache_v, float *__restrict__ out,
                              uint32_t n_tokens, uint32_t p0, uint32_t seq, uint32_t n_heads, uint32_t n_kv,
@@ -655,40 +659,40 @@ prefill_attention_mma_kernel(const float *__restrict__ q, const uint16_t *__rest
     constexpr uint32_t d = 128;
     extern __shared__ __align__(16) uint8_t pf_smem[];
     uint16_t *Qs = reinterpret_cast<uint16_t *>(pf_smem);                 // [3][64][pitch]
-    uint8_t *tiles = pf_smem + kPfQBytes;                                 // [2 buffers][K, V][32][pitch]
+    uint8_t *tiles = pf_smem + kPfQBytes;                                 // [K, V][32][pitch]
     const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32, g = lane >> 2, t = lane & 3;
     const uint32_t group = n_heads / n_kv, subs = group / hw;             // CTAs per kv head and position range
-    const uint32_t kvh = blockIdx.y / subs, hsub = blockIdx.y % subs;
+    // the last tokens see the most keys: they go first, all heads of a block of tokens side by side
+    const uint32_t per_block = n_kv * subs, hy = blockIdx.x % per_block;
+    const uint32_t block = gridDim.x / per_block - 1 - blockIdx.x / per_block;
+    const uint32_t kvh = hy / subs, hsub = hy % subs;
     const uint32_t pbs = 4 / hw;                                          // 16-position blocks per CTA
     const uint32_t head = kvh * group + hsub * hw + warp % hw;
-    const uint32_t tok0 = (blockIdx.x * pbs + warp / hw) * 16;            // this warp's first token
-    const uint32_t cta_tok_end = min(n_tokens, (blockIdx.x + 1) * pbs * 16);
+    const uint32_t tok0 = (block * pbs + warp / hw) * 16;                 // this warp's first token
+    const uint32_t cta_tok_end = min(n_tokens, (block + 1) * pbs * 16);
     const uint32_t n_tiles = (p0 + cta_tok_end + kPfKeys - 1) / kPfKeys;  // keys 0 .. p0 + last token
     const float scale = 1.0f / sqrtf((float)d);
 
     const uint16_t *kb = cache_k + ((size_t)seq * n_kv + kvh) * s_max * d;
     const uint16_t *vb = cache_v + ((size_t)seq * n_kv + kvh) * s_max * d;
-    auto fetch = [&](uint32_t jt, uint32_t buf) {
-        uint8_t *kt = tiles + buf * 2 * kPfTileBytes, *vt = kt + kPfTileBytes;
-        // 32 keys x 16 pieces of 16 bytes, for K and for V: 8 of each per thread
+    auto fetch = [&](const uint16_t *src, uint8_t *dst, uint32_t jt) {  // K or V of a tile: four pieces of 16 bytes a thread
+        if (jt < n_tiles)
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-            const uint32_t idx = threadIdx.x + 128 * i, key = idx / 16, piece = idx % 16;
-            const uint32_t j = jt * kPfKeys + key;
-            const uint32_t src_j = min(j, s_max - 1);              // a valid address even when unused
-            const uint32_t bytes = j < p0 + cta_tok_end ? 16u : 0u;  // 0: zero-filled
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
-                             (uint32_t)__cvta_generic_to_shared(kt + (key * kPfPitch + piece * 8) * 2)),
-                         "l"(kb + (size_t)src_j * d + piece * 8), "r"(bytes)
-                         : "memory");
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
-                             (uint32_t)__cvta_generic_to_shared(vt + (key * kPfPitch + piece * 8) * 2)),
-                         "l"(vb + (size_t)src_j * d + piece * 8), "r"(bytes)
-                         : "memory");
-        }
+            for (int i = 0; i < 4; ++i) {
+                const uint32_t idx = threadIdx.x + 128 * i, key = idx / 16, piece = idx % 16;
+                const uint32_t j = jt * kPfKeys + key;
+                const uint32_t src_j = min(j, s_max - 1);              // a valid address even when unused
+                const uint32_t bytes = j < p0 + cta_tok_end ? 16u : 0u;  // 0: zero-filled
+                asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
+                                 (uint32_t)__cvta_generic_to_shared(dst + (key * kPfPitch + piece * 8) * 2)),
+                             "l"(src + (size_t)src_j * d + piece * 8), "r"(bytes)
+                             : "memory");
+            }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    fetch(0, 0);
+    uint8_t *k_tile = tiles, *v_tile = tiles + kPfTileBytes;
+    fetch(kb, k_tile, 0);
+    fetch(vb, v_tile, 0);
 
     // ---- this warp's 16 query rows, scaled and split into three bfloat16 terms
     for (uint32_t idx = lane; idx < 16 * (d / 4); idx += 32) {
@@ -714,21 +718,16 @@ prefill_attention_mma_kernel(const float *__restrict__ q, const uint16_t *__rest
     const uint32_t q_addr0 = (uint32_t)__cvta_generic_to_shared(
         Qs + ((size_t)warp * 16 + (lane & 7) + ((lane >> 3) & 1) * 8) * kPfPitch + (lane >> 4) * 8);
 
+    const uint32_t kt_addr = (uint32_t)__cvta_generic_to_shared(k_tile), vt_addr = (uint32_t)__cvta_generic_to_shared(v_tile);
+    // K and V of a tile have one buffer each: K of the next tile comes in during the second product, V during the first
     for (uint32_t jt = 0; jt < n_tiles; ++jt) {
-        const uint32_t buf = jt & 1;
-        if (jt + 1 < n_tiles) {
-            fetch(jt + 1, buf ^ 1);
-            asm volatile("cp.async.wait_group 1;" ::: "memory");
-        } else {
-            asm volatile("cp.async.wait_group 0;" ::: "memory");
-        }
-        __syncthreads();  // tile jt has landed for every thread
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();  // K of the tile has landed for every thread
         const uint32_t j0 = jt * kPfKeys;
-        if (tok0 < n_tokens && j0 <= warp_last) {  // warp-uniform: the tile holds keys this warp sees
-            const uint32_t kt_addr = (uint32_t)__cvta_generic_to_shared(tiles + buf * 2 * kPfTileBytes);
-            const uint32_t vt_addr = kt_addr + kPfTileBytes;
+        const bool live = tok0 < n_tokens && j0 <= warp_last;  // warp-uniform: the tile holds keys this warp sees
+        float sacc[4][4];
+        if (live) {
             // ---- S = q k^T for 32 keys: four 8-key tiles
-            float sacc[4][4];
 #pragma unroll
             for (int nt = 0; nt < 4; ++nt) sacc[nt][0] = sacc[nt][1] = sacc[nt][2] = sacc[nt][3] = 0.f;
             // (a k-step's fragments are fetched while the step before is multiplied)
@@ -752,6 +751,11 @@ prefill_attention_mma_kernel(const float *__restrict__ q, const uint16_t *__rest
                         mma_bf16_full(sacc[nt], qf[ks & 1][term], kf[ks & 1][nt / 2][(nt % 2) * 2],
                                       kf[ks & 1][nt / 2][(nt % 2) * 2 + 1]);
             }
+        }
+        __syncthreads();
+        fetch(kb, k_tile, jt + 1);
+        uint32_t pa[3][2][4];  // [term][16-key step][A fragment]
+        if (live) {
             // ---- causal mask and online softmax (rows g and g + 8; columns 2t, 2t+1 of each tile)
             float mx[2] = {-INFINITY, -INFINITY};
 #pragma unroll
@@ -773,7 +777,6 @@ prefill_attention_mma_kernel(const float *__restrict__ q, const uint16_t *__rest
                 alpha[r] = m_new == -INFINITY ? 1.f : expf(m_row[r] - m_new);
                 m_row[r] = m_new;
             }
-            uint32_t pa[3][2][4];  // [term][16-key step][A fragment]
             float psum[2] = {0.f, 0.f};
 #pragma unroll
             for (int nt = 0; nt < 4; ++nt) {
@@ -802,6 +805,10 @@ prefill_attention_mma_kernel(const float *__restrict__ q, const uint16_t *__rest
                 o[nd][2] *= alpha[1];
                 o[nd][3] *= alpha[1];
             }
+        }
+        asm volatile("cp.async.wait_group 1;" ::: "memory");
+        __syncthreads();  // V of the tile has landed for every thread
+        if (live) {
             // ---- O += P V: two 16-key steps, sixteen 8-channel tiles, four of them at a time: a tile's three terms are
             // added one after the other, with three other tiles between two of them
             uint32_t vf[2][2][4];  // [parity][pair of the four][B fragments of channel tiles nd, nd + 1]
@@ -824,7 +831,8 @@ prefill_attention_mma_kernel(const float *__restrict__ q, const uint16_t *__rest
                         mma_bf16_full(o[nd + i], pa[term][kk], vf[step & 1][i / 2][i % 2 * 2], vf[step & 1][i / 2][i % 2 * 2 + 1]);
             }
         }
-        __syncthreads();  // the buffer may be refilled by the next iteration's fetch
+        __syncthreads();
+        fetch(vb, v_tile, jt + 1);
     }
     // ---- normalise and store (token-major)
 #pragma unroll
@@ -1537,7 +1545,7 @@ qk_status qk_prefill_attention(qk_ctx *ctx, const float *q, const void *cache_k,
         QK_LAUNCHED(c);
     }
     const size_t hw = group < 4 ? group : 4, pbs = 4 / hw;
-    dim3 grid((unsigned)qk::ceil_div(n_tokens, 16 * pbs), (unsigned)(n_kv_heads * (group / hw)));
+    const dim3 grid((unsigned)(qk::ceil_div(n_tokens, 16 * pbs) * n_kv_heads * (group / hw)));
     QK_CUDA(cudaFuncSetAttribute(prefill_attention_mma_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)kPfSmem));
     QK_PDL(c, prefill_attention_mma_kernel, grid, dim3(128), (size_t)kPfSmem, q, (const uint16_t *)cache_k,
