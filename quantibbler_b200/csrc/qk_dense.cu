@@ -712,15 +712,19 @@ dense_norm_rows_kernel(InputArgs in, uint16_t *__restrict__ dst) {
 // float32 accumulators through distributed shared memory, each CTA finishing its share of the
 // columns.  Weights depend on no other kernel: the first stages' copies start before the
 // dependency wait.  Warp 0 issues the copies, warp 1 the MMAs, warps 2..5 finish.
+// More CTAs than SMs: half the stages each, two to an SM, so that one streams while the other finishes its tile or begins
+// (as many weight bytes in flight): 64 rows, the gated pair of a 14336-wide MLP of 4096, 224 tiles, 84 -> 65.5 us, of sixteen
+// such experts half as wide, 1792 tiles, 339 -> 317 (5.9 TB/s).
 template <int BN> struct NarrowShape {
     static constexpr uint32_t kABytes = 128 * kTcK * 2, kBBytes = BN * kTcK * 2, kStage = kABytes + kBBytes;
-    static constexpr int kStages = BN >= 128 ? 6 : 8;
+    static constexpr uint32_t kStages = BN >= 128 ? 6 : 8, kHalf = kStages / 2;
     static constexpr uint32_t kTmemCols = BN < 32 ? 32 : BN;
-    static constexpr size_t kSmem = 1024 + kStages * kStage + (2 * kStages + 2) * 8 + 32;
-    static_assert(128 * BN * 4 + 2 * 32 * BN * 4 <= kStages * kStage, "the accumulators must fit the drained stages");
+    static constexpr size_t smem(uint32_t stages) { return 1024 + stages * kStage + (2 * kStages + 2) * 8 + 32; }
+    static_assert(128 * BN * 4 + 2 * 32 * BN * 4 <= kHalf * kStage, "the accumulators must fit the drained stages");
+    static_assert(2 * (smem(kHalf) + 1024) <= 227 * 1024, "two CTAs of half the stages fit an SM");
 };
 struct NarrowArgs {
-    uint32_t n_tokens, rows, k_chunks, splits, wait_limit;
+    uint32_t n_tokens, rows, k_chunks, splits, stages, wait_limit;
     int *error;
     const int32_t *offsets;  // rows sorted by expert: [experts + 1]; null: one matrix
     uint32_t tiles;          // weight tiles of an expert
@@ -730,16 +734,17 @@ __device__ __forceinline__ void cluster_sync_all() {
 }
 
 template <int BN>
-__global__ void __launch_bounds__(kTcThreads, 1)
+__global__ void __launch_bounds__(kTcThreads, 2)
 dense_narrow_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_constant__ CUtensorMap x_map,
                     NarrowArgs g, OutputArgs out) {
     using S = NarrowShape<BN>;
     qk::pdl_launch();
     extern __shared__ __align__(1024) uint8_t nr_smem[];
     uint8_t *tiles = reinterpret_cast<uint8_t *>(((uintptr_t)nr_smem + 1023) & ~(uintptr_t)1023);
-    uint64_t *full = reinterpret_cast<uint64_t *>(tiles + S::kStages * S::kStage);
-    uint64_t *empty = full + S::kStages;
-    uint64_t *acc_full = empty + S::kStages;
+    const uint32_t stages = g.stages;
+    uint64_t *full = reinterpret_cast<uint64_t *>(tiles + stages * S::kStage);
+    uint64_t *empty = full + stages;
+    uint64_t *acc_full = empty + stages;
     uint64_t *drain = acc_full + 1;
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(drain + 1);
     volatile int *abort_flag = reinterpret_cast<volatile int *>(tmem_slot + 1);
@@ -763,7 +768,7 @@ dense_narrow_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
     const uint32_t per = (g.k_chunks + g.splits - 1) / g.splits;
     const uint32_t kc0 = min(split * per, g.k_chunks), kc1 = min(kc0 + per, g.k_chunks);
     if (threadIdx.x == 0) {
-        for (int s = 0; s < S::kStages; ++s) {
+        for (uint32_t s = 0; s < stages; ++s) {
             mbar_init(&full[s], 1);
             mbar_init(&empty[s], 1);
         }
@@ -782,7 +787,7 @@ dense_narrow_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     __syncthreads();
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-    const uint32_t ahead = min((uint32_t)S::kStages, kc1 - kc0);
+    const uint32_t ahead = min(stages, kc1 - kc0);
     if (warp == 0 && lane == 0)
         for (uint32_t i = 0; i < ahead; ++i) {
             asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(smem_u32(&full[i])),
@@ -798,8 +803,8 @@ dense_narrow_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
         uint32_t gc = 0;
         bool dead = false;
         for (uint32_t kc = kc0; kc < kc1; ++kc, ++gc) {
-            const uint32_t s = gc % S::kStages;
-            if (gc >= ahead && !mbar_wait(&empty[s], ((gc / S::kStages) & 1) ^ 1, abort_flag, g.wait_limit)) {
+            const uint32_t s = gc % stages;
+            if (gc >= ahead && !mbar_wait(&empty[s], ((gc / stages) & 1) ^ 1, abort_flag, g.wait_limit)) {
                 dead = true;
                 break;
             }
@@ -817,15 +822,15 @@ dense_narrow_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
         }
         if (dead) *abort_flag = 1;
         if (*abort_flag)  // the copies still in flight
-            for (uint32_t i = gc > (uint32_t)S::kStages ? gc - S::kStages : 0; i < gc; ++i)
-                (void)mbar_wait(&full[i % S::kStages], (i / S::kStages) & 1, never, g.wait_limit);
+            for (uint32_t i = gc > stages ? gc - stages : 0; i < gc; ++i)
+                (void)mbar_wait(&full[i % stages], (i / stages) & 1, never, g.wait_limit);
     } else if (warp == 1) {
         const uint32_t idesc = tc_idesc(BN);
         uint32_t gc = 0;
         bool dead = false;
         for (uint32_t kc = kc0; kc < kc1; ++kc, ++gc) {
-            const uint32_t s = gc % S::kStages;
-            if (!mbar_wait(&full[s], (gc / S::kStages) & 1, abort_flag, g.wait_limit)) {
+            const uint32_t s = gc % stages;
+            if (!mbar_wait(&full[s], (gc / stages) & 1, abort_flag, g.wait_limit)) {
                 dead = true;
                 break;
             }
@@ -883,16 +888,29 @@ dense_narrow_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
         const uint32_t c_begin = split * share, c_end = min(min(c_begin + share, (uint32_t)BN), n_rows);
         float *ups = own + 128 * BN;  // [2][BN][32]: up rows for their gate rows
         const uint32_t n = tile * 128 + row, lane_addr = tmem_base + ((quarter * 32) << 16);
-        auto value = [&](uint32_t c) -> float {  // (splits > 1) the sum over the cluster, in split order
-            float v = 0.f;
-            for (uint32_t p = 0; p < g.splits; ++p) {
-                uint32_t remote;
-                float x;
-                asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(own + c * 128 + row)), "r"(p));
-                asm volatile("ld.shared::cluster.f32 %0, [%1];" : "=f"(x) : "r"(remote) : "memory");
-                v += x;
+        // (splits > 1: two, four or eight) eight columns from c on, summed over the cluster in split order; two CTAs' values
+        // are fetched together: a value at a time waited for the other SM each time (6144 rows of 4096 on 64: 29 -> 26.6 us)
+        auto values = [&](uint32_t c, float (&v)[8]) {
+#pragma unroll
+            for (int e = 0; e < 8; ++e) v[e] = 0.f;
+            for (uint32_t p = 0; p < g.splits; p += 2) {
+                float x[2][8];
+#pragma unroll
+                for (int q = 0; q < 2; ++q) {
+                    uint32_t remote;
+                    asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(remote) : "r"(smem_u32(own + row)), "r"(p + q));
+#pragma unroll
+                    for (int e = 0; e < 8; ++e)
+                        asm volatile("ld.shared::cluster.f32 %0, [%1];"
+                                     : "=f"(x[q][e])
+                                     : "r"(remote + min(c + e, (uint32_t)BN - 1) * 512)
+                                     : "memory");
+                }
+#pragma unroll
+                for (int q = 0; q < 2; ++q)
+#pragma unroll
+                    for (int e = 0; e < 8; ++e) v[e] += x[q][e];
             }
-            return v;
         };
         auto done = [&](uint32_t c, float v) {
             if (pair) {
@@ -915,12 +933,15 @@ dense_narrow_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
                     if ((uint32_t)(c0 + j) < c_end) done(c0 + j, __uint_as_float(v[j]));
                 }
             }
-        } else if (!pair) {
-#pragma unroll 4
-            for (uint32_t c = c_begin; c < c_end; ++c) done(c, value(c));
-        } else if (quarter & 1) {
-#pragma unroll 4
-            for (uint32_t c = c_begin; c < c_end; ++c) done(c, value(c));
+        } else if (!pair || (quarter & 1)) {
+#pragma unroll 1
+            for (uint32_t c = c_begin; c < c_end; c += 8) {
+                float v[8];
+                values(c, v);
+#pragma unroll
+                for (int e = 0; e < 8; ++e)
+                    if (c + e < c_end) done(c + e, v[e]);
+            }
         }
         if (pair) {
             asm volatile("bar.sync 1, %0;" ::"r"(kTcEpiWarps * 32) : "memory");
@@ -945,9 +966,14 @@ dense_narrow_kernel(const __grid_constant__ CUtensorMap w_map, const __grid_cons
                         }
                     }
                 } else {
-#pragma unroll 4
-                    for (uint32_t c = c_begin; c < c_end; ++c)
-                        finish_pair(out, t0 + c, j, value(c), ups[((quarter >> 1) * BN + c) * 32 + lane]);
+#pragma unroll 1
+                    for (uint32_t c = c_begin; c < c_end; c += 8) {
+                        float v[8];
+                        values(c, v);
+#pragma unroll
+                        for (int e = 0; e < 8; ++e)
+                            if (c + e < c_end) finish_pair(out, t0 + c + e, j, v[e], ups[((quarter >> 1) * BN + c + e) * 32 + lane]);
+                    }
                 }
             }
         }
@@ -1048,11 +1074,13 @@ qk_status launch_narrow(qk_ctx *c, const void *x, size_t x_stride, const qk_dens
                              (size_t)c->sm_count);
     g.wait_limit = c->wait_limit ? c->wait_limit : kTcWaitDefault;
     g.error = (int *)c->d_err.ptr;
-    QK_CUDA(cudaFuncSetAttribute(dense_narrow_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::kSmem));
+    g.stages = tiles * g.splits > (uint32_t)c->sm_count ? S::kHalf : S::kStages;
+    QK_CUDA(cudaFuncSetAttribute(dense_narrow_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                 (int)S::smem(S::kStages)));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(tiles * g.splits);
     cfg.blockDim = dim3(kTcThreads);
-    cfg.dynamicSmemBytes = S::kSmem;
+    cfg.dynamicSmemBytes = S::smem(g.stages);
     cfg.stream = c->stream;
     cudaLaunchAttribute attr[2];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
