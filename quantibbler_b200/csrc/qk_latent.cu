@@ -34,7 +34,10 @@ __device__ __forceinline__ void lt_load8(const float *p, float (&w)[8]) {
 struct LatentArgs {
     const int32_t *positions, *slots;
     const float *q;
-    float *absorbed;   // [tokens][heads][kv_stride]
+    // [tokens][heads][kv_stride] (steps 0), or for the tensor cores their A fragments in two bfloat16
+    // terms: [tokens][sixteens of heads][steps of 16 channels][term][lane][4]
+    float *absorbed;
+    uint32_t steps;
     float *partial;    // [tokens][heads][n_splits][kv_stride + 8]: sums, then maximum and weight
     void *out;
     uint32_t tokens, heads, dim, dim_stride, vdim, vdim_stride, kv_stride, window, ring, n_splits, q_stride, out_stride;
@@ -54,7 +57,7 @@ __device__ __forceinline__ SplitKeys split_keys(const LatentArgs &a, int pos, ui
 }
 
 // ------------------------------------------------------------------ absorbed: W_uk^T q
-constexpr int kAbsRows = 4, kAbsWarps = 8, kAbsAhead = 8;
+constexpr int kAbsMany = 4, kAbsWarps = 8, kAbsAhead = 8;
 __device__ __forceinline__ void lt_fetch8(const uint16_t *p, uint4 (&w)[1]) { w[0] = *reinterpret_cast<const uint4 *>(p); }
 __device__ __forceinline__ void lt_fetch8(const float *p, uint4 (&w)[2]) {
     w[0] = *reinterpret_cast<const uint4 *>(p);
@@ -77,12 +80,14 @@ __device__ __forceinline__ void lt_open8(const uint4 (&v)[2], float (&w)[8]) {
         w[4 * i + 3] = __uint_as_float(v[i].w);
     }
 }
-template <typename W>
+// kAbsRows rows share the weights that a block reads.  A step of one row has a form of its own: with the
+// products of three rows that are not there it took 4.1 us from the wait, 2.5 without (16 heads of 128 x 512).
+template <typename W, int kAbsRows>
 __global__ void __launch_bounds__(kAbsWarps * 32)
 absorb_query_kernel(LatentArgs a, const W *__restrict__ uk) {
     qk::pdl_launch();
-    extern __shared__ float ab_smem[];  // [kAbsRows][dim] queries, [kAbsWarps][256] sums
-    float *qs = ab_smem, *sums = ab_smem + kAbsRows * a.dim;
+    extern __shared__ __align__(16) float ab_smem[];  // [kAbsWarps][256] sums, [kAbsRows][dim] queries
+    float *sums = ab_smem, *qs = ab_smem + kAbsWarps * 256;
     const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32, h = blockIdx.y;
     const uint32_t c0 = blockIdx.x * 256 + lane * 8, t0 = blockIdx.z * kAbsRows;
     const bool live = c0 < a.kv_stride;
@@ -122,11 +127,29 @@ absorb_query_kernel(LatentArgs a, const W *__restrict__ uk) {
 #pragma unroll
     for (int r = 0; r < kAbsRows; ++r) {
         if (t0 + r >= a.tokens) break;
-#pragma unroll
-        for (int e = 0; e < 8; ++e) sums[warp * 256 + lane * 8 + e] = acc[r][e];
+        for (int e = 0; e < 8; e += 4)
+            *reinterpret_cast<float4 *>(sums + warp * 256 + lane * 8 + e) =
+                make_float4(acc[r][e], acc[r][e + 1], acc[r][e + 2], acc[r][e + 3]);
         __syncthreads();
-        const uint32_t c = blockIdx.x * 256 + threadIdx.x;
-        if (c < a.kv_stride) {
+        if (a.steps) {  // (kv_stride is even)
+            const uint32_t i = 2 * threadIdx.x, c = blockIdx.x * 256 + i;
+            if (i < 256 && c < a.kv_stride) {
+                float2 v = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int w = 0; w < kAbsWarps; ++w) {
+                    const float2 x = *reinterpret_cast<const float2 *>(sums + w * 256 + i);
+                    v.x += x.x;
+                    v.y += x.y;
+                }
+                uint32_t hi, lo;
+                split_bf16(v.x * a.scale, v.y * a.scale, hi, lo);
+                const size_t block = ((size_t)(t0 + r) * ((a.heads + 15) / 16) + h / 16) * a.steps + c / 16;
+                uint32_t *dst = reinterpret_cast<uint32_t *>(a.absorbed) + block * 256 + (h % 8 * 4 + c % 8 / 2) * 4 +
+                                h % 16 / 8 + c % 16 / 8 * 2;
+                dst[0] = hi;
+                dst[128] = lo;
+            }
+        } else if (const uint32_t c = blockIdx.x * 256 + threadIdx.x; c < a.kv_stride) {
             float v = 0.f;
 #pragma unroll
             for (int w = 0; w < kAbsWarps; ++w) v += sums[w * 256 + threadIdx.x];
@@ -236,16 +259,19 @@ latent_mma_kernel(LatentArgs a, const uint16_t *__restrict__ cache, uint32_t clu
     using S = LatShape<KV>;
     constexpr int kQ = S::kQuarter, kSteps = kQ / 16, kTilesPerWarp = kQ / 8;
     qk::pdl_launch();
-    qk::pdl_wait();
     extern __shared__ __align__(16) uint8_t lat_smem[];
     const uint32_t split = blockIdx.x, h0 = blockIdx.y * 16, t = blockIdx.z;
     const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32, g = lane >> 2, c4 = lane & 3;
+    // (positions and slots are written by copies and ordinary launches in front of the step, none of
+    // which lets a kernel start early)
     const int pos = a.positions[t];
+    const uint32_t slot = (uint32_t)a.slots[t];
+    qk::pdl_wait();
     if (pos < 0) return;  // (the whole cluster works on one row)
     uint8_t *ring = lat_smem + warp * S::kBufs * S::kTileBytes;
     float *scores = reinterpret_cast<float *>(lat_smem + S::kSmem - S::kScores);  // [2][warp][16][pitch]
     const SplitKeys keys = split_keys(a, pos, split);
-    const uint16_t *base = cache + (size_t)a.slots[t] * a.ring * a.kv_stride + warp * kQ;
+    const uint16_t *base = cache + (size_t)slot * a.ring * a.kv_stride + warp * kQ;
     const uint32_t ring0 = keys.first % a.ring, n_tiles = (keys.count + kLatKeys - 1) / kLatKeys;
     auto fetch = [&](uint32_t tile) {
         if (tile < n_tiles) {
@@ -262,19 +288,29 @@ latent_mma_kernel(LatentArgs a, const uint16_t *__restrict__ cache, uint32_t clu
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
-    fetch(0);
-    // this warp's quarter of the query, as A fragments in two bfloat16 terms
+    // This warp's quarter of the query, as A fragments in two bfloat16 terms, asked for before the first
+    // keys.  (Gathered from float32 rows, eight of them per load, they took 4 us of the 14 that a launch of one
+    // row and one tile per block had after its wait; as fragments 1.1.)
     uint32_t qh[kSteps][4], ql[kSteps][4];
+    {
+        const uint4 *src = reinterpret_cast<const uint4 *>(a.absorbed) +
+                           (((size_t)t * gridDim.y + blockIdx.y) * a.steps + warp * kSteps) * 64 + lane;
+        uint4 x[kSteps][2];
 #pragma unroll
-    for (int ks = 0; ks < kSteps; ++ks)
+        for (int ks = 0; ks < kSteps; ++ks)
 #pragma unroll
-        for (int e = 0; e < 4; ++e) {
-            const uint32_t r = g + (e & 1) * 8, c = warp * kQ + ks * 16 + 2 * c4 + (e >> 1) * 8;
-            float2 v = make_float2(0.f, 0.f);
-            if (h0 + r < a.heads && c < a.kv_stride)  // (kv_stride is even)
-                v = *reinterpret_cast<const float2 *>(a.absorbed + ((size_t)t * a.heads + h0 + r) * a.kv_stride + c);
-            split_bf16(v.x, v.y, qh[ks][e], ql[ks][e]);
-        }
+            for (int term = 0; term < TERMS; ++term) x[ks][term] = src[ks * 64 + term * 32];
+        fetch(0);
+#pragma unroll
+        for (int ks = 0; ks < kSteps; ++ks)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {  // (what lies past the heads or the channels has not been written)
+                const bool live = h0 + g + (e & 1) * 8 < a.heads && warp * kQ + ks * 16 + (e >> 1) * 8 < a.kv_stride;
+                const auto &h = x[ks][0], &l = x[ks][TERMS - 1];
+                qh[ks][e] = live ? (e == 0 ? h.x : e == 1 ? h.y : e == 2 ? h.z : h.w) : 0u;
+                ql[ks][e] = live ? (e == 0 ? l.x : e == 1 ? l.y : e == 2 ? l.z : l.w) : 0u;
+            }
+    }
     float o[kTilesPerWarp][4];
 #pragma unroll
     for (int n = 0; n < kTilesPerWarp; ++n) o[n][0] = o[n][1] = o[n][2] = o[n][3] = 0.f;
@@ -399,34 +435,62 @@ latent_mma_kernel(LatentArgs a, const uint16_t *__restrict__ cache, uint32_t clu
     const uint32_t n_cta = cluster, rank = split % n_cta;
     if (n_cta > 1) lat_cluster_sync();
     else __syncthreads();
+    // Each CTA reads the others' maxima and weights once (a value per thread) and forms the factor of each of
+    // them per head; the sums' reads are under way meanwhile.  (These 32 KB per CTA bound the merge: 2.4 to 3.6 us,
+    // 10 to 14 bytes per clock; 3 to 5 with a branch around each read.  Sent by stores instead of being read,
+    // eight lines per store, they took longer.)
+    constexpr int kPeers = 8, kTurns = 2;
+    float *stats = scores, *factor = stats + 2 * kPeers * 16;  // [2][peer][head], [peer][head]
     const uint32_t share = (KV / 4 + n_cta - 1) / n_cta, p0 = rank * share, p1 = min(p0 + share, (uint32_t)KV / 4);
-    for (uint32_t i = threadIdx.x; i < 16 * share; i += 128) {
-        const uint32_t r = i / share, piece = p0 + i % share, h = h0 + r;
-        if (h >= a.heads || piece >= p1) continue;
-        float mc[8], mx = -INFINITY;
+    {
+        const uint32_t r = threadIdx.x % 16, p = threadIdx.x / 16;
+        stats[threadIdx.x] = p < n_cta ? lat_peer(stat + r, p) : -INFINITY;
+        stats[kPeers * 16 + threadIdx.x] = p < n_cta ? lat_peer(stat + 16 + r, p) : 0.f;
+    }
+#pragma unroll 1
+    for (uint32_t i0 = threadIdx.x; i0 < (16 * share + 127) / 128 * 128; i0 += kTurns * 128) {
+        float4 x[kTurns][kPeers];
 #pragma unroll
-        for (int p = 0; p < 8; ++p) {
-            mc[p] = (uint32_t)p < n_cta ? lat_peer(stat + r, p) : -INFINITY;
-            mx = fmaxf(mx, mc[p]);
-        }
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        float w = 0.f;
+        for (int n = 0; n < kTurns; ++n) {
+            const uint32_t i = min(i0 + n * 128, 16 * share - 1), piece = min(p0 + i % share, (uint32_t)KV / 4 - 1);
 #pragma unroll
-        for (int p = 0; p < 8; ++p) {
-            if ((uint32_t)p >= n_cta || mc[p] == -INFINITY) continue;
-            const float e = expf(mc[p] - mx);
-            const float4 x = lat_peer4(sums + r * kSumPitch + piece * 4, p);
-            v.x = fmaf(e, x.x, v.x);
-            v.y = fmaf(e, x.y, v.y);
-            v.z = fmaf(e, x.z, v.z);
-            v.w = fmaf(e, x.w, v.w);
-            w = fmaf(e, lat_peer(stat + 16 + r, p), w);
+            for (int p = 0; p < kPeers; ++p)
+                if ((uint32_t)p < n_cta) x[n][p] = lat_peer4(sums + i / share * kSumPitch + piece * 4, p);
         }
-        float *dst = a.partial + (((size_t)t * a.heads + h) * (a.n_splits / n_cta) + split / n_cta) * (a.kv_stride + 8);
-        if (piece * 4 < a.kv_stride) *reinterpret_cast<float4 *>(dst + piece * 4) = v;
-        if (piece == 0) {
-            dst[a.kv_stride] = mx;
-            dst[a.kv_stride + 1] = w;
+        if (i0 == threadIdx.x) {  // (uniform: the first turn of the loop)
+            __syncthreads();
+            const uint32_t r = threadIdx.x % 16, p = threadIdx.x / 16;
+            float mx = -INFINITY;
+#pragma unroll
+            for (int q = 0; q < kPeers; ++q) mx = fmaxf(mx, stats[q * 16 + r]);
+            const float mc = stats[p * 16 + r];
+            factor[p * 16 + r] = mc == -INFINITY ? 0.f : expf(mc - mx);
+            __syncthreads();
+        }
+#pragma unroll
+        for (int n = 0; n < kTurns; ++n) {
+            const uint32_t i = i0 + n * 128, r = i / share, piece = p0 + i % share, h = h0 + r;
+            if (i >= 16 * share || h >= a.heads || piece >= p1) continue;
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            float w = 0.f, mx = -INFINITY;
+#pragma unroll
+            for (int p = 0; p < kPeers; ++p) {
+                if ((uint32_t)p >= n_cta) break;
+                const float e = factor[p * 16 + r], mc = stats[p * 16 + r];
+                mx = fmaxf(mx, mc);
+                const bool none = mc == -INFINITY;  // (an empty split)
+                v.x = none ? v.x : fmaf(e, x[n][p].x, v.x);
+                v.y = none ? v.y : fmaf(e, x[n][p].y, v.y);
+                v.z = none ? v.z : fmaf(e, x[n][p].z, v.z);
+                v.w = none ? v.w : fmaf(e, x[n][p].w, v.w);
+                w = none ? w : fmaf(e, stats[(kPeers + p) * 16 + r], w);
+            }
+            float *dst = a.partial + (((size_t)t * a.heads + h) * (a.n_splits / n_cta) + split / n_cta) * (a.kv_stride + 8);
+            if (piece * 4 < a.kv_stride) *reinterpret_cast<float4 *>(dst + piece * 4) = v;
+            if (piece == 0) {
+                dst[a.kv_stride] = mx;
+                dst[a.kv_stride + 1] = w;
+            }
         }
     }
     if (n_cta > 1) lat_cluster_sync();  // no CTA leaves while another still reads its shared memory
@@ -434,7 +498,7 @@ latent_mma_kernel(LatentArgs a, const uint16_t *__restrict__ cache, uint32_t clu
 
 // ------------------------------------------------------------------ absorbed: combine, W_uv
 // A block takes kRows rows of one head: the weights are read once for all of them.
-constexpr int kOutThreads = 256;
+constexpr int kOutThreads = 256, kOutWarps = kOutThreads / 32;
 template <typename W, int kRows>
 __global__ void __launch_bounds__(kOutThreads)
 latent_output_kernel(LatentArgs a, const W *__restrict__ uv, uint32_t per_block) {
@@ -450,7 +514,7 @@ latent_output_kernel(LatentArgs a, const W *__restrict__ uv, uint32_t per_block)
     float *lat = lo_smem, *wt = lo_smem + kRows * a.kv_stride;
     const uint32_t h = blockIdx.x, t0 = blockIdx.z * kRows, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const uint32_t j0 = blockIdx.y * per_block, j1 = min(j0 + per_block, a.vdim), pitch = a.kv_stride + 8;
-    // a warp per row forms its splits' weights (and with several rows its combined latent as well)
+    // a warp per row forms its splits' weights and its combined latent
     for (uint32_t r = warp; r < (uint32_t)kRows; r += kOutThreads / 32) {
         const uint32_t t = t0 + r;
         const bool live = t < a.tokens && a.positions[t] >= 0;  // (an idle row's output is zero)
@@ -467,33 +531,19 @@ latent_output_kernel(LatentArgs a, const W *__restrict__ uv, uint32_t per_block)
         for (int off = 16; off > 0; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
         for (uint32_t s = lane; s < a.n_splits && live; s += 32) wt[r * a.n_splits + s] /= l;
         __syncwarp();
-        if constexpr (kRows > 1)
 #pragma unroll 4
-            for (uint32_t i = lane * 4; i < a.kv_stride; i += 128) {
-                float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-                for (uint32_t s = 0; s < a.n_splits; ++s) {
-                    const float e = wt[r * a.n_splits + s];
-                    if (e == 0.f) continue;  // (an empty split holds no sums)
-                    const float4 x = *reinterpret_cast<const float4 *>(src + (size_t)s * pitch + i);
-                    v = make_float4(fmaf(e, x.x, v.x), fmaf(e, x.y, v.y), fmaf(e, x.z, v.z), fmaf(e, x.w, v.w));
-                }
-                *reinterpret_cast<float4 *>(lat + r * a.kv_stride + i) = v;
+        for (uint32_t i = lane * 4; i < a.kv_stride; i += 128) {
+            float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+            for (uint32_t s = 0; s < a.n_splits; ++s) {
+                const float e = wt[r * a.n_splits + s];
+                if (e == 0.f) continue;  // (an empty split holds no sums)
+                const float4 x = *reinterpret_cast<const float4 *>(src + (size_t)s * pitch + i);
+                v = make_float4(fmaf(e, x.x, v.x), fmaf(e, x.y, v.y), fmaf(e, x.z, v.z), fmaf(e, x.w, v.w));
             }
+            *reinterpret_cast<float4 *>(lat + r * a.kv_stride + i) = v;
+        }
     }
     __syncthreads();
-    if constexpr (kRows == 1) {  // one row: the whole block combines it
-        const float *src = a.partial + ((size_t)t0 * a.heads + h) * a.n_splits * pitch;
-        for (uint32_t i = threadIdx.x; i < a.kv_stride; i += kOutThreads) {
-            float v = 0.f;
-#pragma unroll 8
-            for (uint32_t s = 0; s < a.n_splits; ++s) {
-                const float e = wt[s];
-                if (e != 0.f) v = fmaf(e, src[(size_t)s * pitch + i], v);
-            }
-            lat[i] = v;
-        }
-        __syncthreads();
-    }
     for (uint32_t j = j0 + warp; j < j1; j += kOutThreads / 32) {
         const W *row = uv + ((size_t)h * a.vdim_stride + j) * a.kv_stride;
         float v[kRows];
@@ -516,6 +566,130 @@ latent_output_kernel(LatentArgs a, const W *__restrict__ uv, uint32_t per_block)
             for (int off = 16; off > 0; off >>= 1) v[r] += __shfl_xor_sync(0xffffffffu, v[r], off);
             if (lane == 0 && t0 + r < a.tokens)
                 put(a.out, a.out_bf16, (size_t)(t0 + r) * a.out_stride + h * a.vdim + j, v[r]);
+        }
+    }
+}
+
+// One row of one head.  A launch of this size is a chain of latencies, so that everything is asked for as
+// early as it can be: a warp's first weights before the dependency wait (they depend on no other kernel),
+// the first splits' sums together with the maxima and weights that combine them; every warp works out the
+// splits' weights itself, which leaves one barrier.  At 16 heads of 128 x 512 the time after the wait fell
+// from 8.1 us to 3.2.
+template <typename W>
+__global__ void __launch_bounds__(kOutThreads)
+latent_output_row_kernel(LatentArgs a, const W *__restrict__ uv, uint32_t per_block) {
+    constexpr int kHeld = 8 / sizeof(W), kPieces = 2, kAhead = 8;
+    qk::pdl_launch();
+    extern __shared__ __align__(16) float lo_smem[];  // [kv_stride] combined latent, [n_splits] weights
+    __shared__ float share[kOutWarps][32];
+    float *lat = lo_smem, *wt = lo_smem + a.kv_stride;
+    const uint32_t h = blockIdx.x, t = blockIdx.z, warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const uint32_t j0 = blockIdx.y * per_block, j1 = min(j0 + per_block, a.vdim), pitch = a.kv_stride + 8, n = a.n_splits;
+    const W *base = uv + (size_t)h * a.vdim_stride * a.kv_stride;
+    uint4 held[kHeld][kPieces][sizeof(W) / 2];  // kHeld rows of this warp, 512 entries of each
+    auto fetch = [&](uint32_t j) {
+#pragma unroll
+        for (int q = 0; q < kHeld; ++q)
+#pragma unroll
+            for (int i = 0; i < kPieces; ++i)
+                lt_fetch8(base + (size_t)min(j + q * kOutWarps, a.vdim - 1) * a.kv_stride + min(i * 256 + lane * 8, a.kv_stride - 8),
+                          held[q][i]);
+    };
+    fetch(j0 + warp);
+    const bool live = a.positions[t] >= 0;  // (an idle row's output is zero; see latent_mma_kernel)
+    qk::pdl_wait();
+    const float *src = a.partial + ((size_t)t * a.heads + h) * n * pitch;
+    auto sums = [&](uint32_t i, uint32_t s0, float2 (&x)[kAhead]) {
+#pragma unroll
+        for (int s = 0; s < kAhead; ++s)
+            x[s] = *reinterpret_cast<const float2 *>(src + (size_t)min(s0 + s, n - 1) * pitch + min(i, a.kv_stride - 2));
+    };
+    float2 x[kAhead];
+    sums(2 * threadIdx.x, 0, x);
+    const float *w;  // the splits' weights
+    if (n <= 32) {
+        float ms = -INFINITY, ls = 0.f;
+        if (lane < n && live) {
+            ms = src[(size_t)lane * pitch + a.kv_stride];
+            ls = src[(size_t)lane * pitch + a.kv_stride + 1];
+        }
+        float m = ms;
+        for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+        const float e = ms == -INFINITY ? 0.f : expf(ms - m);
+        float l = e != 0.f ? e * ls : 0.f;
+        for (int off = 16; off > 0; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
+        share[warp][lane] = live ? e / l : 0.f;
+        __syncwarp();
+        w = share[warp];
+    } else {
+        if (warp == 0) {
+            float m = -INFINITY, l = 0.f;
+            for (uint32_t s = lane; s < n && live; s += 32) m = fmaxf(m, src[(size_t)s * pitch + a.kv_stride]);
+            for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
+            for (uint32_t s = lane; s < n; s += 32) {
+                const float ms = live ? src[(size_t)s * pitch + a.kv_stride] : -INFINITY;
+                const float e = ms == -INFINITY ? 0.f : expf(ms - m);
+                wt[s] = e;
+                if (e != 0.f) l += e * src[(size_t)s * pitch + a.kv_stride + 1];
+            }
+            for (int off = 16; off > 0; off >>= 1) l += __shfl_xor_sync(0xffffffffu, l, off);
+            for (uint32_t s = lane; s < n && live; s += 32) wt[s] /= l;
+        }
+        __syncthreads();
+        w = wt;
+    }
+    for (uint32_t i = 2 * threadIdx.x; i < a.kv_stride; i += 2 * kOutThreads) {
+        float2 v = make_float2(0.f, 0.f);
+        for (uint32_t s0 = 0; s0 < n; s0 += kAhead) {
+            if (s0 || i >= 2 * kOutThreads) sums(i, s0, x);
+#pragma unroll
+            for (int s = 0; s < kAhead; ++s) {
+                const float e = s0 + s < n ? w[s0 + s] : 0.f;
+                if (e != 0.f) v = make_float2(fmaf(e, x[s].x, v.x), fmaf(e, x[s].y, v.y));  // (an empty split holds no sums)
+            }
+        }
+        *reinterpret_cast<float2 *>(lat + i) = v;
+    }
+    __syncthreads();
+    for (uint32_t j = j0 + warp; j < j1; j += kHeld * kOutWarps) {
+        float v[kHeld];
+#pragma unroll
+        for (int q = 0; q < kHeld; ++q) v[q] = 0.f;
+#pragma unroll 1
+        for (uint32_t i0 = 0; i0 < a.kv_stride; i0 += kPieces * 256) {
+            uint4 now[kHeld][kPieces][sizeof(W) / 2];
+#pragma unroll
+            for (int q = 0; q < kHeld; ++q)
+#pragma unroll
+                for (int i = 0; i < kPieces; ++i) {
+                    if (i0 == 0) {
+#pragma unroll
+                        for (int z = 0; z < (int)sizeof(W) / 2; ++z) now[q][i][z] = held[q][i][z];
+                    } else {
+                        lt_fetch8(base + (size_t)min(j + q * kOutWarps, a.vdim - 1) * a.kv_stride +
+                                      min(i0 + i * 256 + lane * 8, a.kv_stride - 8), now[q][i]);
+                    }
+                }
+            if (i0 == 0 && j + kHeld * kOutWarps < j1) fetch(j + kHeld * kOutWarps);
+#pragma unroll
+            for (int i = 0; i < kPieces; ++i) {
+                const uint32_t at = i0 + i * 256 + lane * 8;
+                if (at >= a.kv_stride) continue;
+                const float4 p = *reinterpret_cast<const float4 *>(lat + at), y = *reinterpret_cast<const float4 *>(lat + at + 4);
+#pragma unroll
+                for (int q = 0; q < kHeld; ++q) {
+                    float u[8];
+                    lt_open8(now[q][i], u);
+                    v[q] = fmaf(u[0], p.x, fmaf(u[1], p.y, fmaf(u[2], p.z, fmaf(u[3], p.w, v[q]))));
+                    v[q] = fmaf(u[4], y.x, fmaf(u[5], y.y, fmaf(u[6], y.z, fmaf(u[7], y.w, v[q]))));
+                }
+            }
+        }
+#pragma unroll
+        for (int q = 0; q < kHeld; ++q) {
+            for (int off = 16; off > 0; off >>= 1) v[q] += __shfl_xor_sync(0xffffffffu, v[q], off);
+            if (lane == 0 && j + q * kOutWarps < j1)
+                put(a.out, a.out_bf16, (size_t)t * a.out_stride + h * a.vdim + j + q * kOutWarps, v[q]);
         }
     }
 }
@@ -817,6 +991,18 @@ qk_status launch_mma(qk_ctx *c, const LatentArgs &a, const uint16_t *cache, uint
     return a.tokens < kManyRows ? launch_mma_terms<KV, 2>(c, a, cache, cluster) : launch_mma_terms<KV, 1>(c, a, cache, cluster);
 }
 
+// The channels that the tensor-core form stages per key, and the floats per row of the absorbed query: as it
+// is, or (sixteen heads at a time, all staged channels) as fragments.
+constexpr size_t kMaxStaged = 512;
+size_t staged_channels(size_t kv_stride) {
+    size_t n = 64;
+    while (n < kv_stride) n *= 2;
+    return n;
+}
+size_t absorbed_floats(size_t heads, size_t kv_stride) {
+    return kv_stride > kMaxStaged ? heads * kv_stride : qk::ceil_div(heads, (size_t)16) * 16 * staged_channels(kv_stride);
+}
+
 template <int DK, int DV>
 qk_status launch_band(qk_ctx *c, const BandArgs &a) {
     using S = BandShape<DK, DV>;
@@ -831,7 +1017,7 @@ qk_status launch_band(qk_ctx *c, const BandArgs &a) {
 extern "C" {
 
 size_t qk_latent_scratch(size_t tokens, size_t heads, size_t kv_stride, size_t n_splits) {
-    return tokens * heads * (kv_stride + n_splits * (kv_stride + 8)) * sizeof(float);
+    return tokens * (absorbed_floats(heads, kv_stride) + heads * n_splits * (kv_stride + 8)) * sizeof(float);
 }
 
 qk_status qk_latent_attention(qk_ctx *ctx, const qk_latent_call *d) {
@@ -856,7 +1042,7 @@ qk_status qk_latent_attention(qk_ctx *ctx, const qk_latent_call *d) {
     a.slots = d->slots;
     a.q = (const float *)d->q;
     a.absorbed = d->scratch;
-    a.partial = d->scratch + d->tokens * d->heads * d->kv_stride;
+    a.partial = d->scratch + d->tokens * absorbed_floats(d->heads, d->kv_stride);
     a.out = d->out;
     a.tokens = (uint32_t)d->tokens;
     a.heads = (uint32_t)d->heads;
@@ -873,18 +1059,28 @@ qk_status qk_latent_attention(qk_ctx *ctx, const qk_latent_call *d) {
     a.scale = d->scale;
     a.out_bf16 = d->out_dtype == QK_BF16;
     const bool bf16 = d->w_dtype == QK_BF16;
-    const dim3 ag((unsigned)qk::ceil_div(d->kv_stride, 256), (unsigned)d->heads, (unsigned)qk::ceil_div(d->tokens, kAbsRows));
-    const size_t ab_smem = (kAbsRows * d->dim + kAbsWarps * 256) * 4;
-    if (ab_smem > 48 * 1024) return qk::fail(QK_ERR_VALUE, "qk_latent_attention: dim %zu does not fit shared memory", d->dim);
-    if (bf16) QK_LAUNCH(c, absorb_query_kernel<uint16_t>, ag, dim3(kAbsWarps * 32), ab_smem, a, (const uint16_t *)d->uk);
-    else QK_LAUNCH(c, absorb_query_kernel<float>, ag, dim3(kAbsWarps * 32), ab_smem, a, (const float *)d->uk);
-    if (bf16 && d->kv_stride <= 512 && c->decode_attention_kernel != 0) {
+    const dim3 ag((unsigned)qk::ceil_div(d->kv_stride, 256), (unsigned)d->heads, (unsigned)qk::ceil_div(d->tokens, kAbsMany));
+    const bool one = d->tokens == 1;
+    const size_t ab_smem = ((one ? 1 : kAbsMany) * d->dim + kAbsWarps * 256) * 4;
+    if ((kAbsMany * d->dim + kAbsWarps * 256) * 4 > 48 * 1024) return qk::fail(QK_ERR_VALUE, "qk_latent_attention: dim %zu does not fit shared memory", d->dim);
+    const bool mma = bf16 && d->kv_stride <= kMaxStaged && c->decode_attention_kernel != 0;
+    a.steps = mma ? (uint32_t)staged_channels(d->kv_stride) / 16 : 0;
+#define QK_LATENT_ABSORB(W, R) \
+    QK_LAUNCH(c, (absorb_query_kernel<W, R>), ag, dim3(kAbsWarps * 32), ab_smem, a, (const W *)d->uk)
+    if (bf16 && one) QK_LATENT_ABSORB(uint16_t, 1);
+    else if (bf16) QK_LATENT_ABSORB(uint16_t, kAbsMany);
+    else if (one) QK_LATENT_ABSORB(float, 1);
+    else QK_LATENT_ABSORB(float, kAbsMany);
+#undef QK_LATENT_ABSORB
+    if (mma) {
         const uint16_t *cache = (const uint16_t *)d->cache;
         const uint32_t cluster = a.n_splits % 8 == 0 ? 8 : a.n_splits % 4 == 0 ? 4 : a.n_splits % 2 == 0 ? 2 : 1;
-        if (d->kv_stride <= 64) st = launch_mma<64>(c, a, cache, cluster);
-        else if (d->kv_stride <= 128) st = launch_mma<128>(c, a, cache, cluster);
-        else if (d->kv_stride <= 256) st = launch_mma<256>(c, a, cache, cluster);
-        else st = launch_mma<512>(c, a, cache, cluster);
+        switch (staged_channels(d->kv_stride)) {
+            case 64: st = launch_mma<64>(c, a, cache, cluster); break;
+            case 128: st = launch_mma<128>(c, a, cache, cluster); break;
+            case 256: st = launch_mma<256>(c, a, cache, cluster); break;
+            default: st = launch_mma<512>(c, a, cache, cluster); break;
+        }
         if (st != QK_OK) return st;
         a.n_splits /= cluster;  // (what is left for the last launch to combine)
     } else {
@@ -911,15 +1107,21 @@ qk_status qk_latent_attention(qk_ctx *ctx, const qk_latent_call *d) {
         QK_CUDA(cudaFuncSetAttribute(latent_output_kernel<W, R>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)); \
         QK_LAUNCH(c, (latent_output_kernel<W, R>), og, dim3(kOutThreads), smem, a, (const W *)d->uv, per);                  \
     } while (0)
+#define QK_LATENT_OUT_ROW(W)                                                                                                \
+    do {                                                                                                                    \
+        QK_CUDA(cudaFuncSetAttribute(latent_output_row_kernel<W>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024)); \
+        QK_LAUNCH(c, latent_output_row_kernel<W>, og, dim3(kOutThreads), smem, a, (const W *)d->uv, per);                   \
+    } while (0)
     const size_t mma_smem = 2 * 16 * (d->kv_stride + 8) * 2;
     if (bf16 && tiled && d->kv_stride % 16 == 0 && mma_smem <= 200 * 1024 && c->decode_attention_kernel != 0) {
         QK_CUDA(cudaFuncSetAttribute(latent_output_mma_kernel<2>, cudaFuncAttributeMaxDynamicSharedMemorySize, 200 * 1024));
         QK_LAUNCH(c, latent_output_mma_kernel<2>, dim3(a.heads, (a.tokens + 15) / 16), dim3(kOutThreads), mma_smem, a,
                   (const uint16_t *)d->uv);
     } else if (bf16 && tiled) QK_LATENT_OUT(uint16_t, 8);
-    else if (bf16) QK_LATENT_OUT(uint16_t, 1);
     else if (tiled) QK_LATENT_OUT(float, 8);
-    else QK_LATENT_OUT(float, 1);
+    else if (bf16) QK_LATENT_OUT_ROW(uint16_t);
+    else QK_LATENT_OUT_ROW(float);
+#undef QK_LATENT_OUT_ROW
 #undef QK_LATENT_OUT
     return QK_OK;
 }

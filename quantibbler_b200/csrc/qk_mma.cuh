@@ -27,13 +27,14 @@ __device__ __forceinline__ void copy16(void *smem, const void *gmem, uint32_t by
                  : "memory");
 }
 __device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
-    return (uint32_t)float_to_bf16_bits(lo) | ((uint32_t)float_to_bf16_bits(hi) << 16);
+    uint32_t r;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi), "f"(lo));
+    return r;
 }
 // x as two bfloat16 terms, packed for two neighbouring values
 __device__ __forceinline__ void split_bf16(float a, float b, uint32_t &hi, uint32_t &lo) {
-    const uint16_t ah = float_to_bf16_bits(a), bh = float_to_bf16_bits(b);
-    hi = (uint32_t)ah | ((uint32_t)bh << 16);
-    lo = pack_bf16(a - bf16_bits_to_float(ah), b - bf16_bits_to_float(bh));
+    hi = pack_bf16(a, b);
+    lo = pack_bf16(a - __uint_as_float(hi << 16), b - __uint_as_float(hi & 0xffff0000u));
 }
 
 }  // namespace

@@ -219,6 +219,50 @@ def test_latent_attention_absorbed(dev, heads, dim, vdim, kv, window, splits, bf
         assert float((got - want).abs().max() / want.abs().max()) < (1e-4 if bf16 else 1e-5), (i, p)
 
 
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("tokens,heads,vdim,kv,splits", [
+    (4, 66, 70, 72, 33), (7, 17, 130, 520, 40), (2, 16, 40, 512, 64), (5, 15, 16, 250, 6)])
+def test_latent_attention_of_several_rows(dev, tokens, heads, vdim, kv, splits, bf16):
+    """Rows that share a call: heads that do not fill the last sixteen, channels that do not fill the last
+    step, more value rows than a warp holds at once, more splits than lanes; the last row is idle.  (The
+    bounds are those of one row: two bfloat16 terms leave 2^-17 of a query, of a weight and of a sum.)"""
+    ctx, torch, L = dev
+    g = torch.Generator(device="cuda").manual_seed(tokens)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    dtype = torch.bfloat16 if bf16 else torch.float32
+    dim, ds, vs, ks, window = 24, 32, L.up_to(vdim, 16), L.padded(kv), 200
+    uk, uv = torch.zeros(heads, ds, ks, device="cuda"), torch.zeros(heads, vs, ks, device="cuda")
+    uk[:, :dim, :kv], uv[:, :vdim, :kv] = rnd(heads, dim, kv) / kv ** 0.5, rnd(heads, vdim, kv) / kv ** 0.5
+    uk, uv = uk.to(dtype), uv.to(dtype)
+    lat = torch.zeros(tokens, window, ks, device="cuda")
+    lat[:, :, :kv] = rnd(tokens, window, kv)
+    lat = lat.to(dtype)
+    at = [(37 * i + 1) % window for i in range(tokens - 1)] + [-1]
+    pos = torch.tensor(at, dtype=torch.int32, device="cuda")
+    slots = torch.arange(tokens, dtype=torch.int32, device="cuda").flip(0).contiguous()
+    q = torch.zeros(tokens, heads, ds, device="cuda")
+    q[:, :, :dim] = rnd(tokens, heads, dim) * 3
+    out = torch.full((tokens, L.padded(heads * vdim)), 7.0, device="cuda")
+    scratch = torch.full((_lib.lib().qk_latent_scratch(tokens, heads, ks, splits) // 4,), float("nan"), device="cuda")
+    c = L.LatentCall(tokens=tokens, positions=pos.data_ptr(), slots=slots.data_ptr(), heads=heads, dim=dim, dim_stride=ds,
+                     vdim=vdim, vdim_stride=vs, kv_rank=kv, kv_stride=ks, window=window, ring=window, n_slots=tokens,
+                     scale=dim ** -0.5, q=q.data_ptr(), q_dtype=QK_F32, q_stride=heads * ds,
+                     w_dtype=QK_BF16 if bf16 else QK_F32, uk=uk.data_ptr(), uv=uv.data_ptr(), cache=lat.data_ptr(),
+                     n_splits=splits, scratch=scratch.data_ptr(), out=out.data_ptr(), out_dtype=QK_F32,
+                     out_stride=out.shape[1])
+    check(_lib.lib().qk_latent_attention(ctx.handle, ctypes.byref(c)))
+    ctx.synchronize()
+    got = out[:, :heads * vdim].reshape(tokens, heads, vdim).double()
+    assert not got[-1].any()
+    for t in range(tokens - 1):
+        seen = lat[tokens - 1 - t, :at[t] + 1].double()
+        kk = torch.einsum("hdc,jc->hjd", uk.double()[:, :dim], seen)
+        vv = torch.einsum("hdc,jc->hjd", uv.double()[:, :vdim], seen)
+        pr = torch.softmax(torch.einsum("hd,hjd->hj", q[t, :, :dim].double(), kk) * dim ** -0.5, dim=1)
+        want = torch.einsum("hj,hjd->hd", pr, vv)
+        assert float((got[t] - want).abs().max() / want.abs().max()) < (1e-4 if bf16 else 1e-5), t
+
+
 @pytest.mark.parametrize("dim,vdim,window,p0,tokens", [
     (16, 16, 1, 0, 20), (32, 64, 7, 3, 64), (48, 32, 64, 100, 65), (64, 128, 65, 10, 200), (128, 16, 130, 0, 300),
     (128, 128, 63, 500, 129), (160, 256, 40, 33, 70), (256, 96, 1000, 70, 100)])
