@@ -23,7 +23,7 @@ constexpr int kVecThreads = 256, kVecWarps = kVecThreads / 32;
 constexpr int kRouteTile = 5;  // a tile of qk_route: expert, first and last + 1 place, the expert's first tile, its tiles
 constexpr int kVectorTokens = 4;
 constexpr int kNarrowTokens = 128;
-enum { kRowAny = 0, kRowNorm = 1, kRowPlain = 2 };  // how input rows may be read
+enum { kRowAny = 0, kRowNorm = 1, kRowPlain = 2, kRowGated = 3 };  // how input rows may be read
 constexpr size_t kVecSmemMax = 200 * 1024, kVecSmemSm = 226 * 1024;  // of a block, of an SM
 
 // ------------------------------------------------------------------ vector form
@@ -96,7 +96,7 @@ dense_vector_kernel(InputArgs in, OutputArgs out, const W *__restrict__ w, uint3
     constexpr int HR = R >= 2 ? R / 2 : 1;
     qk::pdl_launch();
     extern __shared__ __align__(16) float xs[];  // [NT][pitch], staged norm weights [2][width]
-    __shared__ float red[kVecWarps];
+    __shared__ __align__(16) float red[2 * kVecWarps];
     __shared__ float part_sum[2][kVecWarps][R * NT];
     const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     const uint32_t k = in.k, pitch = (k + T::kStep - 1) / T::kStep * T::kStep, steps = pitch / T::kStep;
@@ -147,6 +147,7 @@ dense_vector_kernel(InputArgs in, OutputArgs out, const W *__restrict__ w, uint3
             auto at4 = [&](uint32_t p) -> float4 & { return *reinterpret_cast<float4 *>(dst + T::place(4 * p)); };
             if (row_kind == kRowNorm) build_norm_row(in, t_in + t, writer, staged, at4, red);
             else if (row_kind == kRowPlain) build_plain_row(in, t_in + t, at4);
+            else if (row_kind == kRowGated) build_gated_row(in, t_in + t, at4);
             else build_input(in, t_in + t, writer, [&](uint32_t i) -> float & { return dst[T::place(i)]; }, red);
         }
         // what lies between k and the pitch meets zero weights; it must only be finite
@@ -237,14 +238,14 @@ __global__ void __launch_bounds__(256)
 dense_input_kernel(InputArgs in, A *__restrict__ dst, int row_kind) {
     qk::pdl_launch();
     extern __shared__ __align__(16) float row_smem[];  // [k], staged norm weights [2][width]
-    __shared__ float red[8];
+    __shared__ __align__(16) float red[16];
     const uint32_t t = blockIdx.x;
     if (row_kind == kRowNorm) stage_norm_weights(in, row_smem + in.k);
     qk::pdl_wait();
     if (dst) {
-        if (row_kind == kRowNorm)
-            build_norm_row(in, t, true, row_smem + in.k,
-                           [&](uint32_t p) -> float4 & { return *reinterpret_cast<float4 *>(row_smem + 4 * p); }, red);
+        auto at4 = [&](uint32_t p) -> float4 & { return *reinterpret_cast<float4 *>(row_smem + 4 * p); };
+        if (row_kind == kRowNorm) build_norm_row(in, t, true, row_smem + in.k, at4, red);
+        else if (row_kind == kRowGated) build_gated_row(in, t, at4);
         else
             build_input(in, t, true, [&](uint32_t i) -> float & { return row_smem[i]; }, red);
         for (uint32_t j = 0; j < (in.places ? in.top : 1u); ++j) {
@@ -1106,12 +1107,18 @@ qk_status launch_tc(qk_ctx *c, const void *x, size_t x_stride, const qk_dense_ca
     }
 }
 
-// Which of the faster ways to read the input rows applies.
+// Which of the faster ways to read the input rows applies.  (One row in the vector form, from the wait to the
+// finished row, the general way and this one: two of 2048 entries one behind the other 4.0 and 1.5 us, with a
+// pending one 6.8 and 2.5; sixteen gated groups of 128 3.7 to 5.4 and 3.4.)
 int row_kind_of(const InputArgs &a) {
     auto aligned = [](const void *p) { return ((uintptr_t)p & 15) == 0; };
     if (a.width % 4 || a.k % 4 || a.x_stride % 4 || !aligned(a.x)) return kRowAny;
     if (a.kind == QK_INPUT_PLAIN) return kRowPlain;
-    if (a.kind != QK_INPUT_NORM || a.width > 1024 * kNormPieces || !aligned(a.x_out)) return kRowAny;
+    if (a.kind == QK_INPUT_GATED)
+        return a.group % 4 || a.group > 128 || a.width % a.group || a.gate_stride % 4 || !aligned(a.gate) ||
+                       !aligned(a.norm_weight) ? kRowAny : kRowGated;
+    if (a.kind == QK_INPUT_CONCAT && (a.k % 8 || !aligned(a.second))) return kRowAny;
+    if (a.width > 1024 * kNormPieces || !aligned(a.x_out)) return kRowAny;
     if (a.norm != QK_NORM_NONE && !aligned(a.norm_weight)) return kRowAny;
     if (a.pending && (a.pending_stride % 4 || !aligned(a.pending) || !aligned(a.pending_weight))) return kRowAny;
     return kRowNorm;
@@ -1366,7 +1373,8 @@ qk_status launch_input(qk_ctx *c, const InputArgs &in, size_t tokens, A *dst) {
         c->launches++;
         return QK_OK;
     }
-    const int kind = dst && in.k % 4 == 0 && row_kind_of(in) == kRowNorm ? kRowNorm : kRowAny;
+    int kind = dst ? row_kind_of(in) : kRowAny;
+    if (kind == kRowPlain || (kind == kRowNorm && (size_t)in.k * 4 + in.width * 8 > kVecSmemMax)) kind = kRowAny;
     const size_t smem = dst ? (size_t)in.k * 4 + (kind == kRowNorm ? in.width * 8 : 0) : 0;
     if (smem > kVecSmemMax) return qk::fail(QK_ERR_VALUE, "qk_dense: an input vector of %u entries does not fit shared memory", in.k);
     QK_CUDA(cudaFuncSetAttribute(dense_input_kernel<A>, cudaFuncAttributeMaxDynamicSharedMemorySize,

@@ -177,10 +177,19 @@ __device__ __forceinline__ void build_input(const InputArgs &a, uint32_t t, bool
     __syncthreads();
 }
 
-// The same for a normed row of up to 1024 kNormPieces aligned entries, for 256 threads: all loads of the
-// row go out together, the norms' weights have been staged by stage_norm_weights (which depends on no
+// The same for a normed row (with or without a second one behind it) of up to 1024 kNormPieces aligned
+// entries, for 256 threads: all loads of the row go out together, the norms' weights have been staged by stage_norm_weights (which depends on no
 // other kernel).  `at4(p)` is the shared-memory place of entries 4 p .. 4 p + 3.
 constexpr int kNormPieces = 4;
+// The sum over the eight warps of such a block, in the order of block_sum; no barrier after it: the next sum
+// takes other words (red: 16 floats).
+__device__ __forceinline__ float row_sum(float v, float *red) {
+    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
+    if (threadIdx.x % 32 == 0) red[threadIdx.x / 32] = v;
+    __syncthreads();
+    const float4 a = *reinterpret_cast<const float4 *>(red), b = *reinterpret_cast<const float4 *>(red + 4);
+    return ((((((a.x + a.y) + a.z) + a.w) + b.x) + b.y) + b.z) + b.w;
+}
 __device__ __forceinline__ void stage16(float *smem, const float *gmem) {
     asm volatile("cp.async.ca.shared.global [%0], [%1], 16;" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem) : "memory");
 }
@@ -192,27 +201,34 @@ __device__ __forceinline__ void stage_norm_weights(const InputArgs &a, float *st
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
-template <typename At4>
-__device__ __forceinline__ void build_norm_row(const InputArgs &a, uint32_t t, bool writer, const float *staged, At4 &&at4,
-                                               float *red) {
+template <int kPieces, typename At4>
+__device__ __forceinline__ void build_norm_pieces(const InputArgs &a, uint32_t t, bool writer, const float *staged, At4 &&at4,
+                                                  float *red) {
     const uint32_t n = a.width, pieces = n / 4;
     const float4 *xr = reinterpret_cast<const float4 *>(a.x + (size_t)t * a.x_stride);
     const float4 *nw = reinterpret_cast<const float4 *>(staged), *pw = nw + pieces;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    float4 h[kNormPieces];
+    const uint32_t own = (a.kind == QK_INPUT_CONCAT ? a.k / 2 : a.k) / 4;  // pieces of the normed part
+    if (a.kind == QK_INPUT_CONCAT) {
+        const float *second = a.second + (size_t)t * a.x_stride;
+        for (uint32_t p = threadIdx.x; p < pieces; p += 256) stage16(&at4(own + p).x, second + 4 * p);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        for (uint32_t p = own + pieces + threadIdx.x; p < a.k / 4; p += 256) at4(p) = zero;
+    }
+    float4 h[kPieces];
 #pragma unroll
-    for (int j = 0; j < kNormPieces; ++j) {
+    for (int j = 0; j < kPieces; ++j) {
         const uint32_t p = threadIdx.x + 256 * j;
         h[j] = p < pieces ? xr[p] : zero;
     }
     if (a.pending) {
         const uint32_t parts = a.pending_top ? a.pending_top : 1;
-        float4 y[kNormPieces];
+        float4 y[kPieces];
         for (uint32_t c = 0; c < parts; ++c) {
             const float4 *pr = reinterpret_cast<const float4 *>(
                 a.pending_top ? pending_row(a, t, c) : a.pending + (size_t)t * a.pending_stride);
 #pragma unroll
-            for (int j = 0; j < kNormPieces; ++j) {
+            for (int j = 0; j < kPieces; ++j) {
                 const uint32_t p = threadIdx.x + 256 * j;
                 const float4 v = p < pieces ? pr[p] : zero;
                 y[j] = c ? make_float4(y[j].x + v.x, y[j].y + v.y, y[j].z + v.z, y[j].w + v.w) : v;
@@ -221,15 +237,15 @@ __device__ __forceinline__ void build_norm_row(const InputArgs &a, uint32_t t, b
         const float share = a.pending_top ? a.pending_scale : 1.f;
         float ps = 0.f;
 #pragma unroll
-        for (int j = 0; j < kNormPieces; ++j) {
+        for (int j = 0; j < kPieces; ++j) {
             y[j] = make_float4(y[j].x * share, y[j].y * share, y[j].z * share, y[j].w * share);
             ps += y[j].x * y[j].x + y[j].y * y[j].y + y[j].z * y[j].z + y[j].w * y[j].w;
         }
-        const float inv = 1.0f / sqrtf(in_block_sum(ps, red) / (float)n + a.pending_eps);
+        const float inv = 1.0f / sqrtf(row_sum(ps, red) / (float)n + a.pending_eps);
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         float4 *xo = writer && a.x_out ? reinterpret_cast<float4 *>(a.x_out + (size_t)t * a.x_stride) : nullptr;
 #pragma unroll
-        for (int j = 0; j < kNormPieces; ++j) {
+        for (int j = 0; j < kPieces; ++j) {
             const uint32_t p = threadIdx.x + 256 * j;
             if (p >= pieces) continue;
             const float4 w = pw[p];
@@ -242,29 +258,29 @@ __device__ __forceinline__ void build_norm_row(const InputArgs &a, uint32_t t, b
     } else if (writer && a.x_out) {
         float4 *xo = reinterpret_cast<float4 *>(a.x_out + (size_t)t * a.x_stride);
 #pragma unroll
-        for (int j = 0; j < kNormPieces; ++j)
+        for (int j = 0; j < kPieces; ++j)
             if (threadIdx.x + 256 * j < pieces) xo[threadIdx.x + 256 * j] = h[j];
     }
     float mean = 0.f, inv = 1.f;
     if (a.norm == QK_NORM_LAYER) {
         float s = 0.f;
 #pragma unroll
-        for (int j = 0; j < kNormPieces; ++j) s += h[j].x + h[j].y + h[j].z + h[j].w;
-        mean = in_block_sum(s, red) / (float)n;
+        for (int j = 0; j < kPieces; ++j) s += h[j].x + h[j].y + h[j].z + h[j].w;
+        mean = row_sum(s, red + 8) / (float)n;
     }
     if (a.norm != QK_NORM_NONE) {
         float s = 0.f;
 #pragma unroll
-        for (int j = 0; j < kNormPieces; ++j) {
+        for (int j = 0; j < kPieces; ++j) {
             if (threadIdx.x + 256 * j >= pieces) continue;
             const float b = h[j].x - mean, c = h[j].y - mean, d = h[j].z - mean, e = h[j].w - mean;
             s += b * b + c * c + d * d + e * e;
         }
-        inv = 1.0f / sqrtf(in_block_sum(s, red) / (float)n + a.norm_eps);
+        inv = 1.0f / sqrtf(row_sum(s, a.norm == QK_NORM_LAYER ? red : red + 8) / (float)n + a.norm_eps);
     }
     asm volatile("cp.async.wait_group 0;" ::: "memory");
 #pragma unroll
-    for (int j = 0; j < kNormPieces; ++j) {
+    for (int j = 0; j < kPieces; ++j) {
         const uint32_t p = threadIdx.x + 256 * j;
         if (p >= pieces) continue;
         float4 v = h[j];
@@ -274,7 +290,55 @@ __device__ __forceinline__ void build_norm_row(const InputArgs &a, uint32_t t, b
         }
         at4(p) = v;
     }
-    for (uint32_t p = pieces + threadIdx.x; p < a.k / 4; p += 256) at4(p) = zero;
+    for (uint32_t p = pieces + threadIdx.x; p < own; p += 256) at4(p) = zero;
+    __syncthreads();
+}
+// (Half the pieces where they do: at the four blocks per SM of the vector form the others cost time even where
+// no thread has any.  A row of 2048 took 1.9 to 3.1 us from the wait with four pieces and block_sum, 1.4 to 2.6
+// with two and row_sum, with a pending one 3.3 and 2.4.)
+template <typename At4>
+__device__ __forceinline__ void build_norm_row(const InputArgs &a, uint32_t t, bool writer, const float *staged, At4 &&at4,
+                                               float *red) {
+    if (a.width <= 512 * kNormPieces) build_norm_pieces<kNormPieces / 2>(a, t, writer, staged, at4, red);
+    else build_norm_pieces<kNormPieces>(a, t, writer, staged, at4, red);
+}
+// A gated row of groups of up to 128 aligned entries, for 256 threads: a warp takes two groups at a time,
+// a lane four entries of each, all of whose loads go out together.
+template <typename At4>
+__device__ __forceinline__ void build_gated_row(const InputArgs &a, uint32_t t, At4 &&at4) {
+    constexpr uint32_t kBatch = 2, kWarps = 8;
+    const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32, per = a.group / 4, groups = a.width / a.group;
+    const float4 *xr = reinterpret_cast<const float4 *>(a.x + (size_t)t * a.x_stride);
+    const float4 *gr = reinterpret_cast<const float4 *>(a.gate + (size_t)t * a.gate_stride);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const uint32_t own = min(lane, per - 1);
+    const float4 w = reinterpret_cast<const float4 *>(a.norm_weight)[own];
+    for (uint32_t h0 = warp; h0 < groups; h0 += kBatch * kWarps) {
+        float4 x[kBatch], g[kBatch];
+#pragma unroll
+        for (uint32_t j = 0; j < kBatch; ++j) {
+            const uint32_t p = min(h0 + j * kWarps, groups - 1) * per + own;
+            x[j] = xr[p];
+            g[j] = gr[p];
+        }
+        float ss[kBatch];
+#pragma unroll
+        for (uint32_t j = 0; j < kBatch; ++j)
+            ss[j] = lane < per ? x[j].x * x[j].x + x[j].y * x[j].y + x[j].z * x[j].z + x[j].w * x[j].w : 0.f;
+        for (int off = 16; off > 0; off >>= 1)
+#pragma unroll
+            for (uint32_t j = 0; j < kBatch; ++j) ss[j] += __shfl_xor_sync(0xffffffffu, ss[j], off);
+#pragma unroll
+        for (uint32_t j = 0; j < kBatch; ++j) {
+            const float inv = 1.0f / sqrtf(ss[j] / (float)a.group + a.norm_eps);
+            const float4 v = x[j];
+            if (lane < per && h0 + j * kWarps < groups)
+                at4((h0 + j * kWarps) * per + lane) =
+                    make_float4(v.x * inv * w.x * silu_f(g[j].x), v.y * inv * w.y * silu_f(g[j].y),
+                                v.z * inv * w.z * silu_f(g[j].z), v.w * inv * w.w * silu_f(g[j].w));
+        }
+    }
+    for (uint32_t p = a.width / 4 + threadIdx.x; p < a.k / 4; p += 256) at4(p) = zero;
     __syncthreads();
 }
 // A plain row in aligned pieces.

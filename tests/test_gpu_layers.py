@@ -127,6 +127,44 @@ def test_dense_concatenated_and_gated_inputs(dev, tokens, serving, tol):
     assert rel(out[:, :33], v @ m.double().T) < tol
 
 
+@pytest.mark.parametrize("serving,tol", [("float32", 4e-6), ("bfloat16", 1e-2)])
+@pytest.mark.parametrize("tokens", [1, 3, 5])
+@pytest.mark.parametrize("width,group", [(4, 4), (72, 12), (1024, 128), (2048, 64), (2052, 36), (4096, 128)])
+def test_dense_rows_in_aligned_pieces(dev, width, group, tokens, serving, tol):
+    """The ways to read an aligned row, around what a thread holds of it: a pending residual, a norm and a second
+    row behind it; gated groups.  (Bounds as for the rows that are read one by one.)"""
+    ctx, torch, L = dev
+    g = torch.Generator(device="cuda").manual_seed(width)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    w = L.Weights(torch, torch.device("cuda"), serving)
+    stride = L.padded(width)
+    rows = L.Rows(torch, torch.device("cuda"), tokens, stride, w, vector=tokens <= 4)
+    rows.x[:, :width] = rnd(tokens, width) * 2 + 1
+    second, y = torch.zeros(tokens, stride, device="cuda"), torch.zeros(tokens, stride, device="cuda")
+    second[:, :width], y[:, :width] = rnd(tokens, width), rnd(tokens, width) * 3
+    pw, nw = rnd(width) * 0.5 + 1, rnd(width) * 0.3 + 1
+    out = torch.zeros(tokens, 72, device="cuda")
+    h = rows.x[:, :width].double()
+    for pending in ({}, dict(pending=y, pending_stride=stride, pending_weight=pw, pending_eps=1e-3, x_out=rows.x2)):
+        yd = y[:, :width].double()
+        if pending:
+            h = h + yd / (yd.pow(2).mean(1, keepdim=True) + 1e-3).sqrt() * pw.double()
+        c = h - h.mean(1, keepdim=True)
+        normed = c / (c.pow(2).mean(1, keepdim=True) + 1e-4).sqrt() * nw.double()
+        m = (rnd(70, 2 * width) / (2 * width) ** 0.5).bfloat16().float()
+        rows.dense(ctx, w.halves(m, width), input=L.IN_CONCAT, x=rows.x, x_stride=stride, second=second, norm_weight=nw,
+                   norm_eps=1e-4, norm=L.NORM_LAYER, out=out, out_stride=72, **pending)
+        assert rel(out[:, :70], torch.cat([normed, second[:, :width].double()], 1) @ m.double().T) < tol
+    assert rel(rows.x2[:, :width], h) < 2e-6
+    gate, gw = rnd(tokens, stride), rnd(group)
+    m = (rnd(33, width) / width ** 0.5).bfloat16().float()
+    rows.dense(ctx, w.matrix(m), input=L.IN_GATED, x=rows.x, x_stride=stride, gate=gate, gate_stride=stride, group=group,
+               norm_weight=gw, norm_eps=1e-3, out=out, out_stride=72)
+    v = rows.x[:, :width].double().reshape(tokens, width // group, group)
+    v = (v / (v.pow(2).mean(2, keepdim=True) + 1e-3).sqrt() * gw.double()).reshape(tokens, width)
+    assert rel(out[:, :33], (v * silu(gate[:, :width].double())) @ m.double().T) < tol
+
+
 def test_dense_results_do_not_depend_on_the_rest_of_the_batch(dev):
     """Within a form, the bits of a row are the same whatever rows lie beside it."""
     ctx, torch, L = dev
