@@ -266,13 +266,22 @@ latent_mma_kernel(LatentArgs a, const uint16_t *__restrict__ cache, uint32_t clu
     // which lets a kernel start early)
     const int pos = a.positions[t];
     const uint32_t slot = (uint32_t)a.slots[t];
-    qk::pdl_wait();
-    if (pos < 0) return;  // (the whole cluster works on one row)
+    if (pos < 0) {  // (the whole cluster works on one row)
+        qk::pdl_wait();
+        return;
+    }
     uint8_t *ring = lat_smem + warp * S::kBufs * S::kTileBytes;
     float *scores = reinterpret_cast<float *>(lat_smem + S::kSmem - S::kScores);  // [2][warp][16][pitch]
     const SplitKeys keys = split_keys(a, pos, split);
     const uint16_t *base = cache + (size_t)slot * a.ring * a.kv_stride + warp * kQ;
     const uint32_t ring0 = keys.first % a.ring, n_tiles = (keys.count + kLatKeys - 1) / kLatKeys;
+    {   // the first keys are on their way to L2 before the dependency wait
+        uint32_t r = ring0 + min(lane, keys.count ? keys.count - 1 : 0u);
+        if (r >= a.ring) r -= a.ring;
+        for (uint32_t i = 0; i < (uint32_t)kQ && warp * kQ + i < a.kv_stride; i += 64)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(base + (size_t)r * a.kv_stride + i));
+    }
+    qk::pdl_wait();
     auto fetch = [&](uint32_t tile) {
         if (tile < n_tiles) {
             uint8_t *dst = ring + (tile % S::kBufs) * S::kTileBytes;
