@@ -253,6 +253,8 @@ delta_scan_kernel(DeltaArgs a, int vec) {
 // scalars per column is sequential.  The scalars depend on the head alone: the inputs kernel
 // writes them once, 20 floats per token: beta R (k . k) [8], R (k . q) [8], beta, beta P, P, R_8.
 constexpr int kMini = 8, kCoef = 20;
+// Floats between the rows of q and k in shared memory: whole fours, the fours of neighbouring rows in other banks.
+__host__ __device__ constexpr uint32_t inputs_pitch(uint32_t dim) { return (dim + 3) / 4 * 4 + 4; }
 
 // A block takes kTok rows and one key head with the heads it serves.  Thread per channel: convolution
 // and silu of the rows from one window of loads (kTaps bounds the taps), then a warp per row for
@@ -262,8 +264,8 @@ template <int kTaps, int kTok>
 __global__ void __launch_bounds__(256, kTaps <= 4 ? 4 : 2)
 delta_inputs_kernel(DeltaArgs a, uint32_t n_tokens) {
     qk::pdl_launch();
-    extern __shared__ float ci_smem[];  // q, k [kTok][dim + 1], then products, then [ratio][kTok][2] gates
-    const uint32_t t0 = blockIdx.x * kTok, kvh = blockIdx.y, pitch = a.dim + 1, ratio = a.heads / a.kv_heads;
+    extern __shared__ __align__(16) float ci_smem[];  // q, k [kTok][pitch], then products, then [ratio][kTok][2] gates
+    const uint32_t t0 = blockIdx.x * kTok, kvh = blockIdx.y, pitch = inputs_pitch(a.dim), ratio = a.heads / a.kv_heads;
     float *qs = ci_smem, *ks = qs + kTok * pitch, *prod = ks + kTok * pitch, *gate = prod + 2 * kTok * kTok;
     const uint32_t n = min((uint32_t)kTok, n_tokens - t0), warp = threadIdx.x / 32, lane = threadIdx.x % 32;
     // (read before the dependency wait: see delta_scan_kernel)
@@ -334,6 +336,7 @@ delta_inputs_kernel(DeltaArgs a, uint32_t n_tokens) {
         }
         const float iq = 1.0f / sqrtf(sq + a.unit_eps) * (1.0f / sqrtf((float)a.dim));
         const float ik = 1.0f / sqrtf(sk + a.unit_eps);
+        if (a.dim + lane < pitch) qs[warp * pitch + a.dim + lane] = ks[warp * pitch + a.dim + lane] = 0.f;
         float *row = a.qkv + (size_t)(t0 + warp) * a.channels + kvh * a.dim;
         float dot = 0.f;
         for (uint32_t d = lane; d < a.dim; d += 32) {
@@ -358,13 +361,32 @@ delta_inputs_kernel(DeltaArgs a, uint32_t n_tokens) {
     }
     if constexpr (kTok == 1) return;
     __syncthreads();
-    {   // k_i . k_t and k_i . q_t: two threads per product
-        const uint32_t pair = threadIdx.x / 2, half = threadIdx.x % 2, t = pair / kTok % kTok, i = pair % kTok;
-        const float *x = (pair < kTok * kTok ? ks : qs) + t * pitch, *y = ks + i * pitch;
-        float v = 0.f;
-        for (uint32_t d = half; d < a.dim; d += 2) v = fmaf(x[d], y[d], v);
-        v += __shfl_xor_sync(0xffffffffu, v, 1);
-        if (half == 0 && pair < 2 * kTok * kTok) prod[pair] = v;
+    if constexpr (kTok == 8) {
+        // k_i . k_t and k_i . q_t, two rows by two: eight threads a square, each with every eighth group of four
+        // entries.  (With two threads a product, entry by entry, a launch of 2048 rows and 16384 channels took 74 us, now 66.)
+        const uint32_t square = threadIdx.x / 8, part = threadIdx.x % 8, kind = square / 16, t = square / 4 % 4 * 2, i = square % 4 * 2;
+        const float *x = (kind ? qs : ks) + t * pitch, *y = ks + i * pitch;
+        float v[2][2] = {};
+        for (uint32_t d = 4 * part; d < a.dim; d += 32) {
+            float4 xs[2], ys[2];
+#pragma unroll
+            for (int r = 0; r < 2; ++r) {
+                xs[r] = *reinterpret_cast<const float4 *>(x + r * pitch + d);
+                ys[r] = *reinterpret_cast<const float4 *>(y + r * pitch + d);
+            }
+#pragma unroll
+            for (int r = 0; r < 2; ++r)
+#pragma unroll
+                for (int c = 0; c < 2; ++c)
+                    v[r][c] = fmaf(xs[r].x, ys[c].x, fmaf(xs[r].y, ys[c].y, fmaf(xs[r].z, ys[c].z, fmaf(xs[r].w, ys[c].w, v[r][c]))));
+        }
+#pragma unroll
+        for (int off = 4; off > 0; off >>= 1)
+#pragma unroll
+            for (int e = 0; e < 4; ++e) v[e / 2][e % 2] += __shfl_xor_sync(0xffffffffu, v[e / 2][e % 2], off);
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+            if (part == (uint32_t)e) prod[kind * kTok * kTok + (t + e / 2) * kTok + i + e % 2] = v[e / 2][e % 2];
     }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < ratio * kTok; i += 256) {
@@ -460,14 +482,15 @@ delta_chunk_scan_kernel(DeltaArgs a, uint32_t n_tokens, int vec) {
         if (chunk < n_chunks) {
             float *q = cs_smem + (chunk % S::kStages) * S::kFloats, *k = q + kMini * S::kDim, *v = k + kMini * S::kDim;
             float *cf = v + kMini * S::kCols;
-            const uint32_t t0 = chunk * kMini;
+            const uint32_t t0 = chunk * kMini, own = n_tokens - t0;  // rows from `own` on are not there
+            const float *rows = a.qkv + (size_t)t0 * a.channels;
             if (vec) {
 #pragma unroll
                 for (int j = 0; j < kPieces; ++j) {
                     const uint32_t t = piece_at[j] / S::kDim, d = piece_at[j] % S::kDim;
                     if (t >= (uint32_t)kMini) continue;
-                    const uint32_t bytes = t0 + t < n_tokens ? 16 : 0;
-                    const float *src = a.qkv + (size_t)min(t0 + t, n_tokens - 1) * a.channels + kvh * a.dim + d;
+                    const uint32_t bytes = t < own ? 16 : 0;
+                    const float *src = rows + (t < own ? t * a.channels : 0u) + kvh * a.dim + d;
                     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
                                      (uint32_t)__cvta_generic_to_shared(q + t * S::kDim + d)), "l"(src), "r"(bytes) : "memory");
                     asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(
@@ -486,9 +509,8 @@ delta_chunk_scan_kernel(DeltaArgs a, uint32_t n_tokens, int vec) {
             }
             for (uint32_t i = threadIdx.x; i < kMini * S::kCols; i += kChunkWarps * 32) {
                 const uint32_t t = i / S::kCols, j = i % S::kCols;
-                const uint32_t bytes = t0 + t < n_tokens && col0 + j < a.vdim ? 4 : 0;
-                const float *src = a.qkv + (size_t)min(t0 + t, n_tokens - 1) * a.channels + 2 * key0 + h * a.vdim +
-                                   min(col0 + j, a.vdim - 1);
+                const uint32_t bytes = t < own && col0 + j < a.vdim ? 4 : 0;
+                const float *src = rows + (t < own ? t * a.channels : 0u) + 2 * key0 + h * a.vdim + min(col0 + j, a.vdim - 1);
                 asm volatile("cp.async.ca.shared.global [%0], [%1], 4, %2;" ::"r"(
                                  (uint32_t)__cvta_generic_to_shared(v + t * S::kCols + j)), "l"(src), "r"(bytes) : "memory");
             }
@@ -712,8 +734,10 @@ qk_status qk_delta(qk_ctx *ctx, const qk_delta_call *d) {
     const bool portion = d->segments == 1 && d->tokens >= (size_t)kMini;  // eight tokens at a time
     const size_t tok = portion ? kMini : 1;
     const dim3 ig((unsigned)qk::ceil_div(d->tokens, tok), a.kv_heads);
-    const size_t smem = (2 * tok * (d->dim + 1) + 2 * tok * tok + d->heads / d->kv_heads * tok * 2) * 4;
-    if (smem > 200 * 1024) return qk::fail(QK_ERR_VALUE, "qk_delta: %zu heads over %zu key heads", d->heads, d->kv_heads);
+    const size_t scalars = 2 * tok * tok + d->heads / d->kv_heads * tok * 2;
+    if ((2 * tok * (d->dim + 1) + scalars) * 4 > 200 * 1024)
+        return qk::fail(QK_ERR_VALUE, "qk_delta: %zu heads over %zu key heads", d->heads, d->kv_heads);
+    const size_t smem = (2 * tok * inputs_pitch((uint32_t)d->dim) + scalars) * 4;
 #define QK_INPUTS(taps, tok)                                                                                    \
     do {                                                                                                        \
         QK_CUDA(cudaFuncSetAttribute(delta_inputs_kernel<taps, tok>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
