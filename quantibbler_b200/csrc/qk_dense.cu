@@ -617,9 +617,14 @@ template <int kV>
 __global__ void __launch_bounds__(256)
 dense_norm_rows_kernel(InputArgs in, uint16_t *__restrict__ dst) {
     qk::pdl_launch();
-    qk::pdl_wait();
-    __shared__ float red[8];
+    __shared__ __align__(16) float red[16];
     const uint32_t t = blockIdx.x, n = in.width, pieces = n / 4;
+    // the norms' weights depend on no other kernel: on their way to L2 before the dependency wait
+    for (uint32_t i = threadIdx.x * 32; i < n; i += 256 * 32) {
+        if (in.norm != QK_NORM_NONE) asm volatile("prefetch.global.L2 [%0];" ::"l"(in.norm_weight + i));
+        if (in.pending) asm volatile("prefetch.global.L2 [%0];" ::"l"(in.pending_weight + i));
+    }
+    qk::pdl_wait();
     const float4 *xr = reinterpret_cast<const float4 *>(in.x + (size_t)t * in.x_stride);
     float4 h[kV];
 #pragma unroll
@@ -647,7 +652,7 @@ dense_norm_rows_kernel(InputArgs in, uint16_t *__restrict__ dst) {
             y[j] = make_float4(y[j].x * share, y[j].y * share, y[j].z * share, y[j].w * share);
             ps += y[j].x * y[j].x + y[j].y * y[j].y + y[j].z * y[j].z + y[j].w * y[j].w;
         }
-        const float inv = 1.0f / sqrtf(in_block_sum(ps, red) / (float)n + in.pending_eps);
+        const float inv = 1.0f / sqrtf(row_sum(ps, red) / (float)n + in.pending_eps);
         const float4 *pw = reinterpret_cast<const float4 *>(in.pending_weight);
         float4 *xo = in.x_out ? reinterpret_cast<float4 *>(in.x_out + (size_t)t * in.x_stride) : nullptr;
 #pragma unroll
@@ -667,7 +672,7 @@ dense_norm_rows_kernel(InputArgs in, uint16_t *__restrict__ dst) {
         float s = 0.f;
 #pragma unroll
         for (int j = 0; j < kV; ++j) s += h[j].x + h[j].y + h[j].z + h[j].w;
-        mean = in_block_sum(s, red) / (float)n;
+        mean = row_sum(s, red + 8) / (float)n;
     }
     if (in.norm != QK_NORM_NONE) {
         float s = 0.f;
@@ -677,7 +682,7 @@ dense_norm_rows_kernel(InputArgs in, uint16_t *__restrict__ dst) {
             const float a = h[j].x - mean, b = h[j].y - mean, c = h[j].z - mean, d = h[j].w - mean;
             s += a * a + b * b + c * c + d * d;
         }
-        inv = 1.0f / sqrtf(in_block_sum(s, red) / (float)n + in.norm_eps);
+        inv = 1.0f / sqrtf(row_sum(s, in.norm == QK_NORM_LAYER ? red : red + 8) / (float)n + in.norm_eps);
     }
     const uint32_t copies = in.places ? in.top : 1;
     const float4 *nw = reinterpret_cast<const float4 *>(in.norm_weight);
@@ -703,7 +708,10 @@ dense_norm_rows_kernel(InputArgs in, uint16_t *__restrict__ dst) {
             if (in.kind == QK_INPUT_CONCAT) o[half + p] = pack(p < pieces ? second[p] : make_float4(0.f, 0.f, 0.f, 0.f));
         }
     }
-    if (in.append.src) append_latent(in, t, red);
+    if (in.append.src) {
+        __syncthreads();  // (the last sum's words are read)
+        append_latent(in, t, red);
+    }
 }
 
 // ------------------------------------------------------------------ narrow form
@@ -1041,19 +1049,22 @@ qk_status launch_tc_kind(qk_ctx *c, const void *x, size_t x_stride, const qk_den
     return QK_OK;
 }
 
-// CTAs per tile: enough to occupy the SMs without splitting the k range finer than four chunks.
+// CTAs per tile: as many as fit the machine at once, two to an SM (clusters do not find room
+// everywhere), at least four chunks of k each.  More than that come in a second wave; fewer
+// have too little in flight.  Measured, us with 1, 2, 4, 8 CTAs a tile, 64 rows: 2040 x 8192
+// 56.8, 34.2, 22.1, 18.3; 4088 x 4096 33.5, 22.3, 17.6, 16.0 and 4344 x 4096 (272 CTAs of clusters of eight do not fit)
+// 34.5, 22.5, 18.0, 23.0; 8952 x 4096 (280 of clusters of four) 37.0, 26.6, 24.0, 36.0 and 9208 x 2048 (288) 23.5, 18.8, 23.7, 28.7;
+// 18168 x 4096 (284 of two) 44.0, 36.7, 42.5, 61.
 uint32_t narrow_splits(size_t tiles, size_t k_chunks, size_t sms) {
-    uint32_t best = 1;
-    size_t best_cost = ~(size_t)0;
-    for (uint32_t s : {1u, 2u, 4u, 8u}) {
-        if (s > 1 && k_chunks / s < 4) break;
-        // (a cluster of CTAs does not find room on every SM)
-        const size_t room = s == 1 ? sms : s == 2 ? sms - 4 : sms - 20;
-        const size_t waves = qk::ceil_div(tiles * s, room);
-        const size_t cost = waves * (qk::ceil_div(k_chunks, s) + 10) + (s > 1 ? 6 : 0);
-        if (cost < best_cost) best = s, best_cost = cost;
-    }
-    return best;
+    constexpr size_t kOf[] = {8, 4, 2}, kSpare[] = {40, 16, 4};
+    for (int i = 0; i < 3; ++i)
+        if (k_chunks >= 4 * kOf[i] && tiles * kOf[i] + kSpare[i] <= 2 * sms) return (uint32_t)kOf[i];
+    return 1;
+}
+// All the stages, one CTA to an SM, while that many fit (2040 x 8192 as sixteen clusters of eight, which do not:
+// 27.8 us with all stages, 18.3 with half of them; twelve clusters 12.0 and 13.5).
+bool narrow_alone(size_t ctas, uint32_t splits, size_t sms) {
+    return ctas + (splits == 8 ? 52 : splits == 4 ? 20 : splits == 2 ? 4 : 0) <= sms;
 }
 
 template <int BN>
@@ -1075,7 +1086,7 @@ qk_status launch_narrow(qk_ctx *c, const void *x, size_t x_stride, const qk_dens
                              (size_t)c->sm_count);
     g.wait_limit = c->wait_limit ? c->wait_limit : kTcWaitDefault;
     g.error = (int *)c->d_err.ptr;
-    g.stages = tiles * g.splits > (uint32_t)c->sm_count ? S::kHalf : S::kStages;
+    g.stages = narrow_alone((size_t)tiles * g.splits, g.splits, (size_t)c->sm_count) ? S::kStages : S::kHalf;
     QK_CUDA(cudaFuncSetAttribute(dense_narrow_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                  (int)S::smem(S::kStages)));
     cudaLaunchConfig_t cfg = {};
@@ -1374,7 +1385,8 @@ qk_status launch_input(qk_ctx *c, const InputArgs &in, size_t tokens, A *dst) {
         return QK_OK;
     }
     int kind = dst ? row_kind_of(in) : kRowAny;
-    if (kind == kRowPlain || (kind == kRowNorm && (size_t)in.k * 4 + in.width * 8 > kVecSmemMax)) kind = kRowAny;
+    if (kind == kRowPlain) kind = kRowAny;
+    if (in.kind == QK_INPUT_CONCAT && (size_t)in.k * 4 + in.width * 8 > kVecSmemMax) kind = kRowAny;
     const size_t smem = dst ? (size_t)in.k * 4 + (kind == kRowNorm ? in.width * 8 : 0) : 0;
     if (smem > kVecSmemMax) return qk::fail(QK_ERR_VALUE, "qk_dense: an input vector of %u entries does not fit shared memory", in.k);
     QK_CUDA(cudaFuncSetAttribute(dense_input_kernel<A>, cudaFuncAttributeMaxDynamicSharedMemorySize,

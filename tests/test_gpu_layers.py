@@ -165,6 +165,34 @@ def test_dense_rows_in_aligned_pieces(dev, width, group, tokens, serving, tol):
     assert rel(out[:, :33], (v * silu(gate[:, :width].double())) @ m.double().T) < tol
 
 
+@pytest.mark.parametrize("tokens", [5, 64, 128])
+@pytest.mark.parametrize("tiles,width", [(0, 72), (0, 1000), (1, 130), (5, 2100), (17, 2100), (34, 1090), (71, 520),
+                                         (73, 2100), (147, 140)])
+def test_dense_few_rows_by_weight_tiles(dev, tiles, width, tokens):
+    """Few rows on matrices around the numbers of 128-row tiles where a tile gets another number of blocks or an SM
+    a second block, up to more tiles than SMs (0): the last tile is ragged, k ends inside a step, some blocks of a
+    cluster have fewer steps than the others or none."""
+    ctx, torch, L = dev
+    g = torch.Generator(device="cuda").manual_seed(width + tokens)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    w = L.Weights(torch, torch.device("cuda"), "bfloat16")
+    rows_out = 128 * (tiles or torch.cuda.get_device_properties(0).multi_processor_count + 2) - 56
+    stride = L.padded(width)
+    rows = L.Rows(torch, torch.device("cuda"), tokens, stride, w, vector=False)
+    rows.x[:, :width] = rnd(tokens, width)
+    xd = rows.x[:, :width].double()
+    m = (rnd(rows_out, width) / width ** 0.5).bfloat16().float()
+    out = torch.zeros(tokens, L.up_to(rows_out, 8), device="cuda")
+    rows.dense(ctx, w.matrix(m), input=L.IN_PLAIN, x=rows.x, x_stride=stride, out=out, out_stride=out.shape[1])
+    assert rel(out[:, :rows_out], xd @ m.double().T) < 1e-2
+    up = (rnd(rows_out, width) / width ** 0.5).bfloat16().float()
+    pair = w.gated_pair(m, up)
+    act = torch.zeros(tokens, pair.rows // 2, device="cuda")
+    rows.dense(ctx, pair, input=L.IN_PLAIN, x=rows.x, x_stride=stride, output=L.OUT_GLU, activation=L.ACTIVATIONS["silu"],
+               out=act, out_stride=act.shape[1])
+    assert rel(act[:, :rows_out], silu(xd @ m.double().T) * (xd @ up.double().T)) < 1e-2
+
+
 def test_dense_results_do_not_depend_on_the_rest_of_the_batch(dev):
     """Within a form, the bits of a row are the same whatever rows lie beside it."""
     ctx, torch, L = dev
