@@ -214,6 +214,12 @@ def test_norm_inside_the_call(gpu_ctx, d, n_tokens, residual, in_place):
         assert torch.equal(a, b)
 
 
+@pytest.mark.parametrize("d,n_tokens", [(1001, 5), (4094, 2), (4097, 3), (6006, 2)])
+def test_norm_inside_the_call_on_rows_of_no_whole_pieces(gpu_ctx, d, n_tokens):
+    """Rows that do not end with the eight entries of a store, below and above what half the registers hold."""
+    test_norm_inside_the_call(gpu_ctx, d, n_tokens, True, False)
+
+
 def test_norm_inside_the_call_refuses_long_rows(gpu_ctx):
     import torch
     from quantibbler_b200.gpu import apply_prefill_many_normed
