@@ -17,7 +17,9 @@
 // full precision, P quantised at the static 1/127 scale, V per-channel INT8 per key block,
 // integer PV, O = alpha*O + pv*(1/127)*dV, O/l at the end.  Unlike the reference (one thread
 // per query row re-quantising every K/V tile into global scratch), the K, V and Q codes are
-// produced once per call by three small kernels.  Two main kernels share them:
+// produced once per call, by three small kernels or, for the tcgen05 form, by one launch.  The main kernels:
+//   * attention_sage_umma_kernel: QK^T on tcgen05 INT8, PV on tcgen05 float16 over the same whole-number codes,
+//     for head_dim = val_dim = 128 and key blocks of 64 (the default there);
 //   * attention_sage_tc_kernel: both integer products on the INT8 tensor cores (mma.sync
 //     m16n8k32), for head_dim = val_dim in {64, 128} and key blocks of 32, 64 or 128;
 //   * attention_sage_kernel: integer dots with dp4a, any shape.  A key block's P codes all

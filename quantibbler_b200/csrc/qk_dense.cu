@@ -721,7 +721,7 @@ dense_norm_rows_kernel(InputArgs in, uint16_t *__restrict__ dst) {
 // float32 accumulators through distributed shared memory, each CTA finishing its share of the
 // columns.  Weights depend on no other kernel: the first stages' copies start before the
 // dependency wait.  Warp 0 issues the copies, warp 1 the MMAs, warps 2..5 finish.
-// More CTAs than SMs: half the stages each, two to an SM, so that one streams while the other finishes its tile or begins
+// More CTAs than fit one to an SM: half the stages each, two to an SM, so that one streams while the other finishes its tile or begins
 // (as many weight bytes in flight): 64 rows, the gated pair of a 14336-wide MLP of 4096, 224 tiles, 84 -> 65.5 us, of sixteen
 // such experts half as wide, 1792 tiles, 339 -> 317 (5.9 TB/s).
 template <int BN> struct NarrowShape {
