@@ -59,7 +59,9 @@ __device__ __forceinline__ float round_bf16_fast(float v) {  // (a NaN becomes a
 template <bool kRoundBf16, bool kFinal>
 __device__ __forceinline__ void sum_form(const StageParams &p, uint32_t rows_per_block, uint32_t slice_bits, uint32_t rank,
                                          uint32_t n_rank) {
-    extern __shared__ __align__(16) uint8_t smem_dyn[];
+    // (aligned as everywhere in this file: the declarations are one symbol, and the first one decides for all of them; with 16
+    // the streaming kernels' digit tables began half a line off, 163 -> 165 us for a stack of layers)
+    extern __shared__ __align__(128) uint8_t smem_dyn[];
     // (the second stage's input is the float64 intermediate; rounded to bfloat16 it is a float32 too)
     using Entry = typename std::conditional<kFinal && !kRoundBf16, double, float>::type;
     using Bits = typename std::conditional<sizeof(Entry) == 8, unsigned long long, uint32_t>::type;
