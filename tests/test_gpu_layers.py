@@ -165,6 +165,80 @@ def test_dense_rows_in_aligned_pieces(dev, width, group, tokens, serving, tol):
     assert rel(out[:, :33], (v * silu(gate[:, :width].double())) @ m.double().T) < tol
 
 
+@pytest.mark.parametrize("serving", ["float32", "bfloat16"])
+@pytest.mark.parametrize("tokens", [1, 4])
+@pytest.mark.parametrize("width", [4, 72, 1024, 2048, 2052, 4096])
+def test_concatenated_rows_have_the_same_bits_however_they_are_read(dev, width, tokens, serving):
+    """Aligned rows, and the same rows one float further on, which are read entry by entry: a row's sums are formed in
+    one order.  The product by the identity leaves the row as it is."""
+    ctx, torch, L = dev
+    g = torch.Generator(device="cuda").manual_seed(width)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    w = L.Weights(torch, torch.device("cuda"), serving)
+    stride = L.padded(width)
+    rows = L.Rows(torch, torch.device("cuda"), tokens, stride, w, vector=True)
+    few = min(width, 512)       # (the identity's rows: the ends of both halves)
+    eye = torch.zeros(2 * few, 2 * width, device="cuda")
+    eye[torch.arange(few), torch.arange(width - few, width)] = 1
+    eye[few + torch.arange(few), torch.arange(width, width + few)] = 1
+    lin = w.halves(eye, width)
+    second, y = torch.zeros(tokens, stride, device="cuda"), torch.zeros(tokens, stride, device="cuda")
+    second[:, :width], y[:, :width] = rnd(tokens, width), rnd(tokens, width) * 3
+    pw, nw, x = rnd(width) * 0.5 + 1, rnd(width) * 0.3 + 1, rnd(tokens, stride) * 2 + 1
+    for norm in (L.NORM_LAYER, L.NORM_RMS):
+        for pending in (False, True):
+            got = []
+            for shift in (0, 1):
+                buf = torch.zeros(tokens * stride + 4, device="cuda")
+                buf[shift:shift + x.numel()] = x.flatten()
+                out = torch.full((tokens, 2 * few), float("nan"), device="cuda")
+                rows.x2.zero_()
+                more = dict(pending=y, pending_stride=stride, pending_weight=pw, pending_eps=1e-3, x_out=rows.x2) if pending else {}
+                rows.dense(ctx, lin, input=L.IN_CONCAT, x=buf.data_ptr() + 4 * shift, x_stride=stride, second=second, norm=norm,
+                           norm_weight=nw, norm_eps=1e-4, out=out, out_stride=out.shape[1], **more)
+                ctx.synchronize()
+                got.append((out, rows.x2[:, :width].clone()))
+            assert torch.equal(got[0][0], got[1][0]), (norm, pending)
+            assert torch.equal(got[0][1], got[1][1]), (norm, pending)
+            assert bool((got[0][0] != 0).any())
+
+
+@pytest.mark.parametrize("tokens,serving", [(1, "float32"), (3, "bfloat16"), (5, "float32")])
+@pytest.mark.parametrize("width,group", [(4, 4), (72, 18), (1024, 128), (2048, 64), (2052, 36), (1536, 96), (600, 150)])
+def test_gated_rows_are_summed_in_lane_order(dev, width, group, tokens, serving):
+    """The bits of a gated row: a lane adds the squares of its entries 32 apart, the lanes' sums meet in a butterfly,
+    whatever the group's width.  Restated in numpy (a product of two float32 is exact in float64, so that one
+    rounding makes the fused multiply-add); silu(32) is 32, the product by the identity leaves the row as it is."""
+    ctx, torch, L = dev
+    rng = np.random.default_rng(width + tokens)
+    f32 = np.float32
+    w = L.Weights(torch, torch.device("cuda"), serving)
+    stride = L.padded(width)
+    rows = L.Rows(torch, torch.device("cuda"), tokens, stride, w, vector=tokens <= 4)
+    x = (rng.standard_normal((tokens, width)) * 3).astype(f32)
+    nw = (rng.standard_normal(group) + 1).astype(f32)
+    rows.x[:, :width] = torch.from_numpy(x).cuda()
+    gate = torch.full((tokens, stride), 32.0, device="cuda")
+    out = torch.zeros(tokens, L.up_to(width, 8), device="cuda")
+    rows.dense(ctx, w.matrix(torch.eye(width, device="cuda")), input=L.IN_GATED, x=rows.x, x_stride=stride, gate=gate,
+               gate_stride=stride, group=group, norm_weight=torch.from_numpy(nw).cuda(), norm_eps=1e-3, out=out,
+               out_stride=out.shape[1])
+    ctx.synchronize()
+    v = x.reshape(tokens, width // group, group)
+    per = -(-group // 32) * 32
+    lanes = np.zeros((tokens, width // group, per), f32)
+    lanes[..., :group] = v
+    ss = np.zeros((tokens, width // group, 32), f32)
+    for i in range(0, per, 32):
+        e = lanes[..., i:i + 32].astype(np.float64)
+        ss = (e * e + ss.astype(np.float64)).astype(f32)
+    for off in (16, 8, 4, 2, 1):
+        ss = ss + ss[..., np.arange(32) ^ off]
+    inv = f32(1) / np.sqrt(ss[..., :1] / f32(group) + f32(1e-3))
+    want = ((v * inv) * nw * f32(32)).reshape(tokens, width)
+    assert np.array_equal(out[:, :width].cpu().numpy(), want)
+
+
 @pytest.mark.parametrize("tokens", [5, 64, 128])
 @pytest.mark.parametrize("tiles,width", [(0, 72), (0, 1000), (1, 130), (5, 2100), (17, 2100), (34, 1090), (71, 520),
                                          (73, 2100), (147, 140)])
