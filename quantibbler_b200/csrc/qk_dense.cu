@@ -1050,17 +1050,22 @@ qk_status launch_tc_kind(qk_ctx *c, const void *x, size_t x_stride, const qk_den
     return QK_OK;
 }
 
-// CTAs per tile: as many as fit the machine at once, two to an SM (clusters do not find room
-// everywhere), at least four chunks of k each.  More than that come in a second wave; fewer
-// have too little in flight.  Measured, us with 1, 2, 4, 8 CTAs a tile, 64 rows: 2040 x 8192
-// 56.8, 34.2, 22.1, 18.3; 4088 x 4096 33.5, 22.3, 17.6, 16.0 and 4344 x 4096 (272 CTAs of clusters of eight do not fit)
-// 34.5, 22.5, 18.0, 23.0; 8952 x 4096 (280 of clusters of four) 37.0, 26.6, 24.0, 36.0 and 9208 x 2048 (288) 23.5, 18.8, 23.7, 28.7;
-// 18168 x 4096 (284 of two) 44.0, 36.7, 42.5, 61.
+// CTAs per tile: enough to occupy the SMs without splitting the k range finer than four chunks.  The count is part
+// of a result's bits (a CTA's products meet in its accumulator, the CTAs' sums in float32), so it is chosen by the
+// matrix (with experts, by how many of them can have rows) and stays as it is although two CTAs fit an SM by now: with as
+// many as fill the SMs twice, 64 rows on 6136 x 4096 take 20.3 us instead of 24.2, on 12024 x 4096 29.4 instead of 40.3.
 uint32_t narrow_splits(size_t tiles, size_t k_chunks, size_t sms) {
-    constexpr size_t kOf[] = {8, 4, 2}, kSpare[] = {40, 16, 4};
-    for (int i = 0; i < 3; ++i)
-        if (k_chunks >= 4 * kOf[i] && tiles * kOf[i] + kSpare[i] <= 2 * sms) return (uint32_t)kOf[i];
-    return 1;
+    uint32_t best = 1;
+    size_t best_cost = ~(size_t)0;
+    for (uint32_t s : {1u, 2u, 4u, 8u}) {
+        if (s > 1 && k_chunks / s < 4) break;
+        // (a cluster of CTAs does not find room on every SM)
+        const size_t room = s == 1 ? sms : s == 2 ? sms - 4 : sms - 20;
+        const size_t waves = qk::ceil_div(tiles * s, room);
+        const size_t cost = waves * (qk::ceil_div(k_chunks, s) + 10) + (s > 1 ? 6 : 0);
+        if (cost < best_cost) best = s, best_cost = cost;
+    }
+    return best;
 }
 // All the stages, one CTA to an SM, while that many fit (2040 x 8192 as sixteen clusters of eight, which do not:
 // 27.8 us with all stages, 18.3 with half of them; twelve clusters 12.0 and 13.5).

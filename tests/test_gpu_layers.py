@@ -267,6 +267,66 @@ def test_dense_few_rows_by_weight_tiles(dev, tiles, width, tokens):
     assert rel(act[:, :rows_out], silu(xd @ m.double().T) * (xd @ up.double().T)) < 1e-2
 
 
+@pytest.mark.parametrize("tokens", [5, 64, 128])
+@pytest.mark.parametrize("tiles,chunks", [(1, 64), (3, 17), (16, 128), (17, 32), (33, 64), (36, 64), (48, 64), (64, 32), (72, 64),
+                                          (94, 64), (130, 8), (147, 32), (224, 64)])
+def test_dense_few_rows_share_a_tile_among_a_fixed_number_of_blocks(dev, tiles, chunks, tokens):
+    """How many blocks share the k range of a 128-row tile shows in the bits: a block's products meet in its
+    accumulator, where a one is lost beside 2^24, and the blocks' sums are added in float32, in their order."""
+    ctx, torch, L = dev
+    sms, width = torch.cuda.get_device_properties(0).multi_processor_count, 64 * chunks
+    cost = {}
+    for s in (1, 2, 4, 8):
+        if s == 1 or chunks // s >= 4:
+            room = sms - {1: 0, 2: 4, 4: 20, 8: 20}[s]
+            cost[s] = -(-tiles * s // room) * (-(-chunks // s) + 10) + (6 if s > 1 else 0)
+    blocks = min(cost, key=lambda s: (cost[s], s))
+    per, want = -(-chunks // blocks), np.float32(0)
+    for b in range(blocks):
+        first, last = min(b * per, chunks), min((b + 1) * per, chunks)
+        ones = 0 if b == 0 else last - first               # (one by one beside 2^24: lost)
+        want += np.float32((2.0 ** 24 if b == 0 else 0) + ones - (2.0 ** 24 if first < last == chunks else 0))
+    w = L.Weights(torch, torch.device("cuda"), "bfloat16")
+    rows = L.Rows(torch, torch.device("cuda"), tokens, width, w, vector=False)
+    rows.x[:] = 1
+    m = torch.zeros(128 * tiles, width, device="cuda")
+    m[:, 40::64] = 1                                       # (a step of 16 entries of its own)
+    m[:, 0], m[:, -1] = 2.0 ** 24, -2.0 ** 24
+    out = torch.zeros(tokens, 128 * tiles, device="cuda")
+    rows.dense(ctx, w.matrix(m), input=L.IN_PLAIN, x=rows.x, x_stride=width, out=out, out_stride=out.shape[1])
+    assert bool((out == float(want)).all()), (blocks, float(want), out.unique())
+
+
+@pytest.mark.parametrize("tokens", [5, 64, 128])
+@pytest.mark.parametrize("tiles,chunks", [(1, 64), (3, 17), (16, 128), (17, 32), (33, 64), (36, 64), (48, 64), (64, 32), (72, 64),
+                                          (94, 64), (130, 8), (147, 32), (224, 64)])
+def test_dense_few_rows_share_a_tile_among_a_fixed_number_of_blocks(dev, tiles, chunks, tokens):
+    """How many blocks share the k range of a 128-row tile shows in the bits: a block's products meet in its
+    accumulator, where a one is lost beside 2^24, and the blocks' sums are added in float32, in their order."""
+    ctx, torch, L = dev
+    sms, width = torch.cuda.get_device_properties(0).multi_processor_count, 64 * chunks
+    cost = {}
+    for s in (1, 2, 4, 8):
+        if s == 1 or chunks // s >= 4:
+            room = sms - {1: 0, 2: 4, 4: 20, 8: 20}[s]
+            cost[s] = -(-tiles * s // room) * (-(-chunks // s) + 10) + (6 if s > 1 else 0)
+    blocks = min(cost, key=lambda s: (cost[s], s))
+    per, want = -(-chunks // blocks), np.float32(0)
+    for b in range(blocks):
+        first, last = min(b * per, chunks), min((b + 1) * per, chunks)
+        ones = 0 if b == 0 else last - first               # (one by one beside 2^24: lost)
+        want += np.float32((2.0 ** 24 if b == 0 else 0) + ones - (2.0 ** 24 if first < last == chunks else 0))
+    w = L.Weights(torch, torch.device("cuda"), "bfloat16")
+    rows = L.Rows(torch, torch.device("cuda"), tokens, width, w, vector=False)
+    rows.x[:] = 1
+    m = torch.zeros(128 * tiles, width, device="cuda")
+    m[:, 40::64] = 1                                       # (a step of 16 entries of its own)
+    m[:, 0], m[:, -1] = 2.0 ** 24, -2.0 ** 24
+    out = torch.zeros(tokens, 128 * tiles, device="cuda")
+    rows.dense(ctx, w.matrix(m), input=L.IN_PLAIN, x=rows.x, x_stride=width, out=out, out_stride=out.shape[1])
+    assert bool((out == float(want)).all()), (blocks, float(want), out.unique())
+
+
 def test_dense_results_do_not_depend_on_the_rest_of_the_batch(dev):
     """Within a form, the bits of a row are the same whatever rows lie beside it."""
     ctx, torch, L = dev
