@@ -721,9 +721,7 @@ qk_status qk_delta(qk_ctx *ctx, const qk_delta_call *call);
 /* Windowed attention over a latent ring cache (qk_latent_append).  q [tokens][heads][dim_stride]
  * float32; uk [heads*dim_stride][kv_stride] and uv [heads*vdim_stride][kv_stride] in w_dtype.
  * A row at position p sees positions max(0, p - window + 1) .. p; every one of them must still
- * be in the ring.  out [tokens][heads*vdim], stride out_stride.  positions and slots (in qk_delta also the
- * segments) are read before the dependency wait: copies and launches that let nothing start early may write
- * them, as any kernel but this library's own does unless it asks for it. */
+ * be in the ring.  out [tokens][heads*vdim], stride out_stride. */
 typedef struct {
     size_t tokens;
     const int32_t *positions, *slots;

@@ -107,22 +107,18 @@ delta_scan_kernel(DeltaArgs a, int vec) {
     __shared__ __align__(16) float ks[2][kScanTokens][kDim], qs[2][kScanTokens][kDim];
     __shared__ float vs[2][kScanTokens][kScanCols];
     __shared__ __align__(16) float gs[2][kScanTokens][4];
-    // Segments, positions and slots are written by copies and ordinary launches in front of the step, none of
-    // which lets a kernel start early: they are read before the dependency wait, and the state is on its way
-    // to L2 meanwhile.
     const uint32_t h = blockIdx.y, seg = blockIdx.z;
-    const uint32_t first = (uint32_t)a.seg_first[seg], len = (uint32_t)a.seg_len[seg];
-    const int pos0 = len ? a.positions[first] : -1;
-    const uint32_t slot = len ? (uint32_t)a.slots[first] : 0u;
     const uint32_t lane8 = threadIdx.x % 8, col_in = threadIdx.x / 8, col0 = blockIdx.x * kScanCols;
     const uint32_t col = col0 + col_in;
     const bool live = col < a.vdim;
     const uint32_t kvh = h / (a.heads / a.kv_heads), key0 = a.kv_heads * a.dim;
-    float *st = a.state + (((size_t)slot * a.heads + h) * a.vdim + min(col, a.vdim - 1)) * a.dim;
-    if (pos0 > 0)
-        for (uint32_t d = 32 * lane8; d < a.dim; d += 256) asm volatile("prefetch.global.L2 [%0];" ::"l"(st + d));
     qk::pdl_wait();
+    const uint32_t first = (uint32_t)a.seg_first[seg], len = (uint32_t)a.seg_len[seg];
+    if (len == 0) return;
+    const int pos0 = a.positions[first];
+    const uint32_t slot = (uint32_t)a.slots[first];  // (asked for beside the position)
     if (pos0 < 0) return;
+    float *st = a.state + (((size_t)slot * a.heads + h) * a.vdim + min(col, a.vdim - 1)) * a.dim;
 
     // entries past dim stay zero in both buffers
     if (a.dim < (uint32_t)kDim) {
@@ -268,10 +264,9 @@ delta_inputs_kernel(DeltaArgs a, uint32_t n_tokens) {
     const uint32_t t0 = blockIdx.x * kTok, kvh = blockIdx.y, pitch = inputs_pitch(a.dim), ratio = a.heads / a.kv_heads;
     float *qs = ci_smem, *ks = qs + kTok * pitch, *prod = ks + kTok * pitch, *gate = prod + 2 * kTok * kTok;
     const uint32_t n = min((uint32_t)kTok, n_tokens - t0), warp = threadIdx.x / 32, lane = threadIdx.x % 32;
-    // (read before the dependency wait: see delta_scan_kernel)
-    const int pos = a.positions[t0], in_seg = a.seg_row[t0];
-    const uint32_t slot = (uint32_t)a.slots[t0];
     qk::pdl_wait();
+    const int pos = a.positions[t0], in_seg = a.seg_row[t0];
+    const uint32_t slot = (uint32_t)a.slots[t0];  // (all three asked for together)
     if (pos < 0) return;
     const uint32_t key0 = a.kv_heads * a.dim, per = ratio * a.vdim;
 #pragma unroll 1

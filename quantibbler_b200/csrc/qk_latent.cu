@@ -40,7 +40,7 @@ struct LatentArgs {
     uint32_t steps;
     float *partial;    // [tokens][heads][n_splits][kv_stride + 8]: sums, then maximum and weight
     void *out;
-    uint32_t tokens, heads, dim, dim_stride, vdim, vdim_stride, kv_stride, window, ring, n_splits, q_stride, out_stride;
+    uint32_t tokens, heads, dim, dim_stride, vdim, vdim_stride, kv_stride, window, ring, n_slots, n_splits, q_stride, out_stride;
     float scale;
     int out_bf16;
 };
@@ -262,26 +262,25 @@ latent_mma_kernel(LatentArgs a, const uint16_t *__restrict__ cache, uint32_t clu
     extern __shared__ __align__(16) uint8_t lat_smem[];
     const uint32_t split = blockIdx.x, h0 = blockIdx.y * 16, t = blockIdx.z;
     const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32, g = lane >> 2, c4 = lane & 3;
-    // (positions and slots are written by copies and ordinary launches in front of the step, none of
-    // which lets a kernel start early)
-    const int pos = a.positions[t];
-    const uint32_t slot = (uint32_t)a.slots[t];
-    if (pos < 0) {  // (the whole cluster works on one row)
-        qk::pdl_wait();
-        return;
+    // The first keys of the row that the call will most likely name are on their way to L2 before the dependency
+    // wait.  What another kernel may have written is not sure to be seen there: this is a hint, taken inside the cache's
+    // bounds, and nothing else follows from it.
+    if (const uint32_t near = (uint32_t)__ldcg(a.slots + t); near < a.n_slots) {
+        const SplitKeys keys = split_keys(a, max(__ldcg(a.positions + t), 0), split);
+        uint32_t r = keys.first % a.ring + min(lane, keys.count ? keys.count - 1 : 0u);
+        if (r >= a.ring) r -= a.ring;
+        for (uint32_t i = 0; i < (uint32_t)kQ && warp * kQ + i < a.kv_stride; i += 64)
+            asm volatile("prefetch.global.L2 [%0];" ::"l"(cache + ((size_t)near * a.ring + r) * a.kv_stride + warp * kQ + i));
     }
+    qk::pdl_wait();
+    const int pos = __ldcg(a.positions + t);
+    const uint32_t slot = (uint32_t)__ldcg(a.slots + t);
+    if (pos < 0) return;  // (the whole cluster works on one row)
     uint8_t *ring = lat_smem + warp * S::kBufs * S::kTileBytes;
     float *scores = reinterpret_cast<float *>(lat_smem + S::kSmem - S::kScores);  // [2][warp][16][pitch]
     const SplitKeys keys = split_keys(a, pos, split);
     const uint16_t *base = cache + (size_t)slot * a.ring * a.kv_stride + warp * kQ;
     const uint32_t ring0 = keys.first % a.ring, n_tiles = (keys.count + kLatKeys - 1) / kLatKeys;
-    {   // the first keys are on their way to L2 before the dependency wait
-        uint32_t r = ring0 + min(lane, keys.count ? keys.count - 1 : 0u);
-        if (r >= a.ring) r -= a.ring;
-        for (uint32_t i = 0; i < (uint32_t)kQ && warp * kQ + i < a.kv_stride; i += 64)
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(base + (size_t)r * a.kv_stride + i));
-    }
-    qk::pdl_wait();
     auto fetch = [&](uint32_t tile) {
         if (tile < n_tiles) {
             uint8_t *dst = ring + (tile % S::kBufs) * S::kTileBytes;
@@ -605,8 +604,8 @@ latent_output_row_kernel(LatentArgs a, const W *__restrict__ uv, uint32_t per_bl
                           held[q][i]);
     };
     fetch(j0 + warp);
-    const bool live = a.positions[t] >= 0;  // (an idle row's output is zero; see latent_mma_kernel)
     qk::pdl_wait();
+    const bool live = a.positions[t] >= 0;  // (an idle row's output is zero; used once the loads below are out)
     const float *src = a.partial + ((size_t)t * a.heads + h) * n * pitch;
     auto sums = [&](uint32_t i, uint32_t s0, float2 (&x)[kAhead]) {
 #pragma unroll
@@ -617,11 +616,9 @@ latent_output_row_kernel(LatentArgs a, const W *__restrict__ uv, uint32_t per_bl
     sums(2 * threadIdx.x, 0, x);
     const float *w;  // the splits' weights
     if (n <= 32) {
-        float ms = -INFINITY, ls = 0.f;
-        if (lane < n && live) {
-            ms = src[(size_t)lane * pitch + a.kv_stride];
-            ls = src[(size_t)lane * pitch + a.kv_stride + 1];
-        }
+        float ms = src[(size_t)min(lane, n - 1) * pitch + a.kv_stride];
+        const float ls = src[(size_t)min(lane, n - 1) * pitch + a.kv_stride + 1];
+        if (lane >= n || !live) ms = -INFINITY;
         float m = ms;
         for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
         const float e = ms == -INFINITY ? 0.f : expf(ms - m);
@@ -1062,6 +1059,7 @@ qk_status qk_latent_attention(qk_ctx *ctx, const qk_latent_call *d) {
     a.kv_stride = (uint32_t)d->kv_stride;
     a.window = (uint32_t)d->window;
     a.ring = (uint32_t)d->ring;
+    a.n_slots = (uint32_t)std::min<size_t>(d->n_slots, UINT32_MAX);
     a.n_splits = (uint32_t)d->n_splits;
     a.q_stride = (uint32_t)d->q_stride;
     a.out_stride = (uint32_t)d->out_stride;

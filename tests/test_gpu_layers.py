@@ -297,36 +297,6 @@ def test_dense_few_rows_share_a_tile_among_a_fixed_number_of_blocks(dev, tiles, 
     assert bool((out == float(want)).all()), (blocks, float(want), out.unique())
 
 
-@pytest.mark.parametrize("tokens", [5, 64, 128])
-@pytest.mark.parametrize("tiles,chunks", [(1, 64), (3, 17), (16, 128), (17, 32), (33, 64), (36, 64), (48, 64), (64, 32), (72, 64),
-                                          (94, 64), (130, 8), (147, 32), (224, 64)])
-def test_dense_few_rows_share_a_tile_among_a_fixed_number_of_blocks(dev, tiles, chunks, tokens):
-    """How many blocks share the k range of a 128-row tile shows in the bits: a block's products meet in its
-    accumulator, where a one is lost beside 2^24, and the blocks' sums are added in float32, in their order."""
-    ctx, torch, L = dev
-    sms, width = torch.cuda.get_device_properties(0).multi_processor_count, 64 * chunks
-    cost = {}
-    for s in (1, 2, 4, 8):
-        if s == 1 or chunks // s >= 4:
-            room = sms - {1: 0, 2: 4, 4: 20, 8: 20}[s]
-            cost[s] = -(-tiles * s // room) * (-(-chunks // s) + 10) + (6 if s > 1 else 0)
-    blocks = min(cost, key=lambda s: (cost[s], s))
-    per, want = -(-chunks // blocks), np.float32(0)
-    for b in range(blocks):
-        first, last = min(b * per, chunks), min((b + 1) * per, chunks)
-        ones = 0 if b == 0 else last - first               # (one by one beside 2^24: lost)
-        want += np.float32((2.0 ** 24 if b == 0 else 0) + ones - (2.0 ** 24 if first < last == chunks else 0))
-    w = L.Weights(torch, torch.device("cuda"), "bfloat16")
-    rows = L.Rows(torch, torch.device("cuda"), tokens, width, w, vector=False)
-    rows.x[:] = 1
-    m = torch.zeros(128 * tiles, width, device="cuda")
-    m[:, 40::64] = 1                                       # (a step of 16 entries of its own)
-    m[:, 0], m[:, -1] = 2.0 ** 24, -2.0 ** 24
-    out = torch.zeros(tokens, 128 * tiles, device="cuda")
-    rows.dense(ctx, w.matrix(m), input=L.IN_PLAIN, x=rows.x, x_stride=width, out=out, out_stride=out.shape[1])
-    assert bool((out == float(want)).all()), (blocks, float(want), out.unique())
-
-
 def test_dense_results_do_not_depend_on_the_rest_of_the_batch(dev):
     """Within a form, the bits of a row are the same whatever rows lie beside it."""
     ctx, torch, L = dev
@@ -461,6 +431,70 @@ def test_latent_attention_of_several_rows(dev, tokens, heads, vdim, kv, splits, 
         pr = torch.softmax(torch.einsum("hd,hjd->hj", q[t, :, :dim].double(), kk) * dim ** -0.5, dim=1)
         want = torch.einsum("hj,hjd->hd", pr, vv)
         assert float((got[t] - want).abs().max() / want.abs().max()) < (1e-4 if bf16 else 1e-5), t
+
+
+def delta_problem(torch, L, tokens, slots, heads, kv_heads, dim, vdim, segments, seed):
+    """Buffers of one qk_delta call, and the call: rows of one portion (segments 1) or one row of each sequence."""
+    g = torch.Generator(device="cuda").manual_seed(seed)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    i32 = dict(dtype=torch.int32, device="cuda")
+    taps, keys = 4, kv_heads * dim
+    channels, at = 2 * keys + heads * vdim, L.up_to(2 * keys + heads * vdim, 8)
+    stride = L.up_to(at + 2 * heads, 8)
+    b = dict(proj=rnd(tokens, stride), conv_q=rnd(keys, taps), conv_k=rnd(keys, taps), conv_v=rnd(heads * vdim, taps),
+             a_log=rnd(heads) * 0.1 - 1, dt_bias=rnd(heads) * 0.1, conv_state=rnd(slots, taps, channels),
+             state=rnd(slots, heads, vdim, dim), qkv=torch.zeros(tokens, channels, device="cuda"),
+             gates=torch.zeros(L.up_to(tokens, 8), heads, 20, device="cuda"), out=torch.zeros(tokens, heads * vdim, device="cuda"),
+             positions=torch.arange(tokens, **i32) + 5, slots=torch.zeros(tokens, **i32),
+             seg_first=torch.arange(segments, **i32), seg_len=torch.full((segments,), tokens // segments, **i32),
+             seg_row=torch.arange(tokens, **i32) % (tokens // segments))
+    call = L.DeltaCall(tokens=tokens, segments=segments, heads=heads, kv_heads=kv_heads, dim=dim, vdim=vdim, taps=taps,
+                       proj_stride=stride, beta_offset=at, decay_offset=at + heads, unit_eps=1e-6, out_stride=heads * vdim,
+                       **{n: t.data_ptr() for n, t in b.items()})
+    return b, call
+
+
+def test_rows_that_the_kernel_before_names(dev):
+    """Positions and slots written by the kernel right in front of the delta rule and the latent attention, another
+    set each time: the rows are taken from it, as after a synchronisation."""
+    ctx, torch, L = dev
+    tokens, slots = 4, 8
+    b, delta = delta_problem(torch, L, tokens, slots, 4, 2, 64, 64, tokens, 3)
+    g = torch.Generator(device="cuda").manual_seed(9)
+    rnd = lambda *s: torch.randn(*s, device="cuda", generator=g)
+    heads, dim, kv, window, splits = 16, 32, 128, 256, 8
+    half = dict(uk=rnd(heads, dim, kv) / kv ** 0.5, uv=rnd(heads, dim, kv) / kv ** 0.5, cache=rnd(slots, window, kv))
+    half = {n: t.bfloat16() for n, t in half.items()}
+    q, out = rnd(tokens, heads * dim), torch.zeros(tokens, heads * dim, device="cuda")
+    scratch = torch.zeros(_lib.lib().qk_latent_scratch(tokens, heads, kv, splits) // 4, device="cuda")
+    latent = L.LatentCall(tokens=tokens, positions=b["positions"].data_ptr(), slots=b["slots"].data_ptr(), heads=heads, dim=dim,
+                          dim_stride=dim, vdim=dim, vdim_stride=dim, kv_rank=kv, kv_stride=kv, window=window, ring=window,
+                          n_slots=slots, scale=dim ** -0.5, q=q.data_ptr(), q_dtype=QK_F32, q_stride=heads * dim, w_dtype=QK_BF16,
+                          n_splits=splits, scratch=scratch.data_ptr(), out=out.data_ptr(), out_dtype=QK_F32,
+                          out_stride=heads * dim, **{n: t.data_ptr() for n, t in half.items()})
+    state, conv = b["state"].clone(), b["conv_state"].clone()
+    names = [(torch.randint(0, window, (tokens,), device="cuda", generator=g, dtype=torch.int32),
+              torch.randperm(slots, device="cuda", generator=g)[:tokens].to(torch.int32)) for _ in range(6)]
+    one = torch.ones(tokens, dtype=torch.int32, device="cuda")
+
+    def ran(k, wait):
+        got = []
+        for call, entry, result in ((delta, _lib.lib().qk_delta, "delta"), (latent, _lib.lib().qk_latent_attention, "latent")):
+            b["state"].copy_(state), b["conv_state"].copy_(conv), b["positions"].zero_(), b["slots"].zero_()
+            torch.cuda.synchronize()
+            torch.mul(names[k][1], one, out=b["slots"])
+            torch.mul(names[k][0], one, out=b["positions"])
+            if wait:
+                torch.cuda.synchronize()
+            check(entry(ctx.handle, ctypes.byref(call)))
+            ctx.synchronize()
+            got.append((b["out"] if result == "delta" else out).clone())
+        return got + [b["state"].clone()]
+
+    for k in range(len(names)):
+        want = ran(k, True)
+        for _ in range(5):
+            assert all(torch.equal(x, y) for x, y in zip(ran(k, False), want)), k
 
 
 @pytest.mark.parametrize("dim,vdim,window,p0,tokens", [

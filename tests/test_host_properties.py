@@ -1,12 +1,15 @@
 """Property tests of the host-side functions of the library (no GPU): random shapes and
 seeds instead of hand-picked ones.  The oracles are NumPy one-liners or ``oracle/``."""
 
+import os
+import re
+
 import numpy as np
 from hypothesis import given, settings
 from hypothesis import strategies as st
 
 from oracle import itq_np
-from quantibbler_b200 import kernels
+from quantibbler_b200 import _build, kernels
 
 
 @settings(max_examples=60, deadline=None, derandomize=True, database=None)
@@ -51,3 +54,18 @@ def test_joint_itq_equals_the_numpy_oracle(dout, din, rank, seed, max_iter):
         assert np.all(np.abs(want[4][differ]) < 1e-9)
     else:
         assert got[2] == want[2] and got[3] == want[3]
+
+
+def test_kernels_read_what_callers_write_behind_the_dependency_wait():
+    """What the kernel before may have written is visible behind griddepcontrol.wait only: in front of it the delta
+    rule's and the latent attention's kernels read constants (and a hint that nothing but a prefetch follows from)."""
+    csrc = os.path.join(os.path.dirname(_build.__file__), "csrc")
+    for name in ("qk_delta.cu", "qk_latent.cu"):
+        with open(os.path.join(csrc, name)) as f:
+            source = f.read()
+        early = re.findall(r"pdl_launch\(\);(.*?)pdl_wait\(\);", source, re.S)
+        assert early
+        for part in early:
+            assert not re.search(r"a\.(positions|slots|seg_first|seg_len|seg_row|partial|absorbed|proj|q)\[", part), (name, part)
+            for hint in re.findall(r".*__ldcg\(a\.(?:positions|slots).*", part):
+                assert "near" in hint or "split_keys" in hint, hint
