@@ -249,8 +249,10 @@ delta_scan_kernel(DeltaArgs a, int vec) {
 // scalars per column is sequential.  The scalars depend on the head alone: the inputs kernel
 // writes them once, 20 floats per token: beta R (k . k) [8], R (k . q) [8], beta, beta P, P, R_8.
 constexpr int kMini = 8, kCoef = 20;
-// Floats between the rows of q and k in shared memory: whole fours, the fours of neighbouring rows in other banks.
-__host__ __device__ constexpr uint32_t inputs_pitch(uint32_t dim) { return (dim + 3) / 4 * 4 + 4; }
+// A row of q or k in shared memory: its even entries, then its odd ones from inputs_odd on, each padded to whole fours.  The
+// rows lie so that eight threads that read fours of the two halves of four rows two apart meet 32 different banks.
+__host__ __device__ constexpr uint32_t inputs_odd(uint32_t dim) { return ((dim + 1) / 2 + 31) / 32 * 32 + 20; }
+__host__ __device__ constexpr uint32_t inputs_pitch(uint32_t dim) { return 2 * inputs_odd(dim) - 20; }
 
 // A block takes kTok rows and one key head with the heads it serves.  Thread per channel: convolution
 // and silu of the rows from one window of loads (kTaps bounds the taps), then a warp per row for
@@ -264,6 +266,8 @@ delta_inputs_kernel(DeltaArgs a, uint32_t n_tokens) {
     const uint32_t t0 = blockIdx.x * kTok, kvh = blockIdx.y, pitch = inputs_pitch(a.dim), ratio = a.heads / a.kv_heads;
     float *qs = ci_smem, *ks = qs + kTok * pitch, *prod = ks + kTok * pitch, *gate = prod + 2 * kTok * kTok;
     const uint32_t n = min((uint32_t)kTok, n_tokens - t0), warp = threadIdx.x / 32, lane = threadIdx.x % 32;
+    const uint32_t odd = inputs_odd(a.dim);
+    auto at = [&](uint32_t row, uint32_t d) { return row * pitch + d % 2 * odd + d / 2; };
     qk::pdl_wait();
     const int pos = a.positions[t0], in_seg = a.seg_row[t0];
     const uint32_t slot = (uint32_t)a.slots[t0];  // (all three asked for together)
@@ -302,7 +306,7 @@ delta_inputs_kernel(DeltaArgs a, uint32_t n_tokens) {
             if (which == 2) {
                 if (t < (int)n) a.qkv[(size_t)(t0 + t) * a.channels + ch] = y;
             } else {
-                (which == 0 ? qs : ks)[t * pitch + in] = t < (int)n ? y : 0.f;
+                (which == 0 ? qs : ks)[at(t, in)] = t < (int)n ? y : 0.f;
             }
         }
     }
@@ -322,8 +326,9 @@ delta_inputs_kernel(DeltaArgs a, uint32_t n_tokens) {
     if (warp < (uint32_t)kTok) {   // unit vectors: warp = row
         float sq = 0.f, sk = 0.f;
         for (uint32_t d = lane; d < a.dim; d += 32) {
-            sq += qs[warp * pitch + d] * qs[warp * pitch + d];
-            sk += ks[warp * pitch + d] * ks[warp * pitch + d];
+            const uint32_t i = at(warp, d);
+            sq += qs[i] * qs[i];
+            sk += ks[i] * ks[i];
         }
         for (int off = 16; off > 0; off >>= 1) {
             sq += __shfl_xor_sync(0xffffffffu, sq, off);
@@ -331,13 +336,14 @@ delta_inputs_kernel(DeltaArgs a, uint32_t n_tokens) {
         }
         const float iq = 1.0f / sqrtf(sq + a.unit_eps) * (1.0f / sqrtf((float)a.dim));
         const float ik = 1.0f / sqrtf(sk + a.unit_eps);
-        if (a.dim + lane < pitch) qs[warp * pitch + a.dim + lane] = ks[warp * pitch + a.dim + lane] = 0.f;
+        if (a.dim + lane < (a.dim + 7) / 8 * 8) qs[at(warp, a.dim + lane)] = ks[at(warp, a.dim + lane)] = 0.f;
         float *row = a.qkv + (size_t)(t0 + warp) * a.channels + kvh * a.dim;
         float dot = 0.f;
         for (uint32_t d = lane; d < a.dim; d += 32) {
-            const float q = qs[warp * pitch + d] * iq, k = ks[warp * pitch + d] * ik;
-            qs[warp * pitch + d] = q;
-            ks[warp * pitch + d] = k;
+            const uint32_t i = at(warp, d);
+            const float q = qs[i] * iq, k = ks[i] * ik;
+            qs[i] = q;
+            ks[i] = k;
             dot += q * k;
             if (warp < n) {
                 row[d] = q;
@@ -357,31 +363,33 @@ delta_inputs_kernel(DeltaArgs a, uint32_t n_tokens) {
     if constexpr (kTok == 1) return;
     __syncthreads();
     if constexpr (kTok == 8) {
-        // k_i . k_t and k_i . q_t, two rows by two: eight threads a square, each with every eighth group of four
-        // entries.  (With two threads a product, entry by entry, a launch on 2048 rows at width 4096 took 74 us, now 66.)
-        const uint32_t square = threadIdx.x / 8, part = threadIdx.x % 8, kind = square / 16, t = square / 4 % 4 * 2, i = square % 4 * 2;
-        const float *x = (kind ? qs : ks) + t * pitch, *y = ks + i * pitch;
-        float v[2][2] = {};
-        for (uint32_t d = 4 * part; d < a.dim; d += 32) {
-            float4 xs[2], ys[2];
+        // k_i . k_t and k_i . q_t, two rows by two: two threads a square, one adds up the even entries, the other the odd
+        // ones, in their order (two threads a product, entry by entry, give the same bits from four times the reads)
+        if (threadIdx.x < 64) {
+            const uint32_t square = threadIdx.x / 2, kind = square / 16, t = square / 4 % 4 * 2, i = square % 4 * 2;
+            const uint32_t part = threadIdx.x % 2 * odd, own = (a.dim + 1) / 2;
+            const float *x = (kind ? qs : ks) + t * pitch + part, *y = ks + i * pitch + part;
+            float v[2][2] = {};
+#pragma unroll 4
+            for (uint32_t d = 0; d < own; d += 4) {
+                float4 xs[2], ys[2];
 #pragma unroll
-            for (int r = 0; r < 2; ++r) {
-                xs[r] = *reinterpret_cast<const float4 *>(x + r * pitch + d);
-                ys[r] = *reinterpret_cast<const float4 *>(y + r * pitch + d);
+                for (int r = 0; r < 2; ++r) {
+                    xs[r] = *reinterpret_cast<const float4 *>(x + r * pitch + d);
+                    ys[r] = *reinterpret_cast<const float4 *>(y + r * pitch + d);
+                }
+#pragma unroll
+                for (int r = 0; r < 2; ++r)
+#pragma unroll
+                    for (int c = 0; c < 2; ++c)
+                        v[r][c] = fmaf(xs[r].w, ys[c].w, fmaf(xs[r].z, ys[c].z, fmaf(xs[r].y, ys[c].y, fmaf(xs[r].x, ys[c].x, v[r][c]))));
             }
 #pragma unroll
-            for (int r = 0; r < 2; ++r)
-#pragma unroll
-                for (int c = 0; c < 2; ++c)
-                    v[r][c] = fmaf(xs[r].x, ys[c].x, fmaf(xs[r].y, ys[c].y, fmaf(xs[r].z, ys[c].z, fmaf(xs[r].w, ys[c].w, v[r][c]))));
+            for (int e = 0; e < 4; ++e) {
+                const float sum = v[e / 2][e % 2] + __shfl_xor_sync(0xffffffffu, v[e / 2][e % 2], 1);
+                if (e / 2 == (int)(threadIdx.x % 2)) prod[kind * kTok * kTok + (t + e / 2) * kTok + i + e % 2] = sum;
+            }
         }
-#pragma unroll
-        for (int off = 4; off > 0; off >>= 1)
-#pragma unroll
-            for (int e = 0; e < 4; ++e) v[e / 2][e % 2] += __shfl_xor_sync(0xffffffffu, v[e / 2][e % 2], off);
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-            if (part == (uint32_t)e) prod[kind * kTok * kTok + (t + e / 2) * kTok + i + e % 2] = v[e / 2][e % 2];
     }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < ratio * kTok; i += 256) {

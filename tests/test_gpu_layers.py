@@ -454,6 +454,40 @@ def delta_problem(torch, L, tokens, slots, heads, kv_heads, dim, vdim, segments,
     return b, call
 
 
+@pytest.mark.parametrize("tokens", [8, 19])
+@pytest.mark.parametrize("dim", [1, 2, 7, 50, 64, 128, 130, 509, 512])
+def test_delta_scalars_of_a_portion_are_summed_in_one_order(dev, dim, tokens):
+    """The bits of k . k and k . q: one chain of fused multiply-adds over the even entries, one over the odd ones, and their
+    sum.  Restated in numpy (a product of two float32 is exact in float64, so that one rounding makes the fused
+    multiply-add); without decay and with a beta of one the scalars are the products themselves."""
+    ctx, torch, L = dev
+    heads, kv_heads = 2, 1
+    b, call = delta_problem(torch, L, tokens, 1, heads, kv_heads, dim, 16, 1, dim)
+    b["a_log"].fill_(-100.0)                                              # (a decay of exactly one)
+    b["proj"][:, call.beta_offset:call.beta_offset + heads] = 100.0       # (a beta of exactly one)
+    check(_lib.lib().qk_delta(ctx.handle, ctypes.byref(call)))
+    ctx.synchronize()
+    f32, f64 = np.float32, np.float64
+    rows = np.zeros((2, L.up_to(tokens, 8), dim), f32)
+    rows[:, :tokens] = np.moveaxis(b["qkv"].cpu().numpy()[:, :2 * dim].reshape(tokens, 2, dim), 1, 0)
+    q, k = rows.reshape(2, -1, 8, dim)
+
+    def products(x):
+        chains = np.zeros((2, x.shape[0], 8, 8), f32)                     # [parity][chunk][t][i]
+        for d in range(dim):
+            exact = x[:, :, None, d].astype(f64) * k[:, None, :, d].astype(f64)
+            chains[d % 2] = (exact + chains[d % 2].astype(f64)).astype(f32)
+        return chains[0] + chains[1]
+
+    gates = b["gates"].cpu().numpy().reshape(-1, heads, 8, 20)
+    kk, kq = products(k), products(q)
+    for c in range(gates.shape[0]):
+        for t in range(min(8, tokens - 8 * c)):
+            for h in range(heads):
+                assert np.array_equal(gates[c, h, t, :t], kk[c, t, :t]), (c, t)
+                assert np.array_equal(gates[c, h, t, 8:9 + t], kq[c, t, :t + 1]), (c, t)
+
+
 def test_rows_that_the_kernel_before_names(dev):
     """Positions and slots written by the kernel right in front of the delta rule and the latent attention, another
     set each time: the rows are taken from it, as after a synchronisation."""
