@@ -1514,10 +1514,13 @@ attention_sage_umma_kernel(SageArgs a, AttnDims dm, int causal, uint32_t wait_li
                 }
                 __syncwarp();
                 if (!more) continue;
-                ok = mbar_wait(bars->digits_read + g, ((it + 2) >> 1) & 1, abort_flag, limit);
+                // S goes over the P codes: the products that read them must be done (the order of issue holds from one
+                // product to the next for one accumulator and shape only).
+                ok = mbar_wait(bars->digits_read + g, ((it + 2) >> 1) & 1, abort_flag, limit) &&
+                     mbar_wait(bars->pv, it & 1, abort_flag, limit) && mbar_wait(bars->pv + 1, it & 1, abort_flag, limit);
                 if (!ok) break;
                 tc_fence_after();
-                if (elect_one()) issue_s(it + 2);  // (over the P codes, behind the products that read them)
+                if (elect_one()) issue_s(it + 2);
                 __syncwarp();
             }
         } else if (warp == kUCopyWarp) {

@@ -355,6 +355,25 @@ def test_sage_tcgen05_kernel_at_the_edges_of_its_tiles(gpu_ctx, seq, causal):
         assert np.array_equal(codes[name], same[name], equal_nan=True), name
 
 
+def test_sage_tcgen05_kernel_repeats_its_bits(gpu_ctx):
+    """Many iterations of many tiles, over and over: a product issued before the one whose operand it overwrites has
+    read it would show as other bits."""
+    b, h, kvh, seq, d, block = 1, 16, 4, 3072, 128, 64
+    rng = np.random.default_rng(77)
+    q = rng.standard_normal((b, h, seq, d), dtype=np.float32) * 3
+    k, v = (rng.standard_normal((b, kvh, seq, d), dtype=np.float32) for _ in range(2))
+    default = gpu_ctx.set_sage_kernel(1)
+    try:
+        tc = run_sage(gpu_ctx, q, k, v, True, block)
+        gpu_ctx.set_sage_kernel(2)
+        first = run_sage(gpu_ctx, q, k, v, True, block)
+        assert np.abs(first - tc).max() <= 1e-5 * np.abs(tc).max()
+        for _ in range(20):
+            assert np.array_equal(run_sage(gpu_ctx, q, k, v, True, block), first)
+    finally:
+        gpu_ctx.set_sage_kernel(default)
+
+
 def test_attention_on_device_buffers(gpu_ctx):
     import torch
     rng = np.random.default_rng(11)

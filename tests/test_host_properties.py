@@ -69,3 +69,11 @@ def test_kernels_read_what_callers_write_behind_the_dependency_wait():
             assert not re.search(r"a\.(positions|slots|seg_first|seg_len|seg_row|partial|absorbed|proj|q)\[", part), (name, part)
             for hint in re.findall(r".*__ldcg\(a\.(?:positions|slots).*", part):
                 assert "near" in hint or "split_keys" in hint, hint
+
+
+def test_sage_scores_are_issued_behind_the_products_whose_operand_they_overwrite():
+    """The scores of iteration it + 2 take the tensor memory of iteration it's P codes.  tcgen05.mma keeps the order of
+    issue for one accumulator and shape only, so both value products are waited for in between."""
+    with open(os.path.join(os.path.dirname(_build.__file__), "csrc", "qk_attention.cu")) as f:
+        loop = re.search(r"issue_pv\(it, 1\);(.*?)issue_s\(it \+ 2\);", f.read(), re.S).group(1)
+    assert "mbar_wait(bars->pv, it & 1" in loop and "mbar_wait(bars->pv + 1, it & 1" in loop
