@@ -467,6 +467,11 @@ sage_prepare_kernel(const float *__restrict__ q, const float *__restrict__ k, co
     qk::pdl_launch();
     qk::pdl_wait();
     const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32, kv_blocks = 2 * planes * n_blocks;
+    // (a caller's buffers need not lie on sixteen bytes)
+    auto load4 = [](const float *p, bool wide) {
+        return wide ? *reinterpret_cast<const float4 *>(p) : make_float4(p[0], p[1], p[2], p[3]);
+    };
+    auto on16 = [](const float *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; };
     auto peak4 = [](float4 x) { return fmaxf(fmaxf(fabsf(x.x), fabsf(x.y)), fmaxf(fabsf(x.z), fabsf(x.w))); };
     auto warp_max = [](float m) {
         for (int off = 16; off > 0; off >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, off));
@@ -481,7 +486,7 @@ sage_prepare_kernel(const float *__restrict__ q, const float *__restrict__ k, co
         float4 x[4];
 #pragma unroll
         for (int e = 0; e < 4; ++e)
-            x[e] = *reinterpret_cast<const float4 *>(q + (size_t)min(row0 + kPrepWarps * e, q_rows - 1) * 128 + 4 * lane);
+            x[e] = load4(q + (size_t)min(row0 + kPrepWarps * e, q_rows - 1) * 128 + 4 * lane, on16(q));
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
             const uint32_t row = row0 + kPrepWarps * e;
@@ -506,7 +511,7 @@ sage_prepare_kernel(const float *__restrict__ q, const float *__restrict__ k, co
 #pragma unroll
         for (int e = 0; e < 8; ++e) {
             const uint32_t j = warp + kPrepWarps * e;
-            x[e] = *reinterpret_cast<const float4 *>(src + (size_t)min(j, kj - 1) * 128 + 4 * lane);
+            x[e] = load4(src + (size_t)min(j, kj - 1) * 128 + 4 * lane, on16(src));
             if (j >= kj) x[e] = make_float4(0.f, 0.f, 0.f, 0.f);
         }
 #pragma unroll

@@ -374,6 +374,34 @@ def test_sage_tcgen05_kernel_repeats_its_bits(gpu_ctx):
         gpu_ctx.set_sage_kernel(default)
 
 
+@pytest.mark.parametrize("which", ["q", "k", "v"])
+def test_sage_inputs_need_not_lie_on_sixteen_bytes(gpu_ctx, which):
+    """One input after the other on four bytes only: the bits of the aligned call (tcgen05 form)."""
+    import torch
+    b, h, kvh, seq, d, block = 1, 4, 2, 321, 128, 64
+    rng = np.random.default_rng(5)
+    host = dict(q=rng.standard_normal((b, h, seq, d), dtype=np.float32), k=rng.standard_normal((b, kvh, seq, d), dtype=np.float32),
+                v=rng.standard_normal((b, kvh, seq, d), dtype=np.float32))
+    shape, outs = shape_of(*host.values()), []
+    default = gpu_ctx.set_sage_kernel(2)
+    try:
+        for shift in (0, 1):
+            bufs = {}
+            for name, x in host.items():
+                at = shift if name == which else 0
+                buf = torch.zeros(x.size + 4, device="cuda")
+                buf[at:at + x.size] = torch.from_numpy(x).cuda().flatten()
+                bufs[name] = buf[at:]
+            out = torch.zeros(b, h, seq, d, device="cuda")
+            torch.cuda.synchronize()
+            gpu_ctx.attention_dev(shape, *(t.data_ptr() for t in bufs.values()), True, out.data_ptr(), block)
+            gpu_ctx.synchronize()
+            outs.append(out)
+    finally:
+        gpu_ctx.set_sage_kernel(default)
+    assert bool((outs[0] != 0).any()) and torch.equal(*outs)
+
+
 def test_attention_on_device_buffers(gpu_ctx):
     import torch
     rng = np.random.default_rng(11)
