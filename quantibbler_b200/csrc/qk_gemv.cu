@@ -1818,7 +1818,7 @@ SumPlan sum_plan(const qk_ctx *c, const StageShape &s, size_t n_inst, size_t tot
                  bool normed = false) {
     SumPlan pl{};
     pl.ranks = (uint32_t)qk::ceil_div(s.n_bits, (size_t)kSumSlice);
-    if (c->gemv_kernel != 1 || pl.ranks > 8u || (normed && s.n_bits > 8 * kSumThreads) || s.n_groups > 65535 ||
+    if (c->gemv_kernel != 1 || pl.ranks > kSumRanks || s.n_bits > kSumMostEntries || (normed && s.n_bits > 8 * kSumThreads) || s.n_groups > 65535 ||
         (double)total_rows * (double)s.n_bits > sum_most_weights(n_inst, final, bf16))
         return pl;
     pl.slice = pl.ranks == 1 ? (uint32_t)s.n_bits

@@ -16,7 +16,8 @@
 // fetched costs more than a branch.  The weight rows are copied to shared memory before the wait for the kernel
 // before this one.  An SM holds one block (the launch asks for that much shared memory): blocks that came in early
 // beside the kernel before would crowd on some SMs and leave others idle.  Long vectors are split over the CTAs of a
-// cluster, `slice_bits` entries each, on a grid of their own; the CTAs share out the final sums.
+// cluster, `slice_bits` entries each, on one grid, that of the whole vector's largest entry; the CTAs share out the rows, whose
+// whole numbers they add up before they are converted.
 //
 // What bounds it: latencies.  By the clock of block 0, us from the wait to the end: the first stage of a 4096 x 4096 linear of
 // rank 1102 with the norm inside 5.3 (entries 1.7, grid and conversion 0.9, sums 1.7, rows 0.8), its second stage 2.9; a
@@ -29,6 +30,9 @@ namespace {
 constexpr int kSumThreads = 512, kSumEntries = 16;  // entries a thread
 constexpr uint32_t kSumSlice = kSumThreads * kSumEntries;  // most entries of a CTA
 constexpr int kSumLow = 21;                          // bits of lo
+constexpr uint32_t kSumRanks = 8;                    // most CTAs of a cluster
+// |q| <= 2^47: a row's sum over fewer entries than this is a 64-bit integer.
+constexpr uint32_t kSumMostEntries = (1u << 16) - 1;
 
 // Shared memory: [hi of the entries, transposed][lo][the entries][weight rows][partial sums][row sums]
 struct SumLayout {
@@ -68,6 +72,7 @@ __device__ __forceinline__ void sum_form(const StageParams &p, uint32_t rows_per
     constexpr int kWarps = kSumThreads / 32;
     __shared__ __align__(16) float norm_red[kWarps];
     __shared__ Bits top_red[kWarps];
+    __shared__ Bits peer_top[kSumRanks];  // (slices)
     const uint32_t tid = threadIdx.x, warp = tid / 32, lane = tid % 32;
     const uint32_t n_rows = p.n_rows, n_bits = p.n_bits;
     const uint32_t row0 = (blockIdx.x / n_rank) * rows_per_block;
@@ -76,6 +81,7 @@ __device__ __forceinline__ void sum_form(const StageParams &p, uint32_t rows_per
         qk::pdl_wait();
         return;
     }
+    if (n_rank > 1) asm volatile("barrier.cluster.arrive.relaxed.aligned;" ::: "memory");  // (this CTA has begun)
     const uint32_t rows = min(rows_per_block, n_rows - row0);
     const uint32_t k_lo = min(rank * slice_bits, n_bits), k_hi = min(k_lo + slice_bits, n_bits);
     const SumLayout lay = sum_layout(max(1u, k_hi - k_lo), rows_per_block, sizeof(Entry));
@@ -84,7 +90,7 @@ __device__ __forceinline__ void sum_form(const StageParams &p, uint32_t rows_per
     Entry *entries = reinterpret_cast<Entry *>(smem_dyn + lay.entries);
     uint8_t *slab = smem_dyn + lay.slab;
     long long *part = reinterpret_cast<long long *>(smem_dyn + lay.part);  // [row][warp of the vector]; row `rows_per_block`: totals
-    double *row_sum = reinterpret_cast<double *>(smem_dyn + lay.row_sum);  // (slices)
+    long long *row_sum = reinterpret_cast<long long *>(smem_dyn + lay.row_sum);  // (slices)
     const uint32_t z_pitch = lay.lanes + 1, padded = kSumEntries * lay.lanes;
 
     // ---- what depends on no other kernel: the weight rows, the constant vectors
@@ -195,6 +201,22 @@ __device__ __forceinline__ void sum_form(const StageParams &p, uint32_t rows_per
         }
     }
 
+    if (n_rank > 1) {  // the whole vector's largest: every CTA tells every other, once that one has begun
+        asm volatile("barrier.cluster.wait.aligned;" ::: "memory");
+        if (tid < n_rank) {
+            uint32_t there;
+            asm volatile("mapa.shared::cluster.u32 %0, %1, %2;"
+                         : "=r"(there)
+                         : "r"((uint32_t)__cvta_generic_to_shared(peer_top + rank)), "r"(tid));
+            if constexpr (sizeof(Entry) == 4) asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(there), "r"(top) : "memory");
+            else asm volatile("st.shared::cluster.u64 [%0], %1;" ::"r"(there), "l"(top) : "memory");
+        }
+        __syncwarp();
+        asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+        asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+        for (uint32_t c = 0; c < n_rank; ++c) top = peer_top[c] > top ? peer_top[c] : top;
+    }
+
     // ---- the entries on the grid of the largest one.  x = v * 2^(shift - 21) lies within 2^26; q = rint(x * 2^21) =
     // hi * 2^21 + lo with hi = rint(x), exactly.
     const bool nonfinite = top >= FloatBits<Entry>::kBad;  // a NaN or an infinity: every row is NaN, as in the digit forms
@@ -289,11 +311,12 @@ __device__ __forceinline__ void sum_form(const StageParams &p, uint32_t rows_per
     auto row_value = [&](uint32_t r) {
         long long s = 0;
         for (uint32_t w = 0; w < lay.warps; ++w) s += part[r * lay.warps + w];
-        const double n = (double)(2 * s - total);
-        return nonfinite ? nan("") : unit != 0.0 ? n * unit : ldexp(n, oexp);
+        return 2 * s - total;
     };
-    auto finish = [&](uint32_t r, double val) {
+    auto finish = [&](uint32_t r, long long sum) {
         const uint32_t row = row0 + r;
+        const double n = (double)sum;
+        double val = nonfinite ? nan("") : unit != 0.0 ? n * unit : ldexp(n, oexp);
         if (kRoundBf16) val = (double)round_bf16((float)val);
         if (kFinal) {
             // (each thread's first row has its scale and bias at hand)
@@ -317,19 +340,19 @@ __device__ __forceinline__ void sum_form(const StageParams &p, uint32_t rows_per
     asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
 #pragma unroll 1
     for (uint32_t r = rank + n_rank * tid; r < rows; r += n_rank * kSumThreads) {
-        double val = 0.0;
+        long long sum = 0;
         for (uint32_t c = 0; c < n_rank; ++c) {
             // (row_sum lies where the slice's width puts it: the last CTA's may be narrower than the others')
             const uint32_t lo = min(c * slice_bits, n_bits), hi = min(lo + slice_bits, n_bits);
             const uint32_t at = (uint32_t)__cvta_generic_to_shared(smem_dyn) +
                                 sum_layout(max(1u, hi - lo), rows_per_block, sizeof(Entry)).row_sum + 8 * r;
             uint32_t there;
-            double one;
+            long long one;
             asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(there) : "r"(at), "r"(c));
-            asm volatile("ld.shared::cluster.f64 %0, [%1];" : "=d"(one) : "r"(there) : "memory");
-            val += one;
+            asm volatile("ld.shared::cluster.s64 %0, [%1];" : "=l"(one) : "r"(there) : "memory");
+            sum += one;
         }
-        finish(r, val);
+        finish(r, sum);
     }
     // (nobody leaves while a peer may still read its sums)
     asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");

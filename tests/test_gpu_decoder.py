@@ -502,6 +502,36 @@ def test_whole_step_kernel_reproduces_the_step_of_separate_launches(gpu_ctx, ser
     gpu_ctx.set_stream(None)
 
 
+@pytest.mark.parametrize("serving,batch", [("bfloat16", 1), ("float32", 2)])
+def test_whole_step_kernel_on_a_wide_feed_forward(gpu_ctx, serving, batch):
+    """A down projection of more entries than one block of the few-instance form takes: still the bits of the separate
+    launches, and (float32) of one token at a time."""
+    kw = dict(n_layers=2, d_ff=8704, serving=serving, max_batch=batch)
+    weights = random_model(step_cfg(**kw), STEP_RANKS, seed=78)
+    plain, fused = Decoder(gpu_ctx, step_cfg(**kw), weights), Decoder(gpu_ctx, step_cfg(fused_step_max_batch=batch, **kw), weights)
+    assert fused.step_kernel is not None and plain.step_kernel is None
+    first = [9, 41][:batch]
+    for dec in (plain, fused):
+        dec.start(first, [0] * batch)
+    for step in range(6):
+        for dec in (plain, fused):
+            dec.step()
+        gpu_ctx.synchronize()
+        assert np.array_equal(fused.logits.cpu().numpy(), plain.logits.cpu().numpy()), step
+        for dec in (plain, fused):
+            dec.advance()
+    if batch > 1:
+        alone = Decoder(gpu_ctx, step_cfg(**dict(kw, max_batch=1)), weights)
+        want = plain.token_ids.cpu().numpy()
+        for b in range(batch):
+            alone.start(first[b:b + 1], [0])
+            for _ in range(6):
+                alone.step()
+                alone.advance()
+            gpu_ctx.synchronize()
+            assert alone.token_ids.cpu().numpy()[0] == want[b]
+
+
 def torch_equal(a, b):
     import torch
     return bool(torch.equal(a, b))

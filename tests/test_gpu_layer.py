@@ -554,43 +554,117 @@ def test_tokens_of_one_layer_match_single_tokens_and_a_group(gpu_ctx, shape, n_t
 
 @pytest.mark.parametrize("serving", ["float32", "bfloat16"])
 @pytest.mark.parametrize("shape", [(1, 1, 1), (33, 511, 129), (150, 512, 16), (77, 4097, 513), (40, 8192, 300), (300, 8193, 90),
-                                   (37, 20000, 33), (4100, 300, 1030)])
+                                   (37, 20000, 33), (4100, 300, 1030), (70, 14336, 200), (60, 300, 9001), (5, 65535, 5),
+                                   (5, 65536, 5)])
 def test_sums_give_the_bits_of_the_digit_forms(gpu_ctx, shape, serving):
     """Few instances by sums (the default) against the digit tables (selector 3): entries of ordinary range, over sixty
-    powers of two, subnormal, near the end of float32, all equal, zero.  One whole number either way, hence the
-    same bits; vectors of more than 8192 entries are cut into slices with a grid each, where a float32 result may
-    round the other way."""
+    powers of two, subnormal, near the end of float32, all equal, zero, large in one place, a NaN in one.  One whole
+    number either way, hence the same bits, also where a vector of more than 8192 entries is cut into slices."""
     import torch
     dout, din, r = shape
     L = make_layer(dout, din, r, seed=dout + din + r + 1, with_bias=(dout % 2 == 1))
+    if din > 1:     # (the first two columns alike)
+        L["vb_t_rows"][:, 0] = (L["vb_t_rows"][:, 0] & 0xfd) | ((L["vb_t_rows"][:, 0] & 1) << 1)
+        L["s2"][1] = L["s2"][0]
     layer = PackedLayer(gpu_ctx, L["ub_rows"], L["vb_t_rows"], dout, din, r, L["s1"], L["s2"], L["bias"], serving=serving)
     rng = np.random.default_rng(sum(shape))
-    x = rng.standard_normal((6, din))
+    x = rng.standard_normal((9, din))
     x[1] *= 2.0 ** rng.integers(-60, 1, din)
     x[2] *= 1e-39
     x[3] *= 1e35
     x[4] = 0.37
     x[5] = 0.0
+    x[6, din // 3] = 1e12
+    x[7, -1] = np.nan
+    # two entries that cancel: what is left of the others shows the grid that they were put on, that of the largest entry of
+    # the whole vector, wherever a slice ends
+    x[8, 0], x[8, min(1, din - 1)] = 2.0 ** 40, -2.0 ** 40
     xs = torch.from_numpy(x.astype(np.float32)).cuda()
     out = {}
     for which in (1, 3):
         prev = gpu_ctx.set_gemv_kernel(which)
         try:
-            for n in (1, 6):
-                y = torch.full((6, dout), float("nan"), device="cuda")
+            for n in (1, 9):
+                y = torch.full((9, dout), 7.0, device="cuda")
                 torch.cuda.synchronize()
-                for first in range(0, 6, n):
+                for first in range(0, 9, n):
                     layer.apply_device(xs[first].data_ptr(), n, y[first].data_ptr())
                 gpu_ctx.synchronize()
                 out[which, n] = y.cpu().numpy()
         finally:
             gpu_ctx.set_gemv_kernel(prev)
     layer.close()
-    assert np.array_equal(out[1, 1], out[1, 6], equal_nan=True)
-    if din <= 8192:
-        assert np.array_equal(out[1, 1], out[3, 1], equal_nan=True)
-    else:
-        # (the slices' grids are finer than the whole vector's by up to 2^-47 of its largest entry: a rounding to float32
-        # or bfloat16 of t, u or y may turn, by a unit in its last place of the terms' scale)
-        scale = np.abs(out[3, 1]).max(axis=1, keepdims=True)
-        assert (np.abs(out[1, 1] - out[3, 1]) <= (2 ** -8 if serving == "bfloat16" else 2 ** -22) * scale).all()
+    for key in ((1, 9), (3, 1), (3, 9)):
+        assert np.array_equal(out[1, 1], out[key], equal_nan=True), key
+
+
+@pytest.mark.parametrize("serving", ["float32", "bfloat16"])
+@pytest.mark.parametrize("gated", [False, True])
+def test_sums_of_a_plan_of_mixed_shapes(gpu_ctx, gated, serving):
+    """Instances with one slice and with two, ragged and empty ones, in one plan: the bits of the digit forms and (of a plain
+    plan) of each layer alone."""
+    import torch
+    from quantibbler_b200.gpu import LayerPlan
+    shapes = [(300, 300, 40), (70, 8192, 33), (130, 8193, 200), (64, 14336, 90), (1, 1, 1)]
+    rng = np.random.default_rng(41)
+    specs = [make_layer(*shape, seed=80 + i, with_bias=(i == 1)) for i, shape in enumerate(shapes)]
+    layers = [PackedLayer(gpu_ctx, s["ub_rows"], s["vb_t_rows"], *shape, s["s1"], s["s2"], s["bias"], serving=serving)
+              for s, shape in zip(specs, shapes)]
+    x = [rng.standard_normal((2, din)).astype(np.float32) * 3 for _, din, _ in shapes]
+    up = [rng.standard_normal((2, din)).astype(np.float32) for _, din, _ in shapes]
+    tx, tu = ([torch.from_numpy(a).cuda() for a in v] for v in (x, up))
+    out = [torch.full((2, dout), 7.0, device="cuda") for dout, _, _ in shapes]
+    torch.cuda.synchronize()
+    at = lambda i, b: (tx[i][b].data_ptr(), tu[i][b].data_ptr()) if gated else (tx[i][b].data_ptr(),)  # noqa: E731
+    plan = LayerPlan(gpu_ctx, [(layers[i], *at(i, b), out[i][b].data_ptr()) for b in range(2) for i in range(len(shapes))],
+                     gated=gated)
+    got = {}
+    for which in (1, 3):
+        prev = gpu_ctx.set_gemv_kernel(which)
+        try:
+            plan.apply()
+            gpu_ctx.synchronize()
+            got[which] = [y.cpu().numpy() for y in out]
+        finally:
+            gpu_ctx.set_gemv_kernel(prev)
+    for i in range(len(shapes)):
+        assert np.array_equal(got[1][i], got[3][i]), shapes[i]
+        if not gated:
+            for b in range(2):
+                assert np.array_equal(got[1][i][b], layers[i].apply(x[i][b])), (shapes[i], b)
+    plan.close()
+
+
+@pytest.mark.parametrize("serving", ["float32", "bfloat16"])
+@pytest.mark.parametrize("din", [300, 4096])
+def test_sums_of_a_normed_plan(gpu_ctx, din, serving):
+    """The norm inside the first stage, with a residual and the updated stream: the bits of the digit form."""
+    import torch
+    from quantibbler_b200.gpu import LayerPlan
+    shapes = [(500, 130), (90, 33), (90, 33)]
+    rng = np.random.default_rng(din)
+    specs = [make_layer(dout, din, r, seed=90 + i) for i, (dout, r) in enumerate(shapes)]
+    layers = [PackedLayer(gpu_ctx, s["ub_rows"], s["vb_t_rows"], dout, din, r, s["s1"], s["s2"], None, serving=serving)
+              for s, (dout, r) in zip(specs, shapes)]
+    x, res = (torch.from_numpy(rng.standard_normal(din).astype(np.float32)).cuda() for _ in range(2))
+    w = torch.from_numpy((rng.standard_normal(din) * 0.1 + 1).astype(np.float32)).cuda()
+    x_out, out = torch.zeros(din, device="cuda"), [torch.zeros(dout, device="cuda") for dout, _ in shapes]
+    torch.cuda.synchronize()
+    plan = LayerPlan(gpu_ctx, [(layer, x.data_ptr(), y.data_ptr()) for layer, y in zip(layers, out)])
+    plan.set_norm([res.data_ptr()] * 3, w.data_ptr(), 1e-5, [x_out.data_ptr(), None, None])
+    got = {}
+    for which in (1, 3):
+        prev = gpu_ctx.set_gemv_kernel(which)
+        try:
+            for t in (x_out, *out):
+                t.fill_(7.0)
+            torch.cuda.synchronize()
+            plan.apply()
+            gpu_ctx.synchronize()
+            got[which] = [t.cpu().numpy() for t in (x_out, *out)]
+        finally:
+            gpu_ctx.set_gemv_kernel(prev)
+    for a, b in zip(got[1], got[3]):
+        assert np.array_equal(a, b)
+    assert np.array_equal(got[1][0], (x + res).cpu().numpy())
+    plan.close()
