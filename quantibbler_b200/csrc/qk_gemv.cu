@@ -1803,23 +1803,33 @@ struct SumPlan {
     size_t blocks, smem;
 };
 constexpr size_t kSumSmem = 116 * 1024;  // at least: more than half of an SM's, so that it holds one block
-// Most weights of a launch (rows x entries over its instances).  The sums' time grows with them, by 0.24 us a million
-// (bfloat16 serving 0.2), from 2.6 us on; the digit form takes 5 to 10 us for its tables and 0.07 to 0.16 us a million after
-// that.  Measured, us a call, digits -> sums, float32 serving: 4096 x 4096 of rank 1024 on 1, 2, 3, 5 tokens 13.4 -> 8.3,
-// 14.1 -> 9.5, 14.3 -> 11.0, 17.0 -> 13.7 (21e6 weights a stage), on 8 tokens (34e6) 17.6 -> 27; 8192 x 3000 of rank 2560 on one token
-// (21e6) 16.0 -> 12.6; 14336 x 14336 of rank 2560 (37e6) 22.5 -> 22.9, bfloat16 serving 23.5 -> 20.7.  Where many
-// instances share the machine, the second stage's short tables cost little: 2048 outputs of rank 800 on 12 tokens (20e6)
-// take 6 us longer by sums, 1024 of rank 300 on 32 (10e6) 3 us less.
-double sum_most_weights(size_t n_inst, bool final, bool bf16) {
-    if (final && n_inst > 8) return 14e6;
-    return bf16 && n_inst <= 2 ? 50e6 : 30e6;
+// Most weights of a launch (rows x entries over its instances).  The sums' time grows with them, by 0.2 us a million (float32
+// serving 0.25); the digit forms spend 5 to 10 us on their tables and 0.07 to 0.16 us a million.  Measured, us a call, the
+// stage by digits -> by sums, the other stage as this rule has it:
+//   first stage of up to 8192 entries, bfloat16: 2 x 2100 x 4096 (17e6) 22.7 -> 19.4, 4 x 2048 x 4096 (34e6) 17.3 -> 15.3, 6 x 2048 x
+//     4096 (50e6) 18.3 -> 18.3, 12 x 1024 x 4096 (50e6) 17.2 -> 19.6; float32: 16 x 800 x 2048 (26e6) 15.9 -> 15.3, 5 x 2048 x 4096
+//     (42e6) 17.6 -> 18.3
+//   of more (slices) in a plan, bfloat16: 1200 x 14336 (17e6) 13.8 -> 13.9, 800 x 14336 (11e6) 13.3 -> 12.7, 1733 x 14336 (25e6)
+//     14.3 -> 15.2, 2 x 1600 x 9000 (29e6) 13.8 -> 17.0; float32: 800 x 14336 13.6 -> 12.6, 1600 x 9000 (14e6) 13.2 -> 13.8
+//   ... on the tokens of one layer, whose digit form has a table launch and copied records: 1733 x 14336 19.5 -> 15.4 (float32
+//     19.6 -> 16.1), on two tokens (50e6) 19.8 -> 20.0
+//   second stage, bfloat16: 14336 x 2560 (37e6) 15.4 -> 13.7, x 3400 (49e6) 15.8 -> 16.8, 2 x 14336 x 1724 (49e6) 17.8 -> 16.2,
+//     12 x 2048 x 800 (20e6) 14.1 -> 12.3, 16 x 2048 x 800 (26e6) 14.9 -> 14.2, 5 x 4096 x 2048 (42e6) 17.2 -> 17.7; float32
+//     (entries of eight bytes): 4 x 4096 x 1733 (28e6) inside four layers of a step 672 -> 649, 4 x 4096 x 2048 (34e6) 16.6 -> 17.8,
+//     8 x 2048 x 800 (13e6) 12.7 -> 11.3, 8 x 4096 x 600 (20e6) 14.5 -> 15.5
+double sum_most_weights(size_t n_inst, size_t ranks, bool final, bool bf16, bool run) {
+    if (ranks > 1 && !run) return bf16 ? 15e6 : 12e6;
+    if (!final) return bf16 && n_inst <= 2 ? 50e6 : 30e6;
+    if (bf16) return n_inst == 1 ? 40e6 : n_inst == 2 ? 50e6 : 30e6;
+    return n_inst <= 5 ? 30e6 : 16e6;
 }
+// run: the tokens of one layer, whose records come with the launch.
 SumPlan sum_plan(const qk_ctx *c, const StageShape &s, size_t n_inst, size_t total_rows, bool final, bool bf16,
-                 bool normed = false) {
+                 bool run, bool normed = false) {
     SumPlan pl{};
     pl.ranks = (uint32_t)qk::ceil_div(s.n_bits, (size_t)kSumSlice);
     if (c->gemv_kernel != 1 || pl.ranks > kSumRanks || s.n_bits > kSumMostEntries || (normed && s.n_bits > 8 * kSumThreads) || s.n_groups > 65535 ||
-        (double)total_rows * (double)s.n_bits > sum_most_weights(n_inst, final, bf16))
+        (double)total_rows * (double)s.n_bits > sum_most_weights(n_inst, pl.ranks, final, bf16, run))
         return pl;
     pl.slice = pl.ranks == 1 ? (uint32_t)s.n_bits
                              : (uint32_t)(qk::ceil_div(qk::ceil_div(s.n_bits, (size_t)pl.ranks), (size_t)128) * 128);
@@ -1874,7 +1884,7 @@ constexpr size_t kSpreadTableSteps = 16;  // k-steps (of 512 inputs) from which 
 bool run_fits(const qk_ctx *c, const StageShape &s, size_t n_inst, bool final, bool bf16) {
     const StagePlan pl = plan_stage(c, s, n_inst);
     return (pl.smem_digits && s.n_steps < kSpreadTableSteps) ||
-           (n_inst * pl.blocks < (size_t)c->sm_count && sum_plan(c, s, n_inst, n_inst * s.n_rows, final, bf16).fits);
+           (n_inst * pl.blocks < (size_t)c->sm_count && sum_plan(c, s, n_inst, n_inst * s.n_rows, final, bf16, true).fits);
 }
 
 // many: the instances' records on the device; or null, and the instances are the tokens of `run` (run_fits).
@@ -1891,7 +1901,7 @@ qk_status launch_bitslice(qk_ctx *c, const StageParams *many, size_t n_inst, con
     const size_t sk_smem = sk_bytes(sk_warps);
     const bool few = c->gemv_kernel != 3 && n_inst * pl.blocks < (size_t)c->sm_count && s.n_groups <= 65535;
     if (few && !need_few) {
-        const SumPlan sums = sum_plan(c, s, n_inst, n_inst * s.n_rows, kFinal, bf16);
+        const SumPlan sums = sum_plan(c, s, n_inst, n_inst * s.n_rows, kFinal, bf16, !many);
         if (sums.fits) return launch_sums<kFinal>(c, many, n_inst, sums, bf16, run);
     }
     // A long input vector (the down projection's 14336 entries): every block of the few-instance
@@ -2081,7 +2091,7 @@ template <bool kFinal>
 qk_status launch_mixed_stage(qk_ctx *c, const StageParams *many, size_t n_inst, const StageShape &s,
                              bool bf16, size_t total_rows, bool pushed = false) {
     if (!pushed) {
-        const SumPlan sums = sum_plan(c, s, n_inst, total_rows, kFinal, bf16);
+        const SumPlan sums = sum_plan(c, s, n_inst, total_rows, kFinal, bf16, false);
         if (sums.fits) return launch_sums<kFinal>(c, many, n_inst, sums, bf16);
     }
     size_t warps, smem;
@@ -2130,7 +2140,7 @@ bool normed_plan_fits(const qk_ctx *c, const StageShape &s, size_t n_inst, size_
 qk_status launch_normed_stage1(qk_ctx *c, const StageParams *many, size_t n_inst, const StageShape &s, bool bf16,
                                size_t total_rows, bool gathered) {
     if (!gathered) {
-        const SumPlan sums = sum_plan(c, s, n_inst, total_rows, false, bf16, true);
+        const SumPlan sums = sum_plan(c, s, n_inst, total_rows, false, bf16, false, true);
         if (sums.fits) return launch_sums<false>(c, many, n_inst, sums, bf16);
     }
     size_t smem;
