@@ -27,6 +27,7 @@
 //     maximum, once for P and the PV product.
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <string>
@@ -2016,26 +2017,9 @@ qk_status launch_sage_tc_block(qk_ctx *c, const SageArgs &a, const AttnDims &dm,
 
 namespace qk {
 
-// Device-buffer form of the Sage face: quantisers, then the main kernel.  `scratch` holds the
-// codes and scales (sage_scratch_bytes of it).
-size_t sage_scratch_bytes(const qk_attention_shape *s, size_t block_size) {
-    const AttnDims dm = dims_of(s);
-    const size_t S = dm.Skv;
-    if (block_size > S) block_size = S;
-    const size_t n_blocks = qk::ceil_div(S, block_size);
-    const size_t widest = dm.d > dm.dv ? dm.d : dm.dv;
-    const size_t wpl = widest <= 16 ? 1 : widest <= 64 ? 4 : widest <= 128 ? 8 : 16;
-    const size_t dpad = wpl * 16, bpad = qk::ceil_div(block_size, kTK) * kTK;
-    const size_t planes = (size_t)dm.B * dm.KV, qrows = (size_t)dm.B * dm.H * dm.Sq;
-    auto up = [](size_t n) { return (n + 255) / 256 * 256; };
-    return up(qrows * dpad) + up(qrows * 4) + up(planes * S * dpad) + up(planes * S * 4) +
-           up(planes * n_blocks * dm.d * 4) + up(planes * n_blocks * dm.dv * bpad) +
-           up(planes * n_blocks * dm.dv * 4) + up(planes * n_blocks * 8 * dpad) +
-           up(planes * n_blocks * 4) + up(planes * ((n_blocks + 1) / 2) * kURecStride) + 1024;
-}
-
 // Where each piece of the Sage scratch lies, and the padded sizes the kernels use.
 struct SageLayout {
+    size_t bytes;  // of the whole scratch
     size_t block, n_blocks, wpl, dpad, bpad, planes, qrows;
     size_t o_qc, o_qs, o_kc, o_ks, o_km, o_vc, o_vs, o_md, o_ms, o_rec;
     bool tc;    // a tensor-core kernel runs: the mean digit rows are produced
@@ -2056,24 +2040,28 @@ SageLayout sage_layout(const qk_ctx *c, const AttnDims &dm, size_t block_size) {
     auto up = [](size_t n) { return (n + 255) / 256 * 256; };
     size_t off = 0;
     auto take = [&](size_t bytes) { size_t o2 = off; off += up(bytes); return o2; };
+    L.tc = c->sage_kernel != 0 && sage_tc_eligible(dm, block_size);
+    const bool recorded = dm.d == kUD && dm.dv == kUD && block_size == kUBlk;
+    L.umma = L.tc && c->sage_kernel == 2 && recorded;
     L.o_qc = take(L.qrows * L.dpad), L.o_qs = take(L.qrows * 4);
-    L.o_kc = take(L.planes * S * L.dpad), L.o_ks = take(L.planes * S * 4);
     L.o_km = take(L.planes * L.n_blocks * dm.d * 4);
+    // The records of the one form lie where the codes of the others do: the size is that of the shape, whichever runs.
+    L.o_rec = off;
+    L.o_kc = take(L.planes * S * L.dpad), L.o_ks = take(L.planes * S * 4);
     L.o_vc = take(L.planes * L.n_blocks * dm.dv * L.bpad), L.o_vs = take(L.planes * L.n_blocks * dm.dv * 4);
     L.o_md = take(L.planes * L.n_blocks * 8 * L.dpad), L.o_ms = take(L.planes * L.n_blocks * 4);
-    L.o_rec = take(L.planes * ((L.n_blocks + 1) / 2) * kURecStride);  // (+ up to 1023 bytes to align it)
-    L.tc = c->sage_kernel != 0 && sage_tc_eligible(dm, block_size);
-    L.umma = L.tc && c->sage_kernel == 2 && dm.d == kUD && dm.dv == kUD && block_size == kUBlk;
+    if (recorded) off = std::max(off, L.o_rec + up(L.planes * ((L.n_blocks + 1) / 2) * kURecStride + 1024));  // (1024: to align them)
+    L.bytes = off;
     return L;
 }
 
-// The three quantisers (psi_Q, gamma + psi_K, psi_V) into `scratch`.
 uint8_t *sage_records(uint8_t *base, const SageLayout &L) {
     // bulk copies want 16-byte alignment; 1 KB keeps the records on the tiles' own boundary
     uint8_t *p = base + L.o_rec;
     return p + ((1024 - (reinterpret_cast<uintptr_t>(p) & 1023)) & 1023);
 }
 
+// The three quantisers (psi_Q, gamma + psi_K, psi_V) into `base`.
 qk_status sage_quantize_dev(qk_ctx *c, const float *dq, const float *dk, const float *dv,
                             uint8_t *base, const AttnDims &dm, const SageLayout &L) {
     const size_t S = dm.Skv;
@@ -2106,12 +2094,11 @@ qk_status sage_quantize_dev(qk_ctx *c, const float *dq, const float *dk, const f
     return QK_OK;
 }
 
+// Device-buffer form of the Sage face: quantisers, then the main kernel.  `base` holds the codes and scales (L.bytes of it).
 qk_status attention_sage_dev(qk_ctx *c, const float *dq, const float *dk, const float *dv,
-                             float *out, uint8_t *scratch, const qk_attention_shape *shape,
-                             int causal, size_t block_size) {
+                             float *out, uint8_t *base, const qk_attention_shape *shape,
+                             int causal, const SageLayout &L) {
     const AttnDims dm = dims_of(shape);
-    const SageLayout L = sage_layout(c, dm, block_size);
-    uint8_t *base = scratch;
     qk_status st = sage_quantize_dev(c, dq, dk, dv, base, dm, L);
     if (st != QK_OK) return st;
     SageArgs a{(const int8_t *)(base + L.o_qc), (const float *)(base + L.o_qs),
@@ -2252,7 +2239,8 @@ qk_status qk_gpu_attention_sage(qk_ctx *ctx, const qk_attention_shape *shape, co
     auto up = [](size_t n) { return (n + 255) / 256 * 256; };
     const size_t qb = q_len * 4, kb = k_len * 4, vb = v_len * 4, ob = out_len * 4;
     const size_t o_q = 0, o_k = up(qb), o_v = o_k + up(kb), o_scratch = o_v + up(vb);
-    if ((st = c->d_in.reserve(o_scratch + qk::sage_scratch_bytes(shape, block_size))) != QK_OK) return st;
+    const qk::SageLayout L = qk::sage_layout(c, dims_of(shape), block_size);
+    if ((st = c->d_in.reserve(o_scratch + L.bytes)) != QK_OK) return st;
     if ((st = c->d_out.reserve(ob)) != QK_OK) return st;
     uint8_t *base = (uint8_t *)c->d_in.ptr;
     float *dq = (float *)(base + o_q), *dk = (float *)(base + o_k), *dv = (float *)(base + o_v);
@@ -2260,7 +2248,7 @@ qk_status qk_gpu_attention_sage(qk_ctx *ctx, const qk_attention_shape *shape, co
     QK_CUDA(cudaMemcpyAsync(dk, key, kb, cudaMemcpyHostToDevice, c->stream));
     QK_CUDA(cudaMemcpyAsync(dv, value, vb, cudaMemcpyHostToDevice, c->stream));
     if ((st = qk::attention_sage_dev(c, dq, dk, dv, (float *)c->d_out.ptr, base + o_scratch, shape,
-                                     causal != 0, block_size)) != QK_OK)
+                                     causal != 0, L)) != QK_OK)
         return st;
     QK_CUDA(cudaMemcpyAsync(out, c->d_out.ptr, ob, cudaMemcpyDeviceToHost, c->stream));
     QK_CUDA(cudaStreamSynchronize(c->stream));
@@ -2298,9 +2286,9 @@ qk_status qk_gpu_attention_sage_dev(qk_ctx *ctx, const qk_attention_shape *shape
     if ((st = qk::resolve_ctx(ctx, &c)) != QK_OK) return st;
     std::lock_guard<std::mutex> lock(c->mu);
     QK_CUDA(cudaSetDevice(c->device));
-    if ((st = c->d_in.reserve(qk::sage_scratch_bytes(shape, block_size))) != QK_OK) return st;
-    return qk::attention_sage_dev(c, q_dev, k_dev, v_dev, out_dev, (uint8_t *)c->d_in.ptr, shape,
-                                  causal != 0, block_size);
+    const qk::SageLayout L = qk::sage_layout(c, dims_of(shape), block_size);
+    if ((st = c->d_in.reserve(L.bytes)) != QK_OK) return st;
+    return qk::attention_sage_dev(c, q_dev, k_dev, v_dev, out_dev, (uint8_t *)c->d_in.ptr, shape, causal != 0, L);
 }
 
 qk_status qk_gpu_attention_sage_block_dev(qk_ctx *ctx, const qk_attention_shape *shape, const float *q_dev,
@@ -2339,15 +2327,15 @@ qk_status qk_gpu_sage_quantize(qk_ctx *ctx, const qk_attention_shape *shape, con
     auto up = [](size_t n) { return (n + 255) / 256 * 256; };
     const size_t qb = q_len * 4, kb = k_len * 4, vb = v_len * 4;
     const size_t o_k = up(qb), o_v = o_k + up(kb), o_scratch = o_v + up(vb);
-    const size_t scratch_bytes = qk::sage_scratch_bytes(shape, block_size);
+    const AttnDims dm = dims_of(shape);
+    const qk::SageLayout L = qk::sage_layout(c, dm, block_size);
+    const size_t scratch_bytes = L.bytes;
     if ((st = c->d_in.reserve(o_scratch + scratch_bytes)) != QK_OK) return st;
     uint8_t *base = (uint8_t *)c->d_in.ptr;
     float *dq = (float *)base, *dk = (float *)(base + o_k), *dv = (float *)(base + o_v);
     QK_CUDA(cudaMemcpyAsync(dq, query, qb, cudaMemcpyHostToDevice, c->stream));
     QK_CUDA(cudaMemcpyAsync(dk, key, kb, cudaMemcpyHostToDevice, c->stream));
     QK_CUDA(cudaMemcpyAsync(dv, value, vb, cudaMemcpyHostToDevice, c->stream));
-    const AttnDims dm = dims_of(shape);
-    const qk::SageLayout L = qk::sage_layout(c, dm, block_size);
     if ((st = qk::sage_quantize_dev(c, dq, dk, dv, base + o_scratch, dm, L)) != QK_OK) return st;
     std::vector<uint8_t> host(scratch_bytes);
     QK_CUDA(cudaMemcpyAsync(host.data(), base + o_scratch, scratch_bytes, cudaMemcpyDeviceToHost,

@@ -402,6 +402,39 @@ def test_sage_inputs_need_not_lie_on_sixteen_bytes(gpu_ctx, which):
     assert bool((outs[0] != 0).any()) and torch.equal(*outs)
 
 
+@pytest.mark.parametrize("dim,block", [(64, 64), (128, 32), (128, 64)])
+def test_sage_scratch_is_what_the_shape_needs(dim, block):
+    """A fresh context's memory after a first call: codes and scales, and records only where a kernel reads them (heads of
+    128, key blocks of 64: 416 bytes a key), whichever form runs first.  (Two more megabytes twice: an allocation is rounded up
+    to them, and the context's error word takes one.)"""
+    import torch
+    from quantibbler_b200.gpu import GpuContext
+    b, h, kvh, s = 1, 2, 2, 64 * 1024
+    q, k, v = (torch.zeros(b, n, s, dim, device="cuda") for n in (h, kvh, kvh))
+    out, blocks = torch.zeros_like(q), s // block
+    codes = kvh * s * dim + kvh * s * 4 + kvh * blocks * dim * max(block, 64) + kvh * blocks * dim * 4 + kvh * blocks * (8 * dim + 4)
+    common = h * s * dim + h * s * 4 + kvh * blocks * dim * 4
+    most = common + max(codes, kvh * s * 416 if (dim, block) == (128, 64) else 0) + (4 << 20)
+    shape = shape_of(*(t.cpu().numpy() for t in (q, k, v)))
+    ctx = GpuContext.init()
+    try:
+        small = torch.zeros(1, 1, 64, dim, device="cuda")
+        one = shape_of(*(small.cpu().numpy() for _ in range(3)))
+        for which in (2, 1):     # (the kernels are loaded)
+            ctx.set_sage_kernel(which)
+            ctx.attention_dev(one, small.data_ptr(), small.data_ptr(), small.data_ptr(), True, out.data_ptr(), block)
+            ctx.synchronize()
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        for which in (2, 1):
+            ctx.set_sage_kernel(which)
+            ctx.attention_dev(shape, q.data_ptr(), k.data_ptr(), v.data_ptr(), True, out.data_ptr(), block)
+            ctx.synchronize()
+            assert free - torch.cuda.mem_get_info()[0] <= most, which
+    finally:
+        ctx.close()
+
+
 def test_attention_on_device_buffers(gpu_ctx):
     import torch
     rng = np.random.default_rng(11)
