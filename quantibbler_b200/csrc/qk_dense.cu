@@ -148,7 +148,7 @@ dense_vector_kernel(InputArgs in, OutputArgs out, const W *__restrict__ w, uint3
             auto at4 = [&](uint32_t p) -> float4 & { return *reinterpret_cast<float4 *>(dst + T::place(4 * p)); };
             if (row_kind == kRowNorm) build_norm_row(in, t_in + t, writer, staged, at4, red);
             else if (row_kind == kRowPlain) build_plain_row(in, t_in + t, at4);
-            else if (row_kind == kRowGated) build_gated_row(in, t_in + t, at);
+            else if (row_kind == kRowGated) build_gated_row(in, t_in + t, at4);
             else build_input(in, t_in + t, writer, at, red);
         }
         // what lies between k and the pitch meets zero weights; it must only be finite
@@ -247,7 +247,7 @@ dense_input_kernel(InputArgs in, A *__restrict__ dst, int row_kind) {
         auto at = [&](uint32_t i) -> float & { return row_smem[i]; };
         auto at4 = [&](uint32_t p) -> float4 & { return *reinterpret_cast<float4 *>(row_smem + 4 * p); };
         if (row_kind == kRowNorm) build_norm_row(in, t, true, row_smem + in.k, at4, red);
-        else if (row_kind == kRowGated) build_gated_row(in, t, at);
+        else if (row_kind == kRowGated) build_gated_row(in, t, at4);
         else build_input(in, t, true, at, red);
         for (uint32_t j = 0; j < (in.places ? in.top : 1u); ++j) {
             A *o = dst + (size_t)(in.places ? (uint32_t)in.places[t * in.top + j] : t) * in.k;
@@ -1129,9 +1129,11 @@ qk_status launch_tc(qk_ctx *c, const void *x, size_t x_stride, const qk_dense_ca
 // pending one 6.8 and 2.5; sixteen gated groups of 128 3.7 to 5.4 and 3.4.)
 int row_kind_of(const InputArgs &a) {
     auto aligned = [](const void *p) { return ((uintptr_t)p & 15) == 0; };
-    if (a.kind == QK_INPUT_GATED) return a.group <= 128 ? kRowGated : kRowAny;
     if (a.width % 4 || a.k % 4 || a.x_stride % 4 || !aligned(a.x)) return kRowAny;
     if (a.kind == QK_INPUT_PLAIN) return kRowPlain;
+    if (a.kind == QK_INPUT_GATED)
+        return a.group % 4 || a.group > 128 || a.width % a.group || a.gate_stride % 4 || !aligned(a.gate) ||
+                       !aligned(a.norm_weight) ? kRowAny : kRowGated;
     if (a.kind == QK_INPUT_CONCAT && (a.k % 8 || !aligned(a.second))) return kRowAny;
     if (a.width > 1024 * kNormPieces || !aligned(a.x_out)) return kRowAny;
     if (a.norm != QK_NORM_NONE && !aligned(a.norm_weight)) return kRowAny;

@@ -177,9 +177,11 @@ __device__ __forceinline__ void build_input(const InputArgs &a, uint32_t t, bool
     __syncthreads();
 }
 
-// The same for a normed row of up to 1024 kNormPieces aligned entries, for 256 threads: all loads of the row go
-// out together, the norms' weights have been staged by stage_norm_weights (which depends on no other kernel).
-// `at4(p)` is the shared-memory place of entries 4 p .. 4 p + 3.
+// The same for a normed row (with or without a second one behind it) of up to 1024 kNormPieces aligned entries, for
+// 256 threads: all loads of the row go out together, the norms' weights have been staged by stage_norm_weights (which
+// depends on no other kernel).  `at4(p)` is the shared-memory place of entries 4 p .. 4 p + 3.  A row's sums run over a
+// thread's pieces; where a second row follows, they run over the entries tid + 256 j as in build_input (the order that such
+// rows have always had), which change hands in the row's own place.
 constexpr int kNormPieces = 4;
 // The sum over the eight warps of such a block, in the order of block_sum; no barrier after it: the next sum
 // takes other words (red: 16 floats).
@@ -208,6 +210,23 @@ __device__ __forceinline__ void build_norm_pieces(const InputArgs &a, uint32_t t
     const float4 *xr = reinterpret_cast<const float4 *>(a.x + (size_t)t * a.x_stride);
     const float4 *nw = reinterpret_cast<const float4 *>(staged), *pw = nw + pieces;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const uint32_t own = (a.kind == QK_INPUT_CONCAT ? a.k / 2 : a.k) / 4;  // pieces of the normed part
+    if (a.kind == QK_INPUT_CONCAT) {
+        const float *second = a.second + (size_t)t * a.x_stride;
+        for (uint32_t p = threadIdx.x; p < pieces; p += 256) stage16(&at4(own + p).x, second + 4 * p);
+        asm volatile("cp.async.commit_group;" ::: "memory");
+        for (uint32_t p = own + pieces + threadIdx.x; p < a.k / 4; p += 256) at4(p) = zero;
+    }
+    const bool by_entry = a.kind == QK_INPUT_CONCAT;
+    // v to the row's place; then use(entry) for this thread's, in their order
+    auto exchange = [&](const float4 (&v)[kPieces], auto &&use) {
+#pragma unroll
+        for (int j = 0; j < kPieces; ++j)
+            if (threadIdx.x + 256 * j < pieces) at4(threadIdx.x + 256 * j) = v[j];
+        __syncthreads();
+#pragma unroll 4
+        for (uint32_t i = threadIdx.x; i < n; i += 256) use((&at4(i / 4).x)[i % 4]);
+    };
     float4 h[kPieces];
 #pragma unroll
     for (int j = 0; j < kPieces; ++j) {
@@ -232,8 +251,9 @@ __device__ __forceinline__ void build_norm_pieces(const InputArgs &a, uint32_t t
 #pragma unroll
         for (int j = 0; j < kPieces; ++j) {
             y[j] = make_float4(y[j].x * share, y[j].y * share, y[j].z * share, y[j].w * share);
-            ps += y[j].x * y[j].x + y[j].y * y[j].y + y[j].z * y[j].z + y[j].w * y[j].w;
+            if (!by_entry) ps += y[j].x * y[j].x + y[j].y * y[j].y + y[j].z * y[j].z + y[j].w * y[j].w;
         }
+        if (by_entry) exchange(y, [&](float v) { ps += v * v; });
         const float inv = 1.0f / sqrtf(row_sum(ps, red) / (float)n + a.pending_eps);
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         float4 *xo = writer && a.x_out ? reinterpret_cast<float4 *>(a.x_out + (size_t)t * a.x_stride) : nullptr;
@@ -254,18 +274,31 @@ __device__ __forceinline__ void build_norm_pieces(const InputArgs &a, uint32_t t
         for (int j = 0; j < kPieces; ++j)
             if (threadIdx.x + 256 * j < pieces) xo[threadIdx.x + 256 * j] = h[j];
     }
-    float mean = 0.f, inv = 1.f;
+    float mean = 0.f, inv = 1.f, sum = 0.f, sq = 0.f;
+    if (by_entry && a.norm != QK_NORM_NONE)
+        exchange(h, [&](float v) {
+            sum += v;
+            sq += v * v;
+        });
     if (a.norm == QK_NORM_LAYER) {
-        float s = 0.f;
+        if (!by_entry) {
 #pragma unroll
-        for (int j = 0; j < kPieces; ++j) s += h[j].x + h[j].y + h[j].z + h[j].w;
-        mean = row_sum(s, red + 8) / (float)n;
+            for (int j = 0; j < kPieces; ++j) sum += h[j].x + h[j].y + h[j].z + h[j].w;
+        }
+        mean = row_sum(sum, red + 8) / (float)n;
     }
     if (a.norm != QK_NORM_NONE) {
-        float s = 0.f;
+        float s = by_entry && a.norm == QK_NORM_RMS ? sq : 0.f;
+        if (by_entry && a.norm == QK_NORM_LAYER) {
+#pragma unroll 4
+            for (uint32_t i = threadIdx.x; i < n; i += 256) {
+                const float d = (&at4(i / 4).x)[i % 4] - mean;
+                s += d * d;
+            }
+        }
 #pragma unroll
         for (int j = 0; j < kPieces; ++j) {
-            if (threadIdx.x + 256 * j >= pieces) continue;
+            if (by_entry || threadIdx.x + 256 * j >= pieces) continue;
             const float b = h[j].x - mean, c = h[j].y - mean, d = h[j].z - mean, e = h[j].w - mean;
             s += b * b + c * c + d * d + e * e;
         }
@@ -283,84 +316,7 @@ __device__ __forceinline__ void build_norm_pieces(const InputArgs &a, uint32_t t
         }
         at4(p) = v;
     }
-    for (uint32_t p = pieces + threadIdx.x; p < a.k / 4; p += 256) at4(p) = zero;
-    __syncthreads();
-}
-// A normed row with a second one behind it, for 256 threads: the loads of 2048 entries go out together, the second
-// row's copies and the staged weights beside them.  A thread has the entries tid + 256 j and adds them up in the order of
-// build_input: the bits are the same.  (Rows in pieces take another order, which dense_norm_rows_kernel shares.)
-template <typename At4>
-__device__ __forceinline__ void build_concat_row(const InputArgs &a, uint32_t t, bool writer, const float *staged, At4 &&at4,
-                                                 float *red) {
-    constexpr int kOwn = 8;
-    const uint32_t n = a.width, half = a.k / 2;
-    const float *xr = a.x + (size_t)t * a.x_stride, *second = a.second + (size_t)t * a.x_stride, *nw = staged, *pw = staged + n;
-    auto at = [&](uint32_t i) -> float & { return (&at4(i / 4).x)[i % 4]; };
-    auto load = [&](const float *p, uint32_t i0, float (&v)[kOwn]) {
-#pragma unroll
-        for (int j = 0; j < kOwn; ++j) v[j] = p[min(i0 + 256 * j, n - 1)];
-    };
-    for (uint32_t p = threadIdx.x; p < n / 4; p += 256) stage16(&at4(half / 4 + p).x, second + 4 * p);
-    asm volatile("cp.async.commit_group;" ::: "memory");
-    for (uint32_t i = n + threadIdx.x; i < half; i += 256) at(i) = at(half + i) = 0.f;
-    float x[kOwn], inv = 0.f;
-    load(xr, threadIdx.x, x);
-    if (a.pending) {
-        const float share = a.pending_top ? a.pending_scale : 1.f;
-        float ps = 0.f;
-#pragma unroll 1
-        for (uint32_t i0 = threadIdx.x; i0 < n; i0 += 256 * kOwn) {
-            float y[kOwn];
-            load(a.pending_top ? pending_row(a, t, 0) : a.pending + (size_t)t * a.pending_stride, i0, y);
-#pragma unroll 1
-            for (uint32_t c = 1; c < a.pending_top; ++c) {
-                float more[kOwn];
-                load(pending_row(a, t, c), i0, more);
-#pragma unroll
-                for (int j = 0; j < kOwn; ++j) y[j] += more[j];
-            }
-#pragma unroll
-            for (int j = 0; j < kOwn; ++j) {
-                const float v = y[j] * share;
-                if (i0 + 256 * j < n) {
-                    at(i0 + 256 * j) = v;
-                    ps += v * v;
-                }
-            }
-        }
-        // (the staged weights are other threads' copies: they are waited for in front of the sum's barrier)
-        asm volatile("cp.async.wait_group 0;" ::: "memory");
-        inv = 1.0f / sqrtf(row_sum(ps, red) / (float)n + a.pending_eps);
-    }
-    float *xo = writer && a.x_out ? a.x_out + (size_t)t * a.x_stride : nullptr;
-    float sum = 0.f, sq = 0.f, mean = 0.f;
-#pragma unroll 1
-    for (uint32_t i0 = threadIdx.x; i0 < n; i0 += 256 * kOwn) {
-        if (i0 != threadIdx.x) load(xr, i0, x);
-#pragma unroll
-        for (int j = 0; j < kOwn; ++j) {
-            const uint32_t i = i0 + 256 * j;
-            if (i >= n) continue;
-            const float h = a.pending ? x[j] + at(i) * inv * pw[i] : x[j];
-            at(i) = h;
-            if (xo) xo[i] = h;
-            sum += h;
-            sq += h * h;
-        }
-    }
-    asm volatile("cp.async.wait_group 0;" ::: "memory");
-    if (a.norm == QK_NORM_LAYER) {
-        mean = row_sum(sum, red + 8) / (float)n;
-        sq = 0.f;
-        for (uint32_t i = threadIdx.x; i < n; i += 256) {
-            const float d = at(i) - mean;
-            sq += d * d;
-        }
-    }
-    if (a.norm != QK_NORM_NONE) {
-        inv = 1.0f / sqrtf(row_sum(sq, a.norm == QK_NORM_LAYER ? red : red + 8) / (float)n + a.norm_eps);
-        for (uint32_t i = threadIdx.x; i < n; i += 256) at(i) = (at(i) - mean) * inv * nw[i];
-    }
+    for (uint32_t p = pieces + threadIdx.x; p < own; p += 256) at4(p) = zero;
     __syncthreads();
 }
 // (Half the pieces where they do: at the four blocks per SM of the vector form the others cost time even where
@@ -369,51 +325,56 @@ __device__ __forceinline__ void build_concat_row(const InputArgs &a, uint32_t t,
 template <typename At4>
 __device__ __forceinline__ void build_norm_row(const InputArgs &a, uint32_t t, bool writer, const float *staged, At4 &&at4,
                                                float *red) {
-    if (a.kind == QK_INPUT_CONCAT) build_concat_row(a, t, writer, staged, at4, red);
-    else if (a.width <= 512 * kNormPieces) build_norm_pieces<kNormPieces / 2>(a, t, writer, staged, at4, red);
+    if (a.width <= 512 * kNormPieces) build_norm_pieces<kNormPieces / 2>(a, t, writer, staged, at4, red);
     else build_norm_pieces<kNormPieces>(a, t, writer, staged, at4, red);
 }
-// A gated row of groups of up to 128 entries, for 256 threads: a warp takes two groups at a time, all of whose
-// loads go out together.  A lane has the entries lane + 32 q and adds up their squares in the order of
-// build_input: the bits are the same.
-template <typename At>
-__device__ __forceinline__ void build_gated_row(const InputArgs &a, uint32_t t, At &&at) {
-    constexpr uint32_t kBatch = 2, kWarps = 8, kOwn = 4;
-    const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32, g = a.group, groups = a.width / g;
-    const float *xr = a.x + (size_t)t * a.x_stride, *gr = a.gate + (size_t)t * a.gate_stride;
-    float w[kOwn];
-#pragma unroll
-    for (uint32_t q = 0; q < kOwn; ++q) w[q] = a.norm_weight[min(lane + 32 * q, g - 1)];
+// A gated row of groups of up to 128 aligned entries, for 256 threads: a warp takes two groups at a time, a lane four
+// entries of each, all of whose loads go out together.  The squares are added in the order of build_input, a lane's entries
+// lane + 32 q: they change hands in the row's own place.
+template <typename At4>
+__device__ __forceinline__ void build_gated_row(const InputArgs &a, uint32_t t, At4 &&at4) {
+    constexpr uint32_t kBatch = 2, kWarps = 8;
+    const uint32_t warp = threadIdx.x / 32, lane = threadIdx.x % 32, per = a.group / 4, groups = a.width / a.group;
+    const float4 *xr = reinterpret_cast<const float4 *>(a.x + (size_t)t * a.x_stride);
+    const float4 *gr = reinterpret_cast<const float4 *>(a.gate + (size_t)t * a.gate_stride);
+    const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
+    const uint32_t own = min(lane, per - 1);
+    const float4 w = reinterpret_cast<const float4 *>(a.norm_weight)[own];
     for (uint32_t h0 = warp; h0 < groups; h0 += kBatch * kWarps) {
-        float x[kBatch][kOwn], z[kBatch][kOwn];
+        float4 x[kBatch], g[kBatch];
+#pragma unroll
+        for (uint32_t j = 0; j < kBatch; ++j) {
+            const uint32_t p = min(h0 + j * kWarps, groups - 1) * per + own;
+            x[j] = xr[p];
+            g[j] = gr[p];
+        }
 #pragma unroll
         for (uint32_t j = 0; j < kBatch; ++j)
-#pragma unroll
-            for (uint32_t q = 0; q < kOwn; ++q) {
-                const uint32_t i = min(h0 + j * kWarps, groups - 1) * g + min(lane + 32 * q, g - 1);
-                x[j][q] = xr[i];
-                z[j][q] = gr[i];
-            }
+            if (lane < per && h0 + j * kWarps < groups) at4((h0 + j * kWarps) * per + lane) = x[j];
+        __syncwarp();
         float ss[kBatch] = {};
 #pragma unroll
         for (uint32_t j = 0; j < kBatch; ++j)
 #pragma unroll
-            for (uint32_t q = 0; q < kOwn; ++q)
-                if (lane + 32 * q < g) ss[j] += x[j][q] * x[j][q];
+            for (uint32_t q = 0; q < 4; ++q) {
+                const uint32_t i = (h0 + j * kWarps) * a.group + lane + 32 * q;
+                if (lane + 32 * q < a.group && h0 + j * kWarps < groups) ss[j] += (&at4(i / 4).x)[i % 4] * (&at4(i / 4).x)[i % 4];
+            }
+        __syncwarp();
         for (int off = 16; off > 0; off >>= 1)
 #pragma unroll
             for (uint32_t j = 0; j < kBatch; ++j) ss[j] += __shfl_xor_sync(0xffffffffu, ss[j], off);
 #pragma unroll
         for (uint32_t j = 0; j < kBatch; ++j) {
-            const float inv = 1.0f / sqrtf(ss[j] / (float)g + a.norm_eps);
-            if (h0 + j * kWarps >= groups) continue;
-#pragma unroll
-            for (uint32_t q = 0; q < kOwn; ++q)
-                if (lane + 32 * q < g)
-                    at((h0 + j * kWarps) * g + lane + 32 * q) = x[j][q] * inv * w[q] * silu_f(z[j][q]);
+            const float inv = 1.0f / sqrtf(ss[j] / (float)a.group + a.norm_eps);
+            const float4 v = x[j];
+            if (lane < per && h0 + j * kWarps < groups)
+                at4((h0 + j * kWarps) * per + lane) =
+                    make_float4(v.x * inv * w.x * silu_f(g[j].x), v.y * inv * w.y * silu_f(g[j].y),
+                                v.z * inv * w.z * silu_f(g[j].z), v.w * inv * w.w * silu_f(g[j].w));
         }
     }
-    for (uint32_t i = a.width + threadIdx.x; i < a.k; i += 256) at(i) = 0.f;
+    for (uint32_t p = a.width / 4 + threadIdx.x; p < a.k / 4; p += 256) at4(p) = zero;
     __syncthreads();
 }
 // A plain row in aligned pieces.
