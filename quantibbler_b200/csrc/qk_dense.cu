@@ -87,7 +87,12 @@ __device__ __forceinline__ void vec_fma(float (&acc)[NT], const uint4 &w, const 
 // left) find room.
 // (The blocks per SM matter more than a spilled register: they hide each other's prologues.)
 __host__ __device__ constexpr int vec_blocks(int nt, int r) { return nt == 4 && r == 4 ? 2 : r == 1 && nt <= 2 ? 4 : 3; }
-template <typename W, int NT, int R>
+// kWide: a normed row of more than 512 kNormPieces entries, kConcat: with a second one behind it; else any other.  Half the
+// pieces a thread do for shorter rows: one of 2048 took 1.9 to 3.1 us from the wait with four pieces and block_sum, 1.4 to
+// 2.6 with two and row_sum, with a pending one 3.3 and 2.4.  Instances of their own: together in one kernel they spill the
+// registers that hold the first weights, and a spill waits for its load.
+enum { kShort = 0, kWide = 1, kWideConcat = 2 };
+template <typename W, int NT, int R, int kRows>
 __global__ void __launch_bounds__(kVecThreads, vec_blocks(NT, R))
 dense_vector_kernel(InputArgs in, OutputArgs out, const W *__restrict__ w, uint32_t rows, uint32_t w_stride,
                     uint32_t n_tokens, uint32_t ksplit, ChoiceArgs ch, int row_kind) {
@@ -146,7 +151,9 @@ dense_vector_kernel(InputArgs in, OutputArgs out, const W *__restrict__ w, uint3
         if (t < n_tokens) {
             auto at = [&](uint32_t i) -> float & { return dst[T::place(i)]; };
             auto at4 = [&](uint32_t p) -> float4 & { return *reinterpret_cast<float4 *>(dst + T::place(4 * p)); };
-            if (row_kind == kRowNorm) build_norm_row(in, t_in + t, writer, staged, at4, red);
+            if constexpr (kRows != kShort)
+                build_norm_pieces<kNormPieces, kRows == kWideConcat ? 1 : 0>(in, t_in + t, writer, staged, at4, red);
+            else if (row_kind == kRowNorm) build_norm_pieces<kNormPieces / 2, -1>(in, t_in + t, writer, staged, at4, red);
             else if (row_kind == kRowPlain) build_plain_row(in, t_in + t, at4);
             else if (row_kind == kRowGated) build_gated_row(in, t_in + t, at4);
             else build_input(in, t_in + t, writer, at, red);
@@ -246,7 +253,7 @@ dense_input_kernel(InputArgs in, A *__restrict__ dst, int row_kind) {
     if (dst) {
         auto at = [&](uint32_t i) -> float & { return row_smem[i]; };
         auto at4 = [&](uint32_t p) -> float4 & { return *reinterpret_cast<float4 *>(row_smem + 4 * p); };
-        if (row_kind == kRowNorm) build_norm_row(in, t, true, row_smem + in.k, at4, red);
+        if (row_kind == kRowNorm) build_norm_pieces<kNormPieces, -1>(in, t, true, row_smem + in.k, at4, red);
         else if (row_kind == kRowGated) build_gated_row(in, t, at4);
         else build_input(in, t, true, at, red);
         for (uint32_t j = 0; j < (in.places ? in.top : 1u); ++j) {
@@ -1151,15 +1158,17 @@ qk_status launch_vector_r(qk_ctx *c, const InputArgs &in, const OutputArgs &out,
     if (kind == kRowNorm) smem += 8 * d.width;
     const size_t groups = d.output == QK_OUTPUT_GLU ? qk::ceil_div(d.rows / 2, R / 2 ? R / 2 : 1)
                                                     : qk::ceil_div(d.rows, R);
-    QK_CUDA(cudaFuncSetAttribute(dense_vector_kernel<W, NT, R>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                 (int)std::max(smem, (size_t)48 * 1024)));
+    auto kernel = kind != kRowNorm || d.width <= 512 * kNormPieces ? dense_vector_kernel<W, NT, R, kShort>
+                  : in.kind == QK_INPUT_CONCAT                     ? dense_vector_kernel<W, NT, R, kWideConcat>
+                                                                   : dense_vector_kernel<W, NT, R, kWide>;
+    QK_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)std::max(smem, (size_t)48 * 1024)));
     ChoiceArgs ch{};
     if (d.experts) ch = ChoiceArgs{d.table, d.ids, (uint32_t)d.top, (uint32_t)d.vocab, d.by_choice ? 1u : 0u};
     const size_t choices = d.experts ? input_rows(d) : 1;
     // the blocks that stay resident, shared out evenly among the choices
     const size_t per_sm = std::max<size_t>(1, std::min<size_t>(vec_blocks(NT, R), kVecSmemSm / (smem + 2048)));
     const size_t resident = std::max<size_t>(1, per_sm * (size_t)c->sm_count / choices);
-    (void)qk::launch_pdl(c->pdl, dense_vector_kernel<W, NT, R>, dim3((unsigned)std::min(groups, resident), (unsigned)choices),
+    (void)qk::launch_pdl(c->pdl, kernel, dim3((unsigned)std::min(groups, resident), (unsigned)choices),
                          dim3(kVecThreads), smem, c->stream, in, out, (const W *)d.w, (uint32_t)d.rows,
                          (uint32_t)d.w_stride, (uint32_t)n_tokens, ks, ch, kind);
     QK_CUDA(cudaGetLastError());

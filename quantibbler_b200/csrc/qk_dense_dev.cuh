@@ -203,21 +203,22 @@ __device__ __forceinline__ void stage_norm_weights(const InputArgs &a, float *st
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
 }
-template <int kPieces, typename At4>
+// kSecond: whether a second row follows (-1: as the call says).
+template <int kPieces, int kSecond, typename At4>
 __device__ __forceinline__ void build_norm_pieces(const InputArgs &a, uint32_t t, bool writer, const float *staged, At4 &&at4,
                                                   float *red) {
     const uint32_t n = a.width, pieces = n / 4;
+    const bool by_entry = kSecond < 0 ? a.kind == QK_INPUT_CONCAT : kSecond != 0;
     const float4 *xr = reinterpret_cast<const float4 *>(a.x + (size_t)t * a.x_stride);
     const float4 *nw = reinterpret_cast<const float4 *>(staged), *pw = nw + pieces;
     const float4 zero = make_float4(0.f, 0.f, 0.f, 0.f);
-    const uint32_t own = (a.kind == QK_INPUT_CONCAT ? a.k / 2 : a.k) / 4;  // pieces of the normed part
-    if (a.kind == QK_INPUT_CONCAT) {
+    const uint32_t own = (by_entry ? a.k / 2 : a.k) / 4;  // pieces of the normed part
+    if (by_entry) {
         const float *second = a.second + (size_t)t * a.x_stride;
         for (uint32_t p = threadIdx.x; p < pieces; p += 256) stage16(&at4(own + p).x, second + 4 * p);
         asm volatile("cp.async.commit_group;" ::: "memory");
         for (uint32_t p = own + pieces + threadIdx.x; p < a.k / 4; p += 256) at4(p) = zero;
     }
-    const bool by_entry = a.kind == QK_INPUT_CONCAT;
     // v to the row's place; then use(entry) for this thread's, in their order
     auto exchange = [&](const float4 (&v)[kPieces], auto &&use) {
 #pragma unroll
@@ -318,15 +319,6 @@ __device__ __forceinline__ void build_norm_pieces(const InputArgs &a, uint32_t t
     }
     for (uint32_t p = pieces + threadIdx.x; p < own; p += 256) at4(p) = zero;
     __syncthreads();
-}
-// (Half the pieces where they do: at the four blocks per SM of the vector form the others cost time even where
-// no thread has any.  A row of 2048 took 1.9 to 3.1 us from the wait with four pieces and block_sum, 1.4 to 2.6
-// with two and row_sum, with a pending one 3.3 and 2.4.)
-template <typename At4>
-__device__ __forceinline__ void build_norm_row(const InputArgs &a, uint32_t t, bool writer, const float *staged, At4 &&at4,
-                                               float *red) {
-    if (a.width <= 512 * kNormPieces) build_norm_pieces<kNormPieces / 2>(a, t, writer, staged, at4, red);
-    else build_norm_pieces<kNormPieces>(a, t, writer, staged, at4, red);
 }
 // A gated row of groups of up to 128 aligned entries, for 256 threads: a warp takes two groups at a time, a lane four
 // entries of each, all of whose loads go out together.  The squares are added in the order of build_input, a lane's entries
