@@ -1081,17 +1081,17 @@ attention_sage_tc_kernel(SageArgs a, AttnDims dm, int causal) {
 //     floats, and the output warps convert nothing (per score two conversions fewer on a pipe that takes two cycles
 //     for each).  S stays kind::i8: half the operand bytes, one conversion per score.
 //   * The Q . mean shift of a row comes from the blocks' mean digit rows, a product with N = 16 whose result
-//     lies in S's columns before S does (64 ..: free once the scores are P codes).
+//     lies in S's columns before S does (32 .. 47: between the two blocks' P codes, and read before S comes).
 //   * Tensor memory (512 columns): S of the two score groups at 0 and 128, the PV sums of the two blocks at 256 and
 //     384.  The scores, scaled, go back to S's columns between the two passes over them (maximum, exponentials); a block's P
 //     codes (float16, PV's A operand) take the first half of its scores' columns.
 // All waits are bounded (bit 1 of the context's error word on expiry).
 //
 // What bounds it: the chain of an iteration - scores to maximum, maximum to P codes, the products' issue - which two
-// groups in turn hide in part: issue slots 52 % busy, the special-function unit 27 % (4096 tokens).  8192 tokens of 32
-// heads over 8, causal, whole call: 1296 us by sixteen warps in step with both products in kind::i8, 1035 with groups of four
-// warps and one PV region, 978 as it is (944 with the preparation in one launch).  Taking the two tiles of a CTA in turn instead
-// of two iterations: 1146.
+// groups in turn hide in part: issue slots 53 % busy, the special-function unit 29 %, the tensor pipe 20 % (4096 tokens).
+// 8192 tokens of 32 heads over 8, causal, whole call: 1296 us by sixteen warps in step with both products in kind::i8, 1035
+// with groups of four warps and one PV region, 978 with all of them, 944 with the preparation in one launch, 956 since S waits
+// for the products that read P.  Taking the two tiles of a CTA in turn instead of two iterations: 1146.
 constexpr int kUQ = 128, kUBlk = 64, kUKeys = 2 * kUBlk, kUD = 128;
 constexpr int kUThreads = 512, kUGroups = kUThreads / kUQ;
 // The block-scale kernel's issuing warps (their lane 0): S products, record copies, PV products.  Each of
@@ -2050,7 +2050,8 @@ SageLayout sage_layout(const qk_ctx *c, const AttnDims &dm, size_t block_size) {
     L.o_kc = take(L.planes * S * L.dpad), L.o_ks = take(L.planes * S * 4);
     L.o_vc = take(L.planes * L.n_blocks * dm.dv * L.bpad), L.o_vs = take(L.planes * L.n_blocks * dm.dv * 4);
     L.o_md = take(L.planes * L.n_blocks * 8 * L.dpad), L.o_ms = take(L.planes * L.n_blocks * 4);
-    if (recorded) off = std::max(off, L.o_rec + up(L.planes * ((L.n_blocks + 1) / 2) * kURecStride + 1024));  // (1024: to align them)
+    if (recorded)  // (1024: to align them)
+        off = std::max(off, L.o_rec + up(L.planes * ((L.n_blocks + 1) / 2) * kURecStride + 1024));
     L.bytes = off;
     return L;
 }

@@ -364,7 +364,8 @@ delta_inputs_kernel(DeltaArgs a, uint32_t n_tokens) {
     __syncthreads();
     if constexpr (kTok == 8) {
         // k_i . k_t and k_i . q_t, two rows by two: two threads a square, one adds up the even entries, the other the odd
-        // ones, in their order (two threads a product, entry by entry, give the same bits from four times the reads)
+        // ones, in their order.  (Two threads a product, entry by entry, give the same bits from four times the reads: a launch
+        // on 2048 rows at width 4096 takes 65.6 us so, 74.6 that way.)
         if (threadIdx.x < 64) {
             const uint32_t square = threadIdx.x / 2, kind = square / 16, t = square / 4 % 4 * 2, i = square % 4 * 2;
             const uint32_t part = threadIdx.x % 2 * odd, own = (a.dim + 1) / 2;
@@ -470,10 +471,9 @@ delta_chunk_scan_kernel(DeltaArgs a, uint32_t n_tokens, int vec) {
         for (uint32_t i = threadIdx.x; i < S::kStages * S::kFloats; i += kChunkWarps * 32) cs_smem[i] = 0.f;
         __syncthreads();
     }
-    // This thread's 16-byte pieces of a chunk's q and k, the same for every chunk: their place in a
-    // stage, whose rows are a power of two long.  (Worked out
-    // anew for each of them, by two divisions a piece, they took 42 of the 421 us of a scan of 2048 tokens, 32 heads of
-    // 128 x 128.)
+    // This thread's 16-byte pieces of a chunk's q and k, the same for every chunk: their place in a stage, whose rows
+    // are a power of two long.  (Worked out anew for each chunk, by two divisions a piece, they took 42 of the 421 us of a
+    // scan of 2048 tokens, 32 heads of 128 x 128.)
     constexpr int kPieces = kE / 2;
     uint32_t piece_at[kPieces];
 #pragma unroll

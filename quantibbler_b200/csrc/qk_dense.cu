@@ -729,8 +729,8 @@ dense_norm_rows_kernel(InputArgs in, uint16_t *__restrict__ dst) {
 // float32 accumulators through distributed shared memory, each CTA finishing its share of the
 // columns.  Weights depend on no other kernel: the first stages' copies start before the
 // dependency wait.  Warp 0 issues the copies, warp 1 the MMAs, warps 2..5 finish.
-// More CTAs than fit one to an SM: half the stages each, two to an SM, so that one streams while the other finishes its tile or begins
-// (as many weight bytes in flight): 64 rows, the gated pair of a 14336-wide MLP of 4096, 224 tiles, 84 -> 65.5 us, of sixteen
+// More CTAs than fit one to an SM: half the stages each, two to an SM, so that one streams while the other finishes its
+// tile or begins (as many weight bytes in flight): 64 rows, the gated pair of a 14336-wide MLP of 4096, 224 tiles, 84 -> 65.5 us, of sixteen
 // such experts half as wide, 1792 tiles, 339 -> 317 (5.9 TB/s).
 template <int BN> struct NarrowShape {
     static constexpr uint32_t kABytes = 128 * kTcK * 2, kBBytes = BN * kTcK * 2, kStage = kABytes + kBBytes;
@@ -1131,9 +1131,9 @@ qk_status launch_tc(qk_ctx *c, const void *x, size_t x_stride, const qk_dense_ca
     }
 }
 
-// Which of the faster ways to read the input rows applies.  (One row in the vector form, from the wait to the
-// finished row, the general way and this one: two of 2048 entries one behind the other 4.0 and 1.5 us, with a
-// pending one 6.8 and 2.5; sixteen gated groups of 128 3.7 to 5.4 and 3.4.)
+// Which of the faster ways to read the input rows applies.  (A launch of 1184 weight rows on one row, the general way and
+// this one: two of 2048 entries one behind the other 8.7 and 6.7 us, with a pending one 10.8 and 8.1; sixteen gated groups
+// of 128 7.9 and 6.4.)
 int row_kind_of(const InputArgs &a) {
     auto aligned = [](const void *p) { return ((uintptr_t)p & 15) == 0; };
     if (a.width % 4 || a.k % 4 || a.x_stride % 4 || !aligned(a.x)) return kRowAny;

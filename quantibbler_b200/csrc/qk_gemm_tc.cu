@@ -697,8 +697,8 @@ struct NormArgs {
 };
 // kPer: entries a thread, 8 for rows of up to 4096 and 16 for up to 8192.  With 8, three blocks fit an SM: a block is a
 // chain of latencies (the row, the sum, the stores), and rows in flight are what hides them.
-// An eight-layer prompt of 2048 tokens at width 4096 takes 9690 us with sixteen entries and two blocks, 9381 with these (both before the stores
-// were wide).
+// An eight-layer prompt of 2048 tokens at width 4096 takes 9690 us with sixteen entries and two blocks, 9381 with
+// these (both before the stores were wide).
 template <int kPer>
 __global__ void __launch_bounds__(kNormThreads, kPer == 8 ? 3 : 2)
 norm_scale_to_bf16_kernel(NormArgs n, ScaleArgs a, uint32_t n_problems, uint32_t d, uint32_t pitch) {

@@ -1806,17 +1806,18 @@ constexpr size_t kSumSmem = 116 * 1024;  // at least: more than half of an SM's,
 // Most weights of a launch (rows x entries over its instances).  The sums' time grows with them, by 0.2 us a million (float32
 // serving 0.25); the digit forms spend 5 to 10 us on their tables and 0.07 to 0.16 us a million.  Measured, us a call, the
 // stage by digits -> by sums, the other stage as this rule has it:
-//   first stage of up to 8192 entries, bfloat16: 2 x 2100 x 4096 (17e6) 22.7 -> 19.4, 4 x 2048 x 4096 (34e6) 17.3 -> 15.3, 6 x 2048 x
-//     4096 (50e6) 18.3 -> 18.3, 12 x 1024 x 4096 (50e6) 17.2 -> 19.6; float32: 16 x 800 x 2048 (26e6) 15.9 -> 15.3, 5 x 2048 x 4096
-//     (42e6) 17.6 -> 18.3
-//   of more (slices) in a plan, bfloat16: 1200 x 14336 (17e6) 13.8 -> 13.9, 800 x 14336 (11e6) 13.3 -> 12.7, 1733 x 14336 (25e6)
-//     14.3 -> 15.2, 2 x 1600 x 9000 (29e6) 13.8 -> 17.0; float32: 800 x 14336 13.6 -> 12.6, 1600 x 9000 (14e6) 13.2 -> 13.8
-//   ... on the tokens of one layer, whose digit form has a table launch and copied records: 1733 x 14336 19.5 -> 15.4 (float32
-//     19.6 -> 16.1), on two tokens (50e6) 19.8 -> 20.0
-//   second stage, bfloat16: 14336 x 2560 (37e6) 15.4 -> 13.7, x 3400 (49e6) 15.8 -> 16.8, 2 x 14336 x 1724 (49e6) 17.8 -> 16.2,
-//     12 x 2048 x 800 (20e6) 14.1 -> 12.3, 16 x 2048 x 800 (26e6) 14.9 -> 14.2, 5 x 4096 x 2048 (42e6) 17.2 -> 17.7; float32
-//     (entries of eight bytes): 4 x 4096 x 1733 (28e6) inside four layers of a step 672 -> 649, 4 x 4096 x 2048 (34e6) 16.6 -> 17.8,
-//     8 x 2048 x 800 (13e6) 12.7 -> 11.3, 8 x 4096 x 600 (20e6) 14.5 -> 15.5
+//   first stage of up to 8192 entries, bfloat16: 2 x 2100 x 4096 (17e6) 22.7 -> 19.4, 4 x 2048 x 4096 (34e6) 17.3 -> 15.3,
+//     6 x 2048 x 4096 (50e6) 18.3 -> 18.3, 12 x 1024 x 4096 (50e6) 17.2 -> 19.6; float32: 16 x 800 x 2048 (26e6) 15.9 ->
+//     15.3, 5 x 2048 x 4096 (42e6) 17.6 -> 18.3
+//   of more (slices) in a plan, bfloat16: 1200 x 14336 (17e6) 13.8 -> 13.9, 800 x 14336 (11e6) 13.3 -> 12.7, 1733 x 14336
+//     (25e6) 14.3 -> 15.2, 2 x 1600 x 9000 (29e6) 13.8 -> 17.0; float32: 800 x 14336 13.6 -> 12.6, 1600 x 9000 (14e6)
+//     13.2 -> 13.8
+//   ... on the tokens of one layer, whose digit form has a table launch and copied records: 1733 x 14336 19.5 -> 15.4
+//     (float32 19.6 -> 16.1), on two tokens (50e6) 19.8 -> 20.0
+//   second stage, bfloat16: 14336 x 2560 (37e6) 15.4 -> 13.7, 14336 x 3400 (49e6) 15.8 -> 16.8, 2 x 14336 x 1724 (49e6)
+//     17.8 -> 16.2, 12 x 2048 x 800 (20e6) 14.1 -> 12.3, 16 x 2048 x 800 (26e6) 14.9 -> 14.2, 5 x 4096 x 2048 (42e6) 17.2 ->
+//     17.7; float32 (entries of eight bytes): 4 x 4096 x 1733 (28e6) inside four layers of a step 672 -> 649, 4 x 4096 x
+//     2048 (34e6) 16.6 -> 17.8, 8 x 2048 x 800 (13e6) 12.7 -> 11.3, 8 x 4096 x 600 (20e6) 14.5 -> 15.5
 double sum_most_weights(size_t n_inst, size_t ranks, bool final, bool bf16, bool run) {
     if (ranks > 1 && !run) return bf16 ? 15e6 : 12e6;
     if (!final) return bf16 && n_inst <= 2 ? 50e6 : 30e6;

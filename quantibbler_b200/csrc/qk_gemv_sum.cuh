@@ -22,7 +22,7 @@
 // What bounds it: latencies.  By the clock of block 0, us from the wait to the end: the first stage of a 4096 x 4096 linear of
 // rank 1102 with the norm inside 5.3 (entries 1.7, grid and conversion 0.9, sums 1.7, rows 0.8), its second stage 2.9; a
 // boundary between kernels 1.1.  One 4096 x 4096 linear of rank 1024 on one token 13.4 -> 8.0 us, an eight-block step of
-// width 4096 at batch 1 901 -> 731 us.
+// width 4096 at batch 1 901 -> 731 us when it came in.  Issue slots 40 % busy while a block is there.
 #pragma once
 
 namespace {
@@ -89,7 +89,8 @@ __device__ __forceinline__ void sum_form(const StageParams &p, uint32_t rows_per
     int *zl = reinterpret_cast<int *>(smem_dyn + lay.low);
     Entry *entries = reinterpret_cast<Entry *>(smem_dyn + lay.entries);
     uint8_t *slab = smem_dyn + lay.slab;
-    long long *part = reinterpret_cast<long long *>(smem_dyn + lay.part);  // [row][warp of the vector]; row `rows_per_block`: totals
+    // [row][warp of the vector]; row `rows_per_block`: totals
+    long long *part = reinterpret_cast<long long *>(smem_dyn + lay.part);
     long long *row_sum = reinterpret_cast<long long *>(smem_dyn + lay.row_sum);  // (slices)
     const uint32_t z_pitch = lay.lanes + 1, padded = kSumEntries * lay.lanes;
 

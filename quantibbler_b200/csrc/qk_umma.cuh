@@ -45,8 +45,8 @@ __device__ __forceinline__ bool mbar_wait(uint64_t *bar, uint32_t parity, volati
 // and not under a comparison with the lane number: their operands live in uniform registers, and only
 // after elect does the compiler know that one lane is left (otherwise an MMA costs its issuer over a hundred
 // cycles).  Measured where an MMA warp only issues: 64-token step of eight factorized blocks 2537 -> 2461 us,
-// 64-row step of the Virudra design 4135 -> 4009 us, prompts 1 to 2 %.  Not in the INT8 Sage kernels, whose
-// issuing warps also compute: there it came out slower (8192 tokens 1294 -> 1332 us).
+// 64-row step of the Virudra design 4135 -> 4009 us, prompts 1 to 2 %.  Not in the block-scale Sage kernel, whose
+// issuing warps also compute: in a kernel of that form it came out slower (8192 tokens 1294 -> 1332 us).
 __device__ __forceinline__ bool elect_one() {
     uint32_t is;
     asm volatile("{\n .reg .pred p;\n elect.sync _|p, 0xffffffff;\n selp.u32 %0, 1, 0, p;\n}" : "=r"(is));
